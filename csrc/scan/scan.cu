@@ -26,6 +26,11 @@ constexpr int SCAN_THREADS = 128;
 template <typename T> __device__ __forceinline__ float s_ld(const T* p);
 template <> __device__ __forceinline__ float s_ld<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float s_ld<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+// a predicated load that stays in the element's own type: the conversion, and with it the wait for the load, comes where
+// the value is used
+template <typename T> __device__ __forceinline__ T s_raw(bool ok, const T* p) { T v; if (ok) v = *p; else v = T(0.f); return v; }
+__device__ __forceinline__ float s_f(float v) { return v; }
+__device__ __forceinline__ float s_f(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T> __device__ __forceinline__ void s_st(T* p, float v);
 template <> __device__ __forceinline__ void s_st<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void s_st<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
@@ -275,77 +280,101 @@ selective_scan_bwd_kernel(ScanArgs a) {
   }
 }
 
-// ---------------------------------------------------------------------------- lane-per-state scan (N == 16, no fused gate)
-// The thread-per-channel kernels above expose B*D threads (32768 for the Mamba configuration) and every step
-// waits on the previous one: they are latency-bound at a few percent of the machine. Here a lane owns ONE state
-// (channel, n): a warp carries 2 channels x 16 states, 16x the threads, one MUFU ex2 and three FMAs per lane
-// and step. The sum over n that y_t (forward) and d delta_t / d u_t (backward) need is taken 16 steps at a time
-// with a transpose-reduce inside each half-warp (15 shuffles for 16 sums) instead of 4 shuffles per step.
-// u / delta / B / C move through shared-memory tiles filled with coalesced loads while the previous tile is
-// being processed. The checkpoint layout is the one of the kernels above, so either backward can follow either
-// forward.
+// ---------------------------------------------------------------------------- two states per lane (N == 16, no fused gate)
+// The thread-per-channel kernels above expose B*D threads (32768 for the Mamba configuration) and every step waits on
+// the previous one: they are latency-bound at a few percent of the machine. Here a lane owns TWO neighbouring states of
+// a channel: a warp carries 4 channels x 8 lanes. What bounds these kernels is instruction issue, so the two states share
+// every shared-memory load, run as packed fp32 pairs (one FMA / MUL instruction for both) and are added in the lane
+// before the sum over the states, which is taken for 8 or 16 steps at a time with a transpose-reduce over the 8 lanes
+// (14 shuffles for 16 sums). u / delta / B / C move through shared-memory tiles filled with coalesced loads while the
+// previous tile is being processed. The checkpoint layout is the one of the kernels above, so either backward can
+// follow either forward.
 constexpr float SCAN_LOG2E = 1.4426950408889634f;
 __device__ __forceinline__ float scan_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float2 f2mul(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2dup(float v) { return make_float2(v, v); }
 
-// sums 16 per-lane values over the 16 lanes of a half-warp; lane j (mod 16) ends with the total of v[j]
-__device__ __forceinline__ float transpose_reduce16(float (&v)[16], int lane) {
+// Sums 16 per-lane values over 8 neighbouring lanes: lane j (mod 8) ends with the totals of v[2j] (in v[0]) and v[2j + 1].
+__device__ __forceinline__ void transpose_reduce8(float (&v)[16], int lane) {
 #pragma unroll
-  for (int step = 0; step < 4; ++step) {
-    const int half = 8 >> step;
-    const bool upper = (lane & half) != 0;
+  for (int step = 0; step < 3; ++step) {
+    const int half = 8 >> step, bit = 4 >> step;
+    const bool upper = (lane & bit) != 0;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
       const float send = upper ? v[i] : v[i + half];
       const float keep = upper ? v[i + half] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
     }
   }
-  return v[0];
 }
 
+// Measured at 2 x 4096 x 4096 x 16 (bf16): 428 us, one state per lane 528 us; 8 x 1000: 340 against 440 us.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 scan_fwd_lanes_kernel(ScanArgs a) {
-  constexpr int DB = 16, TT = 32;
+  constexpr int DB = 16, TT = 32;                     // channels per block (4 warps x 4), time steps per tile
   __shared__ float2 s_x[2][TT][DB];                   // (delta, delta * u)
-  __shared__ float2 s_BC[2][TT][SCAN_N];
-  __shared__ float s_u[2][TT][DB], s_y[TT][DB];
+  __shared__ float4 s_BC[2][TT][SCAN_N / 2];          // (B of the two states, C of the two states)
+  __shared__ float s_u[2][TT][DB], s_y[TT][DB + 1];
   const int b = blockIdx.y, d0 = blockIdx.x * DB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = lane & 15, ch = warp * 2 + (lane >> 4);
+  const int np = lane & 7, ch = warp * 4 + (lane >> 3);       // state pair, channel
   const int d = d0 + ch;
   const bool active = d < a.D;
-  const float A2 = active ? a.A[(long long)d * SCAN_N + n] * SCAN_LOG2E : 0.f;
+  float2 A2 = make_float2(0.f, 0.f);
+  if (active) A2 = make_float2(a.A[(long long)d * SCAN_N + 2 * np] * SCAN_LOG2E, a.A[(long long)d * SCAN_N + 2 * np + 1] * SCAN_LOG2E);
   const float dsk = (active && a.Dskip) ? a.Dskip[d] : 0.f;
   const int n_ck = (a.S + SCAN_CK - 1) / SCAN_CK;
-  float h = 0.f;
-  // loader role: thread -> (row lt of the tile, channel / state pair lp)
+  float2 h = make_float2(0.f, 0.f);
+  // loader role: thread -> (rows lt, lt + 16 of the tile, channel pair / state pair lp)
   const int lt = threadIdx.x >> 3, lp = threadIdx.x & 7;
   const int ld0 = d0 + 2 * lp, ld1 = ld0 + 1;
   const float db0 = (a.delta_bias && ld0 < a.D) ? a.delta_bias[ld0] : 0.f, db1 = (a.delta_bias && ld1 < a.D) ? a.delta_bias[ld1] : 0.f;
   const long long rb = (long long)b * a.S;
   const T* up = (const T*)a.u; const T* dp = (const T*)a.delta; const T* Bp = (const T*)a.Bm; const T* Cp = (const T*)a.Cm;
-  float r[8];
+  T r[2][8];
   auto load_tile = [&](int t0) {
-    const int t = t0 + lt;
-    const bool ok = t < a.S;
-    const long long row = rb + t;
-    r[0] = (ok && ld0 < a.D) ? s_ld(up + row * a.u_ld + ld0) : 0.f;
-    r[1] = (ok && ld1 < a.D) ? s_ld(up + row * a.u_ld + ld1) : 0.f;
-    float x0 = (ok && ld0 < a.D) ? s_ld(dp + row * a.delta_ld + ld0) + db0 : 0.f;
-    float x1 = (ok && ld1 < a.D) ? s_ld(dp + row * a.delta_ld + ld1) + db1 : 0.f;
-    if (a.delta_softplus) { x0 = softplus20(x0); x1 = softplus20(x1); }
-    r[2] = (ok && ld0 < a.D) ? x0 : 0.f; r[3] = (ok && ld1 < a.D) ? x1 : 0.f;
-    r[4] = ok ? s_ld(Bp + row * a.b_ld + 2 * lp) : 0.f; r[5] = ok ? s_ld(Bp + row * a.b_ld + 2 * lp + 1) : 0.f;
-    r[6] = ok ? s_ld(Cp + row * a.c_ld + 2 * lp) : 0.f; r[7] = ok ? s_ld(Cp + row * a.c_ld + 2 * lp + 1) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int t = t0 + lt + 16 * k;
+      const bool ok = t < a.S;
+      const long long row = rb + t;
+      r[k][0] = s_raw(ok && ld0 < a.D, up + row * a.u_ld + ld0);
+      r[k][1] = s_raw(ok && ld1 < a.D, up + row * a.u_ld + ld1);
+      r[k][2] = s_raw(ok && ld0 < a.D, dp + row * a.delta_ld + ld0);
+      r[k][3] = s_raw(ok && ld1 < a.D, dp + row * a.delta_ld + ld1);
+      r[k][4] = s_raw(ok, Bp + row * a.b_ld + 2 * lp); r[k][5] = s_raw(ok, Bp + row * a.b_ld + 2 * lp + 1);
+      r[k][6] = s_raw(ok, Cp + row * a.c_ld + 2 * lp); r[k][7] = s_raw(ok, Cp + row * a.c_ld + 2 * lp + 1);
+    }
   };
-  auto put_tile = [&](int buf) {
-    s_u[buf][lt][2 * lp] = r[0]; s_u[buf][lt][2 * lp + 1] = r[1];
-    s_x[buf][lt][2 * lp] = make_float2(r[2], r[2] * r[0]); s_x[buf][lt][2 * lp + 1] = make_float2(r[3], r[3] * r[1]);
-    s_BC[buf][lt][2 * lp] = make_float2(r[4], r[6]); s_BC[buf][lt][2 * lp + 1] = make_float2(r[5], r[7]);
+  auto put_tile = [&](int buf, int t0) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int tt = lt + 16 * k;
+      const bool ok = t0 + tt < a.S;
+      const float u0 = s_f(r[k][0]), u1 = s_f(r[k][1]);
+      float x0 = s_f(r[k][2]) + db0, x1 = s_f(r[k][3]) + db1;
+      if (a.delta_softplus) { x0 = softplus20(x0); x1 = softplus20(x1); }
+      x0 = (ok && ld0 < a.D) ? x0 : 0.f; x1 = (ok && ld1 < a.D) ? x1 : 0.f;      // past the end: delta 0 keeps the state
+      s_u[buf][tt][2 * lp] = u0; s_u[buf][tt][2 * lp + 1] = u1;
+      s_x[buf][tt][2 * lp] = make_float2(x0, x0 * u0); s_x[buf][tt][2 * lp + 1] = make_float2(x1, x1 * u1);
+      s_BC[buf][tt][lp] = make_float4(s_f(r[k][4]), s_f(r[k][5]), s_f(r[k][6]), s_f(r[k][7]));
+    }
   };
   const int n_tiles = (a.S + TT - 1) / TT;
-  load_tile(0); put_tile(0);
+  load_tile(0); put_tile(0, 0);
   __syncthreads();
   for (int tile = 0; tile < n_tiles; ++tile) {
     const int cur = tile & 1, t0 = tile * TT;
@@ -356,190 +385,187 @@ scan_fwd_lanes_kernel(ScanArgs a) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int t = half * 16 + i;
-        if ((t % SCAN_CK) == 0 && a.hck && active && t0 + t < a.S)
-          a.hck[(((long long)b * n_ck + (t0 + t) / SCAN_CK) * a.D + d) * SCAN_N + n] = h;      // state BEFORE step t
-        const float2 x = s_x[cur][t][ch], bc = s_BC[cur][t][n];
-        h = fmaf(scan_ex2(x.x * A2), h, x.y * bc.x);
-        p[i] = h * bc.y;
+        if ((t % SCAN_CK) == 0 && a.hck && active && t0 + t < a.S)          // state BEFORE step t
+          *reinterpret_cast<float2*>(a.hck + (((long long)b * n_ck + (t0 + t) / SCAN_CK) * a.D + d) * SCAN_N + 2 * np) = h;
+        const float2 x = s_x[cur][t][ch];
+        const float4 bc = s_BC[cur][t][np];
+        const float2 e = f2mul(f2dup(x.x), A2);
+        h = f2fma(make_float2(scan_ex2(e.x), scan_ex2(e.y)), h, f2mul(f2dup(x.y), make_float2(bc.x, bc.y)));
+        const float2 pr = f2mul(h, make_float2(bc.z, bc.w));
+        p[i] = pr.x + pr.y;
       }
-      const float y = transpose_reduce16(p, lane);         // lane n: sum over the states for step half*16 + n
-      const int t = half * 16 + n;
-      s_y[t][ch] = y + dsk * s_u[cur][t][ch];
+      transpose_reduce8(p, lane);                          // lane np: sums over the states for steps half*16 + 2np, + 1
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int t = half * 16 + 2 * np + k;
+        s_y[t][ch] = p[k] + dsk * s_u[cur][t][ch];
+      }
     }
     __syncthreads();
-    {
-      const int t = t0 + lt;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int tt = lt + 16 * k, t = t0 + tt;
       if (t < a.S) {
         T* yp = (T*)a.y + (rb + t) * a.y_ld;
-        if (ld0 < a.D) s_st(yp + ld0, s_y[lt][2 * lp]);
-        if (ld1 < a.D) s_st(yp + ld1, s_y[lt][2 * lp + 1]);
+        if (ld0 < a.D) s_st(yp + ld0, s_y[tt][2 * lp]);
+        if (ld1 < a.D) s_st(yp + ld1, s_y[tt][2 * lp + 1]);
       }
     }
-    if (tile + 1 < n_tiles) put_tile(cur ^ 1);
+    if (tile + 1 < n_tiles) put_tile(cur ^ 1, t0 + TT);
     __syncthreads();
   }
 }
 
-// Backward. A block owns 64 channels and walks the checkpoint intervals from the last to the first. Per interval
-// each lane re-runs 8 steps of its state from the checkpoint, then runs the adjoint recurrence in reverse; it does so
-// for 4 channels in turn (pass p: channel p*16 + 2*warp + lane/16) so that the per-(t, n) sums dB / dC, which run
-// over ALL channels, gather 4 channels in registers before they touch shuffles, shared memory and finally one atomic
-// per (t, n) and block. The next interval's u / delta / dy / B / C rows and checkpoints are fetched into registers
-// while the current one is processed.
+// Backward. A block owns 32 channels and walks the checkpoint intervals from the last to the first. Per interval each
+// lane re-runs 8 steps of its two states from the checkpoint, then runs the adjoint recurrence in reverse. The per-(t, n)
+// sums dB / dC, which run over ALL channels, are reduced over the warp's channels and the block's warps before one atomic
+// per (t, n) and block. The next interval's u / delta / dy / B / C rows and checkpoints are fetched into registers, in
+// their own type, while the current one is processed (converting them at the load made every interval wait for memory).
+// 32 channels and two blocks per SM: batch 2 x 4096 channels is 256 blocks, one wave on 148 SMs. Measured at 2 x 4096 x
+// 4096 x 16 (bf16): 1.07 ms; one state per lane and 64 channels per block took 2.01 ms (1.31 ms with twice the batch);
+// 64 channels in two passes spill at two blocks per SM (1.98 ms), three blocks per SM spill (2.9 ms).
 template <typename T>
 __global__ void __launch_bounds__(256, 2)
 scan_bwd_lanes_kernel(ScanArgs a) {
-  constexpr int DB = 64, CK = SCAN_CK, WARPS = 8, PASSES = 4;
+  constexpr int DB = 32, CK = SCAN_CK, WARPS = 8;
+  static_assert(256 / DB == CK, "one (row, channel) of an interval per loader thread");
   __shared__ float4 s_in[CK][DB];                    // (delta, delta * u, u, dy) per (t, channel)
   __shared__ float s_draw[CK][DB];                   // delta before softplus
-  __shared__ float2 s_BC[CK][SCAN_N];
+  __shared__ float s_BC[CK][SCAN_N / 2][4];          // (B of the two states, C of the two states)
   __shared__ float2 s_out[CK][DB];                   // (d delta_raw, d u without the skip term)
-  __shared__ float2 s_dBC[WARPS][CK][SCAN_N];
+  __shared__ float s_dBC[WARPS][32][9];              // per warp: lane l holds 8 of the 32 x 8 (t, n) sums
   const int b = blockIdx.y, d0 = blockIdx.x * DB;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = lane & 15, chw = warp * 2 + (lane >> 4);     // channel inside a pass
+  const int np = lane & 7, ch = warp * 4 + (lane >> 3);      // state pair, channel of the block
   const int n_ck = (a.S + CK - 1) / CK;
   const long long rb = (long long)b * a.S;
-  float Araw[PASSES], g_acc[PASSES], dA_acc[PASSES], ddb_acc[PASSES], dD_acc[PASSES], hnext[PASSES];
-#pragma unroll
-  for (int p = 0; p < PASSES; ++p) {
-    const int d = d0 + p * 16 + chw;
-    Araw[p] = d < a.D ? a.A[(long long)d * SCAN_N + n] : 0.f;
-    g_acc[p] = dA_acc[p] = ddb_acc[p] = dD_acc[p] = 0.f;
-  }
-  // loader / storer role: rows lt and lt + 4 of channel lc; threads 0..127 also fetch B, 128..255 C
-  const int lc = threadIdx.x & 63, lt = threadIdx.x >> 6;
+  const int d = d0 + ch;
+  float2 Araw = make_float2(0.f, 0.f), g = Araw, dA = Araw, hnext;
+  float ddb_acc = 0.f, dD_acc = 0.f;
+  if (d < a.D) Araw = make_float2(a.A[(long long)d * SCAN_N + 2 * np], a.A[(long long)d * SCAN_N + 2 * np + 1]);
+  const float2 A2 = f2mul(Araw, f2dup(SCAN_LOG2E));
+  // loader / storer role: row lt of channel lc; threads 0..127 also fetch B, 128..255 C
+  const int lc = threadIdx.x % DB, lt = threadIdx.x / DB;
   const int ldd = d0 + lc;
   const bool ch_ok = ldd < a.D;
   const float dbias = (a.delta_bias && ch_ok) ? a.delta_bias[ldd] : 0.f;
   const float dsk = (a.Dskip && ch_ok) ? a.Dskip[ldd] : 0.f;
   const int bt = (threadIdx.x & 127) >> 4, bn = threadIdx.x & 15;
-  float pu[2], pd[2], pg[2], pbc;
+  T pu, pd, pg, pbc;
   auto prefetch = [&](int c) {
     const int t0 = c * CK;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int t = t0 + lt + 4 * k;
+    {
+      const int t = t0 + lt;
       const bool ok = t < a.S && ch_ok;
       const long long row = rb + t;
-      pu[k] = ok ? s_ld((const T*)a.u + row * a.u_ld + ldd) : 0.f;
-      pd[k] = ok ? s_ld((const T*)a.delta + row * a.delta_ld + ldd) : 0.f;
-      pg[k] = ok ? s_ld((const T*)a.dy + row * a.dy_ld + ldd) : 0.f;
+      pu = s_raw(ok, (const T*)a.u + row * a.u_ld + ldd);
+      pd = s_raw(ok, (const T*)a.delta + row * a.delta_ld + ldd);
+      pg = s_raw(ok, (const T*)a.dy + row * a.dy_ld + ldd);
     }
     const bool okb = t0 + bt < a.S;
-    if (threadIdx.x < 128) pbc = okb ? s_ld((const T*)a.Bm + (rb + t0 + bt) * a.b_ld + bn) : 0.f;
-    else pbc = okb ? s_ld((const T*)a.Cm + (rb + t0 + bt) * a.c_ld + bn) : 0.f;
-#pragma unroll
-    for (int p = 0; p < PASSES; ++p) {
-      const int d = d0 + p * 16 + chw;
-      hnext[p] = d < a.D ? a.hck[(((long long)b * n_ck + c) * a.D + d) * SCAN_N + n] : 0.f;
-    }
+    if (threadIdx.x < 128) pbc = s_raw(okb, (const T*)a.Bm + (rb + t0 + bt) * a.b_ld + bn);
+    else pbc = s_raw(okb, (const T*)a.Cm + (rb + t0 + bt) * a.c_ld + bn);
+    hnext = d < a.D ? *reinterpret_cast<const float2*>(a.hck + (((long long)b * n_ck + c) * a.D + d) * SCAN_N + 2 * np) : make_float2(0.f, 0.f);
   };
   prefetch(n_ck - 1);
   for (int c = n_ck - 1; c >= 0; --c) {
     const int t0 = c * CK;
     __syncthreads();                                  // the previous interval's tiles are no longer read
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int t = t0 + lt + 4 * k;
+    {
+      const int t = t0 + lt;
       const bool ok = t < a.S && ch_ok;
-      const float draw = ok ? pd[k] + dbias : 0.f;
+      const float draw = ok ? s_f(pd) + dbias : 0.f;
       const float dl = ok ? (a.delta_softplus ? softplus20(draw) : draw) : 0.f;
-      s_in[lt + 4 * k][lc] = make_float4(dl, dl * pu[k], pu[k], pg[k]);
-      s_draw[lt + 4 * k][lc] = draw;
+      s_in[lt][lc] = make_float4(dl, dl * s_f(pu), s_f(pu), s_f(pg));
+      s_draw[lt][lc] = draw;
     }
-    if (threadIdx.x < 128) s_BC[bt][bn].x = pbc; else s_BC[bt][bn].y = pbc;
-    float h0[PASSES];
-#pragma unroll
-    for (int p = 0; p < PASSES; ++p) h0[p] = hnext[p];
+    s_BC[bt][bn >> 1][(threadIdx.x < 128 ? 0 : 2) + (bn & 1)] = s_f(pbc);
+    const float2 h0 = hnext;
     __syncthreads();
-    if (c > 0) prefetch(c - 1);                       // in flight during the passes below
-    float dBp[CK], dCp[CK];
-#pragma unroll
-    for (int i = 0; i < CK; ++i) dBp[i] = dCp[i] = 0.f;
-#pragma unroll
-    for (int p = 0; p < PASSES; ++p) {
-      const int ch = p * 16 + chw;
-      const float A2 = Araw[p] * SCAN_LOG2E;
-      float hs[CK + 1], av[CK];
-      hs[0] = h0[p];
-#pragma unroll
-      for (int i = 0; i < CK; ++i) {
-        const float4 x = s_in[i][ch];
-        av[i] = scan_ex2(x.x * A2);
-        hs[i + 1] = fmaf(av[i], hs[i], x.y * s_BC[i][n].x);
-      }
-      float red[16];
-      float g = g_acc[p], dA = dA_acc[p];
-#pragma unroll
-      for (int i = CK - 1; i >= 0; --i) {
-        const float4 x = s_in[i][ch];                 // (dl, dl*u, u, gy)
-        const float2 bc = s_BC[i][n];
-        const float dhn = fmaf(x.w, bc.y, g);
-        const float t1 = dhn * hs[i] * av[i];
-        const float xb = dhn * bc.x;
-        red[i] = fmaf(t1, Araw[p], xb * x.z);         // d delta_t, this state's share
-        red[CK + i] = xb * x.x;                       // d u_t, this state's share
-        dA = fmaf(t1, x.x, dA);
-        dBp[i] = fmaf(dhn, x.y, dBp[i]);
-        dCp[i] = fmaf(x.w, hs[i + 1], dCp[i]);
-        g = dhn * av[i];
-      }
-      g_acc[p] = g; dA_acc[p] = dA;
-      const float tot = transpose_reduce16(red, lane);   // lane j < 8: d delta of step j; j >= 8: d u of step j - 8
-      const int j = lane & 15;
-      if (j < CK) {
-        float ddraw = tot;
-        if (a.delta_softplus) ddraw *= sigmoidf_(s_draw[j][ch]);
-        s_out[j][ch].x = ddraw;
-        ddb_acc[p] += ddraw;
-        const float4 x = s_in[j][ch];
-        dD_acc[p] = fmaf(x.w, x.z, dD_acc[p]);
-      } else {
-        s_out[j - CK][ch].y = tot;
-      }
-    }
+    if (c > 0) prefetch(c - 1);                       // in flight during the work below
+    float2 dBp[CK], dCp[CK];
+    float2 hs[CK + 1], av[CK];
+    hs[0] = h0;
 #pragma unroll
     for (int i = 0; i < CK; ++i) {
-      dBp[i] += __shfl_xor_sync(0xffffffffu, dBp[i], 16);    // the warp's two channel groups
-      dCp[i] += __shfl_xor_sync(0xffffffffu, dCp[i], 16);
-      if (lane < 16) s_dBC[warp][i][n] = make_float2(dBp[i], dCp[i]);
+      const float2 x = *reinterpret_cast<const float2*>(&s_in[i][ch]);
+      const float2 bb = *reinterpret_cast<const float2*>(s_BC[i][np]);
+      const float2 e = f2mul(f2dup(x.x), A2);
+      av[i] = make_float2(scan_ex2(e.x), scan_ex2(e.y));
+      hs[i + 1] = f2fma(av[i], hs[i], f2mul(f2dup(x.y), bb));
+    }
+    float red[16];
+#pragma unroll
+    for (int i = CK - 1; i >= 0; --i) {
+      const float4 x = s_in[i][ch];                 // (dl, dl*u, u, gy)
+      const float4 bc = *reinterpret_cast<const float4*>(s_BC[i][np]);
+      const float2 dhn = f2fma(f2dup(x.w), make_float2(bc.z, bc.w), g);
+      g = f2mul(dhn, av[i]);
+      const float2 t1 = f2mul(g, hs[i]);
+      const float2 xb = f2mul(dhn, make_float2(bc.x, bc.y));
+      const float2 rd = f2mul(t1, Araw);
+      const float xs = xb.x + xb.y;
+      red[2 * i] = fmaf(xs, x.z, rd.x + rd.y);      // d delta_t, these two states' share
+      red[2 * i + 1] = xs * x.x;                    // d u_t, these two states' share
+      dA = f2fma(t1, f2dup(x.x), dA);
+      dBp[i] = f2mul(dhn, f2dup(x.y));
+      dCp[i] = f2mul(f2dup(x.w), hs[i + 1]);
+    }
+    transpose_reduce8(red, lane);                   // lane np: (d delta, d u) of step np
+    {
+      float ddraw = red[0];
+      if (a.delta_softplus) ddraw *= sigmoidf_(s_draw[np][ch]);
+      s_out[np][ch] = make_float2(ddraw, red[1]);
+      ddb_acc += ddraw;
+      const float2 x = *reinterpret_cast<const float2*>(&s_in[np][ch].z);
+      dD_acc = fmaf(x.y, x.x, dD_acc);
+    }
+    // dB / dC over the warp's four channel groups: a transpose-reduce of the 32 values over lane bits 16 and 8 leaves 8
+    // per lane: steps 4 * (lane >> 4) .. + 3, of dB for lanes with bit 8 clear and of dC for the others
+    {
+      const bool hi = (lane & 16) != 0, isc = (lane & 8) != 0;
+      float2 kb[4], kc[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 sb = hi ? dBp[i] : dBp[i + 4], qb = hi ? dBp[i + 4] : dBp[i];
+        const float2 sc = hi ? dCp[i] : dCp[i + 4], qc = hi ? dCp[i + 4] : dCp[i];
+        kb[i] = make_float2(qb.x + __shfl_xor_sync(0xffffffffu, sb.x, 16), qb.y + __shfl_xor_sync(0xffffffffu, sb.y, 16));
+        kc[i] = make_float2(qc.x + __shfl_xor_sync(0xffffffffu, sc.x, 16), qc.y + __shfl_xor_sync(0xffffffffu, sc.y, 16));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 s = isc ? kb[i] : kc[i], q = isc ? kc[i] : kb[i];
+        s_dBC[warp][lane][2 * i] = q.x + __shfl_xor_sync(0xffffffffu, s.x, 8);
+        s_dBC[warp][lane][2 * i + 1] = q.y + __shfl_xor_sync(0xffffffffu, s.y, 8);
+      }
     }
     __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int tt = lt + 4 * k, t = t0 + tt;
+    {
+      const int t = t0 + lt;
       if (t < a.S && ch_ok) {
-        const float2 o = s_out[tt][lc];
+        const float2 o = s_out[lt][lc];
         s_st((T*)a.ddelta + (rb + t) * a.ddelta_ld + ldd, o.x);
-        s_st((T*)a.du + (rb + t) * a.du_ld + ldd, fmaf(dsk, s_in[tt][lc].w, o.y));
+        s_st((T*)a.du + (rb + t) * a.du_ld + ldd, fmaf(dsk, s_in[lt][lc].w, o.y));
       }
     }
     if (t0 + bt < a.S) {
+      const int isc = threadIdx.x < 128 ? 0 : 1;
+      const int sl = (bt >> 2) * 16 + isc * 8 + (bn >> 1), si = (bt & 3) * 2 + (bn & 1);
       float acc = 0.f;
-      if (threadIdx.x < 128) {
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) acc += s_dBC[w][bt][bn].x;
-        atomicAdd(a.dB + (rb + t0 + bt) * SCAN_N + bn, acc);
-      } else {
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) acc += s_dBC[w][bt][bn].y;
-        atomicAdd(a.dC + (rb + t0 + bt) * SCAN_N + bn, acc);
-      }
+      for (int w = 0; w < WARPS; ++w) acc += s_dBC[w][sl][si];
+      atomicAdd((isc ? a.dC : a.dB) + (rb + t0 + bt) * SCAN_N + bn, acc);
     }
   }
+  // per-channel sums are spread over the channel's 8 lanes
 #pragma unroll
-  for (int p = 0; p < PASSES; ++p) {
-    const int d = d0 + p * 16 + chw;
-    float v0 = ddb_acc[p], v1 = dD_acc[p];            // per-channel sums sit in lanes j < 8 of each half-warp
-#pragma unroll
-    for (int o = 8; o; o >>= 1) { v0 += __shfl_xor_sync(0xffffffffu, v0, o); v1 += __shfl_xor_sync(0xffffffffu, v1, o); }
-    if (d < a.D) {
-      atomicAdd(a.dA + (long long)d * SCAN_N + n, dA_acc[p]);
-      if (n == 0) {
-        if (a.ddelta_bias) atomicAdd(a.ddelta_bias + d, v0);
-        if (a.dDskip) atomicAdd(a.dDskip + d, v1);
-      }
+  for (int o = 4; o; o >>= 1) { ddb_acc += __shfl_xor_sync(0xffffffffu, ddb_acc, o); dD_acc += __shfl_xor_sync(0xffffffffu, dD_acc, o); }
+  if (d < a.D) {
+    atomicAdd(a.dA + (long long)d * SCAN_N + 2 * np, dA.x);
+    atomicAdd(a.dA + (long long)d * SCAN_N + 2 * np + 1, dA.y);
+    if (np == 0) {
+      if (a.ddelta_bias) atomicAdd(a.ddelta_bias + d, ddb_acc);
+      if (a.dDskip) atomicAdd(a.dDskip + d, dD_acc);
     }
   }
 }
@@ -671,8 +697,8 @@ int b200_selective_scan_fwd(const ScanArgs* a, int is_bf16, cudaStream_t st) {
   dim3 grid((a->D + SCAN_THREADS - 1) / SCAN_THREADS, a->B);
   if (a->N == SCAN_N && !a->z) {       // lane-per-state kernel
     dim3 g2((a->D + 15) / 16, a->B);
-    if (is_bf16) scan_fwd_lanes_kernel<__nv_bfloat16><<<g2, 256, 0, st>>>(*a);
-    else scan_fwd_lanes_kernel<float><<<g2, 256, 0, st>>>(*a);
+    if (is_bf16) scan_fwd_lanes_kernel<__nv_bfloat16><<<g2, 128, 0, st>>>(*a);
+    else scan_fwd_lanes_kernel<float><<<g2, 128, 0, st>>>(*a);
     return (int)cudaGetLastError();
   }
   if (is_bf16) selective_scan_fwd_kernel<__nv_bfloat16><<<grid, SCAN_THREADS, 0, st>>>(*a);
@@ -684,7 +710,7 @@ int b200_selective_scan_bwd(const ScanArgs* a, int is_bf16, cudaStream_t st) {
   if (a->B <= 0 || a->S <= 0 || a->D <= 0) return 0;
   if (a->N < 1 || a->N > SCAN_N || !a->hck) return -1;
   if (a->N == SCAN_N && !a->z) {       // lane-per-state kernel
-    dim3 g2((a->D + 63) / 64, a->B);
+    dim3 g2((a->D + 31) / 32, a->B);
     if (is_bf16) scan_bwd_lanes_kernel<__nv_bfloat16><<<g2, 256, 0, st>>>(*a);
     else scan_bwd_lanes_kernel<float><<<g2, 256, 0, st>>>(*a);
     return (int)cudaGetLastError();

@@ -51,6 +51,25 @@ def test_selective_scan_fwd_bwd(B, S, D, N, full, dtype):
         assert rel_err(a.grad, b.grad) < gtol, nm
 
 
+@pytest.mark.parametrize("B,S,D", [(1, 1, 1), (2, 7, 31), (1, 8, 32), (3, 9, 33), (1, 33, 17), (2, 65, 64)])
+def test_selective_scan_block_edges(B, S, D):
+    """16 states, no gate: around the 8-step intervals, the 32-step tiles and the 16 / 32 channels of a block. fp32: the
+    kernel's ex2.approx and summation order against the sequential recurrence, ~1e-6 per step over at most 65 steps."""
+    g = torch.Generator(device="cuda").manual_seed(S * 100 + D)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ins = [r(B, S, D), r(B, S, D), -(r(D, 16).abs() + 0.2), r(B, S, 16), r(B, S, 16), r(D), None, r(D) * 0.3]
+    ins_k = [t.clone().requires_grad_(True) if t is not None else None for t in ins]
+    ins_r = [t.clone().requires_grad_(True) if t is not None else None for t in ins]
+    y, yr = SC.selective_scan(*ins_k, True), SC.selective_scan_ref(*ins_r, True)
+    w = r(B, S, D)
+    (y * w).sum().backward()
+    (yr * w).sum().backward()
+    assert rel_err(y, yr) < 2e-4
+    for a, b in zip(ins_k, ins_r):
+        if a is not None:
+            assert rel_err(a.grad, b.grad) < 2e-4
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,S,C,K,act,bias", [(2, 100, 192, 4, "silu", True), (1, 33, 70, 3, "none", False), (2, 64, 128, 2, "silu", False), (1, 200, 64, 4, "none", True)])
 def test_causal_conv1d(B, S, C, K, act, bias, dtype):
