@@ -39,6 +39,10 @@ __device__ __forceinline__ uint32_t lane_id() {
   uint32_t r; asm volatile("mov.u32 %0, %%laneid;" : "=r"(r)); return r;
 }
 
+// One thread of a converged warp. Threads that issue tcgen05.mma are chosen this way, in a branch on a warp index that is
+// uniform by construction (`uniform_warp`): the compiler then keeps the descriptors in uniform registers. Behind a plain
+// `lane == 0` it does not, and back-to-back 128 x 64 x 16 products with A in TMEM took 44 cycles to issue against 29.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
@@ -125,6 +129,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* s
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem)), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
+// global[0 .. bytes) += shared[0 .. bytes) as fp32, added in L2 (untiled: both addresses and the size multiples of 16 bytes)
+__device__ __forceinline__ void bulk_reduce_add_f32(float* dst, const void* smem, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+               ::"l"(dst), "r"(smem_u32(smem)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
@@ -204,6 +213,17 @@ __device__ __forceinline__ void umma_f16_c(uint32_t d_tmem, uint64_t a_desc, uin
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0)
+      : "memory");
+}
+
+// the same with A in tensor memory: row m of A is TMEM lane m, two bf16 along K per 32-bit column (K-major)
+template <bool ACC>
+__device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0)
       : "memory");
 }
 
@@ -338,6 +358,13 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&r)[
         "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------
@@ -368,6 +395,13 @@ __device__ __forceinline__ void fma2_scalar(float& x, float& y, float m, float a
       "mov.b64 v, {%0, %1};\n\tmov.b64 mm, {%2, %2};\n\tmov.b64 aa, {%3, %3};\n\t"
       "fma.rn.f32x2 v, v, mm, aa;\n\t"
       "mov.b64 {%0, %1}, v;\n\t}" : "+f"(x), "+f"(y) : "f"(m), "f"(a));
+}
+// (x, y) <- (x, y) * m + (ax, ay)
+__device__ __forceinline__ void fma2_pair(float& x, float& y, float m, float ax, float ay) {
+  asm("{\n\t.reg .b64 v, mm, aa;\n\t"
+      "mov.b64 v, {%0, %1};\n\tmov.b64 mm, {%2, %2};\n\tmov.b64 aa, {%3, %4};\n\t"
+      "fma.rn.f32x2 v, v, mm, aa;\n\t"
+      "mov.b64 {%0, %1}, v;\n\t}" : "+f"(x), "+f"(y) : "f"(m), "f"(ax), "f"(ay));
 }
 // (sx, sy) += (x, y)
 __device__ __forceinline__ void add2(float& sx, float& sy, float x, float y) {
