@@ -53,7 +53,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* pv_bar = bars + 6;     // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = uniform_warp();
   pdl_trigger();
   const int m_blocks = (p.Sq + BMQ - 1) / BMQ;
   int bid = blockIdx.x;
@@ -131,7 +131,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   };
 
   bool ok = true;
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     mbar_expect_tx(q_bar, Q_BYTES);
 #pragma unroll
     for (int a = 0; a < KA; ++a) tma_load_4d(sQ + a * (BMQ * 128), &tmQ, q_bar, a * 64, h, q0, b);
@@ -225,7 +225,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_fence_before_sync();
     fence_proxy_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       ok = mbar_wait(&v_bar[st], (j >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL);
       if (ok) {
         tc_fence_after_sync();

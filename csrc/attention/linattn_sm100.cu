@@ -444,7 +444,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* q_bar = bars; uint64_t* k_bar = bars + 1; uint64_t* v_bar = bars + 3; uint64_t* a_bar = bars + 4; uint64_t* b_bar = bars + 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const int n_chunks = (p.S + LA_C - 1) / LA_C;
@@ -519,7 +519,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncthreads();
     float den = p.eps;
     if (full) {
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         tc_fence_after_sync();
         la_mma_xyT<HD>(tmem_base + COL_A, sQ, sKc);                                   // A = Q~ K~^T
         la_mma_pw<HD, HD>(tmem_base + COL_NUM, sQ, sShi, HD * 128, false);            // NUM = Q~ S (value + remainder)
@@ -548,7 +548,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     __syncthreads();
     if (full) den += s_part[row] + s_part[LA_C + row];        // both halves add in the same order
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       ok = mbar_wait(v_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL);
       if (ok) {
         tc_fence_after_sync();
@@ -795,7 +795,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint64_t* k_bar = bars; uint64_t* v_bar = bars + 2; uint64_t* a_bar = bars + 3; uint64_t* b_bar = bars + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const int n_chunks = (p.S + LA_C - 1) / LA_C;
@@ -863,7 +863,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     la_phi_half<HD>(sKc, row, hf, valid, p.scale, p.kind);
     fence_proxy_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       la_mma_xyT<HD>(tmem_base + COL_A, sG, sV);                                      // T = G V^T
       la_mma_xwT<HD>(tmem_base + COL_DQ, sG, sShi, false);                            // dQ~ = G S^T (value + remainder)
@@ -883,7 +883,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tc_fence_before_sync();
     fence_proxy_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       la_mma_pw<HD, LA_C>(tmem_base + COL_DQ, sP, sKc, LA_C * 128, true);             // dQ~ += dA K~ (value + remainder)
       if (rem) la_mma_pw<HD, LA_C>(tmem_base + COL_DQ, sPlo, sKc, LA_C * 128, true);
@@ -955,7 +955,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* ld_bar = bars; uint64_t* t_bar = bars + 1; uint64_t* u_bar = bars + 2; uint64_t* b_bar = bars + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const int n_chunks = (p.S + LA_C - 1) / LA_C;
@@ -1025,7 +1025,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     fence_proxy_async_smem();
     __syncthreads();
     if (full) {
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       la_mma_xyT<HD>(tmem_base + COL_T, sK, sQ);                                      // A^T = K~ Q~^T   [key][query]
       tc_commit(t_bar);
@@ -1048,7 +1048,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tc_fence_before_sync();
     fence_proxy_async_smem();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       la_mma_pw<HD, LA_C>(tmem_base + COL_DV, sP, sG, LA_C * 128, true);              // dV += mask(A)^T G
       tc_commit(u_bar);
@@ -1071,7 +1071,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     fence_proxy_async_smem();
     }
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       if (full) la_mma_pw<HD, LA_C>(tmem_base + COL_DK, sP, sQ, LA_C * 128, true);    // dK~ += mask(dA)^T Q~
       la_mma_xTw<HD>(tmem_base + COL_DS, sQ, q_lbo, sG, have_state0 || it > 0);       // dS += Q~^T G

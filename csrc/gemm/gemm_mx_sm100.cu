@@ -110,7 +110,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* acc_full = bars + 2 * STAGES;
   uint64_t* acc_empty = bars + 2 * STAGES + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   const int m_blocks = (p.M + Cf::BM - 1) / Cf::BM, n_blocks = (p.N + Cf::BN - 1) / Cf::BN;
   const int num_kb = p.K / Cf::K_PER_STAGE;
@@ -157,7 +157,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ scale copies + MMA issue
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0, acc_phase = 0; bool ok = true;
       for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         if (!mbar_wait(acc_empty, acc_phase ^ 1, p.status, ST_TIMEOUT_ACC_EMPTY)) { ok = false; break; }

@@ -271,7 +271,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   pdl_trigger();
 
@@ -490,7 +490,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && crank == 0) {                       // of a CTA pair only the even CTA issues
+    if (crank == 0 && elect_one()) {                     // of a CTA pair only the even CTA issues
       constexpr uint32_t idesc = make_idesc(BM * CG, BN, KindOf<T>::CF, KindOf<T>::AF, KindOf<T>::BF,
                                             A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       // K-major: 8-row groups 1024 B apart.  MN-major: 8-k-row groups 1024 B apart, 128B-row atoms
