@@ -121,6 +121,23 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     return buf[..., : t.shape[-1]]
 
 
+def _operand(t: torch.Tensor):
+    """(tensor, batch, rows, columns, row stride, batch stride) of an operand that TMA can read: `t` itself, or the padded
+    copy `_tma_ready` makes of it."""
+    if t.dim() == 2:
+        rows, cols = t.shape
+        ld, inner = t.stride()
+        if inner == 1 and ld >= cols and ld * t.element_size() % 16 == 0 and t.data_ptr() % 16 == 0:
+            return t, 1, rows, cols, ld, rows * ld
+    t = _tma_ready(_as3d(t))
+    return t, t.shape[0], t.shape[1], t.shape[2], t.stride(1), t.stride(0)
+
+
+_KINDS = {(torch.bfloat16, torch.bfloat16): GEMM_BF16, (torch.float32, torch.float32): GEMM_F32,
+          (torch.int8, torch.int8): GEMM_S8S8, (torch.uint8, torch.int8): GEMM_U8S8,
+          (torch.float8_e4m3fn, torch.float8_e4m3fn): GEMM_E4M3}
+
+
 @nv.traced("gemm")
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, dact: str = "none", want_aux: bool = False, alpha: float = 1.0,
@@ -148,12 +165,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             r = (out, r[1]) if want_aux else out
         return r
     lib = nv.cuda()
-    kinds = {(torch.bfloat16, torch.bfloat16): GEMM_BF16, (torch.float32, torch.float32): GEMM_F32,
-             (torch.int8, torch.int8): GEMM_S8S8, (torch.uint8, torch.int8): GEMM_U8S8,
-             (torch.float8_e4m3fn, torch.float8_e4m3fn): GEMM_E4M3}
-    if (a.dtype, b.dtype) not in kinds:
+    kind = _KINDS.get((a.dtype, b.dtype))
+    if kind is None:
         raise TypeError(f"gemm operands must be bf16 x bf16, fp32 x fp32, int8 x int8, uint8 x int8 or e4m3 x e4m3 (got {a.dtype}, {b.dtype})")
-    kind = kinds[(a.dtype, b.dtype)]
     is_f32 = kind == GEMM_F32
     lowp = kind >= GEMM_S8S8
     if lowp and (a_mn or b_mn):
@@ -166,12 +180,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if b_mn:
             b, b_mn = transpose_last2(b), False
     squeeze = a.dim() == 2
-    a3, b3 = _tma_ready(_as3d(a)), _tma_ready(_as3d(b))
-    batch = a3.shape[0]
-    if b3.shape[0] != batch:
+    a3, batch, ar, ac, lda, stride_a = _operand(a)
+    b3, batch_b, br, bc, ldb, stride_b = _operand(b)
+    if batch_b != batch:
         raise ValueError("batch mismatch")
-    M, K = (a3.shape[2], a3.shape[1]) if a_mn else (a3.shape[1], a3.shape[2])
-    N, Kb = (b3.shape[2], b3.shape[1]) if b_mn else (b3.shape[1], b3.shape[2])
+    M, K = (ac, ar) if a_mn else (ar, ac)
+    N, Kb = (bc, br) if b_mn else (br, bc)
     if K != Kb:
         raise ValueError(f"gemm K mismatch: {K} vs {Kb}")
     dev = a.device
@@ -228,12 +242,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise ValueError("split-K needs an fp32 output and a linear epilogue")
         out_mode = OUT_F32_ATOMIC
     if out is None:
-        shape = (batch, M, N)
+        shape = (M, N) if squeeze else (batch, M, N)
         odt = torch.int32 if out_mode == OUT_I32 else torch.float32 if out_mode != OUT_BF16 else torch.bfloat16
         out = torch.zeros(shape, dtype=odt, device=dev) if out_mode == OUT_F32_ATOMIC else torch.empty(shape, dtype=odt, device=dev)
-    out3 = out if out.dim() == 3 else out.view(1, M, N) if batch == 1 else out.view(batch, M, N)
-    ldc = out3.stride(1)
-    aux = torch.empty((batch, M, N), dtype=torch.bfloat16, device=dev) if want_aux else None
+    if out.dim() == 2 and batch == 1 and out.shape[0] == M and out.shape[1] == N:
+        out3, ldc, out_ptr = out, out.stride(0), out.data_ptr()
+        stride_c = M * ldc
+    else:
+        out3 = out if out.dim() == 3 else out.view(1, M, N) if batch == 1 else out.view(batch, M, N)
+        ldc, out_ptr = out3.stride(1), out3.data_ptr()
+        stride_c = out3.stride(0) if batch > 1 else M * ldc
+    aux = torch.empty((M, N) if squeeze else (batch, M, N), dtype=torch.bfloat16, device=dev) if want_aux else None
     if aux_in is not None:
         aux_in = aux_in.contiguous().view(batch, M, N)
         if aux_in.dtype != torch.bfloat16:
@@ -247,24 +266,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if bias is not None and bias.dtype not in (torch.float32, torch.bfloat16):
         raise TypeError("bias must be fp32 or bf16")
 
-    args = nv.GemmArgs()
-    p = args.p
-    p.M, p.N, p.K, p.batch, p.splits = M, N, K, batch, splits
-    p.C, p.ldc, p.strideC = out3.data_ptr(), ldc, out3.stride(0) if batch > 1 else M * ldc
-    p.bias = nv.ptr(bias); p.bias_f32 = 1 if (bias is not None and bias.dtype == torch.float32) else 0
-    p.bias_vec_ok = 1 if (bias is not None and bias.data_ptr() % 16 == 0 and bias.is_contiguous() and N % 4 == 0) else 0
-    p.strideBias = N if (bias is not None and bias.dim() == 2) else 0      # [batch, N] bias: one vector per batch
-    p.residual = nv.ptr(residual)
-    p.ldr = residual.stride(1) if residual is not None else 0
-    p.strideR = residual.stride(0) if residual is not None else 0
-    p.aux_out = nv.ptr(aux); p.aux_in = nv.ptr(aux_in)
-    p.alpha = float(alpha); p.alpha_ptr = nv.ptr(alpha_t.float() if alpha_t is not None and alpha_t.dtype != torch.float32 else alpha_t); p.act = ACT[act]; p.dact = ACT[dact]; p.out_mode = out_mode
-    es_out = 4 if out_mode != OUT_BF16 else 2
-    aux_ok = (aux is None and aux_in is None) or (ldc == N and N % 8 == 0)
-    p.vec_ok = 1 if (ldc * es_out % 16 == 0 and out3.data_ptr() % 16 == 0 and (batch == 1 or p.strideC * es_out % 16 == 0) and aux_ok) else 0
     if (aux is not None or aux_in is not None) and ldc != N:
         raise ValueError("aux tensors need a dense output (ldc == N)")
-    p.res_vec_ok = 1 if (residual is not None and residual.stride(1) % 8 == 0 and residual.data_ptr() % 16 == 0 and (batch == 1 or residual.stride(0) % 8 == 0)) else 0
     if row_scale is not None:
         row_scale = row_scale.float().contiguous()
         if row_scale.numel() != batch * M:
@@ -273,26 +276,38 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         col_scale = col_scale.float().contiguous()
         if col_scale.numel() != N:
             raise ValueError("col_scale needs one value per row of B")
-    p.row_scale, p.col_scale = nv.ptr(row_scale), nv.ptr(col_scale)
-    p.status = nv.status_word(dev).data_ptr()
     for name, t in (("m_valid", m_valid), ("k_valid", k_valid)):
         if t is not None and (t.dtype != torch.int32 or t.numel() != batch or not t.is_cuda):
             raise ValueError(f"{name} must be an int32 device tensor with one entry per batch")
-    p.m_valid, p.k_valid = nv.ptr(m_valid), nv.ptr(k_valid)
-    args.A, args.lda, args.strideA, args.a_mn = a3.data_ptr(), a3.stride(1), a3.stride(0), int(a_mn)
-    args.B, args.ldb, args.strideB, args.b_mn = b3.data_ptr(), b3.stride(1), b3.stride(0), int(b_mn)
-    args.M, args.N, args.K, args.batch, args.dtype = M, N, K, batch, kind
+    if alpha_t is not None and alpha_t.dtype != torch.float32:
+        alpha_t = alpha_t.float()
+    bias_ptr = bias_f32 = bias_vec_ok = bias_stride = 0
+    if bias is not None:
+        bias_ptr, bias_f32 = bias.data_ptr(), int(bias.dtype == torch.float32)
+        bias_vec_ok = int(bias_ptr % 16 == 0 and N % 4 == 0 and bias.is_contiguous())
+        bias_stride = N if bias.dim() == 2 else 0                  # [batch, N] bias: one vector per batch
+    res_ptr = ldr = stride_r = res_vec_ok = 0
+    if residual is not None:
+        res_ptr, ldr, stride_r = residual.data_ptr(), residual.stride(1), residual.stride(0)
+        res_vec_ok = int(ldr % 8 == 0 and res_ptr % 16 == 0 and (batch == 1 or stride_r % 8 == 0))
+    es_out = 4 if out_mode != OUT_BF16 else 2
+    vec_ok = int(ldc * es_out % 16 == 0 and out_ptr % 16 == 0 and (batch == 1 or stride_c * es_out % 16 == 0)
+                 and ((aux is None and aux_in is None) or N % 8 == 0))
+    rec = nv.GEMM_PACK.pack(
+        M, N, K, batch, splits, out_ptr, ldc, stride_c, bias_ptr, bias_f32, bias_vec_ok, bias_stride, res_ptr, ldr, stride_r,
+        nv.ptr(aux), nv.ptr(aux_in), float(alpha), nv.ptr(alpha_t), ACT[act], ACT[dact], out_mode, vec_ok, res_vec_ok,
+        nv.ptr(row_scale), nv.ptr(col_scale), nv.status_ptr(dev), nv.ptr(m_valid), nv.ptr(k_valid),
+        a3.data_ptr(), lda, stride_a, int(a_mn), b3.data_ptr(), ldb, stride_b, int(b_mn), M, N, K, batch, kind)
+    res = out3[0] if (squeeze and out.dim() == 3) else out
     if _prepare:
         # a fused kernel runs this product itself: hand back the filled launch record, the tile width, the results and
         # everything the record points at (kept alive by the caller until the launch has been issued)
-        res = out3[0] if (squeeze and out.dim() == 3) else out
-        return args, bn, res, (aux[0] if (aux is not None and squeeze) else aux), (a3, b3, bias, residual, aux_in, row_scale, col_scale, m_valid, k_valid, out3)
-    rc = lib.b200_gemm_launch(C.byref(args), bn, sms, nv.stream_ptr())
+        return nv.GemmArgs.from_buffer_copy(rec), bn, res, aux, (a3, b3, bias, residual, aux_in, row_scale, col_scale, m_valid, k_valid, out3)
+    rc = lib.b200_gemm_launch(rec, bn, sms, nv.stream_ptr())
     nv.check(rc, "b200_gemm_launch")
     nv.count_launch()
-    res = out3[0] if (squeeze and out.dim() == 3) else out
     if accumulate_into is not None:
         res = accumulate_into
     if want_aux:
-        return res, (aux[0] if squeeze else aux)
+        return res, aux
     return res

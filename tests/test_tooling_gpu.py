@@ -26,6 +26,28 @@ def test_gemv_both_orientations(m, n, dtype):
     assert torch.allclose(yt.double(), 2.0 * (a.double().t() @ xt.double()), rtol=1e-4, atol=1e-3 * math.sqrt(m))
 
 
+@pytest.mark.parametrize("m,n,k,ldc", [(1, 1, 1, 1), (130, 257, 65, 257), (128, 128, 1024, 128), (64, 96, 4097, 96), (40, 50, 60, 64), (300, 300, 1500, 301)])
+def test_sgemm_writes_c_in_place(m, n, k, ldc):
+    """beta = 0 around the split-K rule, with a leading dimension wider than the row (the gap stays untouched), and with C
+    sharing memory with an operand. TF32 drops mantissa bits past the tenth: at most 2^-10 of each factor, 2^-9 of a product."""
+    from rust_neural_network_b200 import blas
+    N = blas.Transpose.NoTrans
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + k)
+    a, b = torch.randn(m * k, generator=g, device="cuda"), torch.randn(k * n, generator=g, device="cuda")
+    c = torch.full((m * ldc,), 7.0, device="cuda")
+    v = c._version
+    assert blas.sgemm(N, N, m, n, k, 1.0, a, k, b, n, 0.0, c, ldc) is c and c._version > v
+    ref = a.view(m, k).double() @ b.view(k, n).double()
+    cv = c.view(m, ldc)
+    assert float((cv[:, :n].double() - ref).norm() / ref.norm()) < 2 ** -9
+    assert bool((cv[:, n:] == 7.0).all())
+    ov = min(m * n, m * k) // 2                                           # C and A in one storage, overlapping by half of the smaller
+    buf = torch.zeros(m * n + m * k, device="cuda")
+    buf[m * n - ov:m * n - ov + m * k] = a
+    blas.sgemm(N, N, m, n, k, 1.0, buf[m * n - ov:], k, b, n, 0.0, buf[:m * n], n)
+    assert float((buf[:m * n].view(m, n).double() - ref).norm() / ref.norm()) < 2 ** -9
+
+
 def test_blas_level1_and_sgemm_gpu():
     torch.manual_seed(0)
     x, y = torch.randn(100003, device=DEV), torch.randn(100003, device=DEV)
