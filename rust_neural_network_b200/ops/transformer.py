@@ -12,14 +12,17 @@ the optimizer's flat fp32 gradient buffer.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
+import struct
 
 import torch
 from torch.autograd import Function
 
+from .. import _native as nv
 from . import kernels as K
 from .functional import _bgrad, _scale_by, _wgrad, lp
-from .gemm import gemm
+from .gemm import _num_sms, gemm
 
 
 def _adjacent(a, b, c):
@@ -142,9 +145,74 @@ class TransformerBlockFn(Function):
                 None, None, None)
 
 
-def transformer_block(x, blk, causal):
-    """Run `blk` (a `models.looped_transformer.TransformerBlock`) through the fused function."""
+nv.register_sigs({"b200_block_fwd": [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]})
+_BLOCK_PACK = struct.Struct("@25P9ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
+
+
+def _shadow_qkv(wq, wk, wv):
+    """bf16 [3d, d] of the three projections. Weights no optimizer has laid out have a shadow each (`functional.lp`): these
+    are moved into one buffer the first time, so that later calls find them adjacent instead of copying them together. Each
+    stays its parameter's own shadow, refreshed when that parameter changes. (Not while a graph is being captured: the
+    buffer would belong to the graph.)"""
+    a, b, c = lp(wq), lp(wk), lp(wv)
+    if _adjacent(a, b, c):
+        return a
+    buf = torch.cat([a, b, c], 0)
+    if not torch.cuda.is_current_stream_capturing() and not any(getattr(w, "_fused_grad", False) for w in (wq, wk, wv)):
+        d = a.shape[0]
+        for i, w in enumerate((wq, wk, wv)):
+            w._lp = buf[i * d:(i + 1) * d]
+    return buf
+
+
+def _plain(*ts) -> bool:
+    return all(t.dtype == torch.float32 and t.is_cuda and t.is_contiguous() for t in ts)
+
+
+def _block_forward(x, blk, causal):
+    """The block without gradients as one native call, or None where its launches cannot be issued that way."""
     at = blk.attn
+    q, k, v, o, f1, f2, n1, n2 = at.q_proj, at.k_proj, at.v_proj, at.out_proj, blk.ff1, blk.ff2, blk.ln1, blk.ln2
+    B, S, d = x.shape
+    ff = f1.weight.shape[0]
+    vecs = (n1.gamma, n1.beta, n2.gamma, n2.beta, q.bias, k.bias, v.bias, o.bias, f1.bias, f2.bias)
+    if (any(t is None for t in vecs) or not _plain(*vecs) or d % 8 or ff % 8 or B * S == 0 or B * S * max(3 * d, ff) >= 2 ** 31
+            or tuple(q.weight.shape) != (d, d) or tuple(k.weight.shape) != (d, d) or tuple(v.weight.shape) != (d, d)
+            or tuple(o.weight.shape) != (d, d) or tuple(f1.weight.shape) != (ff, d) or tuple(f2.weight.shape) != (d, ff)):
+        return None
+    x = x if x.is_contiguous() else x.contiguous()
+    ws = (_shadow_qkv(q.weight, k.weight, v.weight), lp(o.weight), lp(f1.weight), lp(f2.weight))
+    if x.data_ptr() % 16 or any(w.data_ptr() % 16 or not w.is_contiguous() for w in ws):
+        return None
+    T, dev, H = B * S, x.device, at.heads
+    adjacent = _adjacent(q.bias, k.bias, v.bias)
+    # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse, gathered bias (fp32)
+    offs, total = [], 0
+    for nbytes in (2 * T * d, 6 * T * d, 2 * T * d, 2 * T * d, 2 * T * ff, 4 * T, 4 * T, 4 * T * H, 12 * d):
+        offs.append(total)
+        total += (nbytes + 255) & ~255
+    work = torch.empty(total, dtype=torch.uint8, device=dev)
+    y = torch.empty_like(x)
+    w0 = work.data_ptr()
+    g1, be1, g2, be2, bq, bk, bv, bo, b1, b2 = (t.data_ptr() for t in vecs)
+    rec = _BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *(w0 + p for p in offs), *(w.data_ptr() for w in ws),
+                           g1, be1, g2, be2, bq, bk, bv, bo, b1, b2, B, S, d, ff, H, int(causal), int(not adjacent), K.OPS["add"], _num_sms(dev),
+                           float(n1.eps), nv.status_ptr(dev))
+    launches = C.c_int(0)
+    nv.check(nv.cuda().b200_block_fwd(rec, C.byref(launches), nv.stream_ptr()), "block_fwd")
+    nv.count_launch(launches.value)
+    return y
+
+
+def transformer_block(x, blk, causal):
+    """Run `blk` (a `models.looped_transformer.TransformerBlock`) through the fused function. Without gradients (and outside
+    torch.func transforms and forward-mode AD, whose tensors have no memory of their own) the forward is one native call."""
+    at = blk.attn
+    if (not torch.is_grad_enabled() and not nv.NVTX_ENABLED and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0):
+        y = _block_forward(x, blk, causal)
+        if y is not None:
+            return y
     return TransformerBlockFn.apply(
         x, blk.ln1.gamma, blk.ln1.beta, at.q_proj.weight, at.q_proj.bias, at.k_proj.weight, at.k_proj.bias,
         at.v_proj.weight, at.v_proj.bias, at.out_proj.weight, at.out_proj.bias, blk.ln2.gamma, blk.ln2.beta,

@@ -40,6 +40,26 @@ def _clone_to(module, device, dtype):
     return m.to_device(device, dtype)
 
 
+@pytest.mark.parametrize("B,S,d,heads,ff,causal", [(1, 1, 128, 2, 256, True), (1, 333, 128, 1, 264, True), (3, 7, 64, 1, 72, False),
+                                                   (2, 130, 256, 4, 1024, False), (64, 257, 512, 8, 2048, True)])
+def test_block_without_gradients_equals_the_differentiable_one(B, S, d, heads, ff, causal):
+    """The one-call forward issues the kernels the differentiable function issues, on the same operands: equal bit for bit,
+    before and after a weight and a bias change in place."""
+    torch.manual_seed(1)
+    blk = TransformerBlock(d, heads, ff, causal=causal, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16)
+    x = torch.randn(B, S, d, device="cuda").bfloat16()
+    for _ in range(2):
+        with torch.no_grad():
+            y = blk(x)
+            strided = blk(torch.stack([x, x], -1)[..., 0])                # not contiguous
+        assert not y.requires_grad and torch.equal(y, blk(x).detach()) and torch.equal(y, strided)
+        with torch.no_grad():
+            blk.attn.k_proj.weight.mul_(1.5)
+            blk.attn.v_proj.bias.add_(0.25)
+            before = y
+    assert not torch.equal(before, blk(x))
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_fused_block_matches_fp32_reference(causal):
     torch.manual_seed(0)
