@@ -3,9 +3,10 @@
 //   out_t = phi(s q_t) . S_t / (phi(s q_t) . z_t + eps),   S_t = sum_{u<=t} phi(s k_u) (x) v_u,   z_t = sum_{u<=t} phi(s k_u)
 //
 // with phi = ELU + 1 or ReLU^2 (rust-nn src/linear_attention.rs:42-94). The reference runs the causal form as a
-// per-token rank-1 recurrence and its backward stores every S_t (src/linear_attention.rs:214-266, 502-632). Here one
-// CTA owns one (batch, head) and walks its sequence in chunks of 128 tokens; thread t owns token t of the chunk (= TMEM
-// lane t). Per chunk, with Q~ = phi(sQ), K~ = phi(sK) formed in shared memory in place on the TMA tiles:
+// per-token rank-1 recurrence and its backward stores every S_t (src/linear_attention.rs:214-266, 502-632). Here a CTA
+// walks the sequence of one (batch, head), or one of `n_seg` segments of it, in chunks of 128 tokens (a token is a TMEM
+// lane). Segments first take their totals (`state_only`), a small kernel sums them up, and the pass starts each segment from
+// the sum: few heads leave most SMs idle otherwise. Per chunk, with Q~ = phi(sQ), K~ = phi(sK) formed in shared memory in place on the TMA tiles:
 //
 //   forward     A = mask(Q~ K~^T)            NUM = Q~ S + A V          den = rowsum(A) + Q~ . z        out = NUM / (den + eps)
 //               S += K~^T V                  z += colsum(K~)
@@ -33,6 +34,7 @@
 namespace b200 {
 
 constexpr int LA_C = 128;                    // tokens per chunk = rows of every product = TMEM lanes
+constexpr uint32_t LA_X_LBO = LA_C * 128;    // distance of a tile's 64-column atoms
 
 // Sequence-parallel exchange of the slice totals, done by the attention kernels themselves over NVLink peer memory.
 // The state pass of a rank (role 1) writes its total into its OWN symmetric buffer and then raises one flag per
@@ -70,6 +72,8 @@ struct LinAttnArgs {
   int kind;                                  // 0: ELU + 1, 1: ReLU^2
   int state_only;                            // forward: only accumulate the state (reads K, V; writes s_out)
   uint32_t* status;
+  float* seg;                                // n_seg > 1: [B*H][n_seg][hd*hd + hd] fp32 workspace for the states between segments
+  int n_seg, seg_chunks;                     // the sequence is walked as n_seg segments of seg_chunks chunks by as many CTAs
   LaExchange sx;
 };
 
@@ -146,70 +150,6 @@ __device__ __forceinline__ void la_retire(const LinAttnArgs& p, uint32_t epoch) 
 }
 
 __device__ __forceinline__ float la_phi(float x, int kind) { return kind == 0 ? (x > 0.f ? x + 1.f : __expf(x)) : (x > 0.f ? x * x : 0.f); }
-// derivative of phi expressed through its value: ELU+1: 1 for x > 0 (phi > 1) else phi; ReLU^2: 2 sqrt(phi)
-__device__ __forceinline__ float la_dphi_from_phi(float p, int kind) { return kind == 0 ? (p > 1.f ? 1.f : p) : 2.f * sqrtf(p); }
-
-// phi(scale * x) in place on a [128 rows][HD] bf16 tile of 128-byte-swizzled 64-column atoms; thread = row.
-// Rows at or beyond `valid` become zero (TMA fills them with zeros, and phi(0) is 1 for ELU + 1).
-template <int HD>
-__device__ __forceinline__ void la_phi_tile(uint8_t* tile, int row, int valid, float scale, int kind) {
-#pragma unroll
-  for (int a = 0; a < HD / 64; ++a)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint4* p = reinterpret_cast<uint4*>(tile + a * (LA_C * 128) + sw128_offset(row, c));
-      uint4 u = *p;
-      uint32_t* w = &u.x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16x2(w[j]);
-        w[j] = row < valid ? pack_bf16x2(la_phi(f.x * scale, kind), la_phi(f.y * scale, kind)) : 0u;
-      }
-      *p = u;
-    }
-}
-
-// fp32 row of a tile (thread = row) -> registers
-template <int HD>
-__device__ __forceinline__ void la_read_row(const uint8_t* tile, int row, float* out) {
-#pragma unroll
-  for (int a = 0; a < HD / 64; ++a)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const uint4 u = *reinterpret_cast<const uint4*>(tile + a * (LA_C * 128) + sw128_offset(row, c));
-      const uint32_t* w = &u.x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { const float2 f = unpack_bf16x2(w[j]); out[a * 64 + c * 8 + 2 * j] = f.x; out[a * 64 + c * 8 + 2 * j + 1] = f.y; }
-    }
-}
-
-// column sums of a tile: thread k (< HD) returns sum over the 128 rows of element (row, k)
-template <int HD>
-__device__ __forceinline__ float la_colsum(const uint8_t* tile, int k) {
-  const uint8_t* base = tile + (k >> 6) * (LA_C * 128) + (k & 7) * 2;
-  const int chunk = (k & 63) >> 3;
-  float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-  for (int r = 0; r < LA_C; r += 2) {
-    s0 += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + sw128_offset(r, chunk)));
-    s1 += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + sw128_offset(r + 1, chunk)));
-  }
-  return s0 + s1;
-}
-// weighted column sums: sum_r w[r] * tile(r, k)
-template <int HD>
-__device__ __forceinline__ float la_colsum_w(const uint8_t* tile, int k, const float* w) {
-  const uint8_t* base = tile + (k >> 6) * (LA_C * 128) + (k & 7) * 2;
-  const int chunk = (k & 63) >> 3;
-  float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-  for (int r = 0; r < LA_C; r += 2) {
-    s0 += w[r] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + sw128_offset(r, chunk)));
-    s1 += w[r + 1] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + sw128_offset(r + 1, chunk)));
-  }
-  return s0 + s1;
-}
-
 // One fp32 row of HD values -> bf16 "value" tile and bf16 "remainder" tile (row = thread), [rows][HD] swizzled atoms
 // of `rows` rows each.
 template <int HD>
@@ -227,35 +167,6 @@ __device__ __forceinline__ void la_write_hilo(uint8_t* hi, uint8_t* lo, int rows
     const uint32_t off = (g >> 3) * (rows * 128) + sw128_offset(row, g & 7);
     *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
-  }
-}
-
-// fp32 row of 128 values -> bf16 K-major [128][128] tile (two atoms), row = thread
-__device__ __forceinline__ void la_write_row128(uint8_t* tile, int row, const float* v) {
-#pragma unroll
-  for (int g = 0; g < 16; ++g) {
-    const uint4 o = make_uint4(pack_bf16x2(v[g * 8], v[g * 8 + 1]), pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]),
-                               pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]), pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]));
-    *reinterpret_cast<uint4*>(tile + (g >> 3) * (LA_C * 128) + sw128_offset(row, g & 7)) = o;
-  }
-}
-
-// fp32 row of 128 values -> bf16 value tile and bf16 remainder tile (both K-major [128][128]), row = thread
-// (`with_lo` false: the value tile only)
-__device__ __forceinline__ void la_write_row128_hilo(uint8_t* hi, uint8_t* lo, int row, const float* v, bool with_lo) {
-#pragma unroll
-  for (int g = 0; g < 16; ++g) {
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = v[g * 8 + 2 * j], b = v[g * 8 + 2 * j + 1];
-      h[j] = pack_bf16x2(a, b);
-      const float2 r = unpack_bf16x2(h[j]);
-      l[j] = pack_bf16x2(a - r.x, b - r.y);
-    }
-    const uint32_t off = (g >> 3) * (LA_C * 128) + sw128_offset(row, g & 7);
-    *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-    if (with_lo) *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
   }
 }
 
@@ -289,6 +200,14 @@ __device__ __forceinline__ void la_mma_pw(uint32_t d, const uint8_t* p, const ui
     umma_f16(d, sdesc_at<1024>(lp, advp), sdesc_at<1024>(lw, k * 2048), idesc, acc || k > 0);
   }
 }
+// D[128 x HD] += P W over 128 tokens, P in TMEM as `la_put_half128` leaves it (`a`: its first column, + 32 for the remainders)
+template <int HD>
+__device__ __forceinline__ void la_mma_tw(uint32_t d, uint32_t a, const uint8_t* w) {
+  constexpr uint32_t idesc = make_idesc(128, HD, CFMT_F32, FMT_BF16, FMT_BF16, 0, 1);
+  const uint32_t lw = sdesc_lo(smem_u32(w), LA_C * 128);
+#pragma unroll
+  for (int k = 0; k < LA_C / 16; ++k) umma_f16_ta<true>(d, a + (k >> 2) * 64 + (k & 3) * 8, sdesc_at<1024>(lw, k * 2048), idesc);
+}
 // D[128 x HD] (+)= X W^T with X K-major [128][HD] and W K-major [HD rows][HD] (atoms of HD rows)
 template <int HD>
 __device__ __forceinline__ void la_mma_xwT(uint32_t d, const uint8_t* x, const uint8_t* w, bool acc) {
@@ -301,12 +220,11 @@ __device__ __forceinline__ void la_mma_xwT(uint32_t d, const uint8_t* x, const u
   }
 }
 // State update D[128 (d_k, zero-padded) x HD] (+)= X^T W over the 128 tokens: X, W MN-major [128 tokens][HD].
-// `x_lbo` is the distance from X's first 64-column atom to the next one; for HD = 64 it points at a tile of zeros, so
-// that the product has the 128 rows the instruction wants and rows 64..127 of D stay zero.
+// For HD = 64 X's second 64-column atom is the tile behind it (see LaSmem): rows 64..127 of D are not used.
 template <int HD>
-__device__ __forceinline__ void la_mma_xTw(uint32_t d, const uint8_t* x, uint32_t x_lbo, const uint8_t* w, bool acc) {
+__device__ __forceinline__ void la_mma_xTw(uint32_t d, const uint8_t* x, const uint8_t* w, bool acc) {
   constexpr uint32_t idesc = make_idesc(128, HD, CFMT_F32, FMT_BF16, FMT_BF16, 1, 1);
-  const uint32_t lx = sdesc_lo(smem_u32(x), x_lbo), lw = sdesc_lo(smem_u32(w), LA_C * 128);
+  const uint32_t lx = sdesc_lo(smem_u32(x), LA_X_LBO), lw = sdesc_lo(smem_u32(w), LA_C * 128);
 #pragma unroll
   for (int k = 0; k < LA_C / 16; ++k)
     umma_f16(d, sdesc_at<1024>(lx, k * 2048), sdesc_at<1024>(lw, k * 2048), idesc, acc || k > 0);
@@ -315,14 +233,12 @@ __device__ __forceinline__ void la_mma_xTw(uint32_t d, const uint8_t* x, uint32_
 template <int HD>
 struct LaSmem {
   static constexpr int TILE = LA_C * HD * 2;          // one [128][HD] operand tile
-  static constexpr int PT = LA_C * LA_C * 2;          // one [128][128] tile
   static constexpr int ST = HD * HD * 2;              // one state tile [HD][HD]
-  static constexpr int ZERO = HD == 64 ? TILE : 0;    // zero atom that pads the state update to 128 rows
-  // The masked [128][128] tile of a chunk (A in the forward, dA in the dQ kernel) enters its product as value + remainder
-  // like the state does: dQ is a difference of nearly equal sums, and one bf16 copy of the tile costs it ~2 % each way.
-  // With head_dim 64 the remainder tile has its own buffer; with 128 (shared memory is full) it reuses the tile of the
-  // operand that is dead by then (Q~ in the forward, G in the dQ kernel).
-  static constexpr int PLO = HD == 64 ? PT : 0;
+  // Head size 64: 80 KB of tiles and 256 TMEM columns, so that two CTAs share an SM and one's elementwise work runs beside
+  // the other's products and waits. The state update wants 128 rows where there are 64: its second 64-row atom is whatever
+  // tile follows in shared memory, and rows 64..127 of the result are never read.
+  static constexpr uint32_t TMEM = HD == 64 ? 256 : 512;
+  static constexpr int CTAS = HD == 64 ? 2 : 1;
 };
 
 // ---------------------------------------------------------------------------------------------------- forward
@@ -368,22 +284,21 @@ __device__ __forceinline__ float la_dot_half(const uint8_t* tile, int row, int h
     }
   return acc0 + acc1;
 }
-// 64 fp32 values = columns 64 hf .. of this thread's row of a [128][128] tile (atom hf) -> value and remainder tiles
-__device__ __forceinline__ void la_write_half128_hilo(uint8_t* hi, uint8_t* lo, int row, int hf, const float* v, bool with_lo) {
+// 64 fp32 values = columns 64 hf .. of this thread's row of a masked [128][128] tile -> A operand in TMEM, over the fp32
+// columns they were read from (`col` = 64 hf of the tile): the bf16 values in the first 32, the rounding remainders in the
+// next 32. The masked tile enters its product as value + remainder like the state does where the result is a difference
+// of nearly equal sums (one bf16 copy costs dQ ~2 %).
+__device__ __forceinline__ void la_put_half128(uint32_t col, const float* v, bool with_lo) {
+  uint32_t h[32], l[32];
 #pragma unroll
-  for (int g = 0; g < 8; ++g) {
-    uint32_t h[4], l[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float a = v[g * 8 + 2 * j], b = v[g * 8 + 2 * j + 1];
-      h[j] = pack_bf16x2(a, b);
-      const float2 r = unpack_bf16x2(h[j]);
-      l[j] = pack_bf16x2(a - r.x, b - r.y);
-    }
-    const uint32_t off = hf * (LA_C * 128) + sw128_offset(row, g);
-    *reinterpret_cast<uint4*>(hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
-    if (with_lo) *reinterpret_cast<uint4*>(lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+  for (int i = 0; i < 32; ++i) {
+    h[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+    const float2 r = unpack_bf16x2(h[i]);
+    l[i] = pack_bf16x2(v[2 * i] - r.x, v[2 * i + 1] - r.y);
   }
+  tmem_st_x32(col, h);
+  if (with_lo) tmem_st_x32(col + 32, l);
+  tmem_st_wait();
 }
 // HD / 2 fp32 values = columns (HD / 2) hf .. of a state row -> value and remainder tiles ([rows][HD], atoms of `rows` rows)
 template <int HD>
@@ -420,24 +335,21 @@ __device__ __forceinline__ float la_colsum_rows(const uint8_t* tile, int k, int 
 }
 
 template <int HD>
-__global__ void __launch_bounds__(LA_FWD_THREADS, 1)
+__global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;                  // columns of a HD-wide row per thread
   constexpr int ZP = LA_FWD_THREADS / HD;     // row groups of the column sums of K~ (4 or 2)
-  constexpr uint32_t COL_A = 0, COL_NUM = 128, COL_S = 256;
+  constexpr uint32_t COL_A = 0, COL_NUM = 128, COL_S = 128 + HD;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + L::TILE;                 // 2 stages
-  uint8_t* sZero = sK + 2 * L::TILE;          // HD = 64 only
-  uint8_t* sV = sZero + L::ZERO;
-  uint8_t* sP = sV + L::TILE;
-  uint8_t* sShi = sP + L::PT;
+  uint8_t* sV = sK + 2 * L::TILE;
+  uint8_t* sShi = sV + L::TILE;
   uint8_t* sSlo = sShi + L::ST;
-  uint8_t* sPlo = HD == 64 ? sSlo + L::ST : sQ;
-  float* sz = reinterpret_cast<float*>(sSlo + L::ST + L::PLO);      // [HD]
+  float* sz = reinterpret_cast<float*>(sSlo + L::ST);               // [HD]
   float* s_part = sz + HD;                    // [2][128]: the halves' shares of a row's denominator
   float* s_zk = s_part + 2 * LA_C;            // [ZP][HD]: partial column sums of K~
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_zk + LA_FWD_THREADS);
@@ -446,9 +358,11 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const int n_chunks = (p.S + LA_C - 1) / LA_C;
+  const int bh = blockIdx.x / p.n_seg, seg = blockIdx.x % p.n_seg, b = bh / p.H, h = bh % p.H;
+  const int c0 = seg * p.seg_chunks;           // first chunk of this CTA's segment
+  const int n_chunks = min(p.seg_chunks, (p.S + LA_C - 1) / LA_C - c0);
   const bool full = !p.state_only;
+  if (p.n_seg > 1 && !full && seg == p.n_seg - 1) return;      // nothing follows the last segment
   // ELU + 1 features sit near 1, where a bf16 copy of the masked tile loses what the later subtraction needs; ReLU^2
   // features are spread over the exponent range and a single copy is enough (0.3 % measured)
   const bool rem = p.kind == 0;
@@ -458,8 +372,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     fence_barrier_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  if (HD == 64) for (int i = tid; i < L::ZERO / 16; i += LA_FWD_THREADS) reinterpret_cast<uint4*>(sZero)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 0) { tmem_alloc(tmem_slot, L::TMEM); tmem_relinquish(); }
   // state before the first token: TMEM (fp32) and the two bf16 operand tiles
   const size_t st_stride = (size_t)HD * HD + HD;
   const uint32_t sx_epoch = la_epoch(p);
@@ -467,9 +380,9 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (tid < HD) {
     float s0[HD];
 #pragma unroll
-    for (int i = 0; i < HD; ++i) s0[i] = s_in ? s_in[bh * st_stride + (size_t)tid * HD + i] : 0.f;
+    for (int i = 0; i < HD; ++i) s0[i] = s_in ? s_in[blockIdx.x * st_stride + (size_t)tid * HD + i] : 0.f;
     la_write_hilo<HD>(sShi, sSlo, HD, tid, s0);
-    sz[tid] = s_in ? s_in[bh * st_stride + (size_t)HD * HD + tid] : 0.f;
+    sz[tid] = s_in ? s_in[blockIdx.x * st_stride + (size_t)HD * HD + tid] : 0.f;
   }
   tc_fence_before_sync();
   fence_proxy_async_smem();
@@ -482,7 +395,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     for (int c = 0; c < HD / 32; ++c) {
       uint32_t r[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(s_in[bh * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
+      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(s_in[blockIdx.x * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
       tmem_st_x32(trow + COL_S + c * 32, r);
     }
     tmem_st_wait();
@@ -494,9 +407,8 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int chunk) {
     mbar_expect_tx(bar, L::TILE);
 #pragma unroll
-    for (int a = 0; a < KA; ++a) tma_load_4d(dst + a * (LA_C * 128), tm, bar, a * 64, h, chunk * LA_C, b);
+    for (int a = 0; a < KA; ++a) tma_load_4d(dst + a * (LA_C * 128), tm, bar, a * 64, h, (c0 + chunk) * LA_C, b);
   };
-  const uint32_t k_lbo[2] = {HD == 64 ? uint32_t(2 * L::TILE) : uint32_t(LA_C * 128), HD == 64 ? uint32_t(L::TILE) : uint32_t(LA_C * 128)};
   if (tid == 0) {
     if (full) load(sQ, &tmQ, q_bar, 0);
     load(sK, &tmK, &k_bar[0], 0);
@@ -508,7 +420,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   for (int c = 0; c < n_chunks; ++c) {
     const int st = c & 1;
     uint8_t* sKc = sK + st * L::TILE;
-    const int valid = min(LA_C, p.S - c * LA_C);
+    const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
     // ---- phi in place
     if (full && !mbar_wait(q_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (ok && !mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
@@ -531,7 +443,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (!mbar_wait(a_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
       if (__syncthreads_or(!ok)) { ok = false; break; }
       tc_fence_after_sync();
-      if (HD == 64 && tid == 0 && c + 1 < n_chunks) load(sQ, &tmQ, q_bar, c + 1);  // Q~ has been consumed
+      if (tid == 0 && c + 1 < n_chunks) load(sQ, &tmQ, q_bar, c + 1);            // Q~ has been consumed
       float a[64];
       la_tmem_row<64>(trow + COL_A + hf * 64, a);
       float r0 = 0.f, r1 = 0.f;
@@ -542,9 +454,8 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         r0 += a[i]; r1 += a[i + 1];
       }
       s_part[hf * LA_C + row] = part + (r0 + r1);
-      la_write_half128_hilo(sP, sPlo, row, hf, a, rem);
+      la_put_half128(trow + COL_A + hf * 64, a, rem);
       tc_fence_before_sync();
-      fence_proxy_async_smem();
     }
     __syncthreads();
     if (full) den += s_part[row] + s_part[LA_C + row];        // both halves add in the same order
@@ -553,10 +464,10 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (ok) {
         tc_fence_after_sync();
         if (full) {                                                                                    // NUM += A V (value + remainder)
-          la_mma_pw<HD, LA_C>(tmem_base + COL_NUM, sP, sV, LA_C * 128, true);
-          if (rem) la_mma_pw<HD, LA_C>(tmem_base + COL_NUM, sPlo, sV, LA_C * 128, true);
+          la_mma_tw<HD>(tmem_base + COL_NUM, tmem_base + COL_A, sV);
+          if (rem) la_mma_tw<HD>(tmem_base + COL_NUM, tmem_base + COL_A + 32, sV);
         }
-        la_mma_xTw<HD>(tmem_base + COL_S, sKc, k_lbo[st], sV, have_state0 || c > 0);                   // S += K~^T V
+        la_mma_xTw<HD>(tmem_base + COL_S, sKc, sV, have_state0 || c > 0);                   // S += K~^T V
         tc_commit(b_bar);
       }
     }
@@ -566,14 +477,13 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
     if (tid == 0) {                                                           // K~ and V of this chunk are free
-      if (HD == 128 && full && c + 1 < n_chunks) load(sQ, &tmQ, q_bar, c + 1);  // (its buffer held the remainder tile)
       if (c + 1 < n_chunks) load(sV, &tmV, v_bar, c + 1);
       if (c + 2 < n_chunks) load(sKc, &tmK, &k_bar[st], c + 2);
     }
     if (full) {
       float num[HH];
       la_tmem_row<HH>(trow + COL_NUM + hf * HH, num);
-      const int tok = c * LA_C + row;
+      const int tok = (c0 + c) * LA_C + row;
       if (tok < p.S) {
         const float inv = 1.f / den;
         __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o.ptr) + (long long)b * p.o.sb + (long long)tok * p.o.ss + (long long)h * p.o.sh + hf * HH;
@@ -610,83 +520,23 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     __syncthreads();
   }
   float* s_out = la_publish_begin<HD>(p, bh, sx_epoch, p.s_out);      // the caller's buffer, or this rank's slot of the exchange
-  if (ok && s_out && hf == 0) {
+  const size_t out_idx = full ? bh : blockIdx.x;
+  if (ok && s_out && hf == 0 && (!full || seg == p.n_seg - 1)) {
     tc_fence_after_sync();
     float srow[HD];
     la_tmem_row<HD>(trow + COL_S, srow);
     if (row < HD) {
 #pragma unroll
       for (int i = 0; i < HD; i += 4)
-        *reinterpret_cast<float4*>(s_out + bh * st_stride + (size_t)row * HD + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
-      s_out[bh * st_stride + (size_t)HD * HD + row] = sz[row];
+        *reinterpret_cast<float4*>(s_out + out_idx * st_stride + (size_t)row * HD + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
+      s_out[out_idx * st_stride + (size_t)HD * HD + row] = sz[row];
     }
   }
   la_publish_end(p, bh, sx_epoch);
   la_retire(p, sx_epoch);
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
-}
-
-// dO and O rows of one token -> G = dO / D (bf16 tile row), returns dden = -(dO . O) / D. Tokens past the end give zeros.
-template <int HD>
-__device__ __forceinline__ float la_load_g(const LinAttnArgs& p, int b, int h, int tok, uint8_t* sG, int row) {
-  uint32_t g[HD / 2];
-  float dden = 0.f;
-  if (tok < p.S) {
-    const __nv_bfloat16* dp = reinterpret_cast<const __nv_bfloat16*>(p.dout.ptr) + (long long)b * p.dout.sb + (long long)tok * p.dout.ss + (long long)h * p.dout.sh;
-    const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o.ptr) + (long long)b * p.o.sb + (long long)tok * p.o.ss + (long long)h * p.o.sh;
-    const __nv_bfloat16* lp = p.o_lo.ptr ? reinterpret_cast<const __nv_bfloat16*>(p.o_lo.ptr) + (long long)b * p.o_lo.sb + (long long)tok * p.o_lo.ss + (long long)h * p.o_lo.sh : nullptr;
-    const float inv = 1.f / p.den[((long long)b * p.H + h) * p.S + tok];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < HD; i += 8) {
-      const uint4 du = *reinterpret_cast<const uint4*>(dp + i), ou = *reinterpret_cast<const uint4*>(op + i);
-      const uint4 lu = lp ? *reinterpret_cast<const uint4*>(lp + i) : make_uint4(0, 0, 0, 0);
-      const uint32_t* dw = &du.x; const uint32_t* ow = &ou.x; const uint32_t* lw = &lu.x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 d2 = unpack_bf16x2(dw[j]), o2 = unpack_bf16x2(ow[j]), l2 = unpack_bf16x2(lw[j]);
-        // the SAME rounded G enters G V^T on the tensor core and the dot product here, so that the two halves of
-        // dA = G . (V_s - O_t) see one dO; O carries its remainder
-        const uint32_t gp = pack_bf16x2(d2.x * inv, d2.y * inv);
-        const float2 gr = unpack_bf16x2(gp);
-        g[(i >> 1) + j] = gp;
-        dot = fmaf(gr.x, o2.x + l2.x, dot); dot = fmaf(gr.y, o2.y + l2.y, dot);
-      }
-    }
-    dden = -dot;
-  } else {
-#pragma unroll
-    for (int i = 0; i < HD / 2; ++i) g[i] = 0u;
-  }
-#pragma unroll
-  for (int gi = 0; gi < HD / 8; ++gi)
-    *reinterpret_cast<uint4*>(sG + (gi >> 3) * (LA_C * 128) + sw128_offset(row, gi & 7)) =
-        make_uint4(g[gi * 4], g[gi * 4 + 1], g[gi * 4 + 2], g[gi * 4 + 3]);
-  return dden;
-}
-
-// grad[i] <- scale * phi'(scale * x_i) * grad[i] with x the raw (bf16) row in global memory, then store as bf16
-template <int HD>
-__device__ __forceinline__ void la_store_dphi(const AttnTensor& x, const AttnTensor& dx, int b, int h, int tok, const float* grad, float scale, int kind) {
-  const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (long long)b * x.sb + (long long)tok * x.ss + (long long)h * x.sh;
-  __nv_bfloat16* gp = reinterpret_cast<__nv_bfloat16*>(dx.ptr) + (long long)b * dx.sb + (long long)tok * dx.ss + (long long)h * dx.sh;
-#pragma unroll
-  for (int i = 0; i < HD; i += 8) {
-    const uint4 xu = *reinterpret_cast<const uint4*>(xp + i);
-    const uint32_t* xw = &xu.x;
-    uint32_t o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 x2 = unpack_bf16x2(xw[j]);
-      const float a = x2.x * scale, c = x2.y * scale;
-      const float da = kind == 0 ? (a > 0.f ? 1.f : __expf(a)) : (a > 0.f ? 2.f * a : 0.f);
-      const float dc = kind == 0 ? (c > 0.f ? 1.f : __expf(c)) : (c > 0.f ? 2.f * c : 0.f);
-      o[j] = pack_bf16x2(grad[i + 2 * j] * da * scale, grad[i + 2 * j + 1] * dc * scale);
-    }
-    *reinterpret_cast<uint4*>(gp + i) = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, L::TMEM); }
 }
 
 // ---------------------------------------------------------------------------------------------------- backward helpers (8 warps)
@@ -771,23 +621,20 @@ __device__ __forceinline__ float la_colsum_w_rows(const uint8_t* tile, int k, co
 // ---------------------------------------------------------------------------------------------------- backward 1: dQ
 // Same 8-warp mapping as the forward: warp w owns rows 32 (w & 3) .. and column half w >> 2.
 template <int HD>
-__global__ void __launch_bounds__(LA_FWD_THREADS, 1)
+__global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;
   constexpr int ZP = LA_FWD_THREADS / HD;
-  constexpr uint32_t COL_A = 0, COL_DQ = 128, COL_S = 256;
+  constexpr uint32_t COL_A = 0, COL_DQ = 128, COL_S = 128 + HD;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sG = smem;
   uint8_t* sK = sG + L::TILE;                 // 2 stages
-  uint8_t* sZero = sK + 2 * L::TILE;
-  uint8_t* sV = sZero + L::ZERO;
-  uint8_t* sP = sV + L::TILE;
-  uint8_t* sShi = sP + L::PT;
+  uint8_t* sV = sK + 2 * L::TILE;
+  uint8_t* sShi = sV + L::TILE;
   uint8_t* sSlo = sShi + L::ST;
-  uint8_t* sPlo = HD == 64 ? sSlo + L::ST : sG;
-  float* sz = reinterpret_cast<float*>(sSlo + L::ST + L::PLO);
+  float* sz = reinterpret_cast<float*>(sSlo + L::ST);
   float* s_part = sz + HD;                    // [2][128]: the halves' shares of dden; later in the chunk: partial column sums
   float* s_zk = s_part;                       // (two barriers lie between the last read of one use and the first write of the other)
   float* s_dden = s_part + 2 * LA_C;          // [128]
@@ -797,8 +644,9 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const int n_chunks = (p.S + LA_C - 1) / LA_C;
+  const int bh = blockIdx.x / p.n_seg, seg = blockIdx.x % p.n_seg, b = bh / p.H, h = bh % p.H;
+  const int c0 = seg * p.seg_chunks;           // first chunk of this CTA's segment
+  const int n_chunks = min(p.seg_chunks, (p.S + LA_C - 1) / LA_C - c0);
   const bool rem = p.kind == 0;                // see the forward kernel
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
@@ -806,15 +654,14 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     fence_barrier_init();
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  if (HD == 64) for (int i = tid; i < L::ZERO / 16; i += LA_FWD_THREADS) reinterpret_cast<uint4*>(sZero)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 0) { tmem_alloc(tmem_slot, L::TMEM); tmem_relinquish(); }
   const size_t st_stride = (size_t)HD * HD + HD;
   if (tid < HD) {
     float s0[HD];
 #pragma unroll
-    for (int i = 0; i < HD; ++i) s0[i] = p.s_in ? p.s_in[bh * st_stride + (size_t)tid * HD + i] : 0.f;
+    for (int i = 0; i < HD; ++i) s0[i] = p.s_in ? p.s_in[blockIdx.x * st_stride + (size_t)tid * HD + i] : 0.f;
     la_write_hilo<HD>(sShi, sSlo, HD, tid, s0);
-    sz[tid] = p.s_in ? p.s_in[bh * st_stride + (size_t)HD * HD + tid] : 0.f;
+    sz[tid] = p.s_in ? p.s_in[blockIdx.x * st_stride + (size_t)HD * HD + tid] : 0.f;
   }
   tc_fence_before_sync();
   fence_proxy_async_smem();
@@ -827,7 +674,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     for (int c = 0; c < HD / 32; ++c) {
       uint32_t r[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(p.s_in[bh * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
+      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(p.s_in[blockIdx.x * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
       tmem_st_x32(trow + COL_S + c * 32, r);
     }
     tmem_st_wait();
@@ -839,9 +686,8 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int chunk) {
     mbar_expect_tx(bar, L::TILE);
 #pragma unroll
-    for (int a = 0; a < KA; ++a) tma_load_4d(dst + a * (LA_C * 128), tm, bar, a * 64, h, chunk * LA_C, b);
+    for (int a = 0; a < KA; ++a) tma_load_4d(dst + a * (LA_C * 128), tm, bar, a * 64, h, (c0 + chunk) * LA_C, b);
   };
-  const uint32_t k_lbo[2] = {HD == 64 ? uint32_t(2 * L::TILE) : uint32_t(LA_C * 128), HD == 64 ? uint32_t(L::TILE) : uint32_t(LA_C * 128)};
   if (tid == 0) {
     load(sK, &tmK, &k_bar[0], 0);
     load(sV, &tmV, v_bar, 0);
@@ -852,8 +698,8 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   for (int c = 0; c < n_chunks; ++c) {
     const int st = c & 1;
     uint8_t* sKc = sK + st * L::TILE;
-    const int valid = min(LA_C, p.S - c * LA_C);
-    const int tok = c * LA_C + row;
+    const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
+    const int tok = (c0 + c) * LA_C + row;
     // this half of G and its share of dden come straight from global memory while the TMA tiles land
     s_part[hf * LA_C + row] = la_load_g_half<HD>(p, b, h, tok, sG, row, hf);
     if (!mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
@@ -878,16 +724,15 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       la_tmem_row<64>(trow + COL_A + hf * 64, a);
 #pragma unroll
       for (int i = 0; i < 64; ++i) a[i] = (hf * 64 + i > row) ? 0.f : a[i] + dden;
-      la_write_half128_hilo(sP, sPlo, row, hf, a, rem);
+      la_put_half128(trow + COL_A + hf * 64, a, rem);
     }
     tc_fence_before_sync();
-    fence_proxy_async_smem();
     __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
-      la_mma_pw<HD, LA_C>(tmem_base + COL_DQ, sP, sKc, LA_C * 128, true);             // dQ~ += dA K~ (value + remainder)
-      if (rem) la_mma_pw<HD, LA_C>(tmem_base + COL_DQ, sPlo, sKc, LA_C * 128, true);
-      la_mma_xTw<HD>(tmem_base + COL_S, sKc, k_lbo[st], sV, have_state0 || c > 0);    // S += K~^T V
+      la_mma_tw<HD>(tmem_base + COL_DQ, tmem_base + COL_A, sKc);                      // dQ~ += dA K~ (value + remainder)
+      if (rem) la_mma_tw<HD>(tmem_base + COL_DQ, tmem_base + COL_A + 32, sKc);
+      la_mma_xTw<HD>(tmem_base + COL_S, sKc, sV, have_state0 || c > 0);    // S += K~^T V
       tc_commit(b_bar);
     }
     s_zk[tid] = la_colsum_rows(sKc, tid % HD, (tid / HD) * (LA_C / ZP), LA_C / ZP);
@@ -925,27 +770,27 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, L::TMEM); }
 }
 
 // ---------------------------------------------------------------------------------------------------- backward 2: dK, dV
 template <int HD>
-__global__ void __launch_bounds__(LA_FWD_THREADS, 1)
+__global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;
   constexpr int ZP = LA_FWD_THREADS / HD;
-  constexpr uint32_t COL_T = 0, COL_DV = 128, COL_DK = 128 + HD, COL_DS = 128 + 2 * HD;
+  constexpr uint32_t COL_T = 0, COL_DV = 128, COL_DK = 128 + HD, COL_DS = HD == 64 ? COL_T : 128 + 2 * HD;
+  // Head size 64 keeps dS in registers (a chunk's share goes through T's columns): 256 TMEM columns hold T, dV and dK
+  constexpr bool DS_REG = HD == 64;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
-  uint8_t* sZero = sQ + L::TILE;               // HD = 64: pads Q~^T G to 128 rows
-  uint8_t* sK = sZero + L::ZERO;
+  uint8_t* sK = sQ + L::TILE;
   uint8_t* sV = sK + L::TILE;
   uint8_t* sG = sV + L::TILE;
-  uint8_t* sP = sG + L::TILE;
-  uint8_t* sDhi = sP + L::PT;
+  uint8_t* sDhi = sG + L::TILE;
   uint8_t* sDlo = sDhi + L::ST;
   float* sdz = reinterpret_cast<float*>(sDlo + L::ST);     // [HD]
   float* sdden = sdz + HD;                                  // [128]
@@ -957,26 +802,27 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const int n_chunks = (p.S + LA_C - 1) / LA_C;
+  const int bh = blockIdx.x / p.n_seg, seg = blockIdx.x % p.n_seg, b = bh / p.H, h = bh % p.H;
+  const int c0 = seg * p.seg_chunks;           // first chunk of this CTA's segment
+  const int n_chunks = min(p.seg_chunks, (p.S + LA_C - 1) / LA_C - c0);
   const bool full = !p.state_only;               // state_only: only dS / dz of this slice (reads Q, dO, O)
+  if (p.n_seg > 1 && !full && seg == 0) return;  // nothing precedes the first segment
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
     mbar_init(ld_bar, 1); mbar_init(t_bar, 1); mbar_init(u_bar, 1); mbar_init(b_bar, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
-  if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  if (HD == 64) for (int i = tid; i < L::ZERO / 16; i += LA_FWD_THREADS) reinterpret_cast<uint4*>(sZero)[i] = make_uint4(0, 0, 0, 0);
+  if (warp == 0) { tmem_alloc(tmem_slot, L::TMEM); tmem_relinquish(); }
   const size_t st_stride = (size_t)HD * HD + HD;
   const uint32_t sx_epoch = la_epoch(p);
   const float* ds_in = la_consume<HD>(p, bh, sx_epoch, p.ds_in);     // the caller's dS, or the higher ranks' totals
   if (tid < HD) {
     float s0[HD];
 #pragma unroll
-    for (int i = 0; i < HD; ++i) s0[i] = ds_in ? ds_in[bh * st_stride + (size_t)tid * HD + i] : 0.f;
+    for (int i = 0; i < HD; ++i) s0[i] = ds_in ? ds_in[blockIdx.x * st_stride + (size_t)tid * HD + i] : 0.f;
     la_write_hilo<HD>(sDhi, sDlo, HD, tid, s0);
-    sdz[tid] = ds_in ? ds_in[bh * st_stride + (size_t)HD * HD + tid] : 0.f;
+    sdz[tid] = ds_in ? ds_in[blockIdx.x * st_stride + (size_t)HD * HD + tid] : 0.f;
   }
   tc_fence_before_sync();
   fence_proxy_async_smem();
@@ -984,12 +830,17 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t trow = tmem_base + (uint32_t(quad * 32) << 16);
-  if (ds_in && hf == 0) {
+  float ds_acc[DS_REG ? HH : 1];                                                      // DS_REG: this thread's half row of dS
+  if (DS_REG) {
+#pragma unroll
+    for (int i = 0; i < (DS_REG ? HH : 1); ++i) ds_acc[i] = (ds_in && row < HD) ? ds_in[blockIdx.x * st_stride + (size_t)row * HD + hf * HH + i] : 0.f;
+  }
+  if (!DS_REG && ds_in && hf == 0) {
 #pragma unroll
     for (int c = 0; c < HD / 32; ++c) {
       uint32_t r[32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(ds_in[bh * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
+      for (int i = 0; i < 32; ++i) r[i] = row < HD ? __float_as_uint(ds_in[blockIdx.x * st_stride + (size_t)row * HD + c * 32 + i]) : 0u;
       tmem_st_x32(trow + COL_DS + c * 32, r);
     }
     tmem_st_wait();
@@ -1002,20 +853,19 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     mbar_expect_tx(ld_bar, 3 * L::TILE);
 #pragma unroll
     for (int a = 0; a < KA; ++a) {
-      tma_load_4d(sQ + a * (LA_C * 128), &tmQ, ld_bar, a * 64, h, chunk * LA_C, b);
-      tma_load_4d(sK + a * (LA_C * 128), &tmK, ld_bar, a * 64, h, chunk * LA_C, b);
-      tma_load_4d(sV + a * (LA_C * 128), &tmV, ld_bar, a * 64, h, chunk * LA_C, b);
+      tma_load_4d(sQ + a * (LA_C * 128), &tmQ, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
+      tma_load_4d(sK + a * (LA_C * 128), &tmK, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
+      tma_load_4d(sV + a * (LA_C * 128), &tmV, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
     }
   };
-  const uint32_t q_lbo = HD == 64 ? uint32_t(L::TILE) : uint32_t(LA_C * 128);
   if (tid == 0) load_all(n_chunks - 1);
   bool ok = true;
   const bool have_state0 = ds_in != nullptr;
   uint32_t t_phase = 0;
   for (int it = 0; it < n_chunks; ++it) {
     const int c = n_chunks - 1 - it;
-    const int valid = min(LA_C, p.S - c * LA_C);
-    const int tok = c * LA_C + row;
+    const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
+    const int tok = (c0 + c) * LA_C + row;
     s_part[hf * LA_C + row] = la_load_g_half<HD>(p, b, h, tok, sG, row, hf);
     if (!mbar_wait(ld_bar, it & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
@@ -1043,16 +893,15 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       la_tmem_row<64>(trow + COL_T + hf * 64, a);
 #pragma unroll
       for (int i = 0; i < 64; ++i) if (hf * 64 + i < row) a[i] = 0.f;                // keep queries at or after this key
-      la_write_half128_hilo(sP, sP, row, hf, a, false);
+      la_put_half128(trow + COL_T + hf * 64, a, false);
     }
     tc_fence_before_sync();
-    fence_proxy_async_smem();
     __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
-      la_mma_pw<HD, LA_C>(tmem_base + COL_DV, sP, sG, LA_C * 128, true);              // dV += mask(A)^T G
+      la_mma_tw<HD>(tmem_base + COL_DV, tmem_base + COL_T, sG);                       // dV += mask(A)^T G
       tc_commit(u_bar);
-      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);                                      // (G V^T)^T = V G^T   [key][query]
+      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);                                      // (G V^T)^T = V G^T   [key][query], over the tile dV has read
       tc_commit(t_bar);
     }
     if (!mbar_wait(t_bar, t_phase, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;      // implies u_bar: the tensor core runs in order
@@ -1065,16 +914,15 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       la_tmem_row<64>(trow + COL_T + hf * 64, a);
 #pragma unroll
       for (int i = 0; i < 64; ++i) a[i] = (hf * 64 + i < row) ? 0.f : a[i] + sdden[hf * 64 + i];
-      la_write_half128_hilo(sP, sP, row, hf, a, false);
+      la_put_half128(trow + COL_T + hf * 64, a, false);
     }
     tc_fence_before_sync();
-    fence_proxy_async_smem();
     }
     __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
-      if (full) la_mma_pw<HD, LA_C>(tmem_base + COL_DK, sP, sQ, LA_C * 128, true);    // dK~ += mask(dA)^T Q~
-      la_mma_xTw<HD>(tmem_base + COL_DS, sQ, q_lbo, sG, have_state0 || it > 0);       // dS += Q~^T G
+      if (full) la_mma_tw<HD>(tmem_base + COL_DK, tmem_base + COL_T, sQ);             // dK~ += mask(dA)^T Q~
+      la_mma_xTw<HD>(tmem_base + COL_DS, sQ, sG, !DS_REG && (have_state0 || it > 0)); // dS += Q~^T G
       tc_commit(b_bar);
     }
     // dz += Q~^T dden in fp32: ZP row groups per column, combined after the barriers below
@@ -1107,41 +955,51 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       for (int g = 0; g < ZP; ++g) dzk += s_zk[g * HD + tid];
       sdz[tid] += dzk;
     }
-    if (full && c > 0 && quad * 32 < HD) {
+    if (quad * 32 < HD && (DS_REG || (full && c > 0))) {
       float srow[HH];
       la_tmem_row<HH>(trow + COL_DS + hf * HH, srow);
-      if (row < HD) la_write_hilo_half<HD>(sDhi, sDlo, HD, row, hf, srow);
+      if constexpr (DS_REG) {
+#pragma unroll
+        for (int i = 0; i < HH; ++i) srow[i] = ds_acc[i] += srow[i];
+      }
+      if (full && c > 0 && row < HD) la_write_hilo_half<HD>(sDhi, sDlo, HD, row, hf, srow);
       fence_proxy_async_smem();
     }
     tc_fence_before_sync();
     __syncthreads();
   }
   float* ds_out = la_publish_begin<HD>(p, bh, sx_epoch, p.ds_out);
-  if (ok && ds_out && hf == 0) {
+  const size_t out_idx = full ? bh : blockIdx.x;
+  if (ok && ds_out && (!full || seg == 0)) {
     tc_fence_after_sync();
-    float srow[HD];
-    la_tmem_row<HD>(trow + COL_DS, srow);
+    float srow[HH];
+    if constexpr (DS_REG) {
+#pragma unroll
+      for (int i = 0; i < HH; ++i) srow[i] = ds_acc[i];
+    } else {
+      la_tmem_row<HH>(trow + COL_DS + hf * HH, srow);
+    }
     if (row < HD) {
 #pragma unroll
-      for (int i = 0; i < HD; i += 4)
-        *reinterpret_cast<float4*>(ds_out + bh * st_stride + (size_t)row * HD + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
-      ds_out[bh * st_stride + (size_t)HD * HD + row] = sdz[row];
+      for (int i = 0; i < HH; i += 4)
+        *reinterpret_cast<float4*>(ds_out + out_idx * st_stride + (size_t)row * HD + hf * HH + i) = make_float4(srow[i], srow[i + 1], srow[i + 2], srow[i + 3]);
+      if (hf == 0) ds_out[out_idx * st_stride + (size_t)HD * HD + row] = sdz[row];
     }
   }
   la_publish_end(p, bh, sx_epoch);
   la_retire(p, sx_epoch);
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, L::TMEM); }
 }
 
 // ---------------------------------------------------------------------------------------------------- host side
-template <int HD> constexpr int la_fwd_smem() { return 4 * LaSmem<HD>::TILE + LaSmem<HD>::ZERO + LaSmem<HD>::PT + LaSmem<HD>::PLO + 2 * LaSmem<HD>::ST + HD * 4 + 128; }
+template <int HD> constexpr int la_fwd_smem() { return 4 * LaSmem<HD>::TILE + 2 * LaSmem<HD>::ST + HD * 4 + 128; }
 // the forward kernel also keeps [2][128] denominator shares and 256 partial column sums
 template <int HD> constexpr int la_fwd8_smem() { return la_fwd_smem<HD>() + 2 * LA_C * 4 + LA_FWD_THREADS * 4; }
 // dQ: [2][128] dden shares (reused for the partial column sums) + [128] dden; dK / dV: the same shares beside its [128] dden
 template <int HD> constexpr int la_dq8_smem() { return la_fwd_smem<HD>() + 3 * LA_C * 4; }
-template <int HD> constexpr int la_dkv_smem() { return 4 * LaSmem<HD>::TILE + LaSmem<HD>::ZERO + LaSmem<HD>::PT + 2 * LaSmem<HD>::ST + (HD + LA_C) * 4 + 2 * LA_C * 4 + 128; }
+template <int HD> constexpr int la_dkv_smem() { return 4 * LaSmem<HD>::TILE + 2 * LaSmem<HD>::ST + (HD + LA_C) * 4 + 2 * LA_C * 4 + 128; }
 
 static int la_maps(const LinAttnArgs& a, CUtensorMap* tq, CUtensorMap* tk, CUtensorMap* tv) {
   const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -1163,14 +1021,46 @@ static int la_set_attrs() {
   return 0;
 }
 
+// The states between segments: in place, seg[bh][s] <- base[bh] + the totals of the segments before s (`reverse`: behind s).
+__global__ void la_segment_prefix_kernel(float* __restrict__ seg, const float* __restrict__ base, int n_seg, int n, int reverse) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float* p = seg + (size_t)blockIdx.y * n_seg * n + i;
+  float acc = base ? base[(size_t)blockIdx.y * n + i] : 0.f;
+  for (int k0 = 0; k0 < n_seg; k0 += 8) {            // eight loads in flight: the sum is the only serial part
+    float t[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)                      // (the last one's total was not taken)
+      t[k] = k0 + k + 1 < n_seg ? p[(size_t)(reverse ? n_seg - 1 - k0 - k : k0 + k) * n] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k0 + k < n_seg) { p[(size_t)(reverse ? n_seg - 1 - k0 - k : k0 + k) * n] = acc; acc += t[k]; }
+  }
+}
+
 template <int HD>
 static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
   if (la_set_attrs<HD>()) return 104;
+  if (a.n_seg > 1 && !a.state_only && a.s_in != a.seg && a.ds_in != a.seg) {
+    // segments: their totals, the prefix over them (the forward's serves the dQ pass too), then the pass itself from there
+    LinAttnArgs t = a;
+    if (which != 1) {
+      t.state_only = 1; t.s_in = t.ds_in = nullptr; t.s_out = t.ds_out = a.seg;
+      if (int rc = la_launch<HD>(t, which, st)) return rc;
+      constexpr int N = HD * HD + HD;
+      la_segment_prefix_kernel<<<dim3((N + 255) / 256, a.B * a.H), 256, 0, st>>>(a.seg, which == 0 ? a.s_in : a.ds_in, a.n_seg, N, which == 2);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return 400 + (int)e;
+    }
+    t = a;
+    if (which == 2) t.ds_in = a.seg; else t.s_in = a.seg;
+    return la_launch<HD>(t, which, st);
+  }
   CUtensorMap tq, tk, tv;
   const bool need_q = which != 1 && !(which == 0 && a.state_only);
   if (int rc = la_maps(a, need_q ? &tq : nullptr, &tk, &tv)) return rc;
   if (!need_q) tq = tk;
-  const unsigned grid = (unsigned)(a.B * a.H);
+  const unsigned grid = (unsigned)(a.B * a.H * a.n_seg);
   if (which == 0) linattn_fwd_kernel<HD><<<grid, LA_FWD_THREADS, la_fwd8_smem<HD>(), st>>>(tq, tk, tv, a);
   else if (which == 1) linattn_bwd_dq_kernel<HD><<<grid, LA_FWD_THREADS, la_dq8_smem<HD>(), st>>>(tk, tv, a);
   else linattn_bwd_dkv_kernel<HD><<<grid, LA_FWD_THREADS, la_dkv_smem<HD>(), st>>>(tq, tk, tv, a);
@@ -1184,7 +1074,8 @@ static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
 extern "C" int b200_linattn(const b200::LinAttnArgs* a, int which, cudaStream_t st) {
   using namespace b200;
   if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
-  if (which < 0 || which > 2) return -2;
+  if (which < 0 || which > 2 || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
+  if ((long long)a->n_seg * a->seg_chunks < (a->S + LA_C - 1) / LA_C || (long long)(a->n_seg - 1) * a->seg_chunks >= (a->S + LA_C - 1) / LA_C) return -2;
   if (a->hd == 64) return la_launch<64>(*a, which, st);
   if (a->hd == 128) return la_launch<128>(*a, which, st);
   return -3;

@@ -21,16 +21,16 @@ Inputs are [B, S, H, d] (any strides); output [B, S, H, d].
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 
 import torch
 from torch.autograd import Function
 
-import ctypes as C
-
 from .. import _native as nv
 from . import kernels as K
 from .functional import matmul
+from .gemm import _num_sms
 
 CHUNK = 128
 
@@ -51,7 +51,8 @@ class LinAttnArgs(C.Structure):
                 ("dout", nv.AttnTensor), ("dq", nv.AttnTensor), ("dk", nv.AttnTensor), ("dv", nv.AttnTensor), ("o_lo", nv.AttnTensor),
                 ("den", C.c_void_p), ("s_in", C.c_void_p), ("s_out", C.c_void_p), ("ds_in", C.c_void_p), ("ds_out", C.c_void_p),
                 ("B", C.c_int), ("H", C.c_int), ("S", C.c_int), ("hd", C.c_int), ("scale", C.c_float), ("eps", C.c_float),
-                ("kind", C.c_int), ("state_only", C.c_int), ("status", C.c_void_p), ("sx", LaExchange)]
+                ("kind", C.c_int), ("state_only", C.c_int), ("status", C.c_void_p),
+                ("seg", C.c_void_p), ("n_seg", C.c_int), ("seg_chunks", C.c_int), ("sx", LaExchange)]
 
 
 nv.register_sigs({"b200_linattn": [C.POINTER(LinAttnArgs), C.c_int, C.c_void_p], "b200_linattn_init": []})
@@ -74,7 +75,7 @@ def fused_supported(q, causal) -> bool:
 
 @nv.traced("linear_attention")
 def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=None, dk=None, dv=None, s_in=None, s_out=None,
-            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None):
+            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None, seg=None, n_seg=1):
     """`sx = (SPContext, dir, role)` lets the kernel itself exchange the slice totals with the other ranks (see
     `LaExchange`); it returns the local buffer the consume pass leaves the summed state in."""
     B, S, H, d = q.shape
@@ -89,10 +90,21 @@ def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=No
     a.den, a.s_in, a.s_out, a.ds_in, a.ds_out = nv.ptr(den), nv.ptr(s_in), nv.ptr(s_out), nv.ptr(ds_in), nv.ptr(ds_out)
     a.B, a.H, a.S, a.hd, a.scale, a.eps = B, H, S, d, float(scale), float(eps)
     a.kind, a.state_only = (0 if kind == "elu" else 1), int(state_only)
-    a.status = nv.status_word(q.device).data_ptr()
+    a.status = nv.status_ptr(q.device)
+    n_chunks = -(-S // CHUNK)
+    a.seg, a.n_seg, a.seg_chunks = nv.ptr(seg), n_seg, -(-n_chunks // n_seg)
     nv.check(nv.cuda().b200_linattn(C.byref(a), which, nv.stream_ptr()), "linattn")
-    nv.count_launch()
+    nv.count_launch(1 if n_seg == 1 or which == 1 else 3)
     return prefix
+
+
+def _segments(bh: int, n_chunks: int, hd: int, sms: int) -> int:
+    """Into how many segments the sequence of every (batch, head) is cut: as many as still run at once (two CTAs per SM at
+    head size 64, one at 128). A segment costs a pass over its K and V (Q, dO, O in the backward) for its total, so segments
+    that would queue lose: 8 x 16 heads, 4096 tokens, head size 128, forward + backward 1.70 ms whole, 2.11 ms in two; while
+    1 x 8 heads x 16384 x 128 takes 6.32 ms whole and 0.69 ms in 16, 1 x 16 x 1000 x 128 0.34 and 0.17 ms in 8."""
+    n = max(1, min((2 if hd == 64 else 1) * sms // max(bh, 1), n_chunks, 64))
+    return -(-n_chunks // -(-n_chunks // n))                     # no empty last segment
 
 
 class FusedCausalLinearAttnFn(Function):
@@ -124,7 +136,10 @@ class FusedCausalLinearAttnFn(Function):
             pre = _launch(0, q, k, v, scale, eps, kind, o=o, den=den, o_lo=o_lo, sx=(sp, 0, 2))
             s_in = pre.clone() if (sp.rank > 0 and need_grad) else None      # the buffer is reused by the next call
         else:
-            _launch(0, q, k, v, scale, eps, kind, o=o, den=den, s_in=s_in, o_lo=o_lo)
+            n_seg = 1 if sp is not None else _segments(B * H, -(-S // CHUNK), d, _num_sms(dev))
+            seg = torch.empty((B * H, n_seg, d * d + d), dtype=torch.float32, device=dev) if n_seg > 1 else None
+            _launch(0, q, k, v, scale, eps, kind, o=o, den=den, s_in=s_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
+            s_in = s_in if seg is None else seg                  # the states the backward's dQ pass starts from
         ctx.save_for_backward(q, k, v, o, den, s_in if s_in is not None else torch.empty(0), o_lo if o_lo is not None else torch.empty(0))
         ctx.cfg = (scale, eps, kind, sp)
         return o
@@ -134,11 +149,12 @@ class FusedCausalLinearAttnFn(Function):
         q, k, v, o, den, s_in, o_lo = ctx.saved_tensors
         scale, eps, kind, sp = ctx.cfg
         s_in = s_in if s_in.numel() else None
+        n_seg = s_in.shape[1] if (s_in is not None and s_in.dim() == 3) else 1
         o_lo = o_lo if o_lo.numel() else None
         B, S, H, d = q.shape
         dout = dout if (_tma_ok(dout) and dout.dtype == torch.bfloat16) else dout.to(torch.bfloat16).contiguous()
         dq, dk, dv = torch.empty_like(o), torch.empty_like(o), torch.empty_like(o)
-        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, s_in=s_in, o_lo=o_lo)
+        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, s_in=None if n_seg > 1 else s_in, o_lo=o_lo, seg=s_in if n_seg > 1 else None, n_seg=n_seg)
         ds_in = None
         if sp is not None and sp.world > 1 and sp.backend == "fused":
             _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, state_only=True, o_lo=o_lo, sx=(sp, 1, 1))
@@ -148,7 +164,8 @@ class FusedCausalLinearAttnFn(Function):
             tot = torch.empty((B * H, d * d + d), dtype=torch.float32, device=q.device)
             _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, ds_out=tot, state_only=True, o_lo=o_lo)
             ds_in = sp._exchange(tot, 1)                        # sum of the higher ranks' totals
-        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo)
+        seg = torch.empty_like(s_in) if n_seg > 1 else None
+        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
         return dq, dk, dv, None, None, None, None
 
 

@@ -115,3 +115,32 @@ def test_run_twice_is_bit_identical():
         res.append((out.detach().clone(), qi.grad.clone(), ki.grad.clone(), vi.grad.clone()))
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("S,hd,kind,n", [(129, 64, "elu", 2), (1000, 64, "relu2", 3), (1000, 128, "elu", 8), (2049, 128, "relu2", 4), (640, 64, "elu", 5)])
+def test_segments_equal_one_walk(S, hd, kind, n, monkeypatch):
+    """A sequence walked in segments (short last segment, short last chunk) against the same kernels walking it whole. Only
+    the order of the fp32 state sums differs (~1e-6), which moves a bf16 result by at most one rounding: 2^-9."""
+    from rust_neural_network_b200 import _native as nv
+    from rust_neural_network_b200.ops import linear_attention as LA
+    q, k, v, w = _inputs(2, S, 3, hd, seed=S)
+    run = lambda: _grads(lambda a, b, c: LA.linear_attention(a, b, c, scale=hd ** -0.5, causal=True, kind=kind), q, k, v, w, False)
+    n_chunks = -(-S // LA.CHUNK)
+    assert n_chunks > (n - 1) * -(-n_chunks // n)
+    monkeypatch.setattr(LA, "_segments", lambda *a: 1)
+    o1, g1 = run()
+    monkeypatch.setattr(LA, "_segments", lambda *a: n)
+    o2, g2 = run()
+    torch.cuda.synchronize(); nv.check_status()
+    for a, b in zip([o2] + g2, [o1] + g1):
+        assert _rel(a, b) < 2 ** -9
+
+
+def test_segment_rule_leaves_no_empty_segment():
+    from rust_neural_network_b200.ops.linear_attention import _segments
+    for bh in (1, 3, 16, 128, 1000):
+        for n_chunks in list(range(1, 70)) + [511, 4096]:
+            for hd in (64, 128):
+                n = _segments(bh, n_chunks, hd, 148)
+                per = -(-n_chunks // n)
+                assert 1 <= n <= 64 and n * per >= n_chunks > (n - 1) * per
