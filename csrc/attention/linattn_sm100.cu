@@ -59,10 +59,12 @@ struct LaExchange {
 struct LinAttnArgs {
   AttnTensor q, k, v, o;                     // bf16 [B, S, H, hd] (any strides, hd contiguous)
   AttnTensor dout, dq, dk, dv;               // backward
+  AttnTensor g;                              // backward scratch, bf16: G = dO / D (written by the G pass, read by both gradient kernels)
   AttnTensor o_lo;                           // optional bf16 remainder O - bf16(O): written by forward, read by backward.
                                              // dden = -(dO . O) / D is one half of a difference of nearly equal terms
                                              // (S^T G against (G . O) z); 8 mantissa bits of O are not enough for it
   float* den;                                // [B, H, S] fp32: denominators incl. eps (written by forward, read by backward)
+  float* dden;                               // backward scratch, [B, H, S] fp32: -(G . O)
   const float* s_in;                         // optional [B*H][hd*hd + hd] fp32: state (row-major [d_k][d_v]) then z
   float* s_out;                              // optional, same layout: state after the last token (forward / state pass)
   const float* ds_in;                        // backward 2, optional: dS, dz flowing in from the tokens after this slice
@@ -149,7 +151,17 @@ __device__ __forceinline__ void la_retire(const LinAttnArgs& p, uint32_t epoch) 
   if (atomicAdd(x.words + 1, 1u) == gridDim.x - 1) { x.words[1] = 0u; __threadfence(); x.words[0] = epoch; }
 }
 
-__device__ __forceinline__ float la_phi(float x, int kind) { return kind == 0 ? (x > 0.f ? x + 1.f : __expf(x)) : (x > 0.f ? x * x : 0.f); }
+// Both sides of a feature map are computed and one is selected: as a branch per element, the exponentials of one tile took
+// 2550 cycles. (An overflowing exponential is never the selected side; a NaN is.)
+__device__ __forceinline__ float la_exp(float x) { return ex2_approx(x * 1.4426950408889634f); }
+__device__ __forceinline__ float la_phi(float x, int kind) {
+  const float e = la_exp(x), p = x + 1.f, q = x * x;
+  return x > 0.f ? (kind == 0 ? p : q) : (kind == 0 ? e : 0.f);
+}
+__device__ __forceinline__ float la_dphi(float x, int kind) {
+  const float e = la_exp(x), q = 2.f * x;
+  return x > 0.f ? (kind == 0 ? 1.f : q) : (kind == 0 ? e : 0.f);
+}
 // One fp32 row of HD values -> bf16 "value" tile and bf16 "remainder" tile (row = thread), [rows][HD] swizzled atoms
 // of `rows` rows each.
 template <int HD>
@@ -334,10 +346,22 @@ __device__ __forceinline__ float la_colsum_rows(const uint8_t* tile, int k, int 
   return (s0 + s1) + (s2 + s3);
 }
 
+// 16-byte piece `i` (of HD / 16) of this thread's half row in a swizzled [128][HD] tile
+template <int HD>
+__device__ __forceinline__ uint4* la_half_piece(uint8_t* tile, int row, int hf, int i) {
+  const int c = hf * (HD / 16) + i;
+  return reinterpret_cast<uint4*>(tile + (c >> 3) * (LA_C * 128) + sw128_offset(row, c & 7));
+}
+// a finished [128][HD] tile to global memory (one thread; tokens past the end are clipped by the tensor map)
+template <int HD>
+__device__ __forceinline__ void la_store_tile(const CUtensorMap* tm, const uint8_t* tile, int h, int tok0, int b) {
+#pragma unroll
+  for (int a = 0; a < HD / 64; ++a) tma_store_4d(tm, tile + a * (LA_C * 128), a * 64, h, tok0, b);
+}
 template <int HD>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
-linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
+linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                   const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmLo, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;                  // columns of a HD-wide row per thread
@@ -476,7 +500,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (!mbar_wait(b_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
-    if (tid == 0) {                                                           // K~ and V of this chunk are free
+    if (tid == 0 && !full) {                                                  // K~ and V of this chunk are free
       if (c + 1 < n_chunks) load(sV, &tmV, v_bar, c + 1);
       if (c + 2 < n_chunks) load(sKc, &tmK, &k_bar[st], c + 2);
     }
@@ -484,25 +508,22 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       float num[HH];
       la_tmem_row<HH>(trow + COL_NUM + hf * HH, num);
       const int tok = (c0 + c) * LA_C + row;
-      if (tok < p.S) {
-        const float inv = 1.f / den;
-        __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o.ptr) + (long long)b * p.o.sb + (long long)tok * p.o.ss + (long long)h * p.o.sh + hf * HH;
-        __nv_bfloat16* lp = p.o_lo.ptr ? reinterpret_cast<__nv_bfloat16*>(p.o_lo.ptr) + (long long)b * p.o_lo.sb + (long long)tok * p.o_lo.ss + (long long)h * p.o_lo.sh + hf * HH : nullptr;
+      const float inv = 1.f / den;
+      // O and its remainder leave as tiles: through V's and K~'s buffers, which this chunk is done with
 #pragma unroll
-        for (int i = 0; i < HH; i += 8) {
-          uint32_t hi[4], lo[4];
+      for (int i = 0; i < HH; i += 8) {
+        uint32_t hi[4], lo[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float x = num[i + 2 * j] * inv, y = num[i + 2 * j + 1] * inv;
-            hi[j] = pack_bf16x2(x, y);
-            const float2 r = unpack_bf16x2(hi[j]);
-            lo[j] = pack_bf16x2(x - r.x, y - r.y);
-          }
-          *reinterpret_cast<uint4*>(op + i) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          if (lp) *reinterpret_cast<uint4*>(lp + i) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        for (int j = 0; j < 4; ++j) {
+          const float x = num[i + 2 * j] * inv, y = num[i + 2 * j + 1] * inv;
+          hi[j] = pack_bf16x2(x, y);
+          const float2 r = unpack_bf16x2(hi[j]);
+          lo[j] = pack_bf16x2(x - r.x, y - r.y);
         }
-        if (p.den && hf == 0) p.den[((long long)b * p.H + h) * p.S + tok] = den;
+        *la_half_piece<HD>(sV, row, hf, i / 8) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (p.o_lo.ptr) *la_half_piece<HD>(sKc, row, hf, i / 8) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
       }
+      if (tok < p.S && p.den && hf == 0) p.den[((long long)b * p.H + h) * p.S + tok] = den;
     }
     if (tid < HD) {
       float zk = 0.f;
@@ -514,11 +535,22 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       float srow[HH];
       la_tmem_row<HH>(trow + COL_S + hf * HH, srow);
       if (row < HD) la_write_hilo_half<HD>(sShi, sSlo, HD, row, hf, srow);
-      fence_proxy_async_smem();
     }
+    fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncthreads();
+    if (full && tid == 0) {
+      la_store_tile<HD>(&tmO, sV, h, (c0 + c) * LA_C, b);
+      if (p.o_lo.ptr) la_store_tile<HD>(&tmLo, sKc, h, (c0 + c) * LA_C, b);
+      tma_store_commit();
+      if (c + 1 < n_chunks) {
+        tma_store_wait_read0();
+        load(sV, &tmV, v_bar, c + 1);
+        if (c + 2 < n_chunks) load(sKc, &tmK, &k_bar[st], c + 2);
+      }
+    }
   }
+  if (tid == 0) tma_store_wait0();
   float* s_out = la_publish_begin<HD>(p, bh, sx_epoch, p.s_out);      // the caller's buffer, or this rank's slot of the exchange
   const size_t out_idx = full ? bh : blockIdx.x;
   if (ok && s_out && hf == 0 && (!full || seg == p.n_seg - 1)) {
@@ -540,67 +572,54 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------------- backward helpers (8 warps)
-// This thread's half of one token: G = dO / D for HD / 2 columns (bf16 tile row), returns its share of -(G . O).
-// Tokens past the end give zeros.
-template <int HD>
-__device__ __forceinline__ float la_load_g_half(const LinAttnArgs& p, int b, int h, int tok, uint8_t* sG, int row, int hf) {
-  constexpr int HH = HD / 2;
-  uint32_t g[HH / 2];
-  float dden = 0.f;
-  if (tok < p.S) {
-    const __nv_bfloat16* dp = reinterpret_cast<const __nv_bfloat16*>(p.dout.ptr) + (long long)b * p.dout.sb + (long long)tok * p.dout.ss + (long long)h * p.dout.sh + hf * HH;
-    const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(p.o.ptr) + (long long)b * p.o.sb + (long long)tok * p.o.ss + (long long)h * p.o.sh + hf * HH;
-    const __nv_bfloat16* lp = p.o_lo.ptr ? reinterpret_cast<const __nv_bfloat16*>(p.o_lo.ptr) + (long long)b * p.o_lo.sb + (long long)tok * p.o_lo.ss + (long long)h * p.o_lo.sh + hf * HH : nullptr;
-    const float inv = 1.f / p.den[((long long)b * p.H + h) * p.S + tok];
-    float dot = 0.f;
+// G = dO / D (bf16) and dden = -(G . O) per token, once for both gradient kernels and their state pass: formed inside them,
+// the three dependent loads cost each chunk 5500 of its 16500 cycles; as a tile G is a TMA load that is under way early.
+// hd / 8 lanes share a token; tokens are enumerated [b][s][h] so that neighbouring lanes read neighbouring memory.
+__global__ void la_g_kernel(const LinAttnArgs p) {
+  const int lpr = p.hd / 8;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long w = t / lpr;
+  const int sub = (int)(t % lpr);
+  const bool ok = w < (long long)p.B * p.H * p.S;
+  const int h = (int)(w % p.H); const long long q = w / p.H; const int s = (int)(q % p.S); const int b = (int)(q / p.S);
+  const long long idx = ((long long)b * p.H + h) * p.S + s;
+  float dot = 0.f;
+  if (ok) {
+    auto at = [&](const AttnTensor& x) { return reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(x.ptr) + b * x.sb + s * x.ss + h * x.sh + sub * 8); };
+    const uint4 du = *at(p.dout), ou = *at(p.o), lu = p.o_lo.ptr ? *at(p.o_lo) : make_uint4(0, 0, 0, 0);
+    const float inv = 1.f / p.den[idx];
+    const uint32_t* dw = &du.x; const uint32_t* ow = &ou.x; const uint32_t* lw = &lu.x;
+    uint32_t g[4];
 #pragma unroll
-    for (int i = 0; i < HH; i += 8) {
-      const uint4 du = *reinterpret_cast<const uint4*>(dp + i), ou = *reinterpret_cast<const uint4*>(op + i);
-      const uint4 lu = lp ? *reinterpret_cast<const uint4*>(lp + i) : make_uint4(0, 0, 0, 0);
-      const uint32_t* dw = &du.x; const uint32_t* ow = &ou.x; const uint32_t* lw = &lu.x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 d2 = unpack_bf16x2(dw[j]), o2 = unpack_bf16x2(ow[j]), l2 = unpack_bf16x2(lw[j]);
-        // the SAME rounded G enters G V^T on the tensor core and the dot product here; O carries its remainder
-        const uint32_t gp = pack_bf16x2(d2.x * inv, d2.y * inv);
-        const float2 gr = unpack_bf16x2(gp);
-        g[(i >> 1) + j] = gp;
-        dot = fmaf(gr.x, o2.x + l2.x, dot); dot = fmaf(gr.y, o2.y + l2.y, dot);
-      }
+    for (int j = 0; j < 4; ++j) {
+      const float2 d2 = unpack_bf16x2(dw[j]), o2 = unpack_bf16x2(ow[j]), l2 = unpack_bf16x2(lw[j]);
+      // the SAME rounded G enters G V^T on the tensor core and the dot product here, so that the two halves of
+      // dA = G . (V_s - O_t) see one dO; O carries its remainder
+      g[j] = pack_bf16x2(d2.x * inv, d2.y * inv);
+      const float2 gr = unpack_bf16x2(g[j]);
+      dot = fmaf(gr.x, o2.x + l2.x, dot); dot = fmaf(gr.y, o2.y + l2.y, dot);
     }
-    dden = -dot;
-  } else {
-#pragma unroll
-    for (int i = 0; i < HH / 2; ++i) g[i] = 0u;
+    *at(p.g) = make_uint4(g[0], g[1], g[2], g[3]);
   }
-#pragma unroll
-  for (int gi = 0; gi < HH / 8; ++gi) {
-    const int gc = hf * (HH / 8) + gi;                 // 16-byte chunk of the full row
-    *reinterpret_cast<uint4*>(sG + (gc >> 3) * (LA_C * 128) + sw128_offset(row, gc & 7)) =
-        make_uint4(g[gi * 4], g[gi * 4 + 1], g[gi * 4 + 2], g[gi * 4 + 3]);
-  }
-  return dden;
+  for (int o = lpr >> 1; o; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (ok && sub == 0) p.dden[idx] = -dot;
 }
-// grad[i] <- scale * phi'(scale * x_i) * grad[i] for this thread's HD / 2 columns of a token, stored as bf16
+// scale * phi'(scale * x) * grad for this thread's half of a token, x the raw (bf16) row in the tile `x`, as bf16 into `dst`
 template <int HD>
-__device__ __forceinline__ void la_store_dphi_half(const AttnTensor& x, const AttnTensor& dx, int b, int h, int tok, int hf, const float* grad, float scale, int kind) {
-  constexpr int HH = HD / 2;
-  const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (long long)b * x.sb + (long long)tok * x.ss + (long long)h * x.sh + hf * HH;
-  __nv_bfloat16* gp = reinterpret_cast<__nv_bfloat16*>(dx.ptr) + (long long)b * dx.sb + (long long)tok * dx.ss + (long long)h * dx.sh + hf * HH;
+__device__ __forceinline__ void la_put_dphi_half(uint8_t* x, uint8_t* dst, int row, int hf, const float* grad, float scale, int kind) {
 #pragma unroll
-  for (int i = 0; i < HH; i += 8) {
-    const uint4 xu = *reinterpret_cast<const uint4*>(xp + i);
+  for (int i = 0; i < HD / 16; ++i) {
+    const uint4 xu = *la_half_piece<HD>(x, row, hf, i);
     const uint32_t* xw = &xu.x;
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 x2 = unpack_bf16x2(xw[j]);
       const float a = x2.x * scale, c = x2.y * scale;
-      const float da = kind == 0 ? (a > 0.f ? 1.f : __expf(a)) : (a > 0.f ? 2.f * a : 0.f);
-      const float dc = kind == 0 ? (c > 0.f ? 1.f : __expf(c)) : (c > 0.f ? 2.f * c : 0.f);
-      o[j] = pack_bf16x2(grad[i + 2 * j] * da * scale, grad[i + 2 * j + 1] * dc * scale);
+      const float da = la_dphi(a, kind), dc = la_dphi(c, kind);
+      o[j] = pack_bf16x2(grad[i * 8 + 2 * j] * da * scale, grad[i * 8 + 2 * j + 1] * dc * scale);
     }
-    *reinterpret_cast<uint4*>(gp + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    *la_half_piece<HD>(dst, row, hf, i) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 // partial weighted column sum: sum over rows [r0, r0 + n) of w[r] * tile(r, k)
@@ -622,7 +641,8 @@ __device__ __forceinline__ float la_colsum_w_rows(const uint8_t* tile, int k, co
 // Same 8-warp mapping as the forward: warp w owns rows 32 (w & 3) .. and column half w >> 2.
 template <int HD>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
-linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
+linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                      const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmDQ, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;
@@ -632,15 +652,14 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint8_t* sG = smem;
   uint8_t* sK = sG + L::TILE;                 // 2 stages
   uint8_t* sV = sK + 2 * L::TILE;
-  uint8_t* sShi = sV + L::TILE;
+  uint8_t* sQr = sV + L::TILE;                // raw Q: phi' needs it
+  uint8_t* sShi = sQr + L::TILE;
   uint8_t* sSlo = sShi + L::ST;
   float* sz = reinterpret_cast<float*>(sSlo + L::ST);
-  float* s_part = sz + HD;                    // [2][128]: the halves' shares of dden; later in the chunk: partial column sums
-  float* s_zk = s_part;                       // (two barriers lie between the last read of one use and the first write of the other)
-  float* s_dden = s_part + 2 * LA_C;          // [128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dden + LA_C);
-  uint64_t* k_bar = bars; uint64_t* v_bar = bars + 2; uint64_t* a_bar = bars + 3; uint64_t* b_bar = bars + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  float* s_zk = sz + HD;                      // [256]: partial column sums of K~
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_zk + LA_FWD_THREADS);
+  uint64_t* k_bar = bars; uint64_t* v_bar = bars + 2; uint64_t* a_bar = bars + 3; uint64_t* b_bar = bars + 4; uint64_t* q_bar = bars + 5; uint64_t* g_bar = bars + 6;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
 
   const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int quad = warp & 3, hf = warp >> 2, row = quad * 32 + lane;
@@ -650,7 +669,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const bool rem = p.kind == 0;                // see the forward kernel
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
-    mbar_init(&k_bar[0], 1); mbar_init(&k_bar[1], 1); mbar_init(v_bar, 1); mbar_init(a_bar, 1); mbar_init(b_bar, 1);
+    mbar_init(&k_bar[0], 1); mbar_init(&k_bar[1], 1); mbar_init(v_bar, 1); mbar_init(a_bar, 1); mbar_init(b_bar, 1); mbar_init(q_bar, 1); mbar_init(g_bar, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -691,21 +710,24 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   if (tid == 0) {
     load(sK, &tmK, &k_bar[0], 0);
     load(sV, &tmV, v_bar, 0);
+    load(sQr, &tmQ, q_bar, 0);
+    load(sG, &tmG, g_bar, 0);
     if (n_chunks > 1) load(sK + L::TILE, &tmK, &k_bar[1], 1);
   }
+  const float* ddp = p.dden + ((long long)b * p.H + h) * p.S;
+  float dden_next = c0 * LA_C + row < p.S ? ddp[c0 * LA_C + row] : 0.f;               // a chunk ahead
   bool ok = true;
   const bool have_state0 = p.s_in != nullptr;
   for (int c = 0; c < n_chunks; ++c) {
     const int st = c & 1;
     uint8_t* sKc = sK + st * L::TILE;
     const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
-    const int tok = (c0 + c) * LA_C + row;
-    // this half of G and its share of dden come straight from global memory while the TMA tiles land
-    s_part[hf * LA_C + row] = la_load_g_half<HD>(p, b, h, tok, sG, row, hf);
+    const float dden = dden_next;
+    if (c + 1 < n_chunks) { const int t = (c0 + c + 1) * LA_C + row; dden_next = t < p.S ? ddp[t] : 0.f; }
     if (!mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (ok && !mbar_wait(v_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
+    if (ok && !mbar_wait(g_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
-    const float dden = s_part[row] + s_part[LA_C + row];
     la_phi_half<HD>(sKc, row, hf, valid, p.scale, p.kind);
     fence_proxy_async_smem();
     __syncthreads();
@@ -719,6 +741,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     if (!mbar_wait(a_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
+    if (tid == 0 && c + 1 < n_chunks) load(sG, &tmG, g_bar, c + 1);                   // both readers of G are done
     {
       float a[64];
       la_tmem_row<64>(trow + COL_A + hf * 64, a);
@@ -739,18 +762,15 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     if (!mbar_wait(b_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
-    if (tid == 0) {
-      if (c + 1 < n_chunks) load(sV, &tmV, v_bar, c + 1);
-      if (c + 2 < n_chunks) load(sKc, &tmK, &k_bar[st], c + 2);
-    }
+    if (tid == 0 && c + 2 < n_chunks) load(sKc, &tmK, &k_bar[st], c + 2);
+    if (!mbar_wait(q_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;          // (landed long ago; its time-out ends the loop above)
+    __syncwarp();
     {
       float dq[HH];
       la_tmem_row<HH>(trow + COL_DQ + hf * HH, dq);
-      if (tok < p.S) {
 #pragma unroll
-        for (int i = 0; i < HH; ++i) dq[i] = fmaf(dden, sz[hf * HH + i], dq[i]);      // z of the chunks before this one
-        la_store_dphi_half<HD>(p.q, p.dq, b, h, tok, hf, dq, p.scale, p.kind);
-      }
+      for (int i = 0; i < HH; ++i) dq[i] = fmaf(dden, sz[hf * HH + i], dq[i]);        // z of the chunks before this one
+      la_put_dphi_half<HD>(sQr, sV, row, hf, dq, p.scale, p.kind);                    // V's buffer takes the result
     }
     __syncthreads();                                                                  // every thread has read the old z
     if (tid < HD) {
@@ -763,11 +783,21 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       float srow[HH];
       la_tmem_row<HH>(trow + COL_S + hf * HH, srow);
       if (row < HD) la_write_hilo_half<HD>(sShi, sSlo, HD, row, hf, srow);
-      fence_proxy_async_smem();
     }
+    fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncthreads();
+    if (tid == 0) {
+      la_store_tile<HD>(&tmDQ, sV, h, (c0 + c) * LA_C, b);
+      tma_store_commit();
+      if (c + 1 < n_chunks) {
+        load(sQr, &tmQ, q_bar, c + 1);
+        tma_store_wait_read0();
+        load(sV, &tmV, v_bar, c + 1);
+      }
+    }
   }
+  if (tid == 0) tma_store_wait0();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) { tc_fence_after_sync(); tmem_dealloc(tmem_base, L::TMEM); }
@@ -777,7 +807,8 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 template <int HD>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                       const __grid_constant__ CUtensorMap tmV, const LinAttnArgs p) {
+                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmDK,
+                       const __grid_constant__ CUtensorMap tmDV, const LinAttnArgs p) {
   using L = LaSmem<HD>;
   constexpr int KA = HD / 64;
   constexpr int HH = HD / 2;
@@ -790,13 +821,13 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint8_t* sK = sQ + L::TILE;
   uint8_t* sV = sK + L::TILE;
   uint8_t* sG = sV + L::TILE;
-  uint8_t* sDhi = sG + L::TILE;
+  uint8_t* sKr = sG + L::TILE;                 // raw K: phi' needs it
+  uint8_t* sDhi = sKr + L::TILE;
   uint8_t* sDlo = sDhi + L::ST;
   float* sdz = reinterpret_cast<float*>(sDlo + L::ST);     // [HD]
   float* sdden = sdz + HD;                                  // [128]
-  float* s_part = sdden + LA_C;                             // [2][128] dden shares; later in the chunk: partial column sums
-  float* s_zk = s_part;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_part + 2 * LA_C);
+  float* s_zk = sdden + LA_C;                               // [256]: partial column sums
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_zk + LA_FWD_THREADS);
   uint64_t* ld_bar = bars; uint64_t* t_bar = bars + 1; uint64_t* u_bar = bars + 2; uint64_t* b_bar = bars + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
 
@@ -849,27 +880,38 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after_sync();
 
-  auto load_all = [&](int chunk) {                      // Q, K, V tiles of one chunk on one barrier
-    mbar_expect_tx(ld_bar, 3 * L::TILE);
+  // The tiles of a chunk arrive on one barrier: Q and G as soon as the previous chunk's products are done, K (twice: phi' needs
+  // it raw) and V once the results that leave through their buffers have been read
+  auto load_qg = [&](int chunk) {
+    mbar_expect_tx(ld_bar, (full ? 5 : 2) * L::TILE);
 #pragma unroll
     for (int a = 0; a < KA; ++a) {
       tma_load_4d(sQ + a * (LA_C * 128), &tmQ, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
+      tma_load_4d(sG + a * (LA_C * 128), &tmG, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
+    }
+  };
+  auto load_kv = [&](int chunk) {
+#pragma unroll
+    for (int a = 0; a < KA; ++a) {
       tma_load_4d(sK + a * (LA_C * 128), &tmK, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
+      tma_load_4d(sKr + a * (LA_C * 128), &tmK, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
       tma_load_4d(sV + a * (LA_C * 128), &tmV, ld_bar, a * 64, h, (c0 + chunk) * LA_C, b);
     }
   };
-  if (tid == 0) load_all(n_chunks - 1);
+  if (tid == 0) { load_qg(n_chunks - 1); if (full) load_kv(n_chunks - 1); }
+  const float* ddp = p.dden + ((long long)b * p.H + h) * p.S;
+  auto dden_of = [&](int chunk) { const int t = (c0 + chunk) * LA_C + tid; return tid < LA_C && t < p.S ? ddp[t] : 0.f; };
+  float dden_next = dden_of(n_chunks - 1);                                            // a chunk ahead
   bool ok = true;
   const bool have_state0 = ds_in != nullptr;
   uint32_t t_phase = 0;
   for (int it = 0; it < n_chunks; ++it) {
     const int c = n_chunks - 1 - it;
     const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
-    const int tok = (c0 + c) * LA_C + row;
-    s_part[hf * LA_C + row] = la_load_g_half<HD>(p, b, h, tok, sG, row, hf);
+    if (tid < LA_C) sdden[tid] = dden_next;
+    if (c > 0) dden_next = dden_of(c - 1);
     if (!mbar_wait(ld_bar, it & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
-    if (hf == 0) sdden[row] = s_part[row] + s_part[LA_C + row];
     la_phi_half<HD>(sQ, row, hf, LA_C, p.scale, p.kind);
     if (full) la_phi_half<HD>(sK, row, hf, valid, p.scale, p.kind);
     fence_proxy_async_smem();
@@ -930,23 +972,18 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (!mbar_wait(b_bar, it & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
-    if (tid == 0 && c > 0) load_all(c - 1);
+    if (tid == 0 && c > 0) load_qg(c - 1);
     if (full) {
       float g[HH];
       la_tmem_row<HH>(trow + COL_DV + hf * HH, g);
-      if (tok < p.S) {
-        __nv_bfloat16* vp = reinterpret_cast<__nv_bfloat16*>(p.dv.ptr) + (long long)b * p.dv.sb + (long long)tok * p.dv.ss + (long long)h * p.dv.sh + hf * HH;
 #pragma unroll
-        for (int i = 0; i < HH; i += 8)
-          *reinterpret_cast<uint4*>(vp + i) = make_uint4(pack_bf16x2(g[i], g[i + 1]), pack_bf16x2(g[i + 2], g[i + 3]),
-                                                         pack_bf16x2(g[i + 4], g[i + 5]), pack_bf16x2(g[i + 6], g[i + 7]));
-      }
+      for (int i = 0; i < HH; i += 8)                                                 // dV and dK leave through V's and K~'s buffers
+        *la_half_piece<HD>(sV, row, hf, i / 8) = make_uint4(pack_bf16x2(g[i], g[i + 1]), pack_bf16x2(g[i + 2], g[i + 3]),
+                                                            pack_bf16x2(g[i + 4], g[i + 5]), pack_bf16x2(g[i + 6], g[i + 7]));
       la_tmem_row<HH>(trow + COL_DK + hf * HH, g);
-      if (tok < p.S) {
 #pragma unroll
-        for (int i = 0; i < HH; ++i) g[i] += sdz[hf * HH + i];                         // dz of the chunks after this one
-        la_store_dphi_half<HD>(p.k, p.dk, b, h, tok, hf, g, p.scale, p.kind);
-      }
+      for (int i = 0; i < HH; ++i) g[i] += sdz[hf * HH + i];                           // dz of the chunks after this one
+      la_put_dphi_half<HD>(sKr, sK, row, hf, g, p.scale, p.kind);
     }
     __syncthreads();                                                                  // every thread has read the old dz
     if (tid < HD) {
@@ -963,11 +1000,18 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         for (int i = 0; i < HH; ++i) srow[i] = ds_acc[i] += srow[i];
       }
       if (full && c > 0 && row < HD) la_write_hilo_half<HD>(sDhi, sDlo, HD, row, hf, srow);
-      fence_proxy_async_smem();
     }
+    fence_proxy_async_smem();
     tc_fence_before_sync();
     __syncthreads();
+    if (full && tid == 0) {
+      la_store_tile<HD>(&tmDV, sV, h, (c0 + c) * LA_C, b);
+      la_store_tile<HD>(&tmDK, sK, h, (c0 + c) * LA_C, b);
+      tma_store_commit();
+      if (c > 0) { tma_store_wait_read0(); load_kv(c - 1); }
+    }
   }
+  if (tid == 0) tma_store_wait0();
   float* ds_out = la_publish_begin<HD>(p, bh, sx_epoch, p.ds_out);
   const size_t out_idx = full ? bh : blockIdx.x;
   if (ok && ds_out && (!full || seg == 0)) {
@@ -997,16 +1041,12 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 template <int HD> constexpr int la_fwd_smem() { return 4 * LaSmem<HD>::TILE + 2 * LaSmem<HD>::ST + HD * 4 + 128; }
 // the forward kernel also keeps [2][128] denominator shares and 256 partial column sums
 template <int HD> constexpr int la_fwd8_smem() { return la_fwd_smem<HD>() + 2 * LA_C * 4 + LA_FWD_THREADS * 4; }
-// dQ: [2][128] dden shares (reused for the partial column sums) + [128] dden; dK / dV: the same shares beside its [128] dden
-template <int HD> constexpr int la_dq8_smem() { return la_fwd_smem<HD>() + 3 * LA_C * 4; }
-template <int HD> constexpr int la_dkv_smem() { return 4 * LaSmem<HD>::TILE + 2 * LaSmem<HD>::ST + (HD + LA_C) * 4 + 2 * LA_C * 4 + 128; }
+// dQ, dK / dV: a raw tile and partial column sums; dK / dV: [128] dden
+template <int HD> constexpr int la_dq8_smem() { return la_fwd_smem<HD>() + LaSmem<HD>::TILE + LA_FWD_THREADS * 4; }
+template <int HD> constexpr int la_dkv_smem() { return 5 * LaSmem<HD>::TILE + 2 * LaSmem<HD>::ST + (HD + LA_C) * 4 + LA_FWD_THREADS * 4 + 128; }
 
-static int la_maps(const LinAttnArgs& a, CUtensorMap* tq, CUtensorMap* tk, CUtensorMap* tv) {
-  const auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  if (tq && make_tmap_attn(tq, a.q.ptr, BF, 2, a.hd, a.H, a.S, a.B, a.q.sh, a.q.ss, a.q.sb, 64, LA_C, CU_TENSOR_MAP_SWIZZLE_128B)) return 101;
-  if (make_tmap_attn(tk, a.k.ptr, BF, 2, a.hd, a.H, a.S, a.B, a.k.sh, a.k.ss, a.k.sb, 64, LA_C, CU_TENSOR_MAP_SWIZZLE_128B)) return 102;
-  if (make_tmap_attn(tv, a.v.ptr, BF, 2, a.hd, a.H, a.S, a.B, a.v.sh, a.v.ss, a.v.sb, 64, LA_C, CU_TENSOR_MAP_SWIZZLE_128B)) return 103;
-  return 0;
+static int la_map(CUtensorMap* m, const LinAttnArgs& a, const AttnTensor& t) {
+  return make_tmap_attn(m, t.ptr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.hd, a.H, a.S, a.B, t.sh, t.ss, t.sb, 64, LA_C, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int HD>
@@ -1041,7 +1081,7 @@ __global__ void la_segment_prefix_kernel(float* __restrict__ seg, const float* _
 template <int HD>
 static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
   if (la_set_attrs<HD>()) return 104;
-  if (a.n_seg > 1 && !a.state_only && a.s_in != a.seg && a.ds_in != a.seg) {
+  if (which != 3 && a.n_seg > 1 && !a.state_only && a.s_in != a.seg && a.ds_in != a.seg) {
     // segments: their totals, the prefix over them (the forward's serves the dQ pass too), then the pass itself from there
     LinAttnArgs t = a;
     if (which != 1) {
@@ -1056,25 +1096,42 @@ static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
     if (which == 2) t.ds_in = a.seg; else t.s_in = a.seg;
     return la_launch<HD>(t, which, st);
   }
-  CUtensorMap tq, tk, tv;
-  const bool need_q = which != 1 && !(which == 0 && a.state_only);
-  if (int rc = la_maps(a, need_q ? &tq : nullptr, &tk, &tv)) return rc;
-  if (!need_q) tq = tk;
+  if (which == 3) {
+    const long long n = (long long)a.B * a.H * a.S * (HD / 8);
+    la_g_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 400 + (int)e;
+  }
+  CUtensorMap tq, tk, tv, tg, t0, t1;                   // t0, t1: results
   const unsigned grid = (unsigned)(a.B * a.H * a.n_seg);
-  if (which == 0) linattn_fwd_kernel<HD><<<grid, LA_FWD_THREADS, la_fwd8_smem<HD>(), st>>>(tq, tk, tv, a);
-  else if (which == 1) linattn_bwd_dq_kernel<HD><<<grid, LA_FWD_THREADS, la_dq8_smem<HD>(), st>>>(tk, tv, a);
-  else linattn_bwd_dkv_kernel<HD><<<grid, LA_FWD_THREADS, la_dkv_smem<HD>(), st>>>(tq, tk, tv, a);
+  if (la_map(&tk, a, a.k)) return 102;
+  if (la_map(&tv, a, a.v)) return 103;
+  tq = tg = t0 = t1 = tk;
+  if (which != 0 && la_map(&tg, a, a.g)) return 104;
+  const bool state = a.state_only != 0 && which != 1;
+  if (!(which == 0 && state) && la_map(&tq, a, a.q)) return 101;
+  if (which == 0) {
+    if (!state && la_map(&t0, a, a.o)) return 105;
+    if (!state && a.o_lo.ptr && la_map(&t1, a, a.o_lo)) return 106;
+    linattn_fwd_kernel<HD><<<grid, LA_FWD_THREADS, la_fwd8_smem<HD>(), st>>>(tq, tk, tv, t0, t1, a);
+  } else if (which == 1) {
+    if (la_map(&t0, a, a.dq)) return 105;
+    linattn_bwd_dq_kernel<HD><<<grid, LA_FWD_THREADS, la_dq8_smem<HD>(), st>>>(tq, tk, tv, tg, t0, a);
+  } else {
+    if (!state && (la_map(&t0, a, a.dk) || la_map(&t1, a, a.dv))) return 105;
+    linattn_bwd_dkv_kernel<HD><<<grid, LA_FWD_THREADS, la_dkv_smem<HD>(), st>>>(tq, tk, tv, tg, t0, t1, a);
+  }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
 }
 
 }  // namespace b200
 
-// which: 0 forward (or state-only pass), 1 backward dQ, 2 backward dK / dV. Causal form; hd 64 or 128; bf16.
+// which: 0 forward (or state-only pass), 3 the backward's G pass, then 1 dQ and 2 dK / dV. Causal form; hd 64 or 128; bf16.
 extern "C" int b200_linattn(const b200::LinAttnArgs* a, int which, cudaStream_t st) {
   using namespace b200;
   if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
-  if (which < 0 || which > 2 || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
+  if (which < 0 || which > 3 || (which > 0 && (!a->g.ptr || !a->dden)) || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
   if ((long long)a->n_seg * a->seg_chunks < (a->S + LA_C - 1) / LA_C || (long long)(a->n_seg - 1) * a->seg_chunks >= (a->S + LA_C - 1) / LA_C) return -2;
   if (a->hd == 64) return la_launch<64>(*a, which, st);
   if (a->hd == 128) return la_launch<128>(*a, which, st);

@@ -48,8 +48,8 @@ class LaExchange(C.Structure):
 
 class LinAttnArgs(C.Structure):
     _fields_ = [("q", nv.AttnTensor), ("k", nv.AttnTensor), ("v", nv.AttnTensor), ("o", nv.AttnTensor),
-                ("dout", nv.AttnTensor), ("dq", nv.AttnTensor), ("dk", nv.AttnTensor), ("dv", nv.AttnTensor), ("o_lo", nv.AttnTensor),
-                ("den", C.c_void_p), ("s_in", C.c_void_p), ("s_out", C.c_void_p), ("ds_in", C.c_void_p), ("ds_out", C.c_void_p),
+                ("dout", nv.AttnTensor), ("dq", nv.AttnTensor), ("dk", nv.AttnTensor), ("dv", nv.AttnTensor), ("g", nv.AttnTensor), ("o_lo", nv.AttnTensor),
+                ("den", C.c_void_p), ("dden", C.c_void_p), ("s_in", C.c_void_p), ("s_out", C.c_void_p), ("ds_in", C.c_void_p), ("ds_out", C.c_void_p),
                 ("B", C.c_int), ("H", C.c_int), ("S", C.c_int), ("hd", C.c_int), ("scale", C.c_float), ("eps", C.c_float),
                 ("kind", C.c_int), ("state_only", C.c_int), ("status", C.c_void_p),
                 ("seg", C.c_void_p), ("n_seg", C.c_int), ("seg_chunks", C.c_int), ("sx", LaExchange)]
@@ -75,11 +75,17 @@ def fused_supported(q, causal) -> bool:
 
 @nv.traced("linear_attention")
 def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=None, dk=None, dv=None, s_in=None, s_out=None,
-            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None, seg=None, n_seg=1):
+            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None, seg=None, n_seg=1, g=None):
     """`sx = (SPContext, dir, role)` lets the kernel itself exchange the slice totals with the other ranks (see
-    `LaExchange`); it returns the local buffer the consume pass leaves the summed state in."""
+    `LaExchange`); it returns the local buffer the consume pass leaves the summed state in. `g`: what `_g_pass` returned
+    for this backward (made here when a gradient kernel is launched without it)."""
     B, S, H, d = q.shape
     a = LinAttnArgs()
+    if which in (1, 2):
+        gt, dden = g if g is not None else _g_pass(q, k, v, o, den, dout, o_lo)
+        a.g, a.dden = _attn_t(gt), dden.data_ptr()
+    elif which == 3:
+        a.g, a.dden = _attn_t(g[0]), g[1].data_ptr()
     prefix = None
     if sx is not None:
         prefix = sx[0].fill_exchange(a.sx, B * H, d * d + d, sx[1], sx[2])
@@ -96,6 +102,14 @@ def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=No
     nv.check(nv.cuda().b200_linattn(C.byref(a), which, nv.stream_ptr()), "linattn")
     nv.count_launch(1 if n_seg == 1 or which == 1 else 3)
     return prefix
+
+
+def _g_pass(q, k, v, o, den, dout, o_lo):
+    """(G = dO / D, dden = -(G . O)): what both gradient kernels start from."""
+    B, S, H, d = q.shape
+    g = (torch.empty((B, S, H, d), dtype=torch.bfloat16, device=q.device), torch.empty((B, H, S), dtype=torch.float32, device=q.device))
+    _launch(3, q, k, v, 1.0, 0.0, "elu", o=o, den=den, dout=dout, o_lo=o_lo, g=g)
+    return g
 
 
 def _segments(bh: int, n_chunks: int, hd: int, sms: int) -> int:
@@ -154,18 +168,19 @@ class FusedCausalLinearAttnFn(Function):
         B, S, H, d = q.shape
         dout = dout if (_tma_ok(dout) and dout.dtype == torch.bfloat16) else dout.to(torch.bfloat16).contiguous()
         dq, dk, dv = torch.empty_like(o), torch.empty_like(o), torch.empty_like(o)
-        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, s_in=None if n_seg > 1 else s_in, o_lo=o_lo, seg=s_in if n_seg > 1 else None, n_seg=n_seg)
+        g = _g_pass(q, k, v, o, den, dout, o_lo)
+        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, g=g, s_in=None if n_seg > 1 else s_in, o_lo=o_lo, seg=s_in if n_seg > 1 else None, n_seg=n_seg)
         ds_in = None
         if sp is not None and sp.world > 1 and sp.backend == "fused":
-            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, state_only=True, o_lo=o_lo, sx=(sp, 1, 1))
-            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dk=dk, dv=dv, o_lo=o_lo, sx=(sp, 1, 2))
+            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, state_only=True, o_lo=o_lo, sx=(sp, 1, 1))
+            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, dk=dk, dv=dv, o_lo=o_lo, sx=(sp, 1, 2))
             return dq, dk, dv, None, None, None, None
         if sp is not None and sp.world > 1:
             tot = torch.empty((B * H, d * d + d), dtype=torch.float32, device=q.device)
-            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, ds_out=tot, state_only=True, o_lo=o_lo)
+            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, ds_out=tot, state_only=True, o_lo=o_lo)
             ds_in = sp._exchange(tot, 1)                        # sum of the higher ranks' totals
         seg = torch.empty_like(s_in) if n_seg > 1 else None
-        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
+        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
         return dq, dk, dv, None, None, None, None
 
 
