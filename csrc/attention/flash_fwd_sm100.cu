@@ -6,12 +6,16 @@
 //
 // One CTA = one (batch, head, 128-query block); 128 threads; thread t owns query row t = TMEM lane t.
 //   S  = Q K_j^T     tcgen05.mma, both operands K-major 128B-swizzled tiles written by TMA   -> TMEM
-//   P  = exp2(S*c - m)  read back with tcgen05.ld (one row per thread: no shuffles), written to
-//                        shared memory as a bf16 K-major swizzled A operand
+//   P  = exp2(S*c - m)  read back with tcgen05.ld (one row per thread: no shuffles), written as bf16 to TMEM over the S
+//                        columns it came from: the A operand of P V
 //   O += P V_j       tcgen05.mma accumulating in TMEM, V consumed MN-major straight from its [kv][hd] layout;
 //                    O is rescaled (TMEM load / store) only when the running maximum grows by > 2^8
-// S_{j+1} is issued right behind P V_j, K/V tiles are double-buffered by TMA, and two CTAs share an SM
-// (TMEM 2 x 256 columns) so one CTA's exponentials overlap the other's MMAs. Every wait is bounded.
+// S_{j+1} is issued right behind P V_j (over P_j: products execute in issue order) and two CTAs share an SM (TMEM 2 x 256
+// columns) so one CTA's exponentials overlap the other's MMAs. Without a P tile in shared memory head_dim 128 has room for
+// blocks of 128 keys (one K and one V stage; 64 keys and two stages before), which halves the waits per key; head_dim 64
+// keeps two stages. What bounds it is the chain wait - load - maximum - exponentials - store per block.
+// Measured, causal (B x H x S x hd): 4 x 16 x 4096 x 128 428 -> 288 us (956 TFLOP/s), 64 x 8 x 1024 x 64 196 -> 175 us; not
+// causal, 16 x 8 x 577 x 64 40.5 -> 35.2 us. Every wait is bounded.
 #include "../common/ptx.cuh"
 #include "../common/launch.cuh"
 #include "../common/tensormap.h"
@@ -28,6 +32,10 @@ struct FwdParams {
   int global_order;      // causal: schedule ALL heads' heaviest query blocks first (only while K and V of all heads fit L2-ish)
 };
 
+// K / V stages that let two CTAs share an SM's shared memory
+constexpr int fwd_stages(int hd, int bn) { return hd * bn > 64 * 128 ? 1 : 2; }
+constexpr int fwd_smem(int hd, int bn) { return 128 * hd * 2 + 2 * fwd_stages(hd, bn) * bn * hd * 2 + 128; }
+
 template <int HD, int BN, bool CAUSAL>
 __global__ void __launch_bounds__(128, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -36,16 +44,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   constexpr int KA = HD / 64;                 // 64-element atoms along head_dim
   constexpr int Q_BYTES = BMQ * HD * 2;
   constexpr int KV_BYTES = BN * HD * 2;
-  constexpr int P_BYTES = BMQ * BN * 2;
+  constexpr int ST = fwd_stages(HD, BN);      // K and V stages
   constexpr uint32_t TMEM_COLS = 256;
   constexpr uint32_t PV_COL = 128;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
-  uint8_t* sK = sQ + Q_BYTES;                 // 2 stages
-  uint8_t* sV = sK + 2 * KV_BYTES;            // 2 stages
-  uint8_t* sP = sV + 2 * KV_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + P_BYTES);
+  uint8_t* sK = sQ + Q_BYTES;                 // ST stages
+  uint8_t* sV = sK + ST * KV_BYTES;           // ST stages
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + ST * KV_BYTES);
   uint64_t* q_bar = bars;          // 1
   uint64_t* k_bar = bars + 1;      // 2
   uint64_t* v_bar = bars + 3;      // 2
@@ -94,13 +101,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   constexpr uint32_t idesc_pv = make_idesc(BMQ, HD, CFMT_F32, FMT_BF16, FMT_BF16, 0, 1);
 
   auto load_k = [&](int j) {
-    const int st = j & 1;
+    const int st = j % ST;
     mbar_expect_tx(&k_bar[st], KV_BYTES);
 #pragma unroll
     for (int a = 0; a < KA; ++a) tma_load_4d(sK + st * KV_BYTES + a * (BN * 128), &tmK, &k_bar[st], a * 64, h, j * BN, b);
   };
   auto load_v = [&](int j) {
-    const int st = j & 1;
+    const int st = j % ST;
     mbar_expect_tx(&v_bar[st], KV_BYTES);
 #pragma unroll
     for (int a = 0; a < KA; ++a) tma_load_4d(sV + st * KV_BYTES + a * (BN * 128), &tmV, &v_bar[st], a * 64, h, j * BN, b);
@@ -108,7 +115,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // MMA issue is one thread's serial instruction stream on the critical path: descriptors are a base word plus
   // an immediate, accumulate flags are compile-time.
   auto issue_s = [&](int j) {   // S = Q K_j^T
-    const int st = j & 1;
+    const int st = j % ST;
     const uint32_t lQ = sdesc_lo(smem_u32(sQ), 0), lK = sdesc_lo(smem_u32(sK + st * KV_BYTES), 0);
 #pragma unroll
     for (int k = 0; k < HD / 16; ++k) {
@@ -119,13 +126,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc_commit(s_bar);
   };
   auto issue_pv = [&](int j) {  // O (+)= P V_j
-    const int st = j & 1;
-    const uint32_t lP = sdesc_lo(smem_u32(sP), 0), mV = sdesc_lo(smem_u32(sV + st * KV_BYTES), BN * 128);
+    const int st = j % ST;
+    const uint32_t mV = sdesc_lo(smem_u32(sV + st * KV_BYTES), BN * 128);
 #pragma unroll
     for (int k = 0; k < BN / 16; ++k) {
-      const uint32_t advp = (k >> 2) * (BMQ * 128) + (k & 3) * 32;
-      if (k == 0 && j == 0) umma_f16_c<false>(tmem_base + PV_COL, sdesc_at<1024>(lP, 0), sdesc_at<1024>(mV, 0), idesc_pv);
-      else umma_f16_c<true>(tmem_base + PV_COL, sdesc_at<1024>(lP, advp), sdesc_at<1024>(mV, k * 2048), idesc_pv);
+      if (k == 0 && j == 0) umma_f16_ta<false>(tmem_base + PV_COL, tmem_base, sdesc_at<1024>(mV, 0), idesc_pv);
+      else umma_f16_ta<true>(tmem_base + PV_COL, tmem_base + k * 8, sdesc_at<1024>(mV, k * 2048), idesc_pv);
     }
     tc_commit(pv_bar);
   };
@@ -136,7 +142,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
     for (int a = 0; a < KA; ++a) tma_load_4d(sQ + a * (BMQ * 128), &tmQ, q_bar, a * 64, h, q0, b);
     load_k(0); load_v(0);
-    if (n_blocks > 1) { load_k(1); load_v(1); }
+    if (ST > 1 && n_blocks > 1) { load_k(1); load_v(1); }
     ok = mbar_wait(q_bar, 0, p.status, ST_TIMEOUT_TMA_FULL) && mbar_wait(&k_bar[0], 0, p.status, ST_TIMEOUT_TMA_FULL);
     if (ok) { tc_fence_after_sync(); issue_s(0); }
   }
@@ -150,14 +156,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const float c = p.scale_log2;
 
   for (int j = 0; j < n_blocks; ++j) {
-    const int st = j & 1;
+    const int st = j % ST;
     if (!mbar_wait(s_bar, j & 1, p.status, ST_TIMEOUT_ACC_FULL)) { ok = false; }      // S_j done, and with it P V_{j-1}
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
-    // K_j has been consumed by S_j and V_{j-1} by P V_{j-1}: refill those buffers (K two blocks ahead, V one)
+    // K_j has been consumed by S_j and V_{j-1} by P V_{j-1}: refill those buffers
     if (tid == 0) {
-      if (j + 2 < n_blocks) load_k(j + 2);
-      if (j >= 1 && j + 1 < n_blocks) load_v(j + 1);
+      if (j + ST < n_blocks) load_k(j + ST);
+      if (j >= 1 && j - 1 + ST < n_blocks) load_v(j - 1 + ST);
     }
     const int kv0 = j * BN;
     const bool need_mask = (kv0 + BN > p.Skv) || (CAUSAL && (kv0 + BN - 1 > q0));
@@ -214,24 +220,24 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       add2(rs2, rs3, s[i + 2], s[i + 3]);
     }
     l_run += (rs0 + rs1) + (rs2 + rs3);
-    // bf16 P tile into shared memory (K-major, 128B swizzle)
+    // P as bf16 into TMEM, over the first half of the S columns it came from: the A operand of P V
 #pragma unroll
-    for (int g = 0; g < BN / 8; ++g) {
-      const int atom = g >> 3, chunk = g & 7;
-      uint4 o = make_uint4(pack_bf16x2(s[g * 8 + 0], s[g * 8 + 1]), pack_bf16x2(s[g * 8 + 2], s[g * 8 + 3]),
-                           pack_bf16x2(s[g * 8 + 4], s[g * 8 + 5]), pack_bf16x2(s[g * 8 + 6], s[g * 8 + 7]));
-      *reinterpret_cast<uint4*>(sP + atom * (BMQ * 128) + sw128_offset(tid, chunk)) = o;
+    for (int cc = 0; cc < BN / 64; ++cc) {
+      uint32_t pk[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(s[cc * 64 + 2 * i], s[cc * 64 + 2 * i + 1]);
+      tmem_st_x32(tmem_row + cc * 32, pk);
     }
+    tmem_st_wait();
     tc_fence_before_sync();
-    fence_proxy_async_smem();
     __syncthreads();
     if (warp == 0 && elect_one()) {
-      ok = mbar_wait(&v_bar[st], (j >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL);
+      ok = mbar_wait(&v_bar[st], (j / ST) & 1, p.status, ST_TIMEOUT_TMA_FULL);
       if (ok) {
         tc_fence_after_sync();
         issue_pv(j);                                              // O (+)= P V_j ; commits pv_bar
         if (j + 1 < n_blocks) {
-          ok = mbar_wait(&k_bar[st ^ 1], ((j + 1) >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL);
+          ok = mbar_wait(&k_bar[(j + 1) % ST], ((j + 1) / ST) & 1, p.status, ST_TIMEOUT_TMA_FULL);
           if (ok) issue_s(j + 1);
         }
       }
@@ -275,7 +281,7 @@ template <int HD, int BN, bool CAUSAL>
 static int fwd_set_attr() {
   static bool done = false;
   if (done) return 0;
-  constexpr int SMEM = 128 * HD * 2 + 4 * BN * HD * 2 + 128 * BN * 2 + 128;
+  constexpr int SMEM = fwd_smem(HD, BN);
   (void)cudaGetLastError();
   if (cudaFuncSetAttribute(flash_fwd_kernel<HD, BN, CAUSAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return 1;
   done = true;
@@ -289,7 +295,7 @@ static int launch_fwd(const FlashArgs& a, cudaStream_t st) {
   if (make_tmap_attn(&tmQ, a.q.ptr, BF, 2, a.hd, a.H, a.Sq, a.B, a.q.sh, a.q.ss, a.q.sb, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B)) return 101;
   if (make_tmap_attn(&tmK, a.k.ptr, BF, 2, a.hd, a.H, a.Skv, a.B, a.k.sh, a.k.ss, a.k.sb, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B)) return 102;
   if (make_tmap_attn(&tmV, a.v.ptr, BF, 2, a.hd, a.H, a.Skv, a.B, a.v.sh, a.v.ss, a.v.sb, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B)) return 103;
-  constexpr int SMEM = 128 * HD * 2 + 4 * BN * HD * 2 + 128 * BN * 2 + 128;
+  constexpr int SMEM = fwd_smem(HD, BN);
   auto kfn = flash_fwd_kernel<HD, BN, CAUSAL>;
   if (fwd_set_attr<HD, BN, CAUSAL>()) return 104;
   FwdParams p;
@@ -308,13 +314,13 @@ static int launch_fwd(const FlashArgs& a, cudaStream_t st) {
 
 extern "C" int b200_flash_fwd_init() {
   using namespace b200;
-  return fwd_set_attr<64, 128, true>() | fwd_set_attr<64, 128, false>() | fwd_set_attr<128, 64, true>() | fwd_set_attr<128, 64, false>();
+  return fwd_set_attr<64, 128, true>() | fwd_set_attr<64, 128, false>() | fwd_set_attr<128, 128, true>() | fwd_set_attr<128, 128, false>();
 }
 
 extern "C" int b200_flash_fwd(const b200::FlashArgs* a, cudaStream_t st) {
   using namespace b200;
   if (a->B <= 0 || a->H <= 0 || a->Sq <= 0 || a->Skv <= 0) return 0;
   if (a->hd == 64) return a->causal ? launch_fwd<64, 128, true>(*a, st) : launch_fwd<64, 128, false>(*a, st);
-  if (a->hd == 128) return a->causal ? launch_fwd<128, 64, true>(*a, st) : launch_fwd<128, 64, false>(*a, st);
+  if (a->hd == 128) return a->causal ? launch_fwd<128, 128, true>(*a, st) : launch_fwd<128, 128, false>(*a, st);
   return -3;
 }
