@@ -41,7 +41,8 @@ struct BwdParams {
 };
 
 // delta[b,h,s] = sum_e dO[b,s,h,e] * O[b,s,h,e]; hd/8 lanes per row, one 16-byte load of each operand per lane. The same
-// pass clears the dQ accumulator (`acc4` vectors of four floats).
+// pass clears the dQ accumulator (`acc4` vectors of four floats). The kernels of this file may be resident before their
+// predecessor has finished, so what it wrote is read past L1 (ld.cg), never through the read-only path.
 __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
                                    const __nv_bfloat16* __restrict__ d, long long d_sb, long long d_ss, long long d_sh,
                                    float* __restrict__ delta, float4* __restrict__ acc, long long acc4, int B, int H, int S, int hd) {
@@ -56,8 +57,8 @@ __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, long lon
   // rows are enumerated [b][s][h] so that neighbouring lanes read neighbouring memory
   const int h = (int)(w % H); const long long r = w / H; const int s = (int)(r % S); const int b = (int)(r / S);
   if (w < total) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(o + b * o_sb + s * o_ss + h * o_sh + sub * 8));
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(d + b * d_sb + s * d_ss + h * d_sh + sub * 8));
+    const uint4 a = __ldcg(reinterpret_cast<const uint4*>(o + b * o_sb + s * o_ss + h * o_sh + sub * 8));
+    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(d + b * d_sb + s * d_ss + h * d_sh + sub * 8));
     const float2 a0 = unpack_bf16x2(a.x), a1 = unpack_bf16x2(a.y), a2 = unpack_bf16x2(a.z), a3 = unpack_bf16x2(a.w);
     const float2 c0 = unpack_bf16x2(c.x), c1 = unpack_bf16x2(c.y), c2 = unpack_bf16x2(c.z), c3 = unpack_bf16x2(c.w);
     sum = a0.x * c0.x + a0.y * c0.y + a1.x * c1.x + a1.y * c1.y + a2.x * c2.x + a2.y * c2.y + a3.x * c3.x + a3.y * c3.y;
@@ -87,7 +88,7 @@ __global__ void flash_dq_convert_kernel(const float* __restrict__ acc, __nv_bflo
     uint32_t o[8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 v = src[j * 32];
+      const float4 v = __ldcg(src + j * 32);
       o[2 * j] = pack_bf16x2(v.x * scale, v.y * scale); o[2 * j + 1] = pack_bf16x2(v.z * scale, v.w * scale);
     }
     uint4* dst = reinterpret_cast<uint4*>(dq + (bh / H) * sb + s * ss + (bh % H) * sh + g * 16);
@@ -482,8 +483,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int k = 0; k < 4; ++k) {
         const int q = q0 + k * 32 + lane;
         const long long idx = (long long)bh * p.Sq + q;
-        lv[k] = q < p.Sq ? __ldg(p.lse + idx) * -1.4426950408889634f : -INFINITY;
-        dv[k] = q < p.Sq ? -__ldg(p.delta + idx) : 0.f;
+        lv[k] = q < p.Sq ? __ldcg(p.lse + idx) * -1.4426950408889634f : -INFINITY;
+        dv[k] = q < p.Sq ? -__ldcg(p.delta + idx) : 0.f;
       }
       if (it >= 2 && !mbar_wait(&st_empty[st], ((it >> 1) - 1) & 1, p.status, ST_TIMEOUT_TMA_EMPTY)) break;
 #pragma unroll

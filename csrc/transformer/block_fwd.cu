@@ -29,11 +29,11 @@ struct BlockArgs {
 };
 
 // out[0 .. 3n) = a | b | c
-__global__ void gather3_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c, float* __restrict__ out, int n) {
+__global__ void gather3_kernel(const float* a, const float* b, const float* c, float* out, int n) {
   pdl_trigger();
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 3 * n) out[i] = i < n ? a[i] : i < 2 * n ? b[i - n] : c[i - 2 * n];
+  if (i < 3 * n) out[i] = __ldcg(i < n ? a + i : i < 2 * n ? b + (i - n) : c + (i - 2 * n));
 }
 
 static int block_gemm(const BlockArgs& b, const void* A, int M, int K, const void* W, int N, const float* bias, int act, const void* residual, void* C, cudaStream_t st) {
