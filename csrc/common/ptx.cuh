@@ -134,6 +134,12 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* s
                ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem)), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
 }
+// the same as an element-wise add in L2 (the tensor map's type: fp32)
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const void* smem, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 // global[0 .. bytes) += shared[0 .. bytes) as fp32, added in L2 (untiled: both addresses and the size multiples of 16 bytes)
 __device__ __forceinline__ void bulk_reduce_add_f32(float* dst, const void* smem, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"

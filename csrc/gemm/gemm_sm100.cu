@@ -156,12 +156,14 @@ __device__ __forceinline__ void panel_store(uint8_t* sbuf, int lane, const float
   }
 }
 
-// Tensor maps of the bf16 outputs (C and the optional pre-activation copy), box {64 columns, 32 rows}: with them a warp
-// hands its 32 x 64 panel to the TMA engine as ONE store instead of reading it back from shared memory and issuing
-// 8 predicated 16-byte stores per thread.
+// Tensor maps of the outputs. bf16 (C and the optional pre-activation copy), box {64 columns, 32 rows}: a warp hands its
+// 32 x 64 panel to the TMA engine as ONE store instead of reading it back from shared memory and issuing 8 predicated
+// 16-byte stores per thread. fp32, box {32, 32}: two stores (or adds in L2) per panel where a thread per row wrote 16 bytes
+// to 32 different rows an instruction. (64 weight gradients of 1024 x 512 over ~770 rows:
+// 116 us each with thread stores.)
 struct OutMaps {
   CUtensorMap c, aux;
-  int use;              // 0: plain stores (fp32 / int32 outputs, unaligned C, narrow tiles)
+  int use;              // 0: plain stores (int32 outputs, unaligned C, narrow tiles), 1: bf16, 2: fp32, 3: fp32 added to C
 };
 
 // GEMM -> reduce-scatter: one map per rank over ITS slot buffer [2 * world][rows_per_rank][N] (peer-mapped), so that a
@@ -185,6 +187,21 @@ __device__ __forceinline__ void panel_store_tma(uint8_t* sbuf, int lane, const f
   fence_proxy_async_smem();
   __syncwarp();
   if (lane == 0) { tma_store_3d(tm, sbuf, col0, row0, b); tma_store_commit(); }
+}
+
+// The same for 32 fp32 columns (v) of a panel; `add`: onto C, in L2
+__device__ __forceinline__ void panel_store_tma_f32(uint8_t* sbuf, int lane, const float* v, const CUtensorMap* tm, int col0, int row0, int b, bool add) {
+  if (lane == 0) tma_store_wait_read0();
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4*>(sbuf + sw128_offset(lane, c)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    if (add) tma_reduce_add_3d(tm, sbuf, col0, row0, b); else tma_store_3d(tm, sbuf, col0, row0, b);
+    tma_store_commit();
+  }
 }
 
 // global (bf16, coalesced) -> row-owner registers: out[c] = 8 bf16 of this lane's row, chunk c
@@ -560,7 +577,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     uint8_t* sbuf = epi_smem + ew * EPI_PANEL_BYTES;
     const float alpha = p.alpha_ptr ? p.alpha * __ldg(p.alpha_ptr) : p.alpha;
     const bool staged = (p.out_mode == OUT_BF16) && p.vec_ok;       // coalesced bf16 path
-    const bool tma_out = staged && PW == 64 && TP != TP_GEMM_RS && om != nullptr && om->use;   // ... through the TMA engine
+    const bool tma_out = staged && PW == 64 && TP != TP_GEMM_RS && om != nullptr && om->use == 1;   // ... through the TMA engine
+    const bool tma_f32 = PW == 64 && TP == TP_NONE && om != nullptr && om->use >= 2;           // fp32 result, ditto
     const bool rs_tma = staged && PW == 64 && TP == TP_GEMM_RS && pm != nullptr && pm->use;    // partial tiles to their owners, ditto
     bool ok = true;
     int it = 0;
@@ -733,6 +751,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
 #pragma unroll
             for (int j = 0; j < PW; ++j) if (j < cols_valid) cp[(long long)lane * p.ldc + j] = __float2bfloat16(f[j]);
           }
+        } else if (PW == 64 && tma_f32) {
+#pragma unroll
+          for (int hh = 0; hh < PW / 32; ++hh)
+            if (col0 + hh * 32 < p.N) panel_store_tma_f32(sbuf, lane, f + hh * 32, &om->c, col0 + hh * 32, row0, b, om->use == 3);
         } else if (row_ok) {
           float* cp = reinterpret_cast<float*>(p.C) + cbase + (long long)lane * p.ldc + col0;
           const bool vec = full && p.vec_ok;
@@ -763,7 +785,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       }
       ++it;
     }
-    if ((tma_out || rs_tma) && lane == 0) {               // this warp's last stores have left shared memory and landed
+    if ((tma_out || rs_tma || tma_f32) && lane == 0) {    // this warp's last stores have left shared memory and landed
       tma_store_wait0();
       if (rs_tma) { fence_proxy_async_all(); __threadfence_system(); }
     }
@@ -1006,11 +1028,19 @@ static int gemm_set_attr() {
 }
 
 static int g_tma_store = -1;     // -1: from the environment on first use (B200NN_GEMM_TMA_STORE=0 turns it off)
-// Output maps for the bf16 store path; `use` stays 0 (plain stores) whenever a rule of the copy engine is not met.
+// Output maps for the TMA store paths; `use` stays 0 (plain stores) whenever a rule of the copy engine is not met.
 static void make_out_maps(OutMaps& om, const GemmParams& p, int BN) {
   om.use = 0;
   if (g_tma_store < 0) { const char* e = getenv("B200NN_GEMM_TMA_STORE"); g_tma_store = (e && e[0] == '0') ? 0 : 1; }
-  if (!g_tma_store || p.out_mode != OUT_BF16 || !p.vec_ok || BN < 128) return;
+  if (!g_tma_store || p.out_mode == OUT_I32 || !p.vec_ok || BN < 128) return;
+  if (p.out_mode != OUT_BF16) {
+    const unsigned long long ld = (unsigned long long)p.ldc * 4, st = (unsigned long long)p.strideC * 4;
+    // (the copy engine clips a row's end to 16 bytes: N must be a multiple of 4, or it would write into the gap behind the row)
+    if (p.N % 4 || ld % 16 || (p.batch > 1 && st % 16) || (reinterpret_cast<uintptr_t>(p.C) & 15)) return;
+    if (make_tmap_3d(&om.c, p.C, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.N, p.M, p.batch, ld, st, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return;
+    om.use = p.out_mode == OUT_F32_ATOMIC ? 3 : 2;
+    return;
+  }
   const unsigned long long ldb = (unsigned long long)p.ldc * 2, sb = (unsigned long long)p.strideC * 2;
   if (ldb % 16 || (p.batch > 1 && sb % 16) || (reinterpret_cast<uintptr_t>(p.C) & 15)) return;
   if (make_tmap_3d(&om.c, p.C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, p.N, p.M, p.batch, ldb, sb, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return;
