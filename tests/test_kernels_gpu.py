@@ -93,6 +93,28 @@ def test_gemm_tf32(a_mn, b_mn):
     assert rel_err(out, ref) < 2e-3
 
 
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("M,N,K_", [(1, 1, 1), (16, 16, 64), (17, 15, 65), (32, 10, 784), (3, 257, 63), (200, 33, 129)])
+def test_gemm_small_fp32(M, N, K_, a_mn, b_mn):
+    """Edges of the 16 x 16 tile and the 64- and 128-long chunks, with leading dimensions wider than the rows, against fp64 on
+    operands cut to TF32 (ten mantissa bits, as the tensor cores read them); fp32 sums: K * 2^-24."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K_)
+    mk = lambda r, c: torch.randn(r, c + 3, generator=g, device=DEV)[:, :c]
+    a, b, bias = mk(*((K_, M) if a_mn else (M, K_))), mk(*((K_, N) if b_mn else (N, K_))), torch.randn(N, generator=g, device=DEV)
+    cut = lambda t: (t.contiguous().view(torch.int32) & ~0x1FFF).view(torch.float32).double()
+    ref = (cut(a).t() if a_mn else cut(a)) @ (cut(b) if b_mn else cut(b).t())
+    scale = torch.full((1,), 0.5, device=DEV)
+    out = torch.full((M, N + 2), 7.0, device=DEV)
+    G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, act="relu", alpha=2.0, alpha_t=scale, out_dtype=torch.float32, out=out[:, :N])
+    tol = max(K_, 8) * 2.0 ** -23
+    assert float((out[:, :N].double() - torch.relu(ref + bias.double())).abs().max()) <= tol * (float(ref.abs().max()) + K_ ** 0.5 + 4)
+    assert bool((out[:, N:] == 7.0).all())
+    acc = torch.ones(M, N, device=DEV)
+    G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, accumulate_into=acc)
+    assert float((acc.double() - 1 - ref).abs().max()) <= tol * (float(ref.abs().max()) + K_ ** 0.5 + 4)
+
+
 def test_gemm_k_edge_cases():
     a = lcg_tensor((1, 8), seed=16).to(DEV).bfloat16()
     b = lcg_tensor((1, 8), seed=17).to(DEV).bfloat16()

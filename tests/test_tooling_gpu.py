@@ -26,7 +26,7 @@ def test_gemv_both_orientations(m, n, dtype):
     assert torch.allclose(yt.double(), 2.0 * (a.double().t() @ xt.double()), rtol=1e-4, atol=1e-3 * math.sqrt(m))
 
 
-@pytest.mark.parametrize("m,n,k,ldc", [(1, 1, 1, 1), (130, 257, 65, 257), (128, 128, 1024, 128), (64, 96, 4097, 96), (40, 50, 60, 64), (300, 300, 1500, 301)])
+@pytest.mark.parametrize("m,n,k,ldc", [(1, 1, 1, 1), (130, 257, 65, 257), (128, 128, 1024, 128), (64, 96, 4097, 96), (40, 50, 60, 64), (300, 300, 1500, 301), (520, 301, 300, 304), (520, 300, 300, 304)])
 def test_sgemm_writes_c_in_place(m, n, k, ldc):
     """beta = 0 around the split-K rule, with a leading dimension wider than the row (the gap stays untouched), and with C
     sharing memory with an operand. TF32 drops mantissa bits past the tenth: at most 2^-10 of each factor, 2^-9 of a product."""
