@@ -43,8 +43,8 @@ struct BwdParams {
 // delta[b,h,s] = sum_e dO[b,s,h,e] * O[b,s,h,e]; hd/8 lanes per row, one 16-byte load of each operand per lane. The same
 // pass clears the dQ accumulator (`acc4` vectors of four floats). The kernels of this file may be resident before their
 // predecessor has finished, so what it wrote is read past L1 (ld.cg), never through the read-only path.
-__global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_sb, long long o_ss, long long o_sh,
-                                   const __nv_bfloat16* __restrict__ d, long long d_sb, long long d_ss, long long d_sh,
+__global__ void flash_delta_kernel(const __nv_bfloat16* o, long long o_sb, long long o_ss, long long o_sh,
+                                   const __nv_bfloat16* d, long long d_sb, long long d_ss, long long d_sh,
                                    float* __restrict__ delta, float4* __restrict__ acc, long long acc4, int B, int H, int S, int hd) {
   pdl_trigger();
   pdl_wait();
@@ -71,7 +71,7 @@ __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, long lon
 // dq[b,s,h,:] (bf16, strided) = scale * dq_accum. The accumulator is laid out the way the dQ warps hand it over: per (b, h),
 // block of 128 queries and 32 rows of it, [hd / 4 column groups][32 rows][4] fp32. A thread converts 16 columns of a row:
 // its four reads are 16 bytes beside its neighbours', its write is a whole 32-byte sector.
-__global__ void flash_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long sb,
+__global__ void flash_dq_convert_kernel(const float* acc, __nv_bfloat16* __restrict__ dq, long long sb,
                                         long long ss, long long sh, float scale, int B, int S, int H, int hd) {
   pdl_trigger();
   pdl_wait();

@@ -6,6 +6,10 @@
 // batch is made of. The rules every kernel launched this way follows:
 //   * `pdl_trigger()` first thing, so that the next kernel can be dispatched early;
 //   * `pdl_wait()` before the first access to global memory (read OR write);
+//   * what a predecessor may have written (activations, gradients, statistics, but also biases, weights and scales: an
+//     optimizer or a gather may have run just before) is read by TMA, with `__ldcg` or by an ordinary load, never with
+//     `__ldg` and not through a `const T* __restrict__` parameter: those say that the memory does not change while the kernel
+//     is resident, so such a load may be moved before the wait or served from a read-only line of the time before it;
 // a kernel that is launched WITHOUT the attribute runs both instructions as no-ops, and a kernel without them that
 // follows on the stream is ordered after the full completion of everything before it, as usual. Inside a stream capture
 // the launches become programmatic dependency edges of the CUDA graph. `b200_set_pdl(0)` turns the attribute off.

@@ -111,7 +111,7 @@ __global__ void unary_kernel(const T* __restrict__ x, T* __restrict__ y, long lo
 
 // y = a (op) b with b broadcast along rows when b_period > 0 (b has b_period elements, index = i % b_period)
 template <typename T>
-__global__ void binary_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long n,
+__global__ void binary_kernel(const T* a, const T* b, T* __restrict__ y, long long n,
                               int op, long long b_period) {
   pdl_trigger();
   pdl_wait();
@@ -159,8 +159,8 @@ __device__ __forceinline__ uint4 gate_pack(const float (&f)[8]) {
 }
 template <bool BWD>
 __global__ void __launch_bounds__(256)
-gate_kernel(const __nv_bfloat16* __restrict__ g, long long ld_g, const __nv_bfloat16* __restrict__ y, long long ld_y,
-            const __nv_bfloat16* __restrict__ z, long long ld_z, __nv_bfloat16* __restrict__ o0, long long ld_0,
+gate_kernel(const __nv_bfloat16* g, long long ld_g, const __nv_bfloat16* y, long long ld_y,
+            const __nv_bfloat16* z, long long ld_z, __nv_bfloat16* __restrict__ o0, long long ld_0,
             __nv_bfloat16* __restrict__ o1, long long ld_1, unsigned rows, unsigned ppr) {
   pdl_trigger();
   pdl_wait();
@@ -173,9 +173,9 @@ gate_kernel(const __nv_bfloat16* __restrict__ g, long long ld_g, const __nv_bflo
       const unsigned k = k0 + u * stride;
       r[u] = k / ppr; col[u] = (k - (unsigned)r[u] * ppr) * 8;
       if (k < total) {
-        b[u] = __ldg(reinterpret_cast<const uint4*>(y + r[u] * ld_y + col[u]));
-        c[u] = __ldg(reinterpret_cast<const uint4*>(z + r[u] * ld_z + col[u]));
-        if (BWD) a[u] = __ldg(reinterpret_cast<const uint4*>(g + r[u] * ld_g + col[u]));
+        b[u] = __ldcg(reinterpret_cast<const uint4*>(y + r[u] * ld_y + col[u]));
+        c[u] = __ldcg(reinterpret_cast<const uint4*>(z + r[u] * ld_z + col[u]));
+        if (BWD) a[u] = __ldcg(reinterpret_cast<const uint4*>(g + r[u] * ld_g + col[u]));
       }
     }
 #pragma unroll
@@ -228,7 +228,7 @@ __global__ void colsum_kernel(const T* __restrict__ x, float* __restrict__ out, 
 // take rows w, w + 8, ... of the block's slab (4 rows in flight per lane), then the warps' partial sums meet in
 // shared memory and leave as one atomic per column. Needs cols % 8 == 0, ld % 8 == 0 and a 16-byte aligned base.
 __global__ void __launch_bounds__(256)
-colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, long long rows, int cols, long long ld, int rows_per_block) {
+colsum_vec_kernel(const __nv_bfloat16* x, float* __restrict__ out, long long rows, int cols, long long ld, int rows_per_block) {
   __shared__ float sh[8][256 + 8];
   pdl_trigger();
   pdl_wait();
@@ -245,7 +245,7 @@ colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, 
     for (; r + 24 < r1; r += 32) {
       uint4 v[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const uint4*>(xp + (r + 8 * j) * ld));
+      for (int j = 0; j < 4; ++j) v[j] = __ldcg(reinterpret_cast<const uint4*>(xp + (r + 8 * j) * ld));
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
@@ -254,7 +254,7 @@ colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, 
       }
     }
     for (; r < r1; r += 8) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(xp + r * ld));
+      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(xp + r * ld));
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) { acc[2 * k] += __uint_as_float(w[k] << 16); acc[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u); }
@@ -276,7 +276,8 @@ colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, 
 // sums of the result. A GEMM epilogue that reads `saved` is latency-bound (each epilogue warp has 4 KB outstanding);
 // as a streaming kernel the same work runs at copy bandwidth, and the column sum costs no extra pass.
 // Same thread layout as colsum_vec_kernel. OP is OP_GELU_BWD / OP_SILU_BWD / OP_RELU_BWD; the derivatives use the
-// hardware tanh / exp approximations (relative error ~2^-11, below the bf16 result's own rounding).
+// hardware tanh / exp approximations (relative error ~2^-11, below the bf16 result's own rounding). Four blocks per SM: what
+// bounds it is bytes in flight, and at more than 64 registers it lost a quarter of them (65536 x 2048: 150 against 131 us).
 template <int OP>
 __device__ __forceinline__ float dact_fast(float a, float s) {
   if constexpr (OP == OP_RELU_BWD) return s > 0.f ? a : 0.f;
@@ -291,8 +292,8 @@ __device__ __forceinline__ float dact_fast(float a, float s) {
   }
 }
 template <int OP>
-__global__ void __launch_bounds__(256)
-dact_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ saved, float* __restrict__ dbias, long long rows, int cols,
+__global__ void __launch_bounds__(256, 4)
+dact_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* saved, float* __restrict__ dbias, long long rows, int cols,
                    long long ld_g, long long ld_s, int rows_per_block) {
   __shared__ float sh[8][256 + 8];
   pdl_trigger();
@@ -324,7 +325,7 @@ dact_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restric
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         gv[j] = *reinterpret_cast<const uint4*>(g + (r + 8 * j) * ld_g + c0);
-        sv[j] = __ldg(reinterpret_cast<const uint4*>(saved + (r + 8 * j) * ld_s + c0));
+        sv[j] = *reinterpret_cast<const uint4*>(saved + (r + 8 * j) * ld_s + c0);
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -337,7 +338,7 @@ dact_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restric
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         gv[j] = *reinterpret_cast<const uint4*>(g + (r + 8 * j) * ld_g + c0);
-        sv[j] = __ldg(reinterpret_cast<const uint4*>(saved + (r + 8 * j) * ld_s + c0));
+        sv[j] = *reinterpret_cast<const uint4*>(saved + (r + 8 * j) * ld_s + c0);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -347,7 +348,7 @@ dact_colsum_kernel(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restric
     }
     for (; r < r1; r += 8) {
       uint4 gv = *reinterpret_cast<const uint4*>(g + r * ld_g + c0);
-      const uint4 sv = __ldg(reinterpret_cast<const uint4*>(saved + r * ld_s + c0));
+      const uint4 sv = *reinterpret_cast<const uint4*>(saved + r * ld_s + c0);
       one(gv, sv);
       *reinterpret_cast<uint4*>(g + r * ld_g + c0) = gv;
     }

@@ -575,7 +575,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     constexpr int PW = CPW >= 64 ? 64 : 32;      // panel width
     constexpr int NPANEL = CPW / PW;
     uint8_t* sbuf = epi_smem + ew * EPI_PANEL_BYTES;
-    const float alpha = p.alpha_ptr ? p.alpha * __ldg(p.alpha_ptr) : p.alpha;
+    const float alpha = p.alpha_ptr ? p.alpha * *p.alpha_ptr : p.alpha;
     const bool staged = (p.out_mode == OUT_BF16) && p.vec_ok;       // coalesced bf16 path
     const bool tma_out = staged && PW == 64 && TP != TP_GEMM_RS && om != nullptr && om->use == 1;   // ... through the TMA engine
     const bool tma_f32 = PW == 64 && TP == TP_NONE && om != nullptr && om->use >= 2;           // fp32 result, ditto
@@ -640,11 +640,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         }
         if (p.row_scale || p.col_scale) {
           // dequantise: per-row scale of A (one per thread's row) and per-column scale of B
-          const float rs = (p.row_scale && row_ok) ? __ldg(p.row_scale + (long long)b * p.M + row) : 1.f;
+          const float rs = (p.row_scale && row_ok) ? p.row_scale[(long long)b * p.M + row] : 1.f;
           if (p.col_scale) {
             const float* cs = p.col_scale + col0;
 #pragma unroll
-            for (int j = 0; j < PW; ++j) f[j] *= rs * ((j < cols_valid) ? __ldg(cs + j) : 0.f);
+            for (int j = 0; j < PW; ++j) f[j] *= rs * ((j < cols_valid) ? cs[j] : 0.f);
           } else {
 #pragma unroll
             for (int j = 0; j < PW; ++j) f[j] *= rs;
@@ -655,13 +655,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             const float4* bp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.bias) + b * p.strideBias + col0);
 #pragma unroll
             for (int j = 0; j < PW / 4; ++j) {
-              const float4 bb = __ldg(bp + j);
+              const float4 bb = bp[j];
               f[4 * j] += bb.x; f[4 * j + 1] += bb.y; f[4 * j + 2] += bb.z; f[4 * j + 3] += bb.w;
             }
           } else if (p.bias_f32) {
             const float* bp = reinterpret_cast<const float*>(p.bias) + b * p.strideBias + col0;
 #pragma unroll
-            for (int j = 0; j < PW; ++j) if (j < cols_valid) f[j] += __ldg(bp + j);
+            for (int j = 0; j < PW; ++j) if (j < cols_valid) f[j] += bp[j];
           } else {
             const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + b * p.strideBias + col0;
 #pragma unroll

@@ -76,10 +76,10 @@ __global__ void layernorm_fwd_kernel(const T* __restrict__ x, const float* __res
 // block-wide barriers line up.
 template <int J2, int W>
 __global__ void __launch_bounds__(256)
-layernorm_fwd_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+layernorm_fwd_vec_kernel(const __nv_bfloat16* x, const float* gamma, const float* beta,
                          __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                          long long rows, int d, float eps,
-                         const __nv_bfloat16* __restrict__ res = nullptr, __nv_bfloat16* __restrict__ sum_out = nullptr) {
+                         const __nv_bfloat16* res = nullptr, __nv_bfloat16* __restrict__ sum_out = nullptr) {
   // with `res`: the normalised row is x + res (rounded to bf16 first, so that it equals what `sum_out` stores and what
   // the backward pass will read); `sum_out` receives that sum. This is the residual add of the layer before, moved
   // out of its GEMM epilogue.
@@ -105,9 +105,13 @@ layernorm_fwd_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __res
     const bool valid = row < rows;
     if (W == 1 && !valid) break;
     const __nv_bfloat16* xr = x + row * d;
-    uint4 xu[J2];
+    uint4 xu[J2], ru[J2];                     // all loads of the row before its first store
 #pragma unroll
-    for (int j = 0; j < J2; ++j) xu[j] = valid ? __ldg(reinterpret_cast<const uint4*>(xr + 8 * lane + 256 * (j * W + wi))) : make_uint4(0u, 0u, 0u, 0u);
+    for (int j = 0; j < J2; ++j) {
+      const int c = 8 * lane + 256 * (j * W + wi);
+      xu[j] = valid ? __ldcg(reinterpret_cast<const uint4*>(xr + c)) : make_uint4(0u, 0u, 0u, 0u);
+      if (res != nullptr) ru[j] = valid ? __ldcg(reinterpret_cast<const uint4*>(res + row * d + c)) : make_uint4(0u, 0u, 0u, 0u);
+    }
     float v[J2][8];
     float s = 0.f;
 #pragma unroll
@@ -117,8 +121,7 @@ layernorm_fwd_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __res
       for (int i = 0; i < 4; ++i) { v[j][2 * i] = __uint_as_float(w[i] << 16); v[j][2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
       if (res != nullptr) {
         const int c = 8 * lane + 256 * (j * W + wi);
-        const uint4 ru = valid ? __ldg(reinterpret_cast<const uint4*>(res + row * d + c)) : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t rw[4] = {ru.x, ru.y, ru.z, ru.w};
+        const uint32_t rw[4] = {ru[j].x, ru[j].y, ru[j].z, ru[j].w};
         uint32_t ow[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -290,9 +293,9 @@ layernorm_bwd_reg_kernel(const T* __restrict__ dy, const T* __restrict__ x, cons
 // [rows, d] gradients) disappear.
 template <int J2, int W, bool SUMS = false>
 __global__ void __launch_bounds__(256)
-layernorm_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
-                         const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                         float* __restrict__ dgamma, float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ dres,
+layernorm_bwd_vec_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* gamma,
+                         const float* mean_in, const float* rstd_in, __nv_bfloat16* __restrict__ dx,
+                         float* __restrict__ dgamma, float* __restrict__ dbeta, const __nv_bfloat16* dres,
                          long long rows, int d, float* __restrict__ sum_dres = nullptr, float* __restrict__ sum_dx = nullptr) {
   constexpr int NS = SUMS ? 4 : 2;
   extern __shared__ float sh[];   // [row groups][NS][d]
@@ -330,9 +333,9 @@ layernorm_bwd_vec_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
       const int c = 8 * lane + 256 * (j * W + wi);
       xu[j] = gu[j] = ru[j] = make_uint4(0u, 0u, 0u, 0u);
       if (valid) {
-        xu[j] = __ldg(reinterpret_cast<const uint4*>(xr + c));
-        gu[j] = __ldg(reinterpret_cast<const uint4*>(gr + c));
-        if (dres) ru[j] = __ldg(reinterpret_cast<const uint4*>(dres + row * d + c));
+        xu[j] = __ldcg(reinterpret_cast<const uint4*>(xr + c));
+        gu[j] = __ldcg(reinterpret_cast<const uint4*>(gr + c));
+        if (dres) ru[j] = __ldcg(reinterpret_cast<const uint4*>(dres + row * d + c));
       }
     }
     const float mean = valid ? mean_in[row] : 0.f, rstd = valid ? rstd_in[row] : 0.f;

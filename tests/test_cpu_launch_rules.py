@@ -1,0 +1,46 @@
+"""Rules of programmatic dependent launch (csrc/common/launch.cuh) that can be read off the kernel sources."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "csrc"
+SOURCES = [p for p in sorted(CSRC.rglob("*.cu")) if "launch_pdl" in p.read_text()]
+
+
+def _code(path):
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", path.read_text(), flags=re.S)
+
+
+def _kernels(code):
+    """(name, parameter list, body) of every `__global__` function."""
+    for m in re.finditer(r"__global__[^;{(]*(?:\([^()]*(?:\([^()]*\))?[^()]*\)\s*)??\b(\w+)\s*\(", code):
+        i = m.end()
+        depth = 1
+        while depth:
+            depth += {"(": 1, ")": -1}.get(code[i], 0)
+            i += 1
+        params = code[m.end():i - 1]
+        b = code.index("{", i)
+        j, depth = b + 1, 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[j], 0)
+            j += 1
+        yield m.group(1), params, code[b:j]
+
+
+def test_the_sources_are_found():
+    assert {"norm.cu", "elementwise.cu", "gemm_sm100.cu", "flash_fwd_sm100.cu", "flash_bwd_sm100.cu", "block_fwd.cu"} <= {p.name for p in SOURCES}
+    waiting = {n for p in SOURCES for n, _, body in _kernels(_code(p)) if "pdl_wait()" in body}
+    assert {"layernorm_fwd_vec_kernel", "layernorm_bwd_vec_kernel", "binary_kernel", "gate_kernel", "colsum_vec_kernel", "dact_colsum_kernel"} <= waiting
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_kernels_launched_early_stay_off_the_read_only_path(path):
+    """A kernel that may be resident before its predecessor has finished must not read what that one writes through L1's
+    read-only path: neither explicitly nor by a `const T* __restrict__` parameter, which lets the compiler take it."""
+    code = _code(path)
+    assert "__ldg(" not in code
+    for name, params, body in _kernels(code):
+        if "pdl_wait()" in body:
+            assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), name

@@ -60,6 +60,66 @@ def test_block_without_gradients_equals_the_differentiable_one(B, S, d, heads, f
     assert not torch.equal(before, blk(x))
 
 
+def _without_early_launches(fn):
+    from rust_neural_network_b200 import _native as nv
+    nv.set_pdl(False)
+    try:
+        r = fn()
+        torch.cuda.synchronize()
+        return r
+    finally:
+        nv.set_pdl(True)
+
+
+def test_blocks_read_what_their_predecessors_wrote():
+    """Blocks with biases of their own, back to back on reused workspaces and on alternating inputs, eager and as a graph:
+    bit for bit what the same kernels give when each starts only after its predecessor has ended."""
+    torch.manual_seed(2)
+    blks = [TransformerBlock(512, 8, 1024, causal=True, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16) for _ in range(4)]
+    for b in blks:
+        for lin in (b.attn.q_proj, b.attn.k_proj, b.attn.v_proj, b.attn.out_proj, b.ff1, b.ff2):
+            lin.bias.data.normal_()
+    xs = [torch.randn(2, 200, 512, device="cuda").bfloat16() for _ in range(2)]
+
+    def forward(x):
+        with torch.no_grad():
+            for b in blks:
+                x = b(x)
+        return x
+
+    ref = _without_early_launches(lambda: [forward(x) for x in xs])
+    static = xs[0].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = forward(static)
+    for i in range(50):
+        assert torch.equal(forward(xs[i % 2]), ref[i % 2])
+        static.copy_(xs[i % 2])
+        graph.replay()
+        assert torch.equal(y, ref[i % 2])
+
+
+def test_bias_free_mlp_step_reads_what_its_predecessors_wrote():
+    """A captured fp32 step whose products, activation gradients and optimizer follow each other without a column sum between
+    them: the weights after 100 replays carry the bits they have without early launches (contractions too short to be split)."""
+    def train():
+        torch.manual_seed(3)
+        m = nn.Sequential()
+        for i in range(3):
+            m.add(nn.Linear(128, 128, bias=False))
+            if i < 2:
+                m.add(nn.ReLU())
+        m.to_device(torch.device("cuda"), torch.float32)
+        t = Trainer(m, Adam(m.parameters(), lr=1e-3), MSELoss(), use_cuda_graph=True)
+        g = torch.Generator(device="cuda").manual_seed(4)
+        data = [(torch.randn(32, 128, generator=g, device="cuda"), torch.randn(32, 128, generator=g, device="cuda")) for _ in range(4)]
+        for i in range(100):
+            t.train_step(*data[i % 4])
+        return t.optimizer.flat.master.clone()
+
+    assert torch.equal(train(), _without_early_launches(train))
+
+
 @pytest.mark.parametrize("causal", [False, True])
 def test_fused_block_matches_fp32_reference(causal):
     torch.manual_seed(0)
