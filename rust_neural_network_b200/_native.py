@@ -64,7 +64,6 @@ class FlashArgs(C.Structure):
 _SIGS = {
     # name: argtypes (restype is always int)
     "b200_gemm_launch": [c_void_p, c_int, c_int, c_void_p],
-    "b200_gemm_small": [c_void_p, c_void_p],
     "b200_flash_fwd": [C.POINTER(FlashArgs), c_void_p],
     "b200_flash_bwd": [C.POINTER(FlashArgs), c_void_p],
     "b200_unary": [c_void_p, c_void_p, c_ll, c_int, c_float, c_float, c_int, c_void_p],

@@ -76,7 +76,7 @@ def sgemm(transa: Transpose, transb: Transpose, m: int, n: int, k: int, alpha: f
         # contraction. Device time, product alone / cleared + split: 512x512x512 10.0 / 8.9 us, x768 11.6 / 8.9, x1024 13.2 / 9.0,
         # x2048 19.6 / 9.4; 64x64x4096 29.2 / 7.1. Below 768 the launch costs what the split saves.
         tiles = -(-m // 128) * -(-n // 128)
-        if k >= 768 and (m * n * k > G.SMALL_MACS or k > G.SMALL_K) and cv.is_contiguous() and tiles < G._num_sms(c.device) // 2:
+        if k >= 768 and cv.is_contiguous() and tiles < G._num_sms(c.device) // 2:
             G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, accumulate_into=cv.zero_())
         else:
             G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, out_dtype=torch.float32, out=cv)

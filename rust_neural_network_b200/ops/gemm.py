@@ -138,34 +138,6 @@ _KINDS = {(torch.bfloat16, torch.bfloat16): GEMM_BF16, (torch.float32, torch.flo
           (torch.float8_e4m3fn, torch.float8_e4m3fn): GEMM_E4M3}
 
 
-# Multiply-adds, and contraction length, up to which an fp32 product runs on csrc/gemm/gemm_small.cu (FMA units) instead of the
-# tensor cores. Device time in us, tensor cores / FMA, both operands K-major | both MN-major (where the tensor-core path
-# transposes first): 128x128x128 5.5 / 2.3 | 9.5 / 2.4; 32x256x784 (6.4 M) 7.7 / 7.1 | 11.2 / 8.2; 512x512x64 (16.8 M)
-# 5.5 / 4.6 | 9.4 / 5.1; 256x256x512 (33.6 M) 8.5 / 9.1 | 11.9 / 12.4; 64x64x4096 7.3 / 28.6 | 11.2 / 32.7.
-SMALL_MACS, SMALL_K = 1 << 23, 1024
-
-
-def _gemm_small(lib, a, b, a_mn, b_mn, bias, act, alpha, alpha_t, accumulate_into, out):
-    """One small fp32 product, both operands read in the order they are stored; None where a check of the general path has to
-    speak (shapes that do not fit, an `out` it would refuse)."""
-    M, K = (a.shape[1], a.shape[0]) if a_mn else a.shape
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else b.shape
-    C, mode = (accumulate_into, OUT_F32_ATOMIC) if accumulate_into is not None else (out, OUT_F32)
-    if K != Kb or K == 0 or M == 0 or N == 0 or b.device != a.device or (bias is not None and bias.numel() != N):
-        return None
-    if C is None:
-        C = torch.empty((M, N), dtype=torch.float32, device=a.device)
-    elif tuple(C.shape) != (M, N) or C.dtype != torch.float32 or C.stride(1) != 1 or (accumulate_into is not None and not C.is_contiguous()):
-        return None
-    if alpha_t is not None and alpha_t.dtype != torch.float32:
-        alpha_t = alpha_t.float()
-    rec = nv.GEMM_PACK.pack(M, N, K, 1, 1, C.data_ptr(), C.stride(0), 0, nv.ptr(bias), 1, 0, 0, 0, 0, 0, 0, 0, float(alpha), nv.ptr(alpha_t), ACT[act], 0,
-                            mode, 0, 0, 0, 0, 0, 0, 0, a.data_ptr(), a.stride(0), 0, int(a_mn), b.data_ptr(), b.stride(0), 0, int(b_mn), M, N, K, 1, GEMM_F32)
-    nv.check(lib.b200_gemm_small(rec, nv.stream_ptr()), "b200_gemm_small")
-    nv.count_launch()
-    return C
-
-
 @nv.traced("gemm")
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, dact: str = "none", want_aux: bool = False, alpha: float = 1.0,
@@ -200,13 +172,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     lowp = kind >= GEMM_S8S8
     if lowp and (a_mn or b_mn):
         raise ValueError("8-bit GEMM operands must be K-major")
-    if (is_f32 and a.dim() == 2 and b.dim() == 2 and a.numel() * (b.shape[1] if b_mn else b.shape[0]) <= SMALL_MACS and a.shape[0 if a_mn else 1] <= SMALL_K and residual is None
-            and aux_in is None and not want_aux and splits <= 1 and row_scale is None and col_scale is None and m_valid is None and k_valid is None
-            and not _prepare and bn == 0 and act in ("none", "relu") and (bias is None or (bias.dim() == 1 and bias.dtype == torch.float32 and bias.is_contiguous()))
-            and out_dtype in (None, torch.float32) and a.stride(1) == 1 and b.stride(1) == 1):
-        r = _gemm_small(lib, a, b, a_mn, b_mn, bias, act, alpha, alpha_t, accumulate_into, out)
-        if r is not None:
-            return r
     if is_f32 and (a_mn or b_mn):
         # TF32 tiles are K-major only; 32-bit MN-major operands are transposed by a kernel first
         from .kernels import transpose_last2

@@ -97,8 +97,8 @@ def test_gemm_tf32(a_mn, b_mn):
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("M,N,K_", [(1, 1, 1), (16, 16, 64), (17, 15, 65), (32, 10, 784), (3, 257, 63), (200, 33, 129)])
 def test_gemm_small_fp32(M, N, K_, a_mn, b_mn):
-    """Edges of the 16 x 16 tile and the 64- and 128-long chunks, with leading dimensions wider than the rows, against fp64 on
-    operands cut to TF32 (ten mantissa bits, as the tensor cores read them); fp32 sums: K * 2^-24."""
+    """A few results up to a few tiles, with leading dimensions wider than the rows, against fp64 on operands cut to TF32 (ten
+    mantissa bits, as the tensor cores read them); fp32 sums: K * 2^-24."""
     g = torch.Generator(device=DEV).manual_seed(M + N + K_)
     mk = lambda r, c: torch.randn(r, c + 3, generator=g, device=DEV)[:, :c]
     a, b, bias = mk(*((K_, M) if a_mn else (M, K_))), mk(*((K_, N) if b_mn else (N, K_))), torch.randn(N, generator=g, device=DEV)
@@ -113,6 +113,19 @@ def test_gemm_small_fp32(M, N, K_, a_mn, b_mn):
     acc = torch.ones(M, N, device=DEV)
     G.gemm(a, b, a_mn=a_mn, b_mn=b_mn, accumulate_into=acc)
     assert float((acc.double() - 1 - ref).abs().max()) <= tol * (float(ref.abs().max()) + K_ ** 0.5 + 4)
+
+
+@pytest.mark.parametrize("N,K_", [(128, 256), (10, 128), (256, 100)])
+def test_gemm_fp32_rows_do_not_depend_on_how_many_there_are(N, K_):
+    """The rows of a small fp32 product carry the bits they have inside a large one: a training step whose ReLUs sit at zero
+    and whose optimizer divides by the gradient's size turns another order of summation into a visible difference."""
+    g = torch.Generator(device=DEV).manual_seed(N + K_)
+    a, b = torch.randn(40000, K_, generator=g, device=DEV), torch.randn(N, K_, generator=g, device=DEV)
+    whole = G.gemm(a, b, out_dtype=torch.float32)
+    for rows in (32, 200):
+        assert torch.equal(G.gemm(a[:rows], b, out_dtype=torch.float32), whole[:rows])
+    at, bt = a[:256].t().contiguous(), b.t().contiguous()
+    assert torch.equal(G.gemm(at, bt, a_mn=True, b_mn=True, out_dtype=torch.float32), whole[:256])
 
 
 def test_gemm_k_edge_cases():
