@@ -44,6 +44,23 @@ def _fused_qkv(wq, wk, wv, getter):
     return torch.cat([a, b, c], 0)
 
 
+def _shadow_qkv(wq, wk, wv):
+    """bf16 [3d, d] of the three projections (`functional.lp`). Weights that have no shadow yet, those no optimizer has laid
+    out, get theirs as neighbours in one buffer, so that no call has to copy them together. A shadow that exists is never
+    moved: a captured graph or another stream may read it, and its memory would be given away under them. (Nor is a buffer
+    made while a graph is being captured, which would own it.)"""
+    ws = (wq, wk, wv)
+    if (all(getattr(w, "_lp", None) is None for w in ws) and len({id(w) for w in ws}) == 3 and len({(w.shape, w.device) for w in ws}) == 1
+            and not (wq.is_cuda and torch.cuda.is_current_stream_capturing())):
+        versions = [w._version for w in ws]
+        with torch.inference_mode(False), torch.no_grad():             # (an inference tensor could not be refreshed outside that mode)
+            buf = torch.cat([w.detach().to(torch.bfloat16) for w in ws], 0)
+            parts = buf.split(wq.shape[0], 0)
+        for w, part, version in zip(ws, parts, versions):
+            w._lp, w._lp_version = part, version
+    return _fused_qkv(wq, wk, wv, lp)
+
+
 def _fused_vec(bq, bk, bv, getter):
     a, b, c = getter(bq), getter(bk), getter(bv)
     if _adjacent(a, b, c):
@@ -63,7 +80,7 @@ class TransformerBlockFn(Function):
         if not x2.is_contiguous():
             x2 = x2.contiguous()
         h1, mean1, rstd1 = K.layernorm_fwd(x2, g1.detach(), be1.detach(), eps)
-        wqkv = _fused_qkv(wq, wk, wv, lp)
+        wqkv = _shadow_qkv(wq, wk, wv)
         bqkv = _fused_vec(bq, bk, bv, lambda t: t.detach())
         qkv = gemm(h1, wqkv, bias=bqkv)                                   # [T, 3d]
         qkv5 = qkv.view(B, S, 3, heads, hd)
@@ -147,22 +164,6 @@ class TransformerBlockFn(Function):
 
 nv.register_sigs({"b200_block_fwd": [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]})
 _BLOCK_PACK = struct.Struct("@25P9ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
-
-
-def _shadow_qkv(wq, wk, wv):
-    """bf16 [3d, d] of the three projections. Weights no optimizer has laid out have a shadow each (`functional.lp`): these
-    are moved into one buffer the first time, so that later calls find them adjacent instead of copying them together. Each
-    stays its parameter's own shadow, refreshed when that parameter changes. (Not while a graph is being captured: the
-    buffer would belong to the graph.)"""
-    a, b, c = lp(wq), lp(wk), lp(wv)
-    if _adjacent(a, b, c):
-        return a
-    buf = torch.cat([a, b, c], 0)
-    if not torch.cuda.is_current_stream_capturing() and not any(getattr(w, "_fused_grad", False) for w in (wq, wk, wv)):
-        d = a.shape[0]
-        for i, w in enumerate((wq, wk, wv)):
-            w._lp = buf[i * d:(i + 1) * d]
-    return buf
 
 
 def _plain(*ts) -> bool:

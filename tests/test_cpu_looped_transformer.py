@@ -149,3 +149,54 @@ def test_more_loops_keep_shape_and_stay_finite():
     for loops in (4, 8):
         y = _raw(LoopedTransformer(4, 8, 2, 16, 4, loops)(x)).detach()
         assert list(y.shape) == [1, 3, 4] and bool(torch.isfinite(y).all())
+
+
+# ----------------------------------------------------------------------------- bf16 shadows of the projections
+def _three(d=16):
+    return [torch.nn.Parameter(torch.randn(d, d, generator=torch.Generator().manual_seed(i))) for i in range(3)]
+
+
+def test_projection_shadows_that_exist_are_never_moved():
+    """A captured graph or another stream may be reading them: a later forward copies them together and leaves them where
+    they are."""
+    from rust_neural_network_b200.ops.functional import lp
+    from rust_neural_network_b200.ops.transformer import _shadow_qkv
+    ws = _three()
+    shadows = [lp(w) for w in ws]
+    where = [s.data_ptr() for s in shadows]
+    with torch.no_grad():
+        packed = _shadow_qkv(*ws)
+    assert torch.equal(packed, torch.cat([w.detach().bfloat16() for w in ws]))
+    assert all(w._lp is s for w, s in zip(ws, shadows)) and [lp(w).data_ptr() for w in ws] == where
+
+
+def test_projection_shadows_are_laid_out_as_neighbours_and_follow_their_weights():
+    from rust_neural_network_b200.ops.transformer import _shadow_qkv
+    ws = _three()
+    first = _shadow_qkv(*ws)
+    again = _shadow_qkv(*ws)
+    assert first.shape == (48, 16) and again.data_ptr() == first.data_ptr() == ws[0]._lp.data_ptr()
+    with torch.no_grad():
+        ws[1].mul_(3.0)
+    assert torch.equal(_shadow_qkv(*ws), torch.cat([w.detach().bfloat16() for w in ws])) and ws[1]._lp.data_ptr() == first[16:].data_ptr()
+    shared = _three(8)
+    assert torch.equal(_shadow_qkv(shared[0], shared[0], shared[1]), torch.cat([shared[i].detach().bfloat16() for i in (0, 0, 1)]))
+
+
+def test_projection_shadows_made_in_inference_mode_can_be_refreshed_outside_it():
+    from rust_neural_network_b200.ops.functional import lp
+    from rust_neural_network_b200.ops.transformer import _shadow_qkv
+    ws = _three()
+    with torch.inference_mode():
+        _shadow_qkv(*ws)
+    with torch.no_grad():
+        ws[2].add_(1.0)
+    assert torch.equal(lp(ws[2]), ws[2].detach().bfloat16())
+    ws = _three()
+    for w in ws:
+        lp(w)
+    with torch.inference_mode():
+        _shadow_qkv(*ws)
+    with torch.no_grad():
+        ws[0].add_(1.0)
+    assert torch.equal(_shadow_qkv(*ws)[:16], ws[0].detach().bfloat16())

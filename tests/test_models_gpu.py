@@ -99,6 +99,26 @@ def test_blocks_read_what_their_predecessors_wrote():
         assert torch.equal(y, ref[i % 2])
 
 
+def test_graph_keeps_its_weights_over_an_eager_forward():
+    """A graph captured on shadows of the projections that are not neighbours replays the same result after a forward without
+    gradients has run outside it and freed memory has been written over."""
+    from rust_neural_network_b200.ops.functional import lp
+    torch.manual_seed(5)
+    blk = TransformerBlock(256, 4, 512, causal=True, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16)
+    for lin in (blk.attn.v_proj, blk.attn.q_proj, blk.attn.k_proj):
+        lp(lin.weight)
+    x = torch.randn(2, 64, 256, device="cuda").bfloat16()
+    ref = blk(x).detach().clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = blk(x)
+    with torch.no_grad():
+        assert torch.equal(blk(x), ref)
+    junk = [torch.full((256, 256), 9.0, device="cuda").bfloat16() for _ in range(16)]
+    graph.replay()
+    assert torch.equal(y, ref) and len(junk) == 16
+
+
 def test_bias_free_mlp_step_reads_what_its_predecessors_wrote():
     """A captured fp32 step whose products, activation gradients and optimizer follow each other without a column sum between
     them: the weights after 100 replays carry the bits they have without early launches (contractions too short to be split)."""
