@@ -71,17 +71,18 @@ def sgemm(transa: Transpose, transb: Transpose, m: int, n: int, k: int, alpha: f
     A = _view2d(a, k, m, lda) if transa.is_trans() else _view2d(a, m, k, lda)          # stored [k, m] -> MN-major
     B = _view2d(b, n, k, ldb) if transb.is_trans() else _view2d(b, k, n, ldb)          # stored [k, n] -> MN-major
     a_mn, b_mn = transa.is_trans(), not transb.is_trans()
-    if beta == 0.0 and _direct(c, cv, a, b):
-        # Straight into C. Split-K adds into a cleared result, one launch more; it pays where a few tiles have a long
-        # contraction. Device time, product alone / cleared + split: 512x512x512 10.0 / 8.9 us, x768 11.6 / 8.9, x1024 13.2 / 9.0,
-        # x2048 19.6 / 9.4; 64x64x4096 29.2 / 7.1. Below 768 the launch costs what the split saves.
-        tiles = -(-m // 128) * -(-n // 128)
-        if k >= 768 and cv.is_contiguous() and tiles < G._num_sms(c.device) // 2:
-            G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, accumulate_into=cv.zero_())
-        else:
-            G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, out_dtype=torch.float32, out=cv)
-            if not c.is_inference():
-                torch.autograd.graph.increment_version(c)       # the kernel's write is an in-place write like any other
+    direct = beta == 0.0 and _direct(c, cv, a, b)
+    # Straight into C. Split-K adds into a cleared result, one launch more; it pays where a few tiles have a long
+    # contraction. Device time, product alone / cleared + split: 512x512x512 10.0 / 8.9 us, x768 11.6 / 8.9, x1024 13.2 / 9.0,
+    # x2048 19.6 / 9.4; 64x64x4096 29.2 / 7.1. Below 768 the launch costs what the split saves. A C with gaps between its rows
+    # cannot be added into: there the split product is copied.
+    split = direct and k >= 768 and -(-m // 128) * -(-n // 128) < G._num_sms(c.device) // 2
+    if split and cv.is_contiguous():
+        G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, accumulate_into=cv.zero_())
+    elif direct and not split:
+        G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, out_dtype=torch.float32, out=cv)
+        if not c.is_inference():
+            torch.autograd.graph.increment_version(c)           # the kernel's write is an in-place write like any other
     elif beta == 0.0:
         out = G.gemm(A, B, a_mn=a_mn, b_mn=b_mn, alpha=alpha, out_dtype=torch.float32)
         cv.copy_(out)

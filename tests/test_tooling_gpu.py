@@ -48,6 +48,21 @@ def test_sgemm_writes_c_in_place(m, n, k, ldc):
     assert float((buf[:m * n].view(m, n).double() - ref).norm() / ref.norm()) < 2 ** -9
 
 
+@pytest.mark.parametrize("k,ldc,straight", [(4096, 80, False), (4096, 64, False), (600, 80, True), (600, 64, True)])
+def test_sgemm_splits_a_long_contraction_whatever_the_rows_of_c_are_apart(monkeypatch, k, ldc, straight):
+    """A product of a few tiles over a long contraction is split over the SMs (64 x 64 x 4096: 29 us in one piece, 7 us split);
+    handed over as `out` it could not be."""
+    from rust_neural_network_b200 import blas
+    N, calls, gemm = blas.Transpose.NoTrans, [], blas.G.gemm
+    monkeypatch.setattr(blas.G, "gemm", lambda *a, **kw: calls.append(kw) or gemm(*a, **kw))
+    a, b, c = (torch.randn(r, device="cuda") for r in (64 * k, k * 64, 64 * ldc))
+    gap = c.view(64, ldc)[:, 64:].clone()
+    blas.sgemm(N, N, 64, 64, k, 1.0, a, k, b, 64, 0.0, c, ldc)
+    assert len(calls) == 1 and ("out" in calls[0]) == straight
+    ref = a.view(64, k).double() @ b.view(k, 64).double()
+    assert float((c.view(64, ldc)[:, :64].double() - ref).norm() / ref.norm()) < 2 ** -9 and torch.equal(c.view(64, ldc)[:, 64:], gap)
+
+
 def test_blas_level1_and_sgemm_gpu():
     torch.manual_seed(0)
     x, y = torch.randn(100003, device=DEV), torch.randn(100003, device=DEV)
