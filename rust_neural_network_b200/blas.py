@@ -49,10 +49,18 @@ def _view2d(t: torch.Tensor, rows: int, cols: int, ld: int) -> torch.Tensor:
     return torch.as_strided(flat, (rows, cols), (ld, 1))
 
 
+_DIRECT_TYPES = {(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)}
+
+
 def _direct(c, cv, a, b) -> bool:
-    """May the product be written into C without a copy: an fp32 GPU tensor outside autograd that does not share its memory
-    with an operand."""
-    if not (c.is_cuda and c.dtype == torch.float32) or c.requires_grad or cv.data_ptr() != c.data_ptr() or a.device != c.device:
+    """May the product be written into C without a copy: an fp32 GPU tensor outside autograd (also outside torch.func transforms
+    and forward-mode AD, which follow a copy but not a kernel's write) that does not share its memory with an operand, and
+    operands whose types the product takes, so that C is not cleared for a call that is then refused."""
+    if not (c.is_cuda and c.dtype == torch.float32) or c.requires_grad or (a.dtype, b.dtype) not in _DIRECT_TYPES:
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    if cv.data_ptr() != c.data_ptr() or a.device != c.device:
         return False
     sc = c.untyped_storage().data_ptr()
     return sc != a.untyped_storage().data_ptr() and sc != b.untyped_storage().data_ptr()

@@ -63,6 +63,25 @@ def test_sgemm_splits_a_long_contraction_whatever_the_rows_of_c_are_apart(monkey
     assert float((c.view(64, ldc)[:, :64].double() - ref).norm() / ref.norm()) < 2 ** -9 and torch.equal(c.view(64, ldc)[:, 64:], gap)
 
 
+def test_sgemm_refused_leaves_c_alone_and_transforms_see_the_write():
+    from rust_neural_network_b200 import blas
+    import torch.autograd.forward_ad as fwad
+    N = blas.Transpose.NoTrans
+    a, b, c = torch.randn(64 * 1024, device="cuda"), torch.randn(1024 * 64, device="cuda"), torch.full((64 * 64,), 7.0, device="cuda")
+    with pytest.raises(TypeError):
+        blas.sgemm(N, N, 64, 64, 1024, 1.0, a, 1024, b.bfloat16(), 64, 0.0, c, 64)
+    assert bool((c == 7.0).all())
+    ref = a.view(64, 1024).double() @ b.view(1024, 64).double()
+    for k in (1024, 512):
+        with fwad.dual_level():
+            dual = fwad.make_dual(c.clone(), torch.ones_like(c))
+            blas.sgemm(N, N, 64, 64, k, 1.0, a, 1024, b, 64, 0.0, dual, 64)
+            value, tangent = fwad.unpack_dual(dual)
+            assert tangent is None or not bool(tangent.any())              # C no longer depends on what it held
+    out = torch.vmap(lambda x: blas.sgemm(N, N, 64, 64, 1024, 1.0, a, 1024, b, 64, 0.0, x, 64))(torch.zeros(2, 64 * 64, device="cuda"))
+    assert float((out[1].view(64, 64).double() - ref).norm() / ref.norm()) < 2 ** -9
+
+
 def test_blas_level1_and_sgemm_gpu():
     torch.manual_seed(0)
     x, y = torch.randn(100003, device=DEV), torch.randn(100003, device=DEV)
