@@ -47,6 +47,11 @@ GEMM_PACK = struct.Struct("@5iPqqPiiqPqqPPfPiiiiiPPPPP" "PqqiPqqi5i0P")
 assert GEMM_PACK.size == C.sizeof(GemmArgs)
 
 
+def f32(v) -> float:
+    """`v` rounded to fp32, infinite past its range: `struct` refuses to round to infinity, a C call does not."""
+    return c_float(float(v)).value
+
+
 class AttnTensor(C.Structure):
     _fields_ = [("ptr", c_void_p), ("sb", c_ll), ("ss", c_ll), ("sh", c_ll)]
 

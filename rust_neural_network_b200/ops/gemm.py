@@ -295,7 +295,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                  and ((aux is None and aux_in is None) or N % 8 == 0))
     rec = nv.GEMM_PACK.pack(
         M, N, K, batch, splits, out_ptr, ldc, stride_c, bias_ptr, bias_f32, bias_vec_ok, bias_stride, res_ptr, ldr, stride_r,
-        nv.ptr(aux), nv.ptr(aux_in), float(alpha), nv.ptr(alpha_t), ACT[act], ACT[dact], out_mode, vec_ok, res_vec_ok,
+        nv.ptr(aux), nv.ptr(aux_in), nv.f32(alpha), nv.ptr(alpha_t), ACT[act], ACT[dact], out_mode, vec_ok, res_vec_ok,
         nv.ptr(row_scale), nv.ptr(col_scale), nv.status_ptr(dev), nv.ptr(m_valid), nv.ptr(k_valid),
         a3.data_ptr(), lda, stride_a, int(a_mn), b3.data_ptr(), ldb, stride_b, int(b_mn), M, N, K, batch, kind)
     res = out3[0] if (squeeze and out.dim() == 3) else out

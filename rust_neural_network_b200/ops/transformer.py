@@ -198,7 +198,7 @@ def _block_forward(x, blk, causal):
     g1, be1, g2, be2, bq, bk, bv, bo, b1, b2 = (t.data_ptr() for t in vecs)
     rec = _BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *(w0 + p for p in offs), *(w.data_ptr() for w in ws),
                            g1, be1, g2, be2, bq, bk, bv, bo, b1, b2, B, S, d, ff, H, int(causal), int(not adjacent), K.OPS["add"], _num_sms(dev),
-                           float(n1.eps), nv.status_ptr(dev))
+                           nv.f32(n1.eps), nv.status_ptr(dev))
     launches = C.c_int(0)
     nv.check(nv.cuda().b200_block_fwd(rec, C.byref(launches), nv.stream_ptr()), "block_fwd")
     nv.count_launch(launches.value)

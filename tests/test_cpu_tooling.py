@@ -381,3 +381,16 @@ def test_examples_run_on_cpu(script, args):
                        cwd=os.path.join(root, "examples"), env=env)
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.strip()
+
+
+def test_launch_record_takes_every_alpha():
+    """A factor past fp32's range is infinite on the device; packing the launch record does not refuse it."""
+    import math
+    from rust_neural_network_b200 import _native as nv
+    fields = list(nv.GemmArgs.from_buffer_copy(bytes(nv.GEMM_PACK.size)).p._fields_)
+    assert ("alpha", nv.c_float) in fields
+    for a in (1e39, -1e39, math.inf, 3.4028235e38, 1e-50, 0, True):
+        r = nv.f32(a)
+        nv.struct.pack("f", r)
+        assert r == torch.tensor(float(a), dtype=torch.float64).float().item()
+    assert math.isnan(nv.f32(math.nan))
