@@ -117,6 +117,8 @@ def _segments(bh: int, n_chunks: int, hd: int, sms: int) -> int:
     head size 64, one at 128). A segment costs a pass over its K and V (Q, dO, O in the backward) for its total, so segments
     that would queue lose: 8 x 16 heads, 4096 tokens, head size 128, forward + backward 1.70 ms whole, 2.11 ms in two; while
     1 x 8 heads x 16384 x 128 takes 6.32 ms whole and 0.69 ms in 16, 1 x 16 x 1000 x 128 0.34 and 0.17 ms in 8."""
+    if n_chunks == 0:
+        return 1
     n = max(1, min((2 if hd == 64 else 1) * sms // max(bh, 1), n_chunks, 64))
     return -(-n_chunks // -(-n_chunks // n))                     # no empty last segment
 

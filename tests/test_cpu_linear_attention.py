@@ -95,3 +95,15 @@ def test_tensor_api_end_to_end_backward():
     q2, k2, v2 = (Tensor.randn([1, 12, 6]).set_requires_grad(True) for _ in range(3))      # the causal ReLU^2 path
     Tensor.linear_attention(q2, k2, v2, 0.5, 1e-6, True, KernelKind.Relu2).sum().backward()
     assert all(t.grad() is not None for t in (q2, k2, v2))
+
+
+def test_segments_cover_every_chunk():
+    """Every chunk lies in one segment and none of them is empty; no tokens are one (empty) segment."""
+    from rust_neural_network_b200.ops.linear_attention import _segments
+    for bh in (0, 1, 7, 16, 148, 296, 4096):
+        for hd in (64, 128):
+            assert _segments(bh, 0, hd, 148) == 1
+            for chunks in (1, 2, 3, 8, 9, 63, 64, 65, 512, 1000):
+                n = _segments(bh, chunks, hd, 148)
+                per = -(-chunks // n)
+                assert 1 <= n <= 64 and (n - 1) * per < chunks <= n * per

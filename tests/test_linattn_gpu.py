@@ -144,3 +144,9 @@ def test_segment_rule_leaves_no_empty_segment():
                 n = _segments(bh, n_chunks, hd, 148)
                 per = -(-n_chunks // n)
                 assert 1 <= n <= 64 and n * per >= n_chunks > (n - 1) * per
+
+
+def test_no_tokens():
+    q, k, v = (torch.zeros(2, 0, 4, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+    o = linear_attention(q, k, v, causal=True, kind="elu")
+    assert o.shape == (2, 0, 4, 64) and all(g.shape == q.shape for g in torch.autograd.grad(o, (q, k, v), torch.zeros_like(o)))
