@@ -431,7 +431,7 @@ scan_bwd_lanes_kernel(ScanArgs a) {
   static_assert(256 / DB == CK, "one (row, channel) of an interval per loader thread");
   __shared__ float4 s_in[CK][DB];                    // (delta, delta * u, u, dy) per (t, channel)
   __shared__ float s_draw[CK][DB];                   // delta before softplus
-  __shared__ float s_BC[CK][SCAN_N / 2][4];          // (B of the two states, C of the two states)
+  __shared__ __align__(16) float s_BC[CK][SCAN_N / 2][4];     // (B of the two states, C of the two states), read as float4
   __shared__ float2 s_out[CK][DB];                   // (d delta_raw, d u without the skip term)
   __shared__ float s_dBC[WARPS][32][9];              // per warp: lane l holds 8 of the 32 x 8 (t, n) sums
   const int b = blockIdx.y, d0 = blockIdx.x * DB;

@@ -44,3 +44,16 @@ def test_kernels_launched_early_stay_off_the_read_only_path(path):
     for name, params, body in _kernels(code):
         if "pdl_wait()" in body:
             assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params), name
+
+
+@pytest.mark.parametrize("path", sorted(CSRC.rglob("*.cu")), ids=lambda p: p.name)
+def test_shared_arrays_read_as_vectors_are_declared_aligned(path):
+    """A `__shared__ float` array is aligned to 4 bytes; reading it as float4 needs the declaration to say 16."""
+    code = _code(path)
+    scalars = {"float", "int", "uint32_t", "unsigned", "__nv_bfloat16", "uint8_t", "char", "half"}
+    for m in re.finditer(r"__shared__\s+((?:__align__\(\d+\)\s*)?)(\w+)\s+([^;]*);", code):
+        align, typ, names = m.groups()
+        if typ not in scalars or align:
+            continue
+        for name in re.findall(r"(\w+)\s*\[", names):
+            assert not re.search(r"reinterpret_cast<(?:const )?(?:float|uint|int)[24]\s*\*>\(\s*&?\s*%s\b" % name, code), (path.name, name)
