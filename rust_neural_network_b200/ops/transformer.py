@@ -177,7 +177,7 @@ def _block_forward(x, blk, causal):
     B, S, d = x.shape
     ff = f1.weight.shape[0]
     vecs = (n1.gamma, n1.beta, n2.gamma, n2.beta, q.bias, k.bias, v.bias, o.bias, f1.bias, f2.bias)
-    if (any(t is None for t in vecs) or not _plain(*vecs) or d % 8 or ff % 8 or B * S == 0 or B * S * max(3 * d, ff) >= 2 ** 31
+    if (any(t is None for t in vecs) or not _plain(*vecs) or d % at.heads or d % 8 or ff % 8 or B * S == 0 or B * S * max(3 * d, ff) >= 2 ** 31
             or tuple(q.weight.shape) != (d, d) or tuple(k.weight.shape) != (d, d) or tuple(v.weight.shape) != (d, d)
             or tuple(o.weight.shape) != (d, d) or tuple(f1.weight.shape) != (ff, d) or tuple(f2.weight.shape) != (d, ff)):
         return None

@@ -99,6 +99,15 @@ def test_blocks_read_what_their_predecessors_wrote():
         assert torch.equal(y, ref[i % 2])
 
 
+def test_block_without_gradients_refuses_heads_that_do_not_divide_the_width():
+    blk = TransformerBlock(584, 8, 64, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16)
+    blk.attn.heads = 9                                                    # 584 // 9 = 64, a head size the kernels know
+    x = torch.zeros(1, 4, 584, device="cuda").bfloat16()
+    for grad in (True, False):
+        with pytest.raises(RuntimeError), torch.set_grad_enabled(grad):
+            blk(x)
+
+
 def test_graph_keeps_its_weights_over_an_eager_forward():
     """A graph captured on shadows of the projections that are not neighbours replays the same result after a forward without
     gradients has run outside it and freed memory has been written over."""
