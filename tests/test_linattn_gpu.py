@@ -147,6 +147,7 @@ def test_segment_rule_leaves_no_empty_segment():
 
 
 def test_no_tokens():
+    from rust_neural_network_b200.ops.linear_attention import linear_attention
     q, k, v = (torch.zeros(2, 0, 4, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
     o = linear_attention(q, k, v, causal=True, kind="elu")
     assert o.shape == (2, 0, 4, 64) and all(g.shape == q.shape for g in torch.autograd.grad(o, (q, k, v), torch.zeros_like(o)))
