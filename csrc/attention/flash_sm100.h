@@ -13,7 +13,7 @@ struct FlashArgs {
   AttnTensor dout, dq, dk, dv;  // bf16 (backward only)
   float* lse;                   // [B, H, Sq] fp32, natural-log log-sum-exp of the scaled scores
   float* delta;                 // [B, H, Sq] fp32 scratch: rowsum(dO * O) (backward only)
-  float* dq_accum;              // [B, H, ceil(Sq / 128) * 128, hd] fp32 scratch in the kernel's own layout, zeroed by the launcher (backward only)
+  float* dq_accum;              // [B, H, ceil(Sq / 32) * 32, hd] fp32 scratch in the kernel's own layout, zeroed by the launcher (backward only; not used when Skv <= 128)
   int B, H, Sq, Skv, hd;
   float scale;
   int causal;

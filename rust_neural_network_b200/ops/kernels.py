@@ -584,16 +584,17 @@ def flash_bwd(dout, q, k, v, o, lse, scale, causal, dq=None, dk=None, dv=None):
     if dk is None: dk = torch.empty((B, Skv, H, hd), dtype=torch.bfloat16, device=dev)
     if dv is None: dv = torch.empty((B, Skv, H, hd), dtype=torch.bfloat16, device=dev)
     delta = torch.empty((B, H, Sq), dtype=torch.float32, device=dev)
-    dq_accum = torch.empty((B, H, (Sq + 127) // 128 * 128, hd), dtype=torch.float32, device=dev)   # the kernel's own layout
+    # the kernel's own layout; one key block adds nothing up and writes dq itself
+    dq_accum = torch.empty((B, H, (Sq + 31) // 32 * 32, hd), dtype=torch.float32, device=dev) if Skv > 128 else None
     a = nv.FlashArgs()
     a.q, a.k, a.v, a.o = _attn_tensor(q), _attn_tensor(k), _attn_tensor(v), _attn_tensor(o)
     a.dout, a.dq, a.dk, a.dv = _attn_tensor(dout), _attn_tensor(dq), _attn_tensor(dk), _attn_tensor(dv)
-    a.lse, a.delta, a.dq_accum = lse.data_ptr(), delta.data_ptr(), dq_accum.data_ptr()
+    a.lse, a.delta, a.dq_accum = lse.data_ptr(), delta.data_ptr(), nv.ptr(dq_accum)
     a.B, a.H, a.Sq, a.Skv, a.hd = B, H, Sq, Skv, hd
     a.scale, a.causal = float(scale), int(causal)
     a.status = nv.status_word(dev).data_ptr()
     nv.check(nv.cuda().b200_flash_bwd(C.byref(a), nv.stream_ptr()), "flash_bwd")
-    nv.count_launch(3)
+    nv.count_launch(3 if Skv > 128 else 2)
     return dq, dk, dv
 
 

@@ -381,6 +381,58 @@ def test_flash_forward_backward(B, S, H, hd, causal):
     assert rel_err(dq, qr.grad) < 2e-2
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("Sq,Skv", [(1, 1), (16, 16), (1, 200), (200, 1), (33, 128), (300, 100), (100, 300), (31, 129), (129, 129), (97, 513), (640, 65)])
+def test_flash_lengths_of_their_own(Sq, Skv, hd, causal):
+    """Queries and keys of different lengths around the blocks of 128 and the groups of 32: key blocks that no query sees, one
+    key block (whose dQ is final), remainders; gradients into views of a wider buffer, which is not written past them."""
+    B, H = 2, 3
+    g = torch.Generator(device=DEV).manual_seed(Sq * 7 + Skv + hd)
+    mk = lambda S: (torch.randn(B, S, H, hd, generator=g, device=DEV) * 0.8).bfloat16()
+    q, k, v, do = mk(Sq), mk(Skv), mk(Skv), mk(Sq)
+    scale = 1.0 / math.sqrt(hd)
+    o, lse = K.flash_fwd(q, k, v, scale, causal)
+    outs = [torch.full((B, S + 1, 2, H, hd), 7.0, device=DEV).bfloat16() for S in (Sq, Skv, Skv)]
+    got = K.flash_bwd(do, q, k, v, o, lse, scale, causal, *(t[:, :-1, 0] for t in outs))
+    ins = [t.float().requires_grad_(True) for t in (q, k, v)]
+    ref = K.attention_ref(*ins, scale, causal)
+    assert rel_err(o, ref) < 1.5e-2
+    for a, r in zip(got, torch.autograd.grad(ref, ins, do.float())):
+        # a single key has a gradient of zero, of which the kernel leaves rounding of terms of the size of dO . V
+        assert float((a.float() - r).norm()) < 2e-2 * float(r.norm()) + 2e-2 * (r.numel() ** 0.5 if min(Sq, Skv) == 1 else 0.0)
+    assert all(bool((t[:, -1] == 7.0).all()) and bool((t[:, :, 1] == 7.0).all()) for t in outs)
+
+
+@pytest.mark.parametrize("hd,S,causal", [(64, 8300, True), (128, 4200, True), (128, 4200, False)])
+def test_flash_long_sequences(hd, S, causal):
+    """Enough bytes that the blocks of a head run together (16 heads: 64 MB of operands in the backward) and pipelines that wrap
+    many times; three heads against fp32."""
+    H = 16
+    g = torch.Generator(device=DEV).manual_seed(S + hd)
+    q, k, v, do = ((torch.randn(1, S, H, hd, generator=g, device=DEV) * 0.8).bfloat16() for _ in range(4))
+    assert 2 * H * S * hd * 4 > 64 * 2 ** 20
+    o, lse = K.flash_fwd(q, k, v, hd ** -0.5, causal)
+    got = K.flash_bwd(do, q, k, v, o, lse, hd ** -0.5, causal)
+    for h in (0, 7, 15):
+        ins = [t[:, :, h:h + 1].float().requires_grad_(True) for t in (q, k, v)]
+        ref = K.attention_ref(*ins, hd ** -0.5, causal)
+        assert rel_err(o[:, :, h:h + 1], ref) < 1.5e-2
+        for a, r in zip(got, torch.autograd.grad(ref, ins, do[:, :, h:h + 1].float())):
+            assert rel_err(a[:, :, h:h + 1], r) < 2e-2
+
+
+def test_flash_backward_scratch_of_short_sequences():
+    """Many short sequences: beside its results the backward needs a few bytes per row, not blocks of 128 rows."""
+    q, k, v, do = (torch.randn(1024, 16, 8, 64, device=DEV).bfloat16() for _ in range(4))
+    o, lse = K.flash_fwd(q, k, v, 0.125, True)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    K.flash_bwd(do, q, k, v, o, lse, 0.125, True)
+    assert torch.cuda.max_memory_allocated() - before < 4 * q.numel() * 2
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,cols,causal", [(64, 37, 0), (256, 1024, 0), (96, 48, 48), (8, 4099, 0)])
 def test_softmax_rows_forward_backward(dtype, rows, cols, causal):
