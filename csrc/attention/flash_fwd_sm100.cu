@@ -13,7 +13,9 @@
 // S_{j+1} is issued right behind P V_j (over P_j: products execute in issue order) and two CTAs share an SM (TMEM 2 x 256
 // columns) so one CTA's exponentials overlap the other's MMAs. Without a P tile in shared memory head_dim 128 has room for
 // blocks of 128 keys (one K and one V stage; 64 keys and two stages before), which halves the waits per key; head_dim 64
-// keeps two stages. What bounds it is the chain wait - load - maximum - exponentials - store per block.
+// keeps two stages. Up to 64 keys blocks of 64 stay the better ones (half the products and exponentials: 2048 x 16 x 16 x 128
+// 627 us in blocks of 128, 516 in blocks of 64; 512 x 16 x 40 x 128 155 and 135). What bounds it is the chain wait - load -
+// maximum - exponentials - store per block.
 // Measured, causal (B x H x S x hd): 4 x 16 x 4096 x 128 428 -> 288 us (956 TFLOP/s), 64 x 8 x 1024 x 64 196 -> 175 us; not
 // causal, 16 x 8 x 577 x 64 40.5 -> 35.2 us. Every wait is bounded.
 #include "../common/ptx.cuh"
@@ -314,13 +316,15 @@ static int launch_fwd(const FlashArgs& a, cudaStream_t st) {
 
 extern "C" int b200_flash_fwd_init() {
   using namespace b200;
-  return fwd_set_attr<64, 128, true>() | fwd_set_attr<64, 128, false>() | fwd_set_attr<128, 128, true>() | fwd_set_attr<128, 128, false>();
+  return fwd_set_attr<64, 128, true>() | fwd_set_attr<64, 128, false>() | fwd_set_attr<128, 128, true>() | fwd_set_attr<128, 128, false>() |
+         fwd_set_attr<128, 64, true>() | fwd_set_attr<128, 64, false>();
 }
 
 extern "C" int b200_flash_fwd(const b200::FlashArgs* a, cudaStream_t st) {
   using namespace b200;
   if (a->B <= 0 || a->H <= 0 || a->Sq <= 0 || a->Skv <= 0) return 0;
   if (a->hd == 64) return a->causal ? launch_fwd<64, 128, true>(*a, st) : launch_fwd<64, 128, false>(*a, st);
+  if (a->hd == 128 && a->Skv <= 64) return a->causal ? launch_fwd<128, 64, true>(*a, st) : launch_fwd<128, 64, false>(*a, st);
   if (a->hd == 128) return a->causal ? launch_fwd<128, 128, true>(*a, st) : launch_fwd<128, 128, false>(*a, st);
   return -3;
 }
