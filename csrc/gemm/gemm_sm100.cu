@@ -507,7 +507,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (crank == 0 && elect_one()) {                     // of a CTA pair only the even CTA issues
+    // Of a CTA pair only the even CTA issues. The elected thread issues faster than lane 0 (8192 x 8192 x 2048 193 against 222 us,
+    // 8192 x 512 x 2048 27.2 against 30.1), but where 256-wide tiles are bound by writing their results it costs: both operands
+    // K-major, 8192 x 32000 x 512 312 against 300 us, 65536 x 2048 x 512 153.5 against 148.5, 65536 x 1536 x 512 118.8 against 114.8.
+    constexpr bool LANE0 = BN == 256 && CG == 1 && !A_MN && !B_MN;
+    if (crank == 0 && (LANE0 ? lane == 0 : elect_one())) {
       constexpr uint32_t idesc = make_idesc(BM * CG, BN, KindOf<T>::CF, KindOf<T>::AF, KindOf<T>::BF,
                                             A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       // K-major: 8-row groups 1024 B apart.  MN-major: 8-k-row groups 1024 B apart, 128B-row atoms
