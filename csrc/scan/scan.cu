@@ -416,6 +416,103 @@ scan_fwd_lanes_kernel(ScanArgs a) {
   }
 }
 
+// Forward with one state per lane (a warp carries 2 channels x 16 states): twice the warps of the kernel above for the same
+// channels. Where there is no more than one block per SM the issue slots are idle and a warp's own chain is what counts:
+// 1 x 4096 x 512 (32 blocks) 218 against 241 us, 2 x 2000 x 1000 (126 blocks) 114 against 121; with 256 blocks both take the
+// same (4 x 1000 x 1024), with 512 the kernel above is the faster one.
+// sums 16 per-lane values over the 16 lanes of a half-warp; lane j (mod 16) ends with the total of v[j]
+__device__ __forceinline__ float transpose_reduce16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int step = 0; step < 4; ++step) {
+    const int half = 8 >> step;
+    const bool upper = (lane & half) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = upper ? v[i] : v[i + half];
+      const float keep = upper ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+    }
+  }
+  return v[0];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+scan_fwd_state_kernel(ScanArgs a) {
+  constexpr int DB = 16, TT = 32;
+  __shared__ float2 s_x[2][TT][DB];                   // (delta, delta * u)
+  __shared__ float2 s_BC[2][TT][SCAN_N];
+  __shared__ float s_u[2][TT][DB], s_y[TT][DB];
+  const int b = blockIdx.y, d0 = blockIdx.x * DB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = lane & 15, ch = warp * 2 + (lane >> 4);
+  const int d = d0 + ch;
+  const bool active = d < a.D;
+  const float A2 = active ? a.A[(long long)d * SCAN_N + n] * SCAN_LOG2E : 0.f;
+  const float dsk = (active && a.Dskip) ? a.Dskip[d] : 0.f;
+  const int n_ck = (a.S + SCAN_CK - 1) / SCAN_CK;
+  float h = 0.f;
+  // loader role: thread -> (row lt of the tile, channel / state pair lp)
+  const int lt = threadIdx.x >> 3, lp = threadIdx.x & 7;
+  const int ld0 = d0 + 2 * lp, ld1 = ld0 + 1;
+  const float db0 = (a.delta_bias && ld0 < a.D) ? a.delta_bias[ld0] : 0.f, db1 = (a.delta_bias && ld1 < a.D) ? a.delta_bias[ld1] : 0.f;
+  const long long rb = (long long)b * a.S;
+  const T* up = (const T*)a.u; const T* dp = (const T*)a.delta; const T* Bp = (const T*)a.Bm; const T* Cp = (const T*)a.Cm;
+  float r[8];
+  auto load_tile = [&](int t0) {
+    const int t = t0 + lt;
+    const bool ok = t < a.S;
+    const long long row = rb + t;
+    r[0] = (ok && ld0 < a.D) ? s_ld(up + row * a.u_ld + ld0) : 0.f;
+    r[1] = (ok && ld1 < a.D) ? s_ld(up + row * a.u_ld + ld1) : 0.f;
+    float x0 = (ok && ld0 < a.D) ? s_ld(dp + row * a.delta_ld + ld0) + db0 : 0.f;
+    float x1 = (ok && ld1 < a.D) ? s_ld(dp + row * a.delta_ld + ld1) + db1 : 0.f;
+    if (a.delta_softplus) { x0 = softplus20(x0); x1 = softplus20(x1); }
+    r[2] = (ok && ld0 < a.D) ? x0 : 0.f; r[3] = (ok && ld1 < a.D) ? x1 : 0.f;
+    r[4] = ok ? s_ld(Bp + row * a.b_ld + 2 * lp) : 0.f; r[5] = ok ? s_ld(Bp + row * a.b_ld + 2 * lp + 1) : 0.f;
+    r[6] = ok ? s_ld(Cp + row * a.c_ld + 2 * lp) : 0.f; r[7] = ok ? s_ld(Cp + row * a.c_ld + 2 * lp + 1) : 0.f;
+  };
+  auto put_tile = [&](int buf) {
+    s_u[buf][lt][2 * lp] = r[0]; s_u[buf][lt][2 * lp + 1] = r[1];
+    s_x[buf][lt][2 * lp] = make_float2(r[2], r[2] * r[0]); s_x[buf][lt][2 * lp + 1] = make_float2(r[3], r[3] * r[1]);
+    s_BC[buf][lt][2 * lp] = make_float2(r[4], r[6]); s_BC[buf][lt][2 * lp + 1] = make_float2(r[5], r[7]);
+  };
+  const int n_tiles = (a.S + TT - 1) / TT;
+  load_tile(0); put_tile(0);
+  __syncthreads();
+  for (int tile = 0; tile < n_tiles; ++tile) {
+    const int cur = tile & 1, t0 = tile * TT;
+    if (tile + 1 < n_tiles) load_tile(t0 + TT);            // in flight while this tile is processed
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float p[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int t = half * 16 + i;
+        if ((t % SCAN_CK) == 0 && a.hck && active && t0 + t < a.S)
+          a.hck[(((long long)b * n_ck + (t0 + t) / SCAN_CK) * a.D + d) * SCAN_N + n] = h;      // state BEFORE step t
+        const float2 x = s_x[cur][t][ch], bc = s_BC[cur][t][n];
+        h = fmaf(scan_ex2(x.x * A2), h, x.y * bc.x);
+        p[i] = h * bc.y;
+      }
+      const float y = transpose_reduce16(p, lane);         // lane n: sum over the states for step half*16 + n
+      const int t = half * 16 + n;
+      s_y[t][ch] = y + dsk * s_u[cur][t][ch];
+    }
+    __syncthreads();
+    {
+      const int t = t0 + lt;
+      if (t < a.S) {
+        T* yp = (T*)a.y + (rb + t) * a.y_ld;
+        if (ld0 < a.D) s_st(yp + ld0, s_y[lt][2 * lp]);
+        if (ld1 < a.D) s_st(yp + ld1, s_y[lt][2 * lp + 1]);
+      }
+    }
+    if (tile + 1 < n_tiles) put_tile(cur ^ 1);
+    __syncthreads();
+  }
+}
+
 // Backward. A block owns 32 channels and walks the checkpoint intervals from the last to the first. Per interval each
 // lane re-runs 8 steps of its two states from the checkpoint, then runs the adjoint recurrence in reverse. The per-(t, n)
 // sums dB / dC, which run over ALL channels, are reduced over the warp's channels and the block's warps before one atomic
@@ -695,8 +792,13 @@ int b200_selective_scan_fwd(const ScanArgs* a, int is_bf16, cudaStream_t st) {
   if (a->B <= 0 || a->S <= 0 || a->D <= 0) return 0;
   if (a->N < 1 || a->N > SCAN_N) return -1;
   dim3 grid((a->D + SCAN_THREADS - 1) / SCAN_THREADS, a->B);
-  if (a->N == SCAN_N && !a->z) {       // lane-per-state kernel
+  if (a->N == SCAN_N && !a->z) {       // the states of a channel over several lanes
     dim3 g2((a->D + 15) / 16, a->B);
+    if ((long long)g2.x * g2.y <= 148) {
+      if (is_bf16) scan_fwd_state_kernel<__nv_bfloat16><<<g2, 256, 0, st>>>(*a);
+      else scan_fwd_state_kernel<float><<<g2, 256, 0, st>>>(*a);
+      return (int)cudaGetLastError();
+    }
     if (is_bf16) scan_fwd_lanes_kernel<__nv_bfloat16><<<g2, 128, 0, st>>>(*a);
     else scan_fwd_lanes_kernel<float><<<g2, 128, 0, st>>>(*a);
     return (int)cudaGetLastError();
@@ -709,7 +811,7 @@ int b200_selective_scan_fwd(const ScanArgs* a, int is_bf16, cudaStream_t st) {
 int b200_selective_scan_bwd(const ScanArgs* a, int is_bf16, cudaStream_t st) {
   if (a->B <= 0 || a->S <= 0 || a->D <= 0) return 0;
   if (a->N < 1 || a->N > SCAN_N || !a->hck) return -1;
-  if (a->N == SCAN_N && !a->z) {       // lane-per-state kernel
+  if (a->N == SCAN_N && !a->z) {       // two states per lane
     dim3 g2((a->D + 31) / 32, a->B);
     if (is_bf16) scan_bwd_lanes_kernel<__nv_bfloat16><<<g2, 256, 0, st>>>(*a);
     else scan_bwd_lanes_kernel<float><<<g2, 256, 0, st>>>(*a);

@@ -51,7 +51,7 @@ def test_selective_scan_fwd_bwd(B, S, D, N, full, dtype):
         assert rel_err(a.grad, b.grad) < gtol, nm
 
 
-@pytest.mark.parametrize("B,S,D", [(1, 1, 1), (2, 7, 31), (1, 8, 32), (3, 9, 33), (1, 33, 17), (2, 65, 64)])
+@pytest.mark.parametrize("B,S,D", [(1, 1, 1), (2, 7, 31), (1, 8, 32), (3, 9, 33), (1, 33, 17), (2, 65, 64), (148, 9, 16), (149, 9, 16), (75, 33, 17), (150, 65, 1)])
 def test_selective_scan_block_edges(B, S, D):
     """16 states, no gate: around the 8-step intervals, the 32-step tiles and the 16 / 32 channels of a block. fp32: the
     kernel's ex2.approx and summation order against the sequential recurrence, ~1e-6 per step over at most 65 steps."""
