@@ -112,15 +112,32 @@ def _g_pass(q, k, v, o, den, dout, o_lo):
     return g
 
 
-def _segments(bh: int, n_chunks: int, hd: int, sms: int) -> int:
-    """Into how many segments the sequence of every (batch, head) is cut: as many as still run at once (two CTAs per SM at
-    head size 64, one at 128). A segment costs a pass over its K and V (Q, dO, O in the backward) for its total, so segments
-    that would queue lose: 8 x 16 heads, 4096 tokens, head size 128, forward + backward 1.70 ms whole, 2.11 ms in two; while
-    1 x 8 heads x 16384 x 128 takes 6.32 ms whole and 0.69 ms in 16, 1 x 16 x 1000 x 128 0.34 and 0.17 ms in 8."""
-    if n_chunks == 0:
+def _segments(bh: int, n_chunks: int, hd: int, sms: int, grad: bool = True) -> int:
+    """Into how many segments the sequence of every (batch, head) is cut: as many as run at once (two CTAs per SM at head size
+    64, one at 128) where that is faster than one. A segment costs a pass over its K and V (Q, G in the backward) for its
+    total and the sum over the totals. Time in us, linear in the chunks that one CTA walks (`per`), fitted to measurements
+    that it meets within about a tenth; whole / cut, forward and forward + backward:
+    1 x 8 heads, head size 64: 256 tokens 15 / 22, 49 / 59; 384 tokens 21 / 22, 68 / 60; 1024 tokens 49 / 22, 159 / 60.
+    1 x 8, 128: 384 tokens 30 / 42, 103 / 120; 640 tokens 47 / 42, 161 / 121; 16384 tokens 1121 / 133, 3812 / 434.
+    8 x 16, 64: 1024 tokens 49 / 66, 184 / 195; 2048 tokens 95 / 108, 352 / 335; 16384 tokens 741 / 694, 2720 / 2268.
+    4 x 16, 128: 512 tokens 38 / 59, 145 / 193; 4096 tokens 285 / 235, 1029 / 760."""
+    n = min((2 if hd == 64 else 1) * sms // max(bh, 1), n_chunks, 64)
+    if n < 2:
         return 1
-    n = max(1, min((2 if hd == 64 else 1) * sms // max(bh, 1), n_chunks, 64))
-    return -(-n_chunks // -(-n_chunks // n))                     # no empty last segment
+    per = -(-n_chunks // n)
+    n = -(-n_chunks // per)                                      # no empty last segment
+    ctas = bh * n
+    if hd == 64:
+        crowded = ctas > sms                                     # two CTAs of an SM share it
+        if grad:
+            whole, cut = 13 + (18.2 + 0.026 * bh) * n_chunks, 38 + (38 if crowded else 22 + 0.035 * ctas) * per
+        else:
+            whole, cut = 4 + 5.7 * n_chunks, 14.5 + 0.03 * ctas + (10.8 if crowded else 7.8) * per
+    elif grad:
+        whole, cut = 16 + (29 + 0.05 * bh) * n_chunks, 88 + (35.5 + 0.06 * ctas) * per
+    else:
+        whole, cut = 4 + 8.7 * n_chunks, 27.5 + 0.045 * ctas + 11.8 * per
+    return n if cut < whole else 1
 
 
 class FusedCausalLinearAttnFn(Function):
@@ -152,7 +169,7 @@ class FusedCausalLinearAttnFn(Function):
             pre = _launch(0, q, k, v, scale, eps, kind, o=o, den=den, o_lo=o_lo, sx=(sp, 0, 2))
             s_in = pre.clone() if (sp.rank > 0 and need_grad) else None      # the buffer is reused by the next call
         else:
-            n_seg = 1 if sp is not None else _segments(B * H, -(-S // CHUNK), d, _num_sms(dev))
+            n_seg = 1 if sp is not None else _segments(B * H, -(-S // CHUNK), d, _num_sms(dev), need_grad)
             seg = torch.empty((B * H, n_seg, d * d + d), dtype=torch.float32, device=dev) if n_seg > 1 else None
             _launch(0, q, k, v, scale, eps, kind, o=o, den=den, s_in=s_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
             s_in = s_in if seg is None else seg                  # the states the backward's dQ pass starts from

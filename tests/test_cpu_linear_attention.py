@@ -101,9 +101,19 @@ def test_segments_cover_every_chunk():
     """Every chunk lies in one segment and none of them is empty; no tokens are one (empty) segment."""
     from rust_neural_network_b200.ops.linear_attention import _segments
     for bh in (0, 1, 7, 16, 148, 296, 4096):
-        for hd in (64, 128):
-            assert _segments(bh, 0, hd, 148) == 1
+        for hd, grad in ((64, True), (64, False), (128, True), (128, False)):
+            assert _segments(bh, 0, hd, 148, grad) == 1
             for chunks in (1, 2, 3, 8, 9, 63, 64, 65, 512, 1000):
-                n = _segments(bh, chunks, hd, 148)
+                n = _segments(bh, chunks, hd, 148, grad)
                 per = -(-chunks // n)
                 assert 1 <= n <= 64 and (n - 1) * per < chunks <= n * per
+
+
+def test_segments_only_where_they_were_measured_to_pay():
+    """(heads, chunks, head size): whole sequences were faster for the first group, cut ones for the second."""
+    from rust_neural_network_b200.ops.linear_attention import _segments
+    whole = [(8, 2, 64, True), (8, 3, 64, False), (8, 3, 128, True), (8, 4, 128, False), (64, 4, 128, True), (128, 8, 64, True), (128, 16, 64, False)]
+    cut = [(8, 3, 64, True), (8, 4, 64, False), (8, 5, 128, True), (8, 5, 128, False), (8, 128, 128, True), (64, 8, 64, True), (64, 32, 128, True),
+           (128, 16, 64, True), (128, 128, 64, True), (128, 128, 64, False), (16, 8, 128, True)]
+    assert [_segments(bh, c, hd, 148, g) for bh, c, hd, g in whole] == [1] * len(whole)
+    assert all(_segments(bh, c, hd, 148, g) > 1 for bh, c, hd, g in cut)
