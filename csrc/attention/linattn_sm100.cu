@@ -76,6 +76,7 @@ struct LinAttnArgs {
   uint32_t* status;
   float* seg;                                // n_seg > 1: [B*H][n_seg][hd*hd + hd] fp32 workspace for the states between segments
   int n_seg, seg_chunks;                     // the sequence is walked as n_seg segments of seg_chunks chunks by as many CTAs
+  float* dseg;                               // whole backward, n_seg > 1: the workspace of dK / dV (`seg` holds the forward's states)
   LaExchange sx;
 };
 
@@ -1081,6 +1082,14 @@ __global__ void la_segment_prefix_kernel(float* __restrict__ seg, const float* _
 template <int HD>
 static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
   if (la_set_attrs<HD>()) return 104;
+  if (which == 4) {                                     // a whole backward: G pass, dQ, dK / dV
+    if (int rc = la_launch<HD>(a, 3, st)) return rc;
+    if (int rc = la_launch<HD>(a, 1, st)) return rc;
+    LinAttnArgs t = a;
+    t.seg = a.dseg;
+    t.s_in = nullptr;
+    return la_launch<HD>(t, 2, st);
+  }
   if (which != 3 && a.n_seg > 1 && !a.state_only && a.s_in != a.seg && a.ds_in != a.seg) {
     // segments: their totals, the prefix over them (the forward's serves the dQ pass too), then the pass itself from there
     LinAttnArgs t = a;
@@ -1127,11 +1136,11 @@ static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
 
 }  // namespace b200
 
-// which: 0 forward (or state-only pass), 3 the backward's G pass, then 1 dQ and 2 dK / dV. Causal form; hd 64 or 128; bf16.
+// which: 0 forward (or state-only pass), 4 backward; its parts: 3 G pass, then 1 dQ and 2 dK / dV. Causal form; hd 64 or 128; bf16.
 extern "C" int b200_linattn(const b200::LinAttnArgs* a, int which, cudaStream_t st) {
   using namespace b200;
   if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
-  if (which < 0 || which > 3 || (which > 0 && (!a->g.ptr || !a->dden)) || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
+  if (which < 0 || which > 4 || (which == 4 && (a->state_only || a->sx.role != 0 || (a->n_seg > 1 && !a->dseg))) || (which > 0 && (!a->g.ptr || !a->dden)) || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
   if ((long long)a->n_seg * a->seg_chunks < (a->S + LA_C - 1) / LA_C || (long long)(a->n_seg - 1) * a->seg_chunks >= (a->S + LA_C - 1) / LA_C) return -2;
   if (a->hd == 64) return la_launch<64>(*a, which, st);
   if (a->hd == 128) return la_launch<128>(*a, which, st);

@@ -11,7 +11,7 @@ denominator for free), between chunks a d x (d+8) state is carried by an exclusi
 
 On a GPU the causal bf16 form with head_dim 64 or 128 runs on the FUSED chunk kernels of
 csrc/attention/linattn_sm100.cu (`FusedCausalLinearAttnFn`): phi in the prologue, all products on tcgen05 with the
-state in TMEM in fp32, the division in the epilogue, one launch forward and two backward. Everything else (non-causal,
+state in TMEM in fp32, the division in the epilogue. Everything else (non-causal,
 other head sizes, fp32, CPU) takes the composition below, in which every
 product is a batched call of the tcgen05 GEMM kernel (NT for (phi Q)(phi K)^T, TN for the chunk states,
 NN for applying them); the feature maps and the mask are this package's elementwise kernels. The
@@ -52,7 +52,7 @@ class LinAttnArgs(C.Structure):
                 ("den", C.c_void_p), ("dden", C.c_void_p), ("s_in", C.c_void_p), ("s_out", C.c_void_p), ("ds_in", C.c_void_p), ("ds_out", C.c_void_p),
                 ("B", C.c_int), ("H", C.c_int), ("S", C.c_int), ("hd", C.c_int), ("scale", C.c_float), ("eps", C.c_float),
                 ("kind", C.c_int), ("state_only", C.c_int), ("status", C.c_void_p),
-                ("seg", C.c_void_p), ("n_seg", C.c_int), ("seg_chunks", C.c_int), ("sx", LaExchange)]
+                ("seg", C.c_void_p), ("n_seg", C.c_int), ("seg_chunks", C.c_int), ("dseg", C.c_void_p), ("sx", LaExchange)]
 
 
 nv.register_sigs({"b200_linattn": [C.POINTER(LinAttnArgs), C.c_int, C.c_void_p], "b200_linattn_init": []})
@@ -75,16 +75,17 @@ def fused_supported(q, causal) -> bool:
 
 @nv.traced("linear_attention")
 def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=None, dk=None, dv=None, s_in=None, s_out=None,
-            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None, seg=None, n_seg=1, g=None):
+            ds_in=None, ds_out=None, state_only=False, o_lo=None, sx=None, seg=None, n_seg=1, g=None, dseg=None):
     """`sx = (SPContext, dir, role)` lets the kernel itself exchange the slice totals with the other ranks (see
     `LaExchange`); it returns the local buffer the consume pass leaves the summed state in. `g`: what `_g_pass` returned
-    for this backward (made here when a gradient kernel is launched without it)."""
+    for this backward (made here when a gradient kernel is launched without it), or the memory for it when the whole backward
+    is launched (`which` 4)."""
     B, S, H, d = q.shape
     a = LinAttnArgs()
     if which in (1, 2):
         gt, dden = g if g is not None else _g_pass(q, k, v, o, den, dout, o_lo)
         a.g, a.dden = _attn_t(gt), dden.data_ptr()
-    elif which == 3:
+    elif which >= 3:
         a.g, a.dden = _attn_t(g[0]), g[1].data_ptr()
     prefix = None
     if sx is not None:
@@ -98,16 +99,20 @@ def _launch(which, q, k, v, scale, eps, kind, o=None, den=None, dout=None, dq=No
     a.kind, a.state_only = (0 if kind == "elu" else 1), int(state_only)
     a.status = nv.status_ptr(q.device)
     n_chunks = -(-S // CHUNK)
-    a.seg, a.n_seg, a.seg_chunks = nv.ptr(seg), n_seg, -(-n_chunks // n_seg)
+    a.seg, a.n_seg, a.seg_chunks, a.dseg = nv.ptr(seg), n_seg, -(-n_chunks // n_seg), nv.ptr(dseg)
     nv.check(nv.cuda().b200_linattn(C.byref(a), which, nv.stream_ptr()), "linattn")
-    nv.count_launch(1 if n_seg == 1 or which == 1 else 3)
+    nv.count_launch((3 if n_seg == 1 else 5) if which == 4 else 1 if n_seg == 1 or which == 1 else 3)
     return prefix
+
+
+def _g_empty(q):
+    B, S, H, d = q.shape
+    return torch.empty((B, S, H, d), dtype=torch.bfloat16, device=q.device), torch.empty((B, H, S), dtype=torch.float32, device=q.device)
 
 
 def _g_pass(q, k, v, o, den, dout, o_lo):
     """(G = dO / D, dden = -(G . O)): what both gradient kernels start from."""
-    B, S, H, d = q.shape
-    g = (torch.empty((B, S, H, d), dtype=torch.bfloat16, device=q.device), torch.empty((B, H, S), dtype=torch.float32, device=q.device))
+    g = _g_empty(q)
     _launch(3, q, k, v, 1.0, 0.0, "elu", o=o, den=den, dout=dout, o_lo=o_lo, g=g)
     return g
 
@@ -141,8 +146,10 @@ def _segments(bh: int, n_chunks: int, hd: int, sms: int, grad: bool = True) -> i
 
 
 class FusedCausalLinearAttnFn(Function):
-    """Causal linear attention on the fused chunk kernels (csrc/attention/linattn_sm100.cu): one forward kernel, two
-    backward kernels (dQ in sequence order, dK / dV in reverse order), state carried in fp32, nothing stored per chunk.
+    """Causal linear attention on the fused chunk kernels (csrc/attention/linattn_sm100.cu): one forward kernel; in the backward
+    a pass that forms G = dO / D and dD, then dQ in sequence order and dK / dV in reverse order. Where the sequence is cut
+    into segments (`_segments`), the forward and dK / dV are each preceded by a pass for the segments' totals and a sum over
+    them. State in fp32; what is stored is one state per segment.
     With `sp` the rank's tokens are one slice of a longer sequence: a state-only pass produces the slice's total state,
     one exchange kernel turns the totals into prefixes (suffixes in the backward), and the main pass starts from them."""
 
@@ -187,19 +194,20 @@ class FusedCausalLinearAttnFn(Function):
         B, S, H, d = q.shape
         dout = dout if (_tma_ok(dout) and dout.dtype == torch.bfloat16) else dout.to(torch.bfloat16).contiguous()
         dq, dk, dv = torch.empty_like(o), torch.empty_like(o), torch.empty_like(o)
-        g = _g_pass(q, k, v, o, den, dout, o_lo)
-        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, g=g, s_in=None if n_seg > 1 else s_in, o_lo=o_lo, seg=s_in if n_seg > 1 else None, n_seg=n_seg)
-        ds_in = None
-        if sp is not None and sp.world > 1 and sp.backend == "fused":
+        if sp is None or sp.world <= 1:                         # one call: preparing a launch from Python takes 20 us
+            _launch(4, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, dk=dk, dv=dv, g=_g_empty(q), s_in=None if n_seg > 1 else s_in,
+                    o_lo=o_lo, seg=s_in if n_seg > 1 else None, dseg=torch.empty_like(s_in) if n_seg > 1 else None, n_seg=n_seg)
+            return dq, dk, dv, None, None, None, None
+        g = _g_pass(q, k, v, o, den, dout, o_lo)                 # a slice of a longer sequence
+        _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, g=g, s_in=s_in, o_lo=o_lo)
+        if sp.backend == "fused":
             _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, state_only=True, o_lo=o_lo, sx=(sp, 1, 1))
             _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, dk=dk, dv=dv, o_lo=o_lo, sx=(sp, 1, 2))
             return dq, dk, dv, None, None, None, None
-        if sp is not None and sp.world > 1:
-            tot = torch.empty((B * H, d * d + d), dtype=torch.float32, device=q.device)
-            _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, ds_out=tot, state_only=True, o_lo=o_lo)
-            ds_in = sp._exchange(tot, 1)                        # sum of the higher ranks' totals
-        seg = torch.empty_like(s_in) if n_seg > 1 else None
-        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
+        tot = torch.empty((B * H, d * d + d), dtype=torch.float32, device=q.device)
+        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, ds_out=tot, state_only=True, o_lo=o_lo)
+        ds_in = sp._exchange(tot, 1)                            # sum of the higher ranks' totals
+        _launch(2, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, g=g, dk=dk, dv=dv, ds_in=ds_in, o_lo=o_lo)
         return dq, dk, dv, None, None, None, None
 
 
