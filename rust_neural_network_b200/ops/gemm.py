@@ -138,6 +138,13 @@ _KINDS = {(torch.bfloat16, torch.bfloat16): GEMM_BF16, (torch.float32, torch.flo
           (torch.float8_e4m3fn, torch.float8_e4m3fn): GEMM_E4M3}
 
 
+def tile_width(M: int, N: int, batch: int, sms: int) -> int:
+    """Columns of a bf16 product's tiles: 256 once such tiles fill the machine."""
+    if N <= 128:
+        return 64 if N <= 64 else 128
+    return 256 if -(-M // 128) * -(-N // 256) * batch >= sms else 128
+
+
 @nv.traced("gemm")
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, act: str = "none",
          residual=None, aux_in=None, dact: str = "none", want_aux: bool = False, alpha: float = 1.0,
@@ -216,17 +223,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     elif lowp:
         bn = 256 if (bn == 256 or (bn == 0 and math.ceil(M / 128) * math.ceil(N / 256) * batch >= sms)) else 128
     elif bn == 0:
-        if N <= 64:
-            bn = 64
-        elif N <= 128:
-            bn = 128
-        else:
+        bn = tile_width(M, N, batch, sms)
+        if N > 128:
             t256 = math.ceil(M / 128) * math.ceil(N / 256) * batch
             # Few tiles and a long K (weight gradients): split-K fills the machine either way, and the wider tile moves
             # a third less operand traffic from L2 per FLOP (measured 167 -> 113 us on 2048 x 512 x 65536).
             splittable = (splits == 0 and out_mode in (OUT_F32, OUT_F32_ATOMIC) and act == "none" and aux_in is None and not want_aux
                           and N >= 256 and K >= 16 * 64 * max(1, sms // max(t256, 1)))
-            bn = 256 if (t256 >= sms or splittable) else 128
+            bn = 256 if splittable else bn
     bk = 32 if is_f32 else 128 if lowp else 64
     num_kb = max(1, math.ceil(K / bk))
     tiles = math.ceil(M / 128) * math.ceil(N / bn) * batch
