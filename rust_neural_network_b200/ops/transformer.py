@@ -209,10 +209,11 @@ def _block_forward(x, blk, causal):
 
 def transformer_block(x, blk, causal):
     """Run `blk` (a `models.looped_transformer.TransformerBlock`) through the fused function. Without gradients (and outside
-    torch.func transforms and forward-mode AD, whose tensors have no memory of their own) the forward is one native call."""
+    torch.func transforms and forward-mode AD, whose tensors have no memory of their own, and tracing, which records a function
+    but not a kernel's writes) the forward is one native call."""
     at = blk.attn
     if (not torch.is_grad_enabled() and not nv.NVTX_ENABLED and torch._C._functorch.peek_interpreter_stack() is None
-            and torch.autograd.forward_ad._current_level < 0):
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None):
         y = _block_forward(x, blk, causal)
         if y is not None:
             return y

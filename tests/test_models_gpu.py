@@ -108,6 +108,15 @@ def test_block_without_gradients_refuses_heads_that_do_not_divide_the_width():
             blk(x)
 
 
+def test_traced_block_runs_on_new_inputs():
+    torch.manual_seed(6)
+    blk = TransformerBlock(128, 2, 256, causal=True, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16)
+    x, x2 = (torch.randn(2, 40, 128, device="cuda").bfloat16() for _ in range(2))
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda t: blk(t) * 1.0, (x,), check_trace=False)
+        assert torch.equal(traced(x2), blk(x2))
+
+
 def test_graph_keeps_its_weights_over_an_eager_forward():
     """A graph captured on shadows of the projections that are not neighbours replays the same result after a forward without
     gradients has run outside it and freed memory has been written over."""
