@@ -185,6 +185,7 @@ class EPContext:
 
 
 _FUSED_LAYER = os.environ.get("B200NN_MOE_FUSED_LAYER", "1") != "0"
+_ALONE_FROM = 1 << 25                # routed elements from which one rank alone takes the separate kernels (see MoEExpertsFn)
 
 
 class MoeFusedArgs(C.Structure):
@@ -267,7 +268,7 @@ class MoEExpertsFn(Function):
         # One rank alone has no transfer to overlap: from about 2^25 routed elements on, the separate kernels (CTA-pair GEMMs) are
         # faster: forward + backward of 8192 x 6 x 1024 1.79 against 1.90 ms, 16384 x 6 x 1024 2.75 against 3.03 ms, 16384 x 6 x 512
         # 1.58 against 1.72 ms; below that the single launch wins (4096 x 6 x 1024 1.48 against 1.55 ms).
-        alone = world == 1 and T * k * d >= 1 << 25
+        alone = world == 1 and T * k * d >= _ALONE_FROM
         if ep.backend == "fused" and x.is_cuda and _FUSED_LAYER and d % 8 == 0 and not alone:
             out, saved = _fused_layer_forward(ep, xc, idx, w, W1, b1, W2, b2, act, cap, xbuf, xptrs, fill, fptrs, ybuf, yptrs, dest)
             ctx.save_for_backward(*saved)

@@ -136,6 +136,32 @@ def test_segments_equal_one_walk(S, hd, kind, n, monkeypatch):
         assert _rel(a, b) < 2 ** -9
 
 
+@pytest.mark.parametrize("hd,kind", [(64, "elu"), (128, "relu2")])
+def test_segments_start_from_a_given_state(hd, kind):
+    """States that flow in (before the first token, behind the last one) and out, with the sequence whole and in segments. The
+    order of the fp32 state sums differs: 2^-9 of a bf16 result, 2^-18 of a state."""
+    from rust_neural_network_b200 import _native as nv
+    from rust_neural_network_b200.ops import linear_attention as LA
+    B, S, H, n = 2, 900, 2, 3
+    q, k, v, w = _inputs(B, S, H, hd, seed=11)
+    g = torch.Generator(device="cuda").manual_seed(12)
+    st = torch.rand(B * H, hd * hd + hd, generator=g, device="cuda") * 40          # about what some hundred tokens leave
+    ds = torch.randn(B * H, hd * hd + hd, generator=g, device="cuda") * 0.1
+    seg = torch.empty(B * H, n, hd * hd + hd, device="cuda")
+    res = []
+    for cut in (False, True):
+        o, s_out, ds_out = torch.empty_like(q), torch.empty_like(st), torch.empty_like(st)
+        den, dq, dk, dv = torch.empty(B, H, S, device="cuda"), *(torch.empty_like(q) for _ in range(3))
+        kw = dict(seg=seg, n_seg=n) if cut else {}
+        LA._launch(0, q, k, v, hd ** -0.5, 1e-6, kind, o=o, den=den, s_in=st, s_out=s_out, **kw)
+        LA._launch(1, q, k, v, hd ** -0.5, 1e-6, kind, o=o, den=den, dout=w, dq=dq, **(kw or dict(s_in=st)))
+        LA._launch(2, q, k, v, hd ** -0.5, 1e-6, kind, o=o, den=den, dout=w, dk=dk, dv=dv, ds_in=ds, ds_out=ds_out, **kw)
+        torch.cuda.synchronize(); nv.check_status()
+        res.append((o, dq, dk, dv, s_out, ds_out))
+    for i, (a, b) in enumerate(zip(*res)):
+        assert _rel(b, a) < (2 ** -9 if i < 4 else 2 ** -18 if i == 4 else 2 ** -9), i
+
+
 def test_segment_rule_leaves_no_empty_segment():
     from rust_neural_network_b200.ops.linear_attention import _segments
     for bh in (1, 3, 16, 128, 1000):

@@ -112,6 +112,10 @@ def test_traced_block_runs_on_new_inputs():
     torch.manual_seed(6)
     blk = TransformerBlock(128, 2, 256, causal=True, init=nn.normal_init(0.05)).to_device(torch.device("cuda"), torch.bfloat16)
     x, x2 = (torch.randn(2, 40, 128, device="cuda").bfloat16() for _ in range(2))
+    with pytest.raises(RuntimeError), torch.no_grad():                    # a trace holds no weights that want gradients
+        torch.jit.trace(lambda t: blk(t) * 1.0, (x,), check_trace=False)
+    for p in blk.parameters():
+        p.requires_grad_(False)
     with torch.no_grad():
         traced = torch.jit.trace(lambda t: blk(t) * 1.0, (x,), check_trace=False)
         assert torch.equal(traced(x2), blk(x2))

@@ -95,6 +95,34 @@ def test_one_kernel_layer_equals_the_separate_kernels(monkeypatch):
     assert rel_err(res[0][0], ref) < 2e-2
 
 
+@pytest.mark.parametrize("T,past", [(16384, True), (16383, False)])
+def test_one_rank_alone_takes_the_separate_kernels_for_many_tokens(monkeypatch, T, past):
+    """On both sides of the rule (16384 x 8 x 256 routed elements): output bit for bit, gradients up to the order over rows."""
+    torch.manual_seed(4)
+    d, hid, E, k = 256, 64, 16, 8
+    assert (T * k * d >= M._ALONE_FROM) == past
+    x = (torch.randn(T, d, device="cuda") * 0.5).bfloat16()
+    idx = torch.topk(torch.randn(T, E, device="cuda"), k)[1].int()
+    w = torch.rand(T, k, device="cuda")
+    ws = [torch.nn.Parameter(torch.randn(*s, device="cuda") * 0.1) for s in ((E, hid, d), (E, hid), (E, d, hid), (E, d))]
+    g = torch.randn(T, d, device="cuda").bfloat16()
+    single, calls = M._fused_layer_forward, []
+    monkeypatch.setattr(M, "_fused_layer_forward", lambda *a: calls.append(1) or single(*a))
+    res = []
+    for limit in (M._ALONE_FROM, 1 << 62):
+        monkeypatch.setattr(M, "_ALONE_FROM", limit)
+        xi, wi = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        for p in ws:
+            p.grad = None
+        out = M.MoEExpertsFn.apply(xi, idx, wi, *ws, "silu", T * k // E + 1024 & ~127, None)
+        out.backward(g)
+        res.append([out.detach(), xi.grad, wi.grad] + [p.grad.clone() for p in ws])
+    assert len(calls) == (1 if past else 2)
+    assert torch.equal(res[0][0], res[1][0])
+    for a, b in zip(res[0][1:], res[1][1:]):
+        assert rel_err(a, b) < 1e-5
+
+
 def test_capacity_drops_are_consistent():
     torch.manual_seed(2)
     T, d, hid, E, k = 256, 64, 64, 4, 1
