@@ -17,7 +17,10 @@
 // bandwidth (operands of the products, dS, the row statistics): P, and for head_dim 64 K and V, are A operands in TMEM,
 // and dQ leaves as 8 KB bulk adds in a private layout ([32-row group][hd / 4][32][4]) that the staging stores write without
 // bank conflicts (the same layout added from registers, 512 bytes per instruction, was slower: 884 against 737 us below).
-// Products that share TMEM columns (S / P, and for head_dim 128 dP / dQ) rely on the tensor core executing in issue order.
+// S of the next block is written over the P that dV has just read, and behind it in issue order. The PTX document orders products
+// of one accumulator and shape, which these two are not: that the tensor core of a CTA executes one thread's products in issue
+// order is an observation (every test and every repeated run agrees), not a promise. A commit and a wait between them would put
+// the completion of dV on the chain of every block, which issuing S early is there to shorten.
 // Every wait is bounded.
 // Measured, kernel alone (B x H x S x hd, causal; earlier form -> this one): 4 x 16 x 4096 x 128 1371 -> 718 us (957 TFLOP/s),
 // 4 x 16 x 4096 x 64 769 -> 449 us, 64 x 8 x 1024 x 64 507 -> 355 us; not causal, 16 x 8 x 577 x 64 92 -> 67 us.
@@ -452,7 +455,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tc_fence_after_sync();
           dv_of(it);
           tc_commit(&do_empty[it % DO_ST]);                    // dP and dV of this block were dO's readers
-          if (more && !next_s(it + 1)) return false;           // over P of this block: products execute in issue order
+          if (more && !next_s(it + 1)) return false;           // over P of this block, behind dV in issue order (see the top)
           if (!mbar_wait(ds_ready, it & 1, p.status, ST_TIMEOUT_ACC_EMPTY)) return false;
           tc_fence_after_sync();
           if (ROOM) {                                          // dP keeps its own columns: first, it is what the softmax warps wait for

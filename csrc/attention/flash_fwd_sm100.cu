@@ -10,8 +10,10 @@
 //                        columns it came from: the A operand of P V
 //   O += P V_j       tcgen05.mma accumulating in TMEM, V consumed MN-major straight from its [kv][hd] layout;
 //                    O is rescaled (TMEM load / store) only when the running maximum grows by > 2^8
-// S_{j+1} is issued right behind P V_j (over P_j: products execute in issue order) and two CTAs share an SM (TMEM 2 x 256
-// columns) so one CTA's exponentials overlap the other's MMAs. Without a P tile in shared memory head_dim 128 has room for
+// S_{j+1} is issued right behind P V_j and written over P_j, without a commit and a wait between them, which would put P V's
+// completion on the chain of every block. That a thread's products execute in issue order is an observation here (PTX promises it
+// for products of one accumulator and shape only). Two CTAs share an SM (TMEM 2 x 256 columns) so one CTA's exponentials overlap
+// the other's MMAs. Without a P tile in shared memory head_dim 128 has room for
 // blocks of 128 keys (one K and one V stage; 64 keys and two stages before), which halves the waits per key; head_dim 64
 // keeps two stages. Up to 64 keys blocks of 64 stay the better ones (half the products and exponentials: 2048 x 16 x 16 x 128
 // 627 us in blocks of 128, 516 in blocks of 64; 512 x 16 x 40 x 128 155 and 135). What bounds it is the chain wait - load -

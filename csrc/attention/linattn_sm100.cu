@@ -837,7 +837,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int bh = blockIdx.x / p.n_seg, seg = blockIdx.x % p.n_seg, b = bh / p.H, h = bh % p.H;
   const int c0 = seg * p.seg_chunks;           // first chunk of this CTA's segment
   const int n_chunks = min(p.seg_chunks, (p.S + LA_C - 1) / LA_C - c0);
-  const bool full = !p.state_only;               // state_only: only dS / dz of this slice (reads Q, dO, O)
+  const bool full = !p.state_only;               // state_only: only dS / dz of this slice (reads Q, G, dden)
   if (p.n_seg > 1 && !full && seg == 0) return;  // nothing precedes the first segment
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
@@ -944,10 +944,12 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       tc_fence_after_sync();
       la_mma_tw<HD>(tmem_base + COL_DV, tmem_base + COL_T, sG);                       // dV += mask(A)^T G
       tc_commit(u_bar);
-      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);                                      // (G V^T)^T = V G^T   [key][query], over the tile dV has read
+      // (G V^T)^T = V G^T [key][query], over the tile that dV reads just before: in issue order, which is an observation (PTX
+      // promises it for one accumulator and shape); waiting for dV here would add its completion to the chain of every chunk
+      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);
       tc_commit(t_bar);
     }
-    if (!mbar_wait(t_bar, t_phase, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;      // implies u_bar: the tensor core runs in order
+    if (!mbar_wait(t_bar, t_phase, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;      // (u_bar has come by then: products are seen to execute in issue order)
     t_phase ^= 1;
     if (ok && !mbar_wait(u_bar, it & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }

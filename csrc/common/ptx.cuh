@@ -40,8 +40,8 @@ __device__ __forceinline__ uint32_t lane_id() {
 }
 
 // One thread of a converged warp. Threads that issue tcgen05.mma are chosen this way, in a branch on a warp index that is
-// uniform by construction (`uniform_warp`): the compiler then keeps the descriptors in uniform registers. Behind a plain
-// `lane == 0` it does not, and back-to-back 128 x 64 x 16 products with A in TMEM took 44 cycles to issue against 29.
+// uniform by construction (`uniform_warp`). Measured with clock64 around a run of back-to-back 128 x 64 x 16 products with A in
+// TMEM: 29 cycles each, 44 behind a plain `lane == 0`. (One exception, measured: 256-wide K-major tiles in gemm_sm100.cu.)
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
