@@ -44,21 +44,29 @@ def _fused_qkv(wq, wk, wv, getter):
     return torch.cat([a, b, c], 0)
 
 
-def _shadow_qkv(wq, wk, wv):
-    """bf16 [3d, d] of the three projections (`functional.lp`). Weights that have no shadow yet, those no optimizer has laid
-    out, get theirs as neighbours in one buffer, so that no call has to copy them together. A shadow that exists is never
+def _shadows_qkv(wq, wk, wv):
+    """bf16 shadows of the three projections (`functional.lp`). Weights that have none yet, those no optimizer has laid out,
+    get theirs as neighbours in one buffer, so that no call has to copy them together. A shadow that exists is never
     moved: a captured graph or another stream may read it, and its memory would be given away under them. (Nor is a buffer
     made while a graph is being captured, which would own it.)"""
-    ws = (wq, wk, wv)
-    if (all(getattr(w, "_lp", None) is None for w in ws) and len({id(w) for w in ws}) == 3 and len({(w.shape, w.device) for w in ws}) == 1
-            and not (wq.is_cuda and torch.cuda.is_current_stream_capturing())):
-        versions = [w._version for w in ws]
-        with torch.inference_mode(False), torch.no_grad():             # (an inference tensor could not be refreshed outside that mode)
-            buf = torch.cat([w.detach().to(torch.bfloat16) for w in ws], 0)
-            parts = buf.split(wq.shape[0], 0)
-        for w, part, version in zip(ws, parts, versions):
-            w._lp, w._lp_version = part, version
-    return _fused_qkv(wq, wk, wv, lp)
+    if getattr(wq, "_lp", None) is None and getattr(wk, "_lp", None) is None and getattr(wv, "_lp", None) is None:
+        ws = (wq, wk, wv)
+        if (len({id(w) for w in ws}) == 3 and len({(w.shape, w.device) for w in ws}) == 1
+                and not (wq.is_cuda and torch.cuda.is_current_stream_capturing())):
+            versions = [w._version for w in ws]
+            with torch.inference_mode(False), torch.no_grad():         # (an inference tensor could not be refreshed outside that mode)
+                parts = torch.cat([w.detach().to(torch.bfloat16) for w in ws], 0).split(wq.shape[0], 0)
+            for w, part, version in zip(ws, parts, versions):
+                w._lp, w._lp_version = part, version
+    return lp(wq), lp(wk), lp(wv)
+
+
+def _shadow_qkv(wq, wk, wv):
+    """The three shadows as one bf16 [3d, d] matrix."""
+    a, b, c = _shadows_qkv(wq, wk, wv)
+    if _adjacent(a, b, c):
+        return torch.as_strided(a, (a.shape[0] * 3, a.shape[1]), (a.shape[1], 1))
+    return torch.cat([a, b, c], 0)
 
 
 def _fused_vec(bq, bk, bv, getter):
@@ -182,11 +190,13 @@ def _block_forward(x, blk, causal):
             or tuple(o.weight.shape) != (d, d) or tuple(f1.weight.shape) != (ff, d) or tuple(f2.weight.shape) != (d, ff)):
         return None
     x = x if x.is_contiguous() else x.contiguous()
-    ws = (_shadow_qkv(q.weight, k.weight, v.weight), lp(o.weight), lp(f1.weight), lp(f2.weight))
+    wqkv = _shadows_qkv(q.weight, k.weight, v.weight)
+    ws = (wqkv[0] if _adjacent(*wqkv) else torch.cat(wqkv, 0), lp(o.weight), lp(f1.weight), lp(f2.weight))
     if x.data_ptr() % 16 or any(w.data_ptr() % 16 or not w.is_contiguous() for w in ws):
         return None
     T, dev, H = B * S, x.device, at.heads
     sms = _num_sms(dev)
+    bn_d = tile_width(T, d, 1, sms)
     adjacent = _adjacent(q.bias, k.bias, v.bias)
     # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse, gathered bias (fp32)
     offs, total = [], 0
@@ -199,7 +209,7 @@ def _block_forward(x, blk, causal):
     g1, be1, g2, be2, bq, bk, bv, bo, b1, b2 = (t.data_ptr() for t in vecs)
     rec = _BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *(w0 + p for p in offs), *(w.data_ptr() for w in ws),
                            g1, be1, g2, be2, bq, bk, bv, bo, b1, b2, B, S, d, ff, H, int(causal), int(not adjacent), K.OPS["add"], sms,
-                           tile_width(T, 3 * d, 1, sms), tile_width(T, d, 1, sms), tile_width(T, ff, 1, sms), tile_width(T, d, 1, sms),
+                           tile_width(T, 3 * d, 1, sms), bn_d, tile_width(T, ff, 1, sms), bn_d,
                            nv.f32(n1.eps), nv.status_ptr(dev))
     launches = C.c_int(0)
     nv.check(nv.cuda().b200_block_fwd(rec, C.byref(launches), nv.stream_ptr()), "block_fwd")
