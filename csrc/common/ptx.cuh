@@ -203,6 +203,12 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t smem_addr, uint32_
   return d;
 }
 
+// MN-major operands of 32-bit elements: 128-byte swizzle in pieces of 32 bytes (CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B); rows of 128 B
+// (32 elements along M/N) per K index, 4-K-row groups `sbo` bytes apart, successive 32-element M/N atoms `lbo` bytes apart.
+__device__ __forceinline__ uint64_t make_sdesc_sw128_b32(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (make_sdesc_sw128(smem_addr, lbo_bytes, sbo_bytes) & ~(static_cast<uint64_t>(7) << 61)) | (static_cast<uint64_t>(1) << 61);
+}
+
 // Cheap descriptor arithmetic for MMA issue loops: all tiles live below 256 KB of shared memory, so the
 // 14-bit address field never carries and a K step is one 32-bit add on the low word. `sdesc_lo` is computed
 // once per operand tile, `sdesc_at(lo, adv_bytes)` yields the descriptor `adv_bytes` further into the tile.
@@ -324,6 +330,30 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }

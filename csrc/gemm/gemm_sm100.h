@@ -12,7 +12,8 @@ enum : int { GEMM_BF16 = 0, GEMM_F32 = 1, GEMM_S8S8 = 2, GEMM_U8S8 = 3, GEMM_E4M
 // Device-visible parameters. Strides are in elements of the respective tensor.
 struct GemmParams {
   int M, N, K, batch;
-  int splits;              // split-K factor; >1 requires OUT_F32_ATOMIC
+  int splits;              // >1: split-K by adding into C, requires OUT_F32_ATOMIC. 0: b200_gemm_launch may divide the contraction over the
+                           // CTAs of a cluster (gemm_cluster_sm100.cu). 1: each sum is formed by one CTA
   void* C; long long ldc, strideC;
   const void* bias; int bias_f32; int bias_vec_ok;   // bias_vec_ok: fp32 bias is 16-byte aligned
   long long strideBias;    // elements between the bias vectors of consecutive batches (0: shared)

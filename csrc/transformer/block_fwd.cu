@@ -24,7 +24,6 @@ struct BlockArgs {
   const void *wqkv, *wo, *w1, *w2;               // bf16, K-major: [3d, d], [d, d], [ff, d], [d, ff]
   const float *g1, *be1, *g2, *be2, *bq, *bk, *bv, *bo, *b1, *b2;
   int B, S, d, ff, heads, causal, bqkv_gather, op_add, num_sms;
-  int bn_qkv, bn_o, bn_1, bn_2;                  // tile widths of the four products
   float eps;
   uint32_t* status;
 };
@@ -37,10 +36,10 @@ __global__ void gather3_kernel(const float* a, const float* b, const float* c, f
   if (i < 3 * n) out[i] = __ldcg(i < n ? a + i : i < 2 * n ? b + (i - n) : c + (i - 2 * n));
 }
 
-static int block_gemm(const BlockArgs& b, const void* A, int M, int K, const void* W, int N, const float* bias, int act, const void* residual, void* C, int bn, cudaStream_t st) {
+static int block_gemm(const BlockArgs& b, const void* A, int M, int K, const void* W, int N, const float* bias, int act, const void* residual, void* C, cudaStream_t st) {
   GemmArgs g = {};
   GemmParams& p = g.p;
-  p.M = g.M = M; p.N = g.N = N; p.K = g.K = K; p.batch = g.batch = 1; p.splits = 1;
+  p.M = g.M = M; p.N = g.N = N; p.K = g.K = K; p.batch = g.batch = 1; p.splits = 0;
   p.C = C; p.ldc = N; p.strideC = (long long)M * N;
   p.bias = bias; p.bias_f32 = 1; p.bias_vec_ok = ((uintptr_t)bias % 16 == 0 && N % 4 == 0) ? 1 : 0;
   p.residual = residual; p.ldr = residual ? N : 0; p.strideR = residual ? (long long)M * N : 0; p.res_vec_ok = residual ? 1 : 0;
@@ -48,7 +47,7 @@ static int block_gemm(const BlockArgs& b, const void* A, int M, int K, const voi
   p.status = b.status;
   g.A = A; g.lda = K; g.strideA = (long long)M * K; g.B = W; g.ldb = K; g.strideB = (long long)N * K;
   g.dtype = GEMM_BF16;
-  return b200_gemm_launch(&g, bn, b.num_sms, st);
+  return b200_gemm_launch(&g, 0, b.num_sms, st);
 }
 
 }  // namespace b200
@@ -66,7 +65,7 @@ extern "C" int b200_block_fwd(const b200::BlockArgs* args, int* launches, cudaSt
     if (e != cudaSuccess) return 400 + (int)e;
     bqkv = b.bqkv; ++n;
   }
-  if (int rc = block_gemm(b, b.h, T, d, b.wqkv, 3 * d, bqkv, ACT_NONE, nullptr, b.qkv, b.bn_qkv, st)) return rc;
+  if (int rc = block_gemm(b, b.h, T, d, b.wqkv, 3 * d, bqkv, ACT_NONE, nullptr, b.qkv, st)) return rc;
   FlashArgs f = {};
   char* qkv = static_cast<char*>(b.qkv);
   AttnTensor* part[3] = {&f.q, &f.k, &f.v};
@@ -75,7 +74,7 @@ extern "C" int b200_block_fwd(const b200::BlockArgs* args, int* launches, cudaSt
   f.lse = b.lse; f.B = b.B; f.H = b.heads; f.Sq = f.Skv = b.S; f.hd = hd;
   f.scale = (float)(1.0 / sqrt((double)hd)); f.causal = b.causal; f.status = b.status;
   if (int rc = b200_flash_fwd(&f, st)) return rc;
-  if (int rc = block_gemm(b, b.o, T, d, b.wo, d, b.bo, ACT_NONE, nullptr, b.h, b.bn_o, st)) return rc;
+  if (int rc = block_gemm(b, b.o, T, d, b.wo, d, b.bo, ACT_NONE, nullptr, b.h, st)) return rc;
   int rc = b200_add_layernorm_fwd(b.h, b.x, b.g2, b.be2, b.y1, b.o, b.mean, b.rstd, T, d, b.eps, st);
   if (rc == -1) {                                            // a width the fused kernel does not take: two kernels
     if ((rc = b200_binary(b.h, b.x, b.y1, (long long)T * d, b.op_add, 0, 1, st))) return rc;
@@ -83,8 +82,8 @@ extern "C" int b200_block_fwd(const b200::BlockArgs* args, int* launches, cudaSt
     ++n;
   }
   if (rc) return rc;
-  if ((rc = block_gemm(b, b.o, T, d, b.w1, b.ff, b.b1, ACT_GELU, nullptr, b.a, b.bn_1, st))) return rc;
-  if ((rc = block_gemm(b, b.a, T, b.ff, b.w2, d, b.b2, ACT_NONE, b.y1, b.y, b.bn_2, st))) return rc;
+  if ((rc = block_gemm(b, b.o, T, d, b.w1, b.ff, b.b1, ACT_GELU, nullptr, b.a, st))) return rc;
+  if ((rc = block_gemm(b, b.a, T, b.ff, b.w2, d, b.b2, ACT_NONE, b.y1, b.y, st))) return rc;
   *launches = n;
   return 0;
 }

@@ -129,9 +129,9 @@ def kernel_matmul(a: torch.Tensor, b: torch.Tensor) -> Tuple[torch.Tensor, GpuBa
 
 def kernel_source(backend: GpuBackendKind) -> str:
     if backend is GpuBackendKind.Nvidia:
-        src = _CSRC / "gemm" / "gemm_sm100.cu"
-        if src.exists():
-            return src.read_text()
+        parts = [_CSRC / "gemm" / f for f in ("gemm_body.cuh", "gemm_sm100.cu")]       # the GEMM body, then the kernels and entry points around it
+        if all(p.exists() for p in parts):
+            return "\n".join(p.read_text() for p in parts)
         return "// gemm_sm100.cu is not shipped with this installation\n"
     return "// No kernel for this platform in this build; the CPU reference path is used.\n"
 

@@ -105,16 +105,19 @@ def _as3d(t: torch.Tensor):
     raise ValueError("gemm operands must be 2-D or 3-D")
 
 
+def _readable(t: torch.Tensor) -> bool:
+    """Can TMA read this 2-D or 3-D operand where it is?"""
+    q = 16 // t.element_size()
+    return (t.stride(-1) == 1 and t.stride(-2) % q == 0 and t.data_ptr() % 16 == 0 and t.stride(-2) >= t.shape[-1]
+            and (t.dim() == 2 or t.shape[0] == 1 or t.stride(0) % q == 0))
+
+
 def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     """Return `t` (3-D view) or a padded copy such that TMA constraints hold:
     innermost stride 1, other strides multiples of 16 bytes, base 16-byte aligned."""
-    es = t.element_size()
-    q = 16 // es
-    ok = t.stride(-1) == 1 and t.stride(-2) % q == 0 and t.data_ptr() % 16 == 0 and t.stride(-2) >= t.shape[-1]
-    if ok and t.shape[0] > 1:
-        ok = t.stride(0) % q == 0
-    if ok:
+    if _readable(t):
         return t
+    q = 16 // t.element_size()
     inner = (t.shape[-1] + q - 1) // q * q
     buf = torch.zeros(t.shape[0], t.shape[1], inner, dtype=t.dtype, device=t.device)
     buf[..., : t.shape[-1]].copy_(t)
@@ -136,13 +139,6 @@ def _operand(t: torch.Tensor):
 _KINDS = {(torch.bfloat16, torch.bfloat16): GEMM_BF16, (torch.float32, torch.float32): GEMM_F32,
           (torch.int8, torch.int8): GEMM_S8S8, (torch.uint8, torch.int8): GEMM_U8S8,
           (torch.float8_e4m3fn, torch.float8_e4m3fn): GEMM_E4M3}
-
-
-def tile_width(M: int, N: int, batch: int, sms: int) -> int:
-    """Columns of a bf16 product's tiles: 256 once such tiles fill the machine."""
-    if N <= 128:
-        return 64 if N <= 64 else 128
-    return 256 if -(-M // 128) * -(-N // 256) * batch >= sms else 128
 
 
 @nv.traced("gemm")
@@ -180,11 +176,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if lowp and (a_mn or b_mn):
         raise ValueError("8-bit GEMM operands must be K-major")
     if is_f32 and (a_mn or b_mn):
-        # TF32 tiles are K-major only; 32-bit MN-major operands are transposed by a kernel first
+        # a transposed fp32 operand that TMA cannot read in place (rows of other than 4 n elements) is transposed by a kernel: one
+        # launch, where padding its rows would take two
         from .kernels import transpose_last2
-        if a_mn:
+        if a_mn and not _readable(a):
             a, a_mn = transpose_last2(a), False
-        if b_mn:
+        if b_mn and not _readable(b):
             b, b_mn = transpose_last2(b), False
     squeeze = a.dim() == 2
     a3, batch, ar, ac, lda, stride_a = _operand(a)
@@ -196,6 +193,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if K != Kb:
         raise ValueError(f"gemm K mismatch: {K} vs {Kb}")
     dev = a.device
+    may_divide = False
     if accumulate_into is not None:
         out = accumulate_into
         if out.dtype != torch.float32 or not out.is_contiguous():
@@ -215,32 +213,35 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                 raise ValueError("`out` must have the result's dtype, size and a unit inner stride")
             if splits > 1:
                 raise ValueError("`out` and split-K do not go together (split-K accumulates into a zeroed fp32 buffer)")
-            splits = splits or 1
-    # tile width and split-K
+            may_divide = splits == 0
+            splits = 1
+    # The launcher chooses the tiles (bn = 0) and may divide a sum over the CTAs of a cluster (0 splits). Here: into how many
+    # parts that are added in memory an fp32 result's contraction is split, on the tiles that go with it.
     sms = _num_sms(dev)
-    if is_f32:
-        bn = 128
-    elif lowp:
-        bn = 256 if (bn == 256 or (bn == 0 and math.ceil(M / 128) * math.ceil(N / 256) * batch >= sms)) else 128
-    elif bn == 0:
-        bn = tile_width(M, N, batch, sms)
-        if N > 128:
-            t256 = math.ceil(M / 128) * math.ceil(N / 256) * batch
-            # Few tiles and a long K (weight gradients): split-K fills the machine either way, and the wider tile moves
-            # a third less operand traffic from L2 per FLOP (measured 167 -> 113 us on 2048 x 512 x 65536).
-            splittable = (splits == 0 and out_mode in (OUT_F32, OUT_F32_ATOMIC) and act == "none" and aux_in is None and not want_aux
-                          and N >= 256 and K >= 16 * 64 * max(1, sms // max(t256, 1)))
-            bn = 256 if splittable else bn
-    bk = 32 if is_f32 else 128 if lowp else 64
-    num_kb = max(1, math.ceil(K / bk))
-    tiles = math.ceil(M / 128) * math.ceil(N / bn) * batch
+    one_cta = _prepare or splits == 1 and not may_divide
     if splits == 0:
         splits = 1
-        if out_mode in (OUT_F32, OUT_F32_ATOMIC) and tiles < sms // 2 and num_kb >= 16 and act == "none" and aux_in is None and not want_aux:
-            splits = max(1, min(sms // tiles, num_kb // 8))
+        num_kb = -(-K // (32 if is_f32 else 128 if lowp else 64))
+        if out_mode in (OUT_F32, OUT_F32_ATOMIC) and num_kb >= (64 if lowp else 16) and act == "none" and aux_in is None and not want_aux:
+            row_tiles = -(-M // 128) * batch
+            t256 = row_tiles * -(-N // 256)
+            # Few tiles and a long K (weight gradients): split-K fills the machine either way, and the wider tile moves
+            # a third less operand traffic from L2 per FLOP (measured 167 -> 113 us on 2048 x 512 x 65536).
+            if bn:
+                sbn = bn
+            elif not is_f32 and not lowp and N >= 256 and (t256 >= sms or K >= 16 * 64 * max(1, sms // t256)):
+                sbn = 256
+            else:
+                sbn = 64 if N <= 64 and not is_f32 and not lowp else 128
+            tiles = row_tiles * -(-N // sbn)
+            if tiles < sms // 2:
+                splits = max(1, min(sms // tiles, num_kb // 8))
+            if splits > 1 or sbn == 256:
+                bn = sbn
     if splits > 1:
-        per = math.ceil(num_kb / splits)
-        splits = math.ceil(num_kb / per)
+        num_kb = -(-K // (32 if is_f32 else 128 if lowp else 64))
+        per = -(-num_kb // splits)
+        splits = -(-num_kb // per)
     if splits > 1:
         if out_mode == OUT_BF16 or act != "none" or aux_in is not None or want_aux:
             raise ValueError("split-K needs an fp32 output and a linear epilogue")
@@ -298,7 +299,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     vec_ok = int(ldc * es_out % 16 == 0 and out_ptr % 16 == 0 and (batch == 1 or stride_c * es_out % 16 == 0)
                  and ((aux is None and aux_in is None) or N % 8 == 0))
     rec = nv.GEMM_PACK.pack(
-        M, N, K, batch, splits, out_ptr, ldc, stride_c, bias_ptr, bias_f32, bias_vec_ok, bias_stride, res_ptr, ldr, stride_r,
+        M, N, K, batch, splits if one_cta or splits > 1 else 0, out_ptr, ldc, stride_c, bias_ptr, bias_f32, bias_vec_ok, bias_stride, res_ptr, ldr, stride_r,
         nv.ptr(aux), nv.ptr(aux_in), nv.f32(alpha), nv.ptr(alpha_t), ACT[act], ACT[dact], out_mode, vec_ok, res_vec_ok,
         nv.ptr(row_scale), nv.ptr(col_scale), nv.status_ptr(dev), nv.ptr(m_valid), nv.ptr(k_valid),
         a3.data_ptr(), lda, stride_a, int(a_mn), b3.data_ptr(), ldb, stride_b, int(b_mn), M, N, K, batch, kind)

@@ -22,7 +22,7 @@ from torch.autograd import Function
 from .. import _native as nv
 from . import kernels as K
 from .functional import _bgrad, _scale_by, _wgrad, lp
-from .gemm import _num_sms, gemm, tile_width
+from .gemm import _num_sms, gemm
 
 
 def _adjacent(a, b, c):
@@ -171,7 +171,7 @@ class TransformerBlockFn(Function):
 
 
 nv.register_sigs({"b200_block_fwd": [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]})
-_BLOCK_PACK = struct.Struct("@25P13ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
+_BLOCK_PACK = struct.Struct("@25P9ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
 
 
 def _plain(*ts) -> bool:
@@ -196,7 +196,6 @@ def _block_forward(x, blk, causal):
         return None
     T, dev, H = B * S, x.device, at.heads
     sms = _num_sms(dev)
-    bn_d = tile_width(T, d, 1, sms)
     adjacent = _adjacent(q.bias, k.bias, v.bias)
     # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse, gathered bias (fp32)
     offs, total = [], 0
@@ -209,7 +208,6 @@ def _block_forward(x, blk, causal):
     g1, be1, g2, be2, bq, bk, bv, bo, b1, b2 = (t.data_ptr() for t in vecs)
     rec = _BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *(w0 + p for p in offs), *(w.data_ptr() for w in ws),
                            g1, be1, g2, be2, bq, bk, bv, bo, b1, b2, B, S, d, ff, H, int(causal), int(not adjacent), K.OPS["add"], sms,
-                           tile_width(T, 3 * d, 1, sms), bn_d, tile_width(T, ff, 1, sms), bn_d,
                            nv.f32(n1.eps), nv.status_ptr(dev))
     launches = C.c_int(0)
     nv.check(nv.cuda().b200_block_fwd(rec, C.byref(launches), nv.stream_ptr()), "block_fwd")

@@ -57,3 +57,9 @@ def test_shared_arrays_read_as_vectors_are_declared_aligned(path):
             continue
         for name in re.findall(r"(\w+)\s*\[", names):
             assert not re.search(r"reinterpret_cast<(?:const )?(?:float|uint|int)[24]\s*\*>\(\s*&?\s*%s\b" % name, code), (path.name, name)
+
+
+@pytest.mark.parametrize("path", [p for p in sorted(CSRC.rglob("*.cuh")) if "pdl_wait()" in p.read_text() and p.name != "launch.cuh"], ids=lambda p: p.name)
+def test_kernel_headers_stay_off_the_read_only_path(path):
+    code = _code(path)
+    assert "__ldg(" not in code and not re.search(r"const\s+\w+\s*\*\s*__restrict__", code)
