@@ -14,6 +14,10 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include "../common/launch.cuh"
+
+using b200::pdl_trigger;
+using b200::pdl_wait;
 
 namespace {
 
@@ -23,6 +27,18 @@ template <> __device__ __forceinline__ float ldf<__nv_bfloat16>(const __nv_bfloa
 template <typename T> __device__ __forceinline__ void stf(T* p, long long i, float v);
 template <> __device__ __forceinline__ void stf<float>(float* p, long long i, float v) { p[i] = v; }
 template <> __device__ __forceinline__ void stf<__nv_bfloat16>(__nv_bfloat16* p, long long i, float v) { p[i] = __float2bfloat16(v); }
+
+// eight neighbouring elements from 16-byte aligned memory
+__device__ __forceinline__ void load8(const float* p, float* v) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float* v) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
 
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
@@ -49,26 +65,78 @@ __device__ __forceinline__ float block_reduce(float v, float* sh) {
 
 // ------------------------------------------------------------------ per-row int8 / e4m3
 // mode 0: int8, scale = absmax/127 (1 when the row is zero); mode 1: e4m3, scale = absmax/448.
-template <typename T>
-__global__ void quant_rows_kernel(const T* __restrict__ x, long long ldx, int cols, uint8_t* __restrict__ q, long long ldq,
-                                  float* __restrict__ scales, int mode) {
+// `inv` ~ 1 / scale. An int8 code is the product's nearest integer wherever that cannot differ from the quotient's: away from halves, the two are
+// 127 * 2^-22 apart at most. (A quotient is 10 instructions: 4096 x 4096 20.3 us with one per element, 18.3 without.)
+__device__ __forceinline__ uint32_t row_code(float x, float scale, float inv, int mode) {
+  if (mode == 0) {
+    const float t = x * inv;
+    if (fabsf(fabsf(t - truncf(t)) - 0.5f) > 1e-4f) return (uint8_t)(int8_t)__float2int_rn(t);      // false for NaN and infinity
+  }
+  const float v = x / scale;
+  if (mode == 0) return (uint8_t)(int8_t)fminf(fmaxf(roundf(v), -128.f), 127.f);
+  return (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+}
+// One block per row. VEC: rows and codes lie on 16 and 8 bytes and the width is a multiple of 8: a row is read once, 16 bytes a load, and
+// kept in registers between the maximum and the codes (MAXV pieces a thread; longer rows are read again). Bound by memory for many rows, by the
+// latency of load - reduction - store for few: 4096 x 4096 bf16 33 -> 18 us, 16 x 4096 6.1 -> 2.4 (element by element before).
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256)
+quant_rows_kernel(const T* x, long long ldx, int cols, uint8_t* q, long long ldq, float* scales, int mode) {
   __shared__ float sh[32];
+  pdl_trigger();
+  pdl_wait();
   const long long r = blockIdx.x;
   const T* xr = x + r * ldx;
-  float m = 0.f;
-  for (int j = threadIdx.x; j < cols; j += blockDim.x) m = fmaxf(m, fabsf(ldf(xr, j)));
-  m = block_reduce<true>(m, sh);
-  const float qmax = mode == 0 ? 127.f : 448.f;
-  const float scale = m > 0.f ? m / qmax : 1.f;
-  if (threadIdx.x == 0) scales[r] = scale;
   uint8_t* qr = q + r * ldq;
-  for (int j = threadIdx.x; j < cols; j += blockDim.x) {
-    const float v = ldf(xr, j) / scale;
-    if (mode == 0) {
-      qr[j] = (uint8_t)(int8_t)fminf(fmaxf(roundf(v), -128.f), 127.f);
-    } else {
-      qr[j] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+  const float qmax = mode == 0 ? 127.f : 448.f;
+  float m = 0.f;
+  if constexpr (VEC) {
+    constexpr int MAXV = 4;
+    const int n8 = cols >> 3, step = blockDim.x;
+    float v[MAXV][8];
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      const int j = threadIdx.x + k * step;
+      if (j < n8) load8(xr + 8 * j, v[k]);
+      else { for (int i = 0; i < 8; ++i) v[k][i] = 0.f; }
     }
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[k][i]));
+    for (int j = threadIdx.x + MAXV * step; j < n8; j += step) {
+      float w[8];
+      load8(xr + 8 * j, w);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(w[i]));
+    }
+    m = block_reduce<true>(m, sh);
+    const float scale = m > 0.f ? m / qmax : 1.f;
+    const float inv = 1.f / scale;
+    if (threadIdx.x == 0) scales[r] = scale;
+    auto put = [&](int j, const float* w) {
+      uint32_t c[2] = {0u, 0u};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i >> 2] |= row_code(w[i], scale, inv, mode) << (8 * (i & 3));
+      *reinterpret_cast<uint2*>(qr + 8 * j) = make_uint2(c[0], c[1]);
+    };
+#pragma unroll
+    for (int k = 0; k < MAXV; ++k) {
+      const int j = threadIdx.x + k * step;
+      if (j < n8) put(j, v[k]);
+    }
+    for (int j = threadIdx.x + MAXV * step; j < n8; j += step) {
+      float w[8];
+      load8(xr + 8 * j, w);
+      put(j, w);
+    }
+  } else {
+    for (int j = threadIdx.x; j < cols; j += blockDim.x) m = fmaxf(m, fabsf(ldf(xr, j)));
+    m = block_reduce<true>(m, sh);
+    const float scale = m > 0.f ? m / qmax : 1.f;
+    const float inv = 1.f / scale;
+    if (threadIdx.x == 0) scales[r] = scale;
+    for (int j = threadIdx.x; j < cols; j += blockDim.x) qr[j] = (uint8_t)row_code(ldf(xr, j), scale, inv, mode);
   }
 }
 
@@ -278,9 +346,9 @@ __global__ void csr_spmm_kernel(const float* __restrict__ vals, const int* __res
   float acc = 0.f;
   const int e0 = row_ptr[r], e1 = row_ptr[r + 1];
   for (int e = e0; e < e1; ++e) {
-    const float v = __ldg(vals + e);
-    const int c = __ldg(col_idx + e);
-    if (j < n) acc += v * __ldg(B + (long long)c * n + j);
+    const float v = vals[e];
+    const int c = col_idx[e];
+    if (j < n) acc += v * B[(long long)c * n + j];
   }
   if (j < n) C[(long long)r * n + j] = acc;
 }
@@ -294,10 +362,14 @@ extern "C" {
 int b200_quant_rows(const void* x, int is_bf16, long long rows, int cols, long long ldx, void* q, long long ldq, float* scales,
                     int mode, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return 0;
-  const int threads = cols >= 1024 ? 256 : 128;
-  if (is_bf16) quant_rows_kernel<__nv_bfloat16><<<(unsigned)rows, threads, 0, st>>>((const __nv_bfloat16*)x, ldx, cols, (uint8_t*)q, ldq, scales, mode);
-  else quant_rows_kernel<float><<<(unsigned)rows, threads, 0, st>>>((const float*)x, ldx, cols, (uint8_t*)q, ldq, scales, mode);
-  return (int)cudaGetLastError();
+  const int es = is_bf16 ? 2 : 4;
+  const bool vec = cols % 8 == 0 && ldx * es % 16 == 0 && ldq % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)q & 7) == 0;
+  const int threads = vec ? (cols >= 2048 ? 256 : 128) : cols >= 1024 ? 256 : 128;
+  auto go = [&](auto kernel, auto* p) { return b200::launch_pdl(kernel, dim3((unsigned)rows), dim3(threads), 0, st, p, ldx, cols, (uint8_t*)q, ldq, scales, mode); };
+  cudaError_t e;
+  if (is_bf16) e = vec ? go(quant_rows_kernel<__nv_bfloat16, true>, (const __nv_bfloat16*)x) : go(quant_rows_kernel<__nv_bfloat16, false>, (const __nv_bfloat16*)x);
+  else e = vec ? go(quant_rows_kernel<float, true>, (const float*)x) : go(quant_rows_kernel<float, false>, (const float*)x);
+  return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }
 
 // absmax: [groups] uint32 scratch, zeroed by this call

@@ -30,7 +30,7 @@ _E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
 class MxGemmArgs(C.Structure):
     _fields_ = [("A", C.c_void_p), ("B", C.c_void_p), ("sfa", C.c_void_p), ("sfb", C.c_void_p), ("C", C.c_void_p), ("ldc", C.c_longlong),
                 ("M", C.c_int), ("N", C.c_int), ("K", C.c_int), ("out_f32", C.c_int), ("alpha", C.c_float), ("kind", C.c_int),
-                ("status", C.c_void_p)]
+                ("bias", C.c_void_p), ("status", C.c_void_p)]
 
 
 nv.register_sigs({
@@ -124,7 +124,7 @@ def quantize_mx(x: torch.Tensor, kind: str = "mxfp8", tensor_scale: float | None
     if x.stride(1) != 1:
         x = x.contiguous()
     data = torch.empty((rows, K if k == 0 else K // 2), dtype=torch.uint8, device=x.device)
-    sf = torch.zeros(_sf_bytes(rows, K, k), dtype=torch.uint8, device=x.device)
+    sf = torch.empty(_sf_bytes(rows, K, k), dtype=torch.uint8, device=x.device)
     nv.check(nv.cuda().b200_mx_quant(x.data_ptr(), int(x.dtype == torch.bfloat16), x.stride(0), rows, K, k, ts, data.data_ptr(),
                                      sf.data_ptr(), nv.stream_ptr()), "mx_quant")
     nv.count_launch()
@@ -154,12 +154,13 @@ def dequantize_mx(t: MxTensor) -> torch.Tensor:
 
 
 @nv.traced("gemm_mx")
-def gemm_mx(a: MxTensor, b: MxTensor, out_dtype=torch.bfloat16) -> torch.Tensor:
-    """a [M, K] x b [N, K] -> [M, N] = a @ b.T, scale factors applied by the tensor core, fp32 accumulation."""
+def gemm_mx(a: MxTensor, b: MxTensor, out_dtype=torch.bfloat16, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """a [M, K] x b [N, K] -> [M, N] = a @ b.T (+ bias), scale factors applied by the tensor core, fp32 accumulation. ``bias``: [N] bf16."""
     if a.kind != b.kind or a.K != b.K:
         raise ValueError("operands must share the format and K")
     if not a.data.is_cuda:
-        return (dequantize_mx(a) @ dequantize_mx(b).t()).to(out_dtype)
+        y = dequantize_mx(a) @ dequantize_mx(b).t()
+        return (y if bias is None else y + bias.float()).to(out_dtype)
     if b.rows % 8 != 0:
         raise ValueError("N must be a multiple of 8")
     from .gemm import _num_sms
@@ -171,6 +172,12 @@ def gemm_mx(a: MxTensor, b: MxTensor, out_dtype=torch.bfloat16) -> torch.Tensor:
     g.out_f32 = int(out_dtype == torch.float32)
     g.alpha = float(a.tensor_scale * b.tensor_scale)
     g.kind = a.kind
+    if bias is not None:
+        if bias.dtype != torch.bfloat16 or bias.shape != (b.rows,):
+            raise ValueError("bias must be a bf16 vector of N elements")
+        if not bias.is_contiguous() or bias.data_ptr() % 16:
+            bias = bias.clone(memory_format=torch.contiguous_format)
+        g.bias = bias.data_ptr()
     g.status = nv.status_word(a.data.device).data_ptr()
     nv.check(nv.cuda().b200_gemm_mx(C.byref(g), _num_sms(a.data.device), nv.stream_ptr()), "gemm_mx")
     nv.count_launch()
@@ -191,9 +198,7 @@ class MxLinear:
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         lead = x.shape[:-1]
         xq = quantize_mx(x.reshape(-1, self.in_features), self.kind)
-        y = gemm_mx(xq, self.weight, torch.bfloat16)
-        if self.bias is not None:
-            y = y + self.bias
+        y = gemm_mx(xq, self.weight, torch.bfloat16, self.bias)
         return y.reshape(*lead, self.out_features)
 
     __call__ = forward

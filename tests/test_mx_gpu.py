@@ -76,3 +76,28 @@ def test_quantized_linear_nvfp4_tensor_core_path():
     assert _rel(ys, ref) < 0.15 and _rel(yh, ref) < 0.2          # the second also quantises the activations to 4 bits
     with pytest.raises(ValueError):
         QuantizedLinear.from_linear(nn.Linear(100, 8).to_device("cuda", torch.float32), QuantFormat.NVFP4, 16, tensor_core=True)
+
+
+@pytest.mark.parametrize("kind", ["mxfp8", "nvfp4"])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (7, 136, 512), (130, 256, 256), (256, 4096, 256), (2100, 1032, 256)])
+def test_narrow_tiles_short_row_blocks_and_bias(kind, M, N, K):
+    """128- and 256-wide tiles, fewer rows than a tile has, column tiles past the end; the bias is added before the result is rounded."""
+    from rust_neural_network_b200.ops import mx
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = mx.quantize_mx(torch.randn(M, K, device="cuda", generator=g), kind), mx.quantize_mx(torch.randn(N, K, device="cuda", generator=g), kind)
+    bias = torch.randn(N, device="cuda", generator=g).bfloat16()
+    want = mx.dequantize_mx(a).double() @ mx.dequantize_mx(b).double().t()
+    assert _rel(mx.gemm_mx(a, b, torch.float32), want) < 1e-4
+    got = mx.gemm_mx(a, b, bias=bias)
+    assert _rel(got, want + bias.double()) < 2.0 ** -8           # half a unit of bf16's 2^-8 per element at most
+    odd = torch.cat([bias, bias])[3:3 + N] if N % 8 else torch.cat([bias[:1], bias])[1:]       # an address off 16 bytes
+    assert _rel(mx.gemm_mx(a, b, torch.float32, bias=odd), want + odd.double()) < 1e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_quantiser_reads_rows_off_16_bytes(dtype):
+    from rust_neural_network_b200.ops import mx
+    base = torch.randn(37, 261, device="cuda").to(dtype)
+    view = base[:, 1:257]
+    a, b = mx.quantize_mx(view), mx.quantize_mx(view.contiguous())
+    assert torch.equal(a.data, b.data) and torch.equal(a.sf, b.sf)

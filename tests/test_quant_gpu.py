@@ -145,3 +145,32 @@ def test_int8_linear_and_quantized_model_gpu():
     a = torch.randint(0, 256, (64, 128), dtype=torch.int32).to(torch.uint8).to(DEV)
     b = torch.randint(-128, 128, (128, 48), dtype=torch.int32).to(torch.int8).to(DEV)
     assert torch.equal(int8.igemm(a, b, 64, 128, 48).cpu(), int8.igemm_scalar(a, b, 64, 128, 48))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode", ["int8", "e4m3"])
+@pytest.mark.parametrize("rows,cols,ld,off", [(3, 8, 8, 0), (5, 2040, 2040, 0), (2, 8200, 8200, 0), (4, 20000, 20000, 0), (3, 100, 104, 0), (3, 96, 100, 0), (3, 64, 80, 1), (2, 7, 7, 0)])
+def test_quant_rows_in_pieces_and_element_by_element(dtype, mode, rows, cols, ld, off):
+    """Rows of 16-byte pieces (some longer than a block keeps in registers), rows that are not, halves exactly between two codes, a row of zeros,
+    one with an infinity and one with subnormal values: the codes of the element-by-element expression."""
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = torch.randn(rows, ld + off, device="cuda", generator=g).to(dtype)[:, off:off + cols]
+    x[0] = torch.randint(-254, 255, (cols,), device="cuda", generator=g).to(dtype) / 2          # quotients near halves of 1 / 127 of the maximum
+    x[0, 0] = 127.0
+    x[1] = 0
+    if rows > 2: x[2, :3] = torch.tensor([1e-39, -3e-39, 0.0], device="cuda").to(dtype)
+    if rows > 3: x[3, 1] = float("inf")
+    q, s = Q.quant_rows(x, mode)
+    xf = x.float()
+    m = xf.abs().amax(-1)
+    qmax = 127.0 if mode == "int8" else 448.0
+    scale = torch.where(m > 0, m / torch.full_like(m, qmax), torch.ones_like(m))      # (torch divides by a number through its reciprocal)
+    assert torch.equal(s, scale)
+    t = xf / scale[:, None]
+    fin = torch.isfinite(t) & torch.isfinite(scale)[:, None]
+    if mode == "int8":
+        want = torch.where(t >= 0, torch.floor(t.double() + 0.5), torch.ceil(t.double() - 0.5)).clamp(-128, 127)
+        assert torch.equal(q.double()[fin], want[fin])
+    else:
+        fin &= (xf == 0) | (xf.abs() > 1e-30)
+        assert torch.equal(q.view(torch.uint8)[fin], t.clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)[fin])
