@@ -25,60 +25,22 @@
 // No state is ever stored per token or per chunk: both backward kernels recompute what they need from Q, K, V, dO, O
 // and the saved denominators.
 //
+// What bounds the kernels is the chain of steps in a chunk (features, products, mask, products, results), two CTAs per SM at head size 64 and one at
+// 128, not the tensor core (a fifth busy) or memory (half busy). So products that need no features (G V^T, G S^T, V dS^T) are issued before
+// the features are formed, the forward forms a chunk's features while the products of the chunk before it run, and a warp reads and
+// converts only the 32 x 32 blocks of a masked tile that it keeps. 8 x 16 x 16384 x 64 forward + backward 2272 -> 1989 us (ELU + 1),
+// 2258 -> 1749 (ReLU^2, whose features cost less); 4 x 16 x 4096 x 128 765 -> 725 and 756 -> 632 us.
+//
 // `s_in` / `s_out` (optional) are the state before the first token and after the last one; a sequence-parallel rank
 // passes the sum of the lower ranks' states in and hands its own total out. Every wait is bounded (status word).
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
-#include "flash_sm100.h"
+#include "linattn_sm100.h"
 
 namespace b200 {
 
 constexpr int LA_C = 128;                    // tokens per chunk = rows of every product = TMEM lanes
 constexpr uint32_t LA_X_LBO = LA_C * 128;    // distance of a tile's 64-column atoms
-
-// Sequence-parallel exchange of the slice totals, done by the attention kernels themselves over NVLink peer memory.
-// The state pass of a rank (role 1) writes its total into its OWN symmetric buffer and then raises one flag per
-// (consumer rank, batch x head); the main pass (role 2) of a consumer waits for the flags of the ranks it depends on,
-// pulls their totals with plain peer loads in rank order (so every run sums in the same order), keeps the sum in
-// `prefix` and acknowledges. A total is double-buffered by call parity and is only overwritten once every consumer has
-// acknowledged the call two earlier. The call counter is a device word that the last CTA of the main pass advances,
-// so a captured graph replays with fresh epochs. All waits are bounded.
-constexpr int LA_MAX_WORLD = 8;
-struct LaExchange {
-  float* state[LA_MAX_WORLD];       // every rank's totals [2][B*H][hd*hd + hd] fp32 (peer-mapped)
-  uint32_t* flags[LA_MAX_WORLD];    // every rank's arrival flags [world][B*H] (peer-mapped): flags[c][r * BH + bh] = epoch
-  uint32_t* acks[LA_MAX_WORLD];     // every rank's release flags [world][B*H] (peer-mapped): acks[r][c * BH + bh] = epoch
-  float* prefix;                    // local [B*H][hd*hd + hd]: the sum the main pass started from (the backward needs it again)
-  uint32_t* words;                  // local: [0] calls so far, [1] retired CTAs of the main pass
-  long long wait_cycles;
-  int rank, world;                  // world <= 1: no exchange
-  int dir;                          // 0: sum over the LOWER ranks (forward states), 1: over the HIGHER ranks (backward)
-  int role;                         // 0: none, 1: publish this slice's total, 2: consume
-};
-
-struct LinAttnArgs {
-  AttnTensor q, k, v, o;                     // bf16 [B, S, H, hd] (any strides, hd contiguous)
-  AttnTensor dout, dq, dk, dv;               // backward
-  AttnTensor g;                              // backward scratch, bf16: G = dO / D (written by the G pass, read by both gradient kernels)
-  AttnTensor o_lo;                           // optional bf16 remainder O - bf16(O): written by forward, read by backward.
-                                             // dden = -(dO . O) / D is one half of a difference of nearly equal terms
-                                             // (S^T G against (G . O) z); 8 mantissa bits of O are not enough for it
-  float* den;                                // [B, H, S] fp32: denominators incl. eps (written by forward, read by backward)
-  float* dden;                               // backward scratch, [B, H, S] fp32: -(G . O)
-  const float* s_in;                         // optional [B*H][hd*hd + hd] fp32: state (row-major [d_k][d_v]) then z
-  float* s_out;                              // optional, same layout: state after the last token (forward / state pass)
-  const float* ds_in;                        // backward 2, optional: dS, dz flowing in from the tokens after this slice
-  float* ds_out;                             // backward 2, optional: dS, dz at the first token (for the slices before it)
-  int B, H, S, hd;
-  float scale, eps;
-  int kind;                                  // 0: ELU + 1, 1: ReLU^2
-  int state_only;                            // forward: only accumulate the state (reads K, V; writes s_out)
-  uint32_t* status;
-  float* seg;                                // n_seg > 1: [B*H][n_seg][hd*hd + hd] fp32 workspace for the states between segments
-  int n_seg, seg_chunks;                     // the sequence is walked as n_seg segments of seg_chunks chunks by as many CTAs
-  float* dseg;                               // whole backward, n_seg > 1: the workspace of dK / dV (`seg` holds the forward's states)
-  LaExchange sx;
-};
 
 __device__ __forceinline__ bool la_wait_flag(const uint32_t* f, uint32_t want, long long budget, uint32_t* status) {
   const long long t0 = clock64();
@@ -152,16 +114,27 @@ __device__ __forceinline__ void la_retire(const LinAttnArgs& p, uint32_t epoch) 
   if (atomicAdd(x.words + 1, 1u) == gridDim.x - 1) { x.words[1] = 0u; __threadfence(); x.words[0] = epoch; }
 }
 
-// Both sides of a feature map are computed and one is selected: as a branch per element, the exponentials of one tile took
-// 2550 cycles. (An overflowing exponential is never the selected side; a NaN is.)
+// The feature maps (KIND 0: ELU + 1, 1: ReLU^2) on pairs. Both sides of ELU + 1 are computed and one is selected: as a branch per element, the
+// exponentials of one tile took 2550 cycles. (An overflowing exponential is never the selected side; a NaN is.)
 __device__ __forceinline__ float la_exp(float x) { return ex2_approx(x * 1.4426950408889634f); }
-__device__ __forceinline__ float la_phi(float x, int kind) {
-  const float e = la_exp(x), p = x + 1.f, q = x * x;
-  return x > 0.f ? (kind == 0 ? p : q) : (kind == 0 ? e : 0.f);
+template <int KIND>
+__device__ __forceinline__ void la_phi2(float& x, float& y, float scale) {
+  mul2(x, y, scale, scale);
+  if constexpr (KIND == 0) {
+    float ex = x, ey = y, px = x, py = y;
+    mul2(ex, ey, 1.4426950408889634f, 1.4426950408889634f);
+    add2(px, py, 1.f, 1.f);
+    ex = ex2_approx(ex); ey = ex2_approx(ey);
+    x = x > 0.f ? px : ex; y = y > 0.f ? py : ey;
+  } else {
+    x = fmaxf(x, 0.f); y = fmaxf(y, 0.f);                 // (0 for a NaN)
+    mul2(x, y, x, y);
+  }
 }
-__device__ __forceinline__ float la_dphi(float x, int kind) {
-  const float e = la_exp(x), q = 2.f * x;
-  return x > 0.f ? (kind == 0 ? 1.f : q) : (kind == 0 ? e : 0.f);
+template <int KIND>
+__device__ __forceinline__ float la_dphi(float x) {
+  if constexpr (KIND == 0) { const float e = la_exp(x); return x > 0.f ? 1.f : e; }
+  else return x > 0.f ? 2.f * x : 0.f;
 }
 // One fp32 row of HD values -> bf16 "value" tile and bf16 "remainder" tile (row = thread), [rows][HD] swizzled atoms
 // of `rows` rows each.
@@ -262,8 +235,8 @@ struct LaSmem {
 constexpr int LA_FWD_THREADS = 256;
 
 // phi(scale * x) in place on this thread's half of its row (4 of the 8 16-byte chunks of every 64-column atom)
-template <int HD>
-__device__ __forceinline__ void la_phi_half(uint8_t* tile, int row, int hf, int valid, float scale, int kind) {
+template <int HD, int KIND>
+__device__ __forceinline__ void la_phi_half(uint8_t* tile, int row, int hf, int valid, float scale) {
 #pragma unroll
   for (int a = 0; a < HD / 64; ++a)
 #pragma unroll
@@ -274,8 +247,9 @@ __device__ __forceinline__ void la_phi_half(uint8_t* tile, int row, int hf, int 
       uint32_t* w = &u.x;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16x2(w[j]);
-        w[j] = row < valid ? pack_bf16x2(la_phi(f.x * scale, kind), la_phi(f.y * scale, kind)) : 0u;
+        float2 f = unpack_bf16x2(w[j]);
+        la_phi2<KIND>(f.x, f.y, scale);
+        w[j] = row < valid ? pack_bf16x2(f.x, f.y) : 0u;
       }
       *p = u;
     }
@@ -297,20 +271,46 @@ __device__ __forceinline__ float la_dot_half(const uint8_t* tile, int row, int h
     }
   return acc0 + acc1;
 }
-// 64 fp32 values = columns 64 hf .. of this thread's row of a masked [128][128] tile -> A operand in TMEM, over the fp32
-// columns they were read from (`col` = 64 hf of the tile): the bf16 values in the first 32, the rounding remainders in the
-// next 32. The masked tile enters its product as value + remainder like the state does where the result is a difference
-// of nearly equal sums (one bf16 copy costs dQ ~2 %).
-__device__ __forceinline__ void la_put_half128(uint32_t col, const float* v, bool with_lo) {
-  uint32_t h[32], l[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    h[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-    const float2 r = unpack_bf16x2(h[i]);
-    l[i] = pack_bf16x2(v[2 * i] - r.x, v[2 * i + 1] - r.y);
+// Columns 64 hf .. of this thread's row of a [128][128] fp32 tile in TMEM, masked, -> A operand over the same columns (`col` = 64 hf of the tile):
+// the bf16 values in the first 32, the rounding remainders (REM) in the next 32. The masked tile enters its product as value + remainder like
+// the state does where the result is a difference of nearly equal sums (one bf16 copy costs dQ ~2 %). A warp's 32 rows meet a 32-column
+// block wholly kept, wholly dropped (not even read) or on the diagonal: LOWER keeps columns <= row, else columns >= row. `f(i, x)` gives the
+// value that column 64 hf + i, which held x, enters with; `g` is given the pairs that are kept.
+template <bool LOWER, bool REM, typename F, typename G>
+__device__ __forceinline__ void la_mask_put(uint32_t col, int quad, int hf, int lane, F f, G g) {
+  const int d0 = LOWER ? 2 * hf - quad : quad - 2 * hf, d1 = LOWER ? d0 + 1 : d0 - 1;       // < 0 kept, 0 diagonal, > 0 dropped
+  // The remainders of the first block lie over the second: both are read first. Without remainders one after the other, in half the registers
+  uint32_t v[REM ? 64 : 32];
+  if constexpr (REM) {
+    if (d0 <= 0) tmem_ld_x32(col, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+    if (d1 <= 0) tmem_ld_x32(col + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+    tmem_ld_wait();
   }
-  tmem_st_x32(col, h);
-  if (with_lo) tmem_st_x32(col + 32, l);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int d = k == 0 ? d0 : d1;
+    uint32_t h[16], l[16];
+    if (d > 0) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) h[i] = l[i] = 0u;
+    } else {
+      constexpr int V1 = REM ? 32 : 0;
+      if constexpr (!REM) { tmem_ld_x32(col + 32 * k, *reinterpret_cast<uint32_t(*)[32]>(&v[0])); tmem_ld_wait(); }
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) {
+        float x = f(32 * k + i, __uint_as_float(v[V1 * k + i])), y = f(32 * k + i + 1, __uint_as_float(v[V1 * k + i + 1]));
+        if (d == 0) {
+          if (LOWER ? i > lane : i < lane) x = 0.f;
+          if (LOWER ? i + 1 > lane : i + 1 < lane) y = 0.f;
+        }
+        g(x, y);
+        h[i / 2] = pack_bf16x2(x, y);
+        if constexpr (REM) { const float2 r = unpack_bf16x2(h[i / 2]); l[i / 2] = pack_bf16x2(x - r.x, y - r.y); }
+      }
+    }
+    tmem_st_x16(col + 16 * k, h);
+    if constexpr (REM) tmem_st_x16(col + 32 + 16 * k, l);
+  }
   tmem_st_wait();
 }
 // HD / 2 fp32 values = columns (HD / 2) hf .. of a state row -> value and remainder tiles ([rows][HD], atoms of `rows` rows)
@@ -359,7 +359,7 @@ __device__ __forceinline__ void la_store_tile(const CUtensorMap* tm, const uint8
 #pragma unroll
   for (int a = 0; a < HD / 64; ++a) tma_store_4d(tm, tile + a * (LA_C * 128), a * 64, h, tok0, b);
 }
-template <int HD>
+template <int HD, int KIND>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmLo, const LinAttnArgs p) {
@@ -390,7 +390,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (p.n_seg > 1 && !full && seg == p.n_seg - 1) return;      // nothing follows the last segment
   // ELU + 1 features sit near 1, where a bf16 copy of the masked tile loses what the later subtraction needs; ReLU^2
   // features are spread over the exponent range and a single copy is enough (0.3 % measured)
-  const bool rem = p.kind == 0;
+  constexpr bool rem = KIND == 0;
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
     mbar_init(q_bar, 1); mbar_init(&k_bar[0], 1); mbar_init(&k_bar[1], 1); mbar_init(v_bar, 1); mbar_init(a_bar, 1); mbar_init(b_bar, 1);
@@ -442,18 +442,19 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   bool ok = true;
   const bool have_state0 = s_in != nullptr;
-  for (int c = 0; c < n_chunks; ++c) {
+  // The features of a chunk are formed one chunk ahead, while the products of the chunk before it run
+  auto phi = [&](int c) {
+    if (full && !mbar_wait(q_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
+    if (ok && !mbar_wait(&k_bar[c & 1], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
+    if (full) la_phi_half<HD, KIND>(sQ, row, hf, LA_C, p.scale);
+    la_phi_half<HD, KIND>(sK + (c & 1) * L::TILE, row, hf, min(LA_C, p.S - (c0 + c) * LA_C), p.scale);
+    fence_proxy_async_smem();
+  };
+  phi(0);
+  if (__syncthreads_or(!ok)) ok = false;
+  for (int c = 0; c < n_chunks && ok; ++c) {
     const int st = c & 1;
     uint8_t* sKc = sK + st * L::TILE;
-    const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
-    // ---- phi in place
-    if (full && !mbar_wait(q_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
-    if (ok && !mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    if (full) la_phi_half<HD>(sQ, row, hf, LA_C, p.scale, p.kind);
-    la_phi_half<HD>(sKc, row, hf, valid, p.scale, p.kind);
-    fence_proxy_async_smem();
-    __syncthreads();
     float den = p.eps;
     if (full) {
       if (warp == 0 && elect_one()) {
@@ -469,17 +470,9 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (__syncthreads_or(!ok)) { ok = false; break; }
       tc_fence_after_sync();
       if (tid == 0 && c + 1 < n_chunks) load(sQ, &tmQ, q_bar, c + 1);            // Q~ has been consumed
-      float a[64];
-      la_tmem_row<64>(trow + COL_A + hf * 64, a);
       float r0 = 0.f, r1 = 0.f;
-#pragma unroll
-      for (int i = 0; i < 64; i += 2) {
-        if (hf * 64 + i > row) a[i] = 0.f;
-        if (hf * 64 + i + 1 > row) a[i + 1] = 0.f;
-        r0 += a[i]; r1 += a[i + 1];
-      }
+      la_mask_put<true, rem>(trow + COL_A + hf * 64, quad, hf, lane, [](int, float x) { return x; }, [&](float x, float y) { add2(r0, r1, x, y); });
       s_part[hf * LA_C + row] = part + (r0 + r1);
-      la_put_half128(trow + COL_A + hf * 64, a, rem);
       tc_fence_before_sync();
     }
     __syncthreads();
@@ -498,6 +491,7 @@ linattn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     // z += colsum(K~) while the products run: ZP row groups per column, combined after the barrier below
     s_zk[tid] = la_colsum_rows(sKc, tid % HD, (tid / HD) * (LA_C / ZP), LA_C / ZP);
+    if (c + 1 < n_chunks) phi(c + 1);
     if (!mbar_wait(b_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
@@ -606,8 +600,8 @@ __global__ void la_g_kernel(const LinAttnArgs p) {
   if (ok && sub == 0) p.dden[idx] = -dot;
 }
 // scale * phi'(scale * x) * grad for this thread's half of a token, x the raw (bf16) row in the tile `x`, as bf16 into `dst`
-template <int HD>
-__device__ __forceinline__ void la_put_dphi_half(uint8_t* x, uint8_t* dst, int row, int hf, const float* grad, float scale, int kind) {
+template <int HD, int KIND>
+__device__ __forceinline__ void la_put_dphi_half(uint8_t* x, uint8_t* dst, int row, int hf, const float* grad, float scale) {
 #pragma unroll
   for (int i = 0; i < HD / 16; ++i) {
     const uint4 xu = *la_half_piece<HD>(x, row, hf, i);
@@ -617,7 +611,7 @@ __device__ __forceinline__ void la_put_dphi_half(uint8_t* x, uint8_t* dst, int r
     for (int j = 0; j < 4; ++j) {
       const float2 x2 = unpack_bf16x2(xw[j]);
       const float a = x2.x * scale, c = x2.y * scale;
-      const float da = la_dphi(a, kind), dc = la_dphi(c, kind);
+      const float da = la_dphi<KIND>(a), dc = la_dphi<KIND>(c);
       o[j] = pack_bf16x2(grad[i * 8 + 2 * j] * da * scale, grad[i * 8 + 2 * j + 1] * dc * scale);
     }
     *la_half_piece<HD>(dst, row, hf, i) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -640,7 +634,7 @@ __device__ __forceinline__ float la_colsum_w_rows(const uint8_t* tile, int k, co
 
 // ---------------------------------------------------------------------------------------------------- backward 1: dQ
 // Same 8-warp mapping as the forward: warp w owns rows 32 (w & 3) .. and column half w >> 2.
-template <int HD>
+template <int HD, int KIND>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                       const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmDQ, const LinAttnArgs p) {
@@ -667,7 +661,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int bh = blockIdx.x / p.n_seg, seg = blockIdx.x % p.n_seg, b = bh / p.H, h = bh % p.H;
   const int c0 = seg * p.seg_chunks;           // first chunk of this CTA's segment
   const int n_chunks = min(p.seg_chunks, (p.S + LA_C - 1) / LA_C - c0);
-  const bool rem = p.kind == 0;                // see the forward kernel
+  constexpr bool rem = KIND == 0;              // see the forward kernel
   if ((smem_u32(smem) & 1023u) != 0) { if (tid == 0 && p.status) atomicCAS(p.status, 0u, (uint32_t)ST_BAD_ARGUMENT); return; }
   if (tid == 0) {
     mbar_init(&k_bar[0], 1); mbar_init(&k_bar[1], 1); mbar_init(v_bar, 1); mbar_init(a_bar, 1); mbar_init(b_bar, 1); mbar_init(q_bar, 1); mbar_init(g_bar, 1);
@@ -725,13 +719,9 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
     const float dden = dden_next;
     if (c + 1 < n_chunks) { const int t = (c0 + c + 1) * LA_C + row; dden_next = t < p.S ? ddp[t] : 0.f; }
-    if (!mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
-    if (ok && !mbar_wait(v_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
+    if (!mbar_wait(v_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (ok && !mbar_wait(g_bar, c & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
-    la_phi_half<HD>(sKc, row, hf, valid, p.scale, p.kind);
-    fence_proxy_async_smem();
-    __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       la_mma_xyT<HD>(tmem_base + COL_A, sG, sV);                                      // T = G V^T
@@ -739,17 +729,15 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       la_mma_xwT<HD>(tmem_base + COL_DQ, sG, sSlo, true);
       tc_commit(a_bar);
     }
+    // K~ while the products that do without it run
+    if (!mbar_wait(&k_bar[st], (c >> 1) & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
+    la_phi_half<HD, KIND>(sKc, row, hf, valid, p.scale);
+    fence_proxy_async_smem();
     if (!mbar_wait(a_bar, c & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
     tc_fence_after_sync();
     if (tid == 0 && c + 1 < n_chunks) load(sG, &tmG, g_bar, c + 1);                   // both readers of G are done
-    {
-      float a[64];
-      la_tmem_row<64>(trow + COL_A + hf * 64, a);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) a[i] = (hf * 64 + i > row) ? 0.f : a[i] + dden;
-      la_put_half128(trow + COL_A + hf * 64, a, rem);
-    }
+    la_mask_put<true, rem>(trow + COL_A + hf * 64, quad, hf, lane, [&](int, float x) { return x + dden; }, [](float, float) {});
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 0 && elect_one()) {
@@ -771,7 +759,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       la_tmem_row<HH>(trow + COL_DQ + hf * HH, dq);
 #pragma unroll
       for (int i = 0; i < HH; ++i) dq[i] = fmaf(dden, sz[hf * HH + i], dq[i]);        // z of the chunks before this one
-      la_put_dphi_half<HD>(sQr, sV, row, hf, dq, p.scale, p.kind);                    // V's buffer takes the result
+      la_put_dphi_half<HD, KIND>(sQr, sV, row, hf, dq, p.scale);                    // V's buffer takes the result
     }
     __syncthreads();                                                                  // every thread has read the old z
     if (tid < HD) {
@@ -805,7 +793,7 @@ linattn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------------- backward 2: dK, dV
-template <int HD>
+template <int HD, int KIND>
 __global__ void __launch_bounds__(LA_FWD_THREADS, LaSmem<HD>::CTAS)
 linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG, const __grid_constant__ CUtensorMap tmDK,
@@ -905,7 +893,6 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   float dden_next = dden_of(n_chunks - 1);                                            // a chunk ahead
   bool ok = true;
   const bool have_state0 = ds_in != nullptr;
-  uint32_t t_phase = 0;
   for (int it = 0; it < n_chunks; ++it) {
     const int c = n_chunks - 1 - it;
     const int valid = min(LA_C, p.S - (c0 + c) * LA_C);
@@ -913,60 +900,46 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     if (c > 0) dden_next = dden_of(c - 1);
     if (!mbar_wait(ld_bar, it & 1, p.status, ST_TIMEOUT_TMA_FULL)) ok = false;
     if (__syncthreads_or(!ok)) { ok = false; break; }
-    la_phi_half<HD>(sQ, row, hf, LA_C, p.scale, p.kind);
-    if (full) la_phi_half<HD>(sK, row, hf, valid, p.scale, p.kind);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (full) {
-    if (warp == 0 && elect_one()) {
+    if (full && warp == 0 && elect_one()) {                                           // the products that do without the features
       tc_fence_after_sync();
-      la_mma_xyT<HD>(tmem_base + COL_T, sK, sQ);                                      // A^T = K~ Q~^T   [key][query]
+      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);                                      // (G V^T)^T = V G^T   [key][query]
       tc_commit(t_bar);
-      la_mma_pw<HD, HD>(tmem_base + COL_DV, sK, sDhi, HD * 128, false);               // dV = K~ dS (value + remainder)
-      la_mma_pw<HD, HD>(tmem_base + COL_DV, sK, sDlo, HD * 128, true);
-      la_mma_xwT<HD>(tmem_base + COL_DK, sV, sDhi, false);                            // dK~ = V dS^T
+      la_mma_xwT<HD>(tmem_base + COL_DK, sV, sDhi, false);                            // dK~ = V dS^T (value + remainder)
       la_mma_xwT<HD>(tmem_base + COL_DK, sV, sDlo, true);
     }
-    if (!mbar_wait(t_bar, t_phase, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
-    t_phase ^= 1;
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc_fence_after_sync();
-    {
-      float a[64];
-      la_tmem_row<64>(trow + COL_T + hf * 64, a);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) if (hf * 64 + i < row) a[i] = 0.f;                // keep queries at or after this key
-      la_put_half128(trow + COL_T + hf * 64, a, false);
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 0 && elect_one()) {
+    la_phi_half<HD, KIND>(sQ, row, hf, LA_C, p.scale);
+    if (full) la_phi_half<HD, KIND>(sK, row, hf, valid, p.scale);
+    fence_proxy_async_smem();
+    if (full) {
+      if (!mbar_wait(t_bar, 0, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;            // (two completions a chunk)
+      if (__syncthreads_or(!ok)) { ok = false; break; }
       tc_fence_after_sync();
-      la_mma_tw<HD>(tmem_base + COL_DV, tmem_base + COL_T, sG);                       // dV += mask(A)^T G
-      tc_commit(u_bar);
-      // (G V^T)^T = V G^T [key][query], over the tile that dV reads just before: in issue order, which is an observation (PTX
-      // promises it for one accumulator and shape); waiting for dV here would add its completion to the chain of every chunk
-      la_mma_xyT<HD>(tmem_base + COL_T, sV, sG);
-      tc_commit(t_bar);
-    }
-    if (!mbar_wait(t_bar, t_phase, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;      // (u_bar has come by then: products are seen to execute in issue order)
-    t_phase ^= 1;
-    if (ok && !mbar_wait(u_bar, it & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
-    if (__syncthreads_or(!ok)) { ok = false; break; }
-    tc_fence_after_sync();
-    {
-      float a[64];
-      la_tmem_row<64>(trow + COL_T + hf * 64, a);
-#pragma unroll
-      for (int i = 0; i < 64; ++i) a[i] = (hf * 64 + i < row) ? 0.f : a[i] + sdden[hf * 64 + i];
-      la_put_half128(trow + COL_T + hf * 64, a, false);
-    }
-    tc_fence_before_sync();
+      // queries at or after this key
+      la_mask_put<false, false>(trow + COL_T + hf * 64, quad, hf, lane, [&](int i, float x) { return x + sdden[hf * 64 + i]; }, [](float, float) {});
+      tc_fence_before_sync();
+      __syncthreads();
+      if (warp == 0 && elect_one()) {
+        tc_fence_after_sync();
+        la_mma_tw<HD>(tmem_base + COL_DK, tmem_base + COL_T, sQ);                     // dK~ += mask(dA)^T Q~
+        tc_commit(u_bar);
+        // A^T = K~ Q~^T, over the tile that dK~ reads just before: in issue order, which is an observation (PTX
+        // promises it for one accumulator and shape); waiting for dK~ here would add its completion to the chain of every chunk
+        la_mma_xyT<HD>(tmem_base + COL_T, sK, sQ);
+        tc_commit(t_bar);
+        la_mma_pw<HD, HD>(tmem_base + COL_DV, sK, sDhi, HD * 128, false);             // dV = K~ dS (value + remainder)
+        la_mma_pw<HD, HD>(tmem_base + COL_DV, sK, sDlo, HD * 128, true);
+      }
+      if (!mbar_wait(t_bar, 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;            // (u_bar has come by then: products are seen to execute in issue order)
+      if (ok && !mbar_wait(u_bar, it & 1, p.status, ST_TIMEOUT_ACC_FULL)) ok = false;
+      if (__syncthreads_or(!ok)) { ok = false; break; }
+      tc_fence_after_sync();
+      la_mask_put<false, false>(trow + COL_T + hf * 64, quad, hf, lane, [](int, float x) { return x; }, [](float, float) {});
+      tc_fence_before_sync();
     }
     __syncthreads();
     if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
-      if (full) la_mma_tw<HD>(tmem_base + COL_DK, tmem_base + COL_T, sQ);             // dK~ += mask(dA)^T Q~
+      if (full) la_mma_tw<HD>(tmem_base + COL_DV, tmem_base + COL_T, sG);             // dV += mask(A)^T G
       la_mma_xTw<HD>(tmem_base + COL_DS, sQ, sG, !DS_REG && (have_state0 || it > 0)); // dS += Q~^T G
       tc_commit(b_bar);
     }
@@ -986,7 +959,7 @@ linattn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       la_tmem_row<HH>(trow + COL_DK + hf * HH, g);
 #pragma unroll
       for (int i = 0; i < HH; ++i) g[i] += sdz[hf * HH + i];                           // dz of the chunks after this one
-      la_put_dphi_half<HD>(sKr, sK, row, hf, g, p.scale, p.kind);
+      la_put_dphi_half<HD, KIND>(sKr, sK, row, hf, g, p.scale);
     }
     __syncthreads();                                                                  // every thread has read the old dz
     if (tid < HD) {
@@ -1052,14 +1025,14 @@ static int la_map(CUtensorMap* m, const LinAttnArgs& a, const AttnTensor& t) {
   return make_tmap_attn(m, t.ptr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.hd, a.H, a.S, a.B, t.sh, t.ss, t.sb, 64, LA_C, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-template <int HD>
+template <int HD, int KIND>
 static int la_set_attrs() {
   static bool done = false;
   if (done) return 0;
   (void)cudaGetLastError();
-  if (cudaFuncSetAttribute(linattn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_fwd8_smem<HD>()) != cudaSuccess) return 1;
-  if (cudaFuncSetAttribute(linattn_bwd_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_dq8_smem<HD>()) != cudaSuccess) return 1;
-  if (cudaFuncSetAttribute(linattn_bwd_dkv_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_dkv_smem<HD>()) != cudaSuccess) return 1;
+  if (cudaFuncSetAttribute(linattn_fwd_kernel<HD, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_fwd8_smem<HD>()) != cudaSuccess) return 1;
+  if (cudaFuncSetAttribute(linattn_bwd_dq_kernel<HD, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_dq8_smem<HD>()) != cudaSuccess) return 1;
+  if (cudaFuncSetAttribute(linattn_bwd_dkv_kernel<HD, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, la_dkv_smem<HD>()) != cudaSuccess) return 1;
   done = true;
   return 0;
 }
@@ -1081,23 +1054,23 @@ __global__ void la_segment_prefix_kernel(float* __restrict__ seg, const float* _
   }
 }
 
-template <int HD>
+template <int HD, int KIND>
 static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
-  if (la_set_attrs<HD>()) return 104;
+  if (la_set_attrs<HD, KIND>()) return 104;
   if (which == 4) {                                     // a whole backward: G pass, dQ, dK / dV
-    if (int rc = la_launch<HD>(a, 3, st)) return rc;
-    if (int rc = la_launch<HD>(a, 1, st)) return rc;
+    if (int rc = la_launch<HD, KIND>(a, 3, st)) return rc;
+    if (int rc = la_launch<HD, KIND>(a, 1, st)) return rc;
     LinAttnArgs t = a;
     t.seg = a.dseg;
     t.s_in = nullptr;
-    return la_launch<HD>(t, 2, st);
+    return la_launch<HD, KIND>(t, 2, st);
   }
   if (which != 3 && a.n_seg > 1 && !a.state_only && a.s_in != a.seg && a.ds_in != a.seg) {
     // segments: their totals, the prefix over them (the forward's serves the dQ pass too), then the pass itself from there
     LinAttnArgs t = a;
     if (which != 1) {
       t.state_only = 1; t.s_in = t.ds_in = nullptr; t.s_out = t.ds_out = a.seg;
-      if (int rc = la_launch<HD>(t, which, st)) return rc;
+      if (int rc = la_launch<HD, KIND>(t, which, st)) return rc;
       constexpr int N = HD * HD + HD;
       la_segment_prefix_kernel<<<dim3((N + 255) / 256, a.B * a.H), 256, 0, st>>>(a.seg, which == 0 ? a.s_in : a.ds_in, a.n_seg, N, which == 2);
       const cudaError_t e = cudaGetLastError();
@@ -1105,7 +1078,7 @@ static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
     }
     t = a;
     if (which == 2) t.ds_in = a.seg; else t.s_in = a.seg;
-    return la_launch<HD>(t, which, st);
+    return la_launch<HD, KIND>(t, which, st);
   }
   if (which == 3) {
     const long long n = (long long)a.B * a.H * a.S * (HD / 8);
@@ -1124,13 +1097,13 @@ static int la_launch(const LinAttnArgs& a, int which, cudaStream_t st) {
   if (which == 0) {
     if (!state && la_map(&t0, a, a.o)) return 105;
     if (!state && a.o_lo.ptr && la_map(&t1, a, a.o_lo)) return 106;
-    linattn_fwd_kernel<HD><<<grid, LA_FWD_THREADS, la_fwd8_smem<HD>(), st>>>(tq, tk, tv, t0, t1, a);
+    linattn_fwd_kernel<HD, KIND><<<grid, LA_FWD_THREADS, la_fwd8_smem<HD>(), st>>>(tq, tk, tv, t0, t1, a);
   } else if (which == 1) {
     if (la_map(&t0, a, a.dq)) return 105;
-    linattn_bwd_dq_kernel<HD><<<grid, LA_FWD_THREADS, la_dq8_smem<HD>(), st>>>(tq, tk, tv, tg, t0, a);
+    linattn_bwd_dq_kernel<HD, KIND><<<grid, LA_FWD_THREADS, la_dq8_smem<HD>(), st>>>(tq, tk, tv, tg, t0, a);
   } else {
     if (!state && (la_map(&t0, a, a.dk) || la_map(&t1, a, a.dv))) return 105;
-    linattn_bwd_dkv_kernel<HD><<<grid, LA_FWD_THREADS, la_dkv_smem<HD>(), st>>>(tq, tk, tv, tg, t0, t1, a);
+    linattn_bwd_dkv_kernel<HD, KIND><<<grid, LA_FWD_THREADS, la_dkv_smem<HD>(), st>>>(tq, tk, tv, tg, t0, t1, a);
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 400 + (int)e;
@@ -1144,8 +1117,8 @@ extern "C" int b200_linattn(const b200::LinAttnArgs* a, int which, cudaStream_t 
   if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
   if (which < 0 || which > 4 || (which == 4 && (a->state_only || a->sx.role != 0 || (a->n_seg > 1 && !a->dseg))) || (which > 0 && (!a->g.ptr || !a->dden)) || a->n_seg < 1 || (a->n_seg > 1 && (!a->seg || a->state_only || a->sx.role != 0))) return -2;
   if ((long long)a->n_seg * a->seg_chunks < (a->S + LA_C - 1) / LA_C || (long long)(a->n_seg - 1) * a->seg_chunks >= (a->S + LA_C - 1) / LA_C) return -2;
-  if (a->hd == 64) return la_launch<64>(*a, which, st);
-  if (a->hd == 128) return la_launch<128>(*a, which, st);
+  if (a->hd == 64) return a->kind == 0 ? la_launch<64, 0>(*a, which, st) : la_launch<64, 1>(*a, which, st);
+  if (a->hd == 128) return a->kind == 0 ? la_launch<128, 0>(*a, which, st) : la_launch<128, 1>(*a, which, st);
   return -3;
 }
-extern "C" int b200_linattn_init() { return b200::la_set_attrs<64>() | b200::la_set_attrs<128>(); }
+extern "C" int b200_linattn_init() { return b200::la_set_attrs<64, 0>() | b200::la_set_attrs<64, 1>() | b200::la_set_attrs<128, 0>() | b200::la_set_attrs<128, 1>(); }

@@ -177,3 +177,26 @@ def test_no_tokens():
     q, k, v = (torch.zeros(2, 0, 4, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
     o = linear_attention(q, k, v, causal=True, kind="elu")
     assert o.shape == (2, 0, 4, 64) and all(g.shape == q.shape for g in torch.autograd.grad(o, (q, k, v), torch.zeros_like(o)))
+
+
+@pytest.mark.parametrize("S", [31, 33, 64, 65, 97, 127, 129, 160])
+@pytest.mark.parametrize("hd,kind", [(64, "elu"), (64, "relu2"), (128, "elu"), (128, "relu2")])
+def test_lengths_around_the_32_wide_blocks_of_the_mask(S, hd, kind):
+    """A masked tile is handled in 32 x 32 blocks that are kept, dropped or on the diagonal; sequences that end inside, at and behind them."""
+    e32, e16 = _check(S, hd, kind, B=1, H=2, seed=S)
+    assert all(e < 6e-3 for e in e16.values()), e16
+
+
+def test_infinite_and_missing_values_stay_where_they_are():
+    """A NaN in one token's query reaches that token's output only; a value reaches the tokens from its own on."""
+    from rust_neural_network_b200.ops.linear_attention import linear_attention
+    q, k, v, _ = _inputs(1, 200, 1, 64, seed=9)
+    clean = linear_attention(q, k, v, scale=0.125, causal=True, kind="elu")
+    q2, v2 = q.clone(), v.clone()
+    q2[0, 70, 0, 3] = float("nan")
+    out = linear_attention(q2, k, v, scale=0.125, causal=True, kind="elu")
+    bad = torch.isnan(out).any(-1)[0, :, 0].nonzero().flatten().tolist()
+    assert bad == [70] and torch.equal(out[:, :70], clean[:, :70]) and torch.equal(out[:, 71:], clean[:, 71:])
+    v2[0, 150, 0, 5] = float("inf")
+    out = linear_attention(q, k, v2, scale=0.125, causal=True, kind="elu")
+    assert torch.equal(out[:, :128], clean[:, :128]) and torch.isfinite(out[:, :128]).all()
