@@ -27,20 +27,9 @@
 #include "../common/ptx.cuh"
 #include "../common/launch.cuh"
 #include "../common/tensormap.h"
+#include "gemm_mx_sm100.h"
 
 namespace b200 {
-
-struct MxGemmArgs {
-  const void* A; const void* B;        // element bytes, K-major
-  const void* sfa; const void* sfb;    // scale chunks (see above); row blocks padded to a multiple of 256 rows
-  void* C; long long ldc;              // [M, N] bf16 or fp32
-  int M, N, K;
-  int out_f32;
-  float alpha;                         // product of the per-tensor scales (NVFP4) or 1
-  int kind;
-  const void* bias;                    // [N] bf16 or null, added in fp32
-  uint32_t* status;
-};
 
 template <int KIND, int BN_>
 struct MxCfg {

@@ -1,12 +1,15 @@
 """In-tree build of the native libraries.
 
-Two shared objects are produced next to this file (under ``lib/``):
+Three shared objects are produced next to this file (under ``lib/``):
 
 * ``libb200nn_cuda.so`` - every hand-written sm_100a kernel (plain CUDA, C ABI, no torch headers);
 * ``libb200nn_host.so`` - the host runtime in C++ (checkpoint reader/writer, tokenizer, parsers,
   tiered store, TCP store, CPU oracles) with no CUDA dependency, so it loads on a CPU-only machine.
 
-Both are loaded through ``ctypes`` (see ``_native.py``). nvcc cross-compiles for
+* ``_b200nn_entry.so`` - the host side of the short GPU calls, a Python extension on torch's C++ tensors (`csrc/entry/`),
+  linked against the kernel library.
+
+The first two are loaded through ``ctypes`` (see ``_native.py``). nvcc cross-compiles for
 ``compute_100a/sm_100a`` without a GPU being present.
 """
 from __future__ import annotations
@@ -72,7 +75,46 @@ def cuda_sources() -> list[Path]:
 
 
 def host_sources() -> list[Path]:
-    return sorted(p for p in CSRC.rglob("*.cpp"))
+    return sorted(p for p in CSRC.rglob("*.cpp") if p.parent.name != "entry")
+
+
+def _entry_flags() -> list[str]:
+    """Compiler flags of the extension: torch's, Python's and CUDA's headers, torch's C++ ABI."""
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", Path(sysconfig.get_paths()["include"]), cuda]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-Werror", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             "-DTORCH_API_INCLUDE_EXTENSION_H", f"-DTORCH_VERSION_TAG=\"{torch.__version__}\""]
+    return flags + [f for d in inc for f in ("-isystem", str(d))]
+
+
+def _compile_entry() -> Path:
+    flags = _entry_flags()
+    src = CSRC / "entry" / "entry.cpp"
+    obj = OBJDIR / f"entry.{_digest(src, ' '.join(flags))}.o"
+    if not obj.exists():
+        for old in OBJDIR.glob("entry.*.o"):
+            old.unlink()
+        r = subprocess.run([os.environ.get("CXX", "g++")] + flags + ["-c", str(src), "-o", str(obj)], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"compile failed: {src}\n{r.stderr}")
+    return obj
+
+
+def _link_entry(obj: Path, cuda_lib: Path) -> Path:
+    """`lib/_b200nn_entry.so`. torch's libraries are loaded by the time it is imported; the kernel library lies next to it."""
+    import torch
+    out = LIBDIR / "_b200nn_entry.so"
+    cudart = Path(_nvcc()).resolve().parent.parent / "lib64"
+    cmd = [os.environ.get("CXX", "g++"), "-shared", "-o", str(out), str(obj), f"-L{cuda_lib.parent}", f"-l:{cuda_lib.name}", "-Wl,-rpath,$ORIGIN",
+           f"-L{Path(torch.__file__).resolve().parent / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{cudart}", "-lcudart"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"link failed\n{r.stderr}")
+    return out
 
 
 def build_all(verbose: bool = False, jobs: int | None = None) -> dict[str, Path]:
@@ -83,9 +125,11 @@ def build_all(verbose: bool = False, jobs: int | None = None) -> dict[str, Path]
     cu, cpp = cuda_sources(), host_sources()
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
         cu_futs = [ex.submit(_compile_one, s, True, verbose) for s in cu]
+        entry_fut = ex.submit(_compile_entry)
         cpp_futs = [ex.submit(_compile_one, s, False, verbose) for s in cpp]
         cu_objs = [f.result() for f in cu_futs]
         cpp_objs = [f.result() for f in cpp_futs]
+        entry_obj = entry_fut.result()
     out = {}
     cuda_lib = LIBDIR / "libb200nn_cuda.so"
     # one CUDA runtime per process: link the shared cudart so the kernels use the same runtime instance
@@ -95,6 +139,7 @@ def build_all(verbose: bool = False, jobs: int | None = None) -> dict[str, Path]
     if r.returncode != 0:
         raise RuntimeError(f"link failed\n{r.stdout}\n{r.stderr}")
     out["cuda"] = cuda_lib
+    out["entry"] = _link_entry(entry_obj, cuda_lib)
     if cpp_objs:
         host_lib = LIBDIR / "libb200nn_host.so"
         cmd = [os.environ.get("CXX", "g++"), "-shared", "-o", str(host_lib)] + [str(o) for o in cpp_objs] + ["-pthread"]

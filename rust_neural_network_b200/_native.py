@@ -104,6 +104,7 @@ _SIGS = {
 }
 
 _cuda_lib = None
+_entry = None
 _host_lib = None
 _launch_count = 0
 
@@ -204,6 +205,23 @@ def host():
     return _host_lib
 
 
+def entry():
+    """The extension that prepares and issues the short GPU calls (csrc/entry/entry.cpp), loaded with the kernel library. Raises if it is missing."""
+    global _entry
+    if _entry is None:
+        cuda()
+        path = LIBDIR / "_b200nn_entry.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: run the in-tree build first (the extension is required on a GPU machine)")
+        from importlib.machinery import ExtensionFileLoader
+        from importlib.util import module_from_spec, spec_from_file_location
+        spec = spec_from_file_location("_b200nn_entry", path, loader=ExtensionFileLoader("_b200nn_entry", str(path)))
+        module = module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _entry = module
+    return _entry
+
+
 def host_available() -> bool:
     return (LIBDIR / "libb200nn_host.so").exists()
 
@@ -223,12 +241,14 @@ def count_launch(n: int = 1) -> None:
 
 
 def launch_count() -> int:
-    return _launch_count
+    return _launch_count + (_entry.launches() if _entry is not None else 0)
 
 
 def reset_launch_count() -> None:
     global _launch_count
     _launch_count = 0
+    if _entry is not None:
+        _entry.reset_launches()
 
 
 def check(rc: int, what: str) -> None:

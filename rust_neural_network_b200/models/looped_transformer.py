@@ -19,7 +19,7 @@ import torch
 from .. import nn
 from ..ops import functional as F
 from ..ops import kernels as K
-from ..ops.transformer import transformer_block
+from ..ops.transformer import block_calls, plain_inference, transformer_block
 
 
 class AttentionKind(enum.Enum):
@@ -95,10 +95,12 @@ class TransformerBlock(nn.Module):
         self.attn.with_attention(kind)
         return self
 
+    def _fused(self, x) -> bool:
+        return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3 and self.attn.kind == AttentionKind.Flash
+                and (x.shape[-1] // self.attn.heads) in (64, 128))
+
     def forward(self, x):
-        fused = (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 3 and self.attn.kind == AttentionKind.Flash
-                 and (x.shape[-1] // self.attn.heads) in (64, 128))
-        if fused:
+        if self._fused(x):
             return transformer_block(x, self, self.causal)
         h = self.attn(self.ln1(x), residual=x)
         a = F.linear(self.ln2(h), self.ff1.weight, self.ff1.bias, "gelu", None)
@@ -173,9 +175,19 @@ class LoopedTransformer(nn.Module):
         tc = self.time_conditioning(h.device, h.dtype)
         loops = 0
         halt_acc = 0.0
+        # without gradients the blocks' weights are looked at once for all loops
+        calls = None
+        if type(self.block) is _BlockStack and plain_inference() and all(type(b) is TransformerBlock and b._fused(h) for b in self.block.blocks):
+            calls = block_calls(h, self.block.blocks)
         for t in range(self.num_loops):
             cond = _add_row(h, tc[t])
-            h = _add(cond, self.block(cond))
+            if calls is None:
+                y = self.block(cond)
+            else:
+                y = cond
+                for call in calls:
+                    y = call(y)
+            h = _add(cond, y)
             loops += 1
             if self.adaptive:
                 hv = torch.sigmoid(self.halt_unit(h).float()).reshape(-1)[0]
@@ -259,11 +271,11 @@ class _AddRowFn(torch.autograd.Function):
 
 
 def _add(a, b):
-    return _AddFn.apply(a, b)
+    return K.binary(a, b, "add") if plain_inference() else _AddFn.apply(a, b)
 
 
 def _add_row(a, row):
-    return _AddRowFn.apply(a, row)
+    return K.binary(a, row.to(a.dtype), "add") if plain_inference() else _AddRowFn.apply(a, row)
 
 
 from .._compat import accept_wrapped as _accept_wrapped  # noqa: E402

@@ -526,17 +526,6 @@ def pointwise_loss(pred, target, kind, delta=1.0, reduction="mean", want_grad=Tr
 
 
 # ----------------------------------------------------------------------------- attention
-def _attn_tensor(t):
-    # t: [B, S, H, hd] view with unit stride on hd
-    a = nv.AttnTensor()
-    a.ptr, a.sb, a.ss, a.sh = t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)
-    return a
-
-
-def _attn_ok(t):
-    return t.stride(3) == 1 and all(s % 8 == 0 for s in (t.stride(0), t.stride(1), t.stride(2))) and t.data_ptr() % 16 == 0
-
-
 def attention_ref(q, k, v, scale, causal):
     """Dense fp32 softmax attention on [B, S, H, hd] tensors."""
     qf, kf, vf = (t.float().permute(0, 2, 1, 3) for t in (q, k, v))
@@ -552,50 +541,16 @@ def attention_ref(q, k, v, scale, causal):
 @nv.traced("flash_attention")
 def flash_fwd(q, k, v, scale, causal):
     """q,k,v: [B, S, H, hd] bf16 views (hd contiguous). Returns (o [B,S,H,hd] bf16, lse [B,H,S] fp32)."""
-    B, Sq, H, hd = q.shape
-    Skv = k.shape[1]
     if not q.is_cuda:
         o = attention_ref(q, k, v, scale, causal)
         return o.to(q.dtype), None
-    if q.dtype != torch.bfloat16:
-        raise TypeError("flash attention kernels take bf16")
-    q, k, v = (t if _attn_ok(t) else t.contiguous() for t in (q, k, v))
-    o = torch.empty((B, Sq, H, hd), dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
-    a = nv.FlashArgs()
-    a.q, a.k, a.v, a.o = _attn_tensor(q), _attn_tensor(k), _attn_tensor(v), _attn_tensor(o)
-    a.lse = lse.data_ptr()
-    a.B, a.H, a.Sq, a.Skv, a.hd = B, H, Sq, Skv, hd
-    a.scale, a.causal = float(scale), int(causal)
-    a.status = nv.status_word(q.device).data_ptr()
-    nv.check(nv.cuda().b200_flash_fwd(C.byref(a), nv.stream_ptr()), "flash_fwd")
-    nv.count_launch()
-    return o, lse
+    return nv.entry().flash_fwd(q, k, v, scale, causal)
 
 
 @nv.traced("flash_attention")
 def flash_bwd(dout, q, k, v, o, lse, scale, causal, dq=None, dk=None, dv=None):
     """Gradients of flash_fwd. dq/dk/dv may be preallocated strided views (e.g. slices of a fused dQKV)."""
-    B, Sq, H, hd = q.shape
-    Skv = k.shape[1]
-    dev = q.device
-    dout = dout if _attn_ok(dout) else dout.contiguous()
-    if dq is None: dq = torch.empty((B, Sq, H, hd), dtype=torch.bfloat16, device=dev)
-    if dk is None: dk = torch.empty((B, Skv, H, hd), dtype=torch.bfloat16, device=dev)
-    if dv is None: dv = torch.empty((B, Skv, H, hd), dtype=torch.bfloat16, device=dev)
-    delta = torch.empty((B, H, Sq), dtype=torch.float32, device=dev)
-    # the kernel's own layout; one key block adds nothing up and writes dq itself
-    dq_accum = torch.empty((B, H, (Sq + 31) // 32 * 32, hd), dtype=torch.float32, device=dev) if Skv > 128 else None
-    a = nv.FlashArgs()
-    a.q, a.k, a.v, a.o = _attn_tensor(q), _attn_tensor(k), _attn_tensor(v), _attn_tensor(o)
-    a.dout, a.dq, a.dk, a.dv = _attn_tensor(dout), _attn_tensor(dq), _attn_tensor(dk), _attn_tensor(dv)
-    a.lse, a.delta, a.dq_accum = lse.data_ptr(), delta.data_ptr(), nv.ptr(dq_accum)
-    a.B, a.H, a.Sq, a.Skv, a.hd = B, H, Sq, Skv, hd
-    a.scale, a.causal = float(scale), int(causal)
-    a.status = nv.status_word(dev).data_ptr()
-    nv.check(nv.cuda().b200_flash_bwd(C.byref(a), nv.stream_ptr()), "flash_bwd")
-    nv.count_launch(3 if Skv > 128 else 2)
-    return dq, dk, dv
+    return nv.entry().flash_bwd(dout, q, k, v, o, lse, scale, causal, dq, dk, dv)
 
 
 # ----------------------------------------------------------------------------- optimizers (flat buffers)

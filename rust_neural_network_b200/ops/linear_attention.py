@@ -145,6 +145,16 @@ def _segments(bh: int, n_chunks: int, hd: int, sms: int, grad: bool = True) -> i
     return n if cut < whole else 1
 
 
+@nv.traced("linear_attention")
+def _fused_forward(q, k, v, scale, eps, kind, need_grad, n_seg):
+    return nv.entry().linattn_fwd(q, k, v, scale, eps, 0 if kind == "elu" else 1, need_grad, n_seg)
+
+
+@nv.traced("linear_attention")
+def _fused_backward(dout, q, k, v, o, den, s_in, o_lo, scale, eps, kind):
+    return nv.entry().linattn_bwd(dout, q, k, v, o, den, s_in, o_lo, scale, eps, 0 if kind == "elu" else 1)
+
+
 class FusedCausalLinearAttnFn(Function):
     """Causal linear attention on the fused chunk kernels (csrc/attention/linattn_sm100.cu): one forward kernel; in the backward
     a pass that forms G = dO / D and dD, then dQ in sequence order and dK / dV in reverse order. Where the sequence is cut
@@ -156,6 +166,14 @@ class FusedCausalLinearAttnFn(Function):
     @staticmethod
     def forward(ctx, q, k, v, scale, eps, kind, sp):
         B, S, H, d = q.shape
+        if sp is None:
+            need_grad = any(t.requires_grad for t in (q, k, v))
+            n_seg = _segments(B * H, -(-S // CHUNK), d, _num_sms(q.device), need_grad)
+            # (the segments' states are what the backward's dQ pass starts from)
+            saved = _fused_forward(q, k, v, scale, eps, kind, need_grad, n_seg)
+            ctx.save_for_backward(*saved)
+            ctx.cfg = (scale, eps, kind, sp)
+            return saved[3]
         q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
         dev = q.device
         o = torch.empty((B, S, H, d), dtype=torch.bfloat16, device=dev)
@@ -176,10 +194,7 @@ class FusedCausalLinearAttnFn(Function):
             pre = _launch(0, q, k, v, scale, eps, kind, o=o, den=den, o_lo=o_lo, sx=(sp, 0, 2))
             s_in = pre.clone() if (sp.rank > 0 and need_grad) else None      # the buffer is reused by the next call
         else:
-            n_seg = 1 if sp is not None else _segments(B * H, -(-S // CHUNK), d, _num_sms(dev), need_grad)
-            seg = torch.empty((B * H, n_seg, d * d + d), dtype=torch.float32, device=dev) if n_seg > 1 else None
-            _launch(0, q, k, v, scale, eps, kind, o=o, den=den, s_in=s_in, o_lo=o_lo, seg=seg, n_seg=n_seg)
-            s_in = s_in if seg is None else seg                  # the states the backward's dQ pass starts from
+            _launch(0, q, k, v, scale, eps, kind, o=o, den=den, s_in=s_in, o_lo=o_lo)
         ctx.save_for_backward(q, k, v, o, den, s_in if s_in is not None else torch.empty(0), o_lo if o_lo is not None else torch.empty(0))
         ctx.cfg = (scale, eps, kind, sp)
         return o
@@ -188,16 +203,13 @@ class FusedCausalLinearAttnFn(Function):
     def backward(ctx, dout):
         q, k, v, o, den, s_in, o_lo = ctx.saved_tensors
         scale, eps, kind, sp = ctx.cfg
+        if sp is None or sp.world <= 1:
+            return (*_fused_backward(dout, q, k, v, o, den, s_in, o_lo, scale, eps, kind), None, None, None, None)
         s_in = s_in if s_in.numel() else None
-        n_seg = s_in.shape[1] if (s_in is not None and s_in.dim() == 3) else 1
         o_lo = o_lo if o_lo.numel() else None
         B, S, H, d = q.shape
         dout = dout if (_tma_ok(dout) and dout.dtype == torch.bfloat16) else dout.to(torch.bfloat16).contiguous()
         dq, dk, dv = torch.empty_like(o), torch.empty_like(o), torch.empty_like(o)
-        if sp is None or sp.world <= 1:                         # one call: preparing a launch from Python takes 20 us
-            _launch(4, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, dk=dk, dv=dv, g=_g_empty(q), s_in=None if n_seg > 1 else s_in,
-                    o_lo=o_lo, seg=s_in if n_seg > 1 else None, dseg=torch.empty_like(s_in) if n_seg > 1 else None, n_seg=n_seg)
-            return dq, dk, dv, None, None, None, None
         g = _g_pass(q, k, v, o, den, dout, o_lo)                 # a slice of a longer sequence
         _launch(1, q, k, v, scale, eps, kind, o=o, den=den, dout=dout, dq=dq, g=g, s_in=s_in, o_lo=o_lo)
         if sp.backend == "fused":

@@ -27,15 +27,7 @@ _KMULT = {0: 128, 1: 256}
 _E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
 
 
-class MxGemmArgs(C.Structure):
-    _fields_ = [("A", C.c_void_p), ("B", C.c_void_p), ("sfa", C.c_void_p), ("sfb", C.c_void_p), ("C", C.c_void_p), ("ldc", C.c_longlong),
-                ("M", C.c_int), ("N", C.c_int), ("K", C.c_int), ("out_f32", C.c_int), ("alpha", C.c_float), ("kind", C.c_int),
-                ("bias", C.c_void_p), ("status", C.c_void_p)]
-
-
 nv.register_sigs({
-    "b200_gemm_mx": [C.POINTER(MxGemmArgs), C.c_int, C.c_void_p],
-    "b200_mx_quant": [C.c_void_p, C.c_int, C.c_longlong, C.c_longlong, C.c_int, C.c_int, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p],
     "b200_mx_dequant": [C.c_void_p, C.c_void_p, C.c_longlong, C.c_int, C.c_int, C.c_float, C.c_void_p, C.c_void_p],
 })
 
@@ -118,16 +110,7 @@ def quantize_mx(x: torch.Tensor, kind: str = "mxfp8", tensor_scale: float | None
     if not x.is_cuda:
         data, sf = _quantize_torch(x.detach(), k, ts)
         return MxTensor(data, sf, rows, K, k, ts)
-    x = x.detach()
-    if x.dtype not in (torch.bfloat16, torch.float32):
-        x = x.float()
-    if x.stride(1) != 1:
-        x = x.contiguous()
-    data = torch.empty((rows, K if k == 0 else K // 2), dtype=torch.uint8, device=x.device)
-    sf = torch.empty(_sf_bytes(rows, K, k), dtype=torch.uint8, device=x.device)
-    nv.check(nv.cuda().b200_mx_quant(x.data_ptr(), int(x.dtype == torch.bfloat16), x.stride(0), rows, K, k, ts, data.data_ptr(),
-                                     sf.data_ptr(), nv.stream_ptr()), "mx_quant")
-    nv.count_launch()
+    data, sf = nv.entry().mx_quant(x.detach(), k, ts, _sf_bytes(rows, K, k))
     return MxTensor(data, sf, rows, K, k, ts)
 
 
@@ -163,25 +146,7 @@ def gemm_mx(a: MxTensor, b: MxTensor, out_dtype=torch.bfloat16, bias: torch.Tens
         return (y if bias is None else y + bias.float()).to(out_dtype)
     if b.rows % 8 != 0:
         raise ValueError("N must be a multiple of 8")
-    from .gemm import _num_sms
-    out = torch.empty((a.rows, b.rows), dtype=out_dtype, device=a.data.device)
-    g = MxGemmArgs()
-    g.A, g.B, g.sfa, g.sfb = a.data.data_ptr(), b.data.data_ptr(), a.sf.data_ptr(), b.sf.data_ptr()
-    g.C, g.ldc = out.data_ptr(), out.stride(0)
-    g.M, g.N, g.K = a.rows, b.rows, a.K
-    g.out_f32 = int(out_dtype == torch.float32)
-    g.alpha = float(a.tensor_scale * b.tensor_scale)
-    g.kind = a.kind
-    if bias is not None:
-        if bias.dtype != torch.bfloat16 or bias.shape != (b.rows,):
-            raise ValueError("bias must be a bf16 vector of N elements")
-        if not bias.is_contiguous() or bias.data_ptr() % 16:
-            bias = bias.clone(memory_format=torch.contiguous_format)
-        g.bias = bias.data_ptr()
-    g.status = nv.status_word(a.data.device).data_ptr()
-    nv.check(nv.cuda().b200_gemm_mx(C.byref(g), _num_sms(a.data.device), nv.stream_ptr()), "gemm_mx")
-    nv.count_launch()
-    return out
+    return nv.entry().gemm_mx(a.data, a.sf, b.data, b.sf, a.rows, b.rows, a.K, a.kind, a.tensor_scale * b.tensor_scale, out_dtype == torch.float32, bias)
 
 
 class MxLinear:

@@ -57,16 +57,7 @@ def quant_rows(x: torch.Tensor, mode: str = "int8"):
         if mode == "int8":
             return round_away(t).clamp(-128, 127).to(torch.int8), scale
         return t.clamp(-448, 448).to(torch.float8_e4m3fn), scale
-    x = _f32_or_bf16(x)
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    rows, cols = x.shape
-    q = torch.empty(rows, cols, dtype=torch.int8 if mode == "int8" else torch.float8_e4m3fn, device=x.device)
-    scales = torch.empty(rows, dtype=torch.float32, device=x.device)
-    nv.check(nv.cuda().b200_quant_rows(x.data_ptr(), _isbf(x), rows, cols, x.stride(0), q.data_ptr(), cols, scales.data_ptr(),
-                                       0 if mode == "int8" else 1, nv.stream_ptr()), "quant_rows")
-    nv.count_launch()
-    return q, scales
+    return nv.entry().quant_rows(x, 0 if mode == "int8" else 1)
 
 
 # ------------------------------------------------------------------ group-wise formats

@@ -178,8 +178,39 @@ def _plain(*ts) -> bool:
     return all(t.dtype == torch.float32 and t.is_cuda and t.is_contiguous() for t in ts)
 
 
-def _block_forward(x, blk, causal):
-    """The block without gradients as one native call, or None where its launches cannot be issued that way."""
+def plain_inference() -> bool:
+    """No gradients, and nothing that follows tensors rather than memory: torch.func transforms and forward-mode AD (their tensors have no
+    memory of their own), tracing (it records a function but not a kernel's writes), NVTX ranges per kernel."""
+    return (not torch.is_grad_enabled() and not nv.NVTX_ENABLED and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None)
+
+
+class _BlockCall:
+    """A block without gradients as one native call: what does not change between the applications of one forward pass (weights, sizes, workspace)
+    is looked at once. Made anew for every forward pass; holds what its record points at."""
+
+    def __init__(self, x, blk, causal, ws, vecs, work, offs):
+        B, S, d = x.shape
+        at = blk.attn
+        w0 = work.data_ptr()
+        self.keep = (ws, vecs, work)
+        self.fields = (*(w0 + p for p in offs), *(w.data_ptr() for w in ws), *(t.data_ptr() for t in vecs), B, S, d, ws[2].shape[0], at.heads, int(causal),
+                       int(not _adjacent(at.q_proj.bias, at.k_proj.bias, at.v_proj.bias)), K.OPS["add"], _num_sms(x.device), nv.f32(blk.ln1.eps),
+                       nv.status_ptr(x.device))
+
+    def __call__(self, x):
+        x = x if x.is_contiguous() else x.contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        y = torch.empty_like(x)
+        launches = C.c_int(0)
+        nv.check(nv.cuda().b200_block_fwd(_BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *self.fields), C.byref(launches), nv.stream_ptr()), "block_fwd")
+        nv.count_launch(launches.value)
+        return y
+
+
+def _block_call(x, blk, causal, work=None):
+    """`_BlockCall` for tensors like `x`, or None where the block's launches cannot be issued that way. `work`: a workspace to share."""
     at = blk.attn
     q, k, v, o, f1, f2, n1, n2 = at.q_proj, at.k_proj, at.v_proj, at.out_proj, blk.ff1, blk.ff2, blk.ln1, blk.ln2
     B, S, d = x.shape
@@ -189,42 +220,41 @@ def _block_forward(x, blk, causal):
             or tuple(q.weight.shape) != (d, d) or tuple(k.weight.shape) != (d, d) or tuple(v.weight.shape) != (d, d)
             or tuple(o.weight.shape) != (d, d) or tuple(f1.weight.shape) != (ff, d) or tuple(f2.weight.shape) != (d, ff)):
         return None
-    x = x if x.is_contiguous() else x.contiguous()
     wqkv = _shadows_qkv(q.weight, k.weight, v.weight)
     ws = (wqkv[0] if _adjacent(*wqkv) else torch.cat(wqkv, 0), lp(o.weight), lp(f1.weight), lp(f2.weight))
-    if x.data_ptr() % 16 or any(w.data_ptr() % 16 or not w.is_contiguous() for w in ws):
+    if any(w.data_ptr() % 16 or not w.is_contiguous() for w in ws):
         return None
-    T, dev, H = B * S, x.device, at.heads
-    sms = _num_sms(dev)
-    adjacent = _adjacent(q.bias, k.bias, v.bias)
+    T = B * S
     # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse, gathered bias (fp32)
     offs, total = [], 0
-    for nbytes in (2 * T * d, 6 * T * d, 2 * T * d, 2 * T * d, 2 * T * ff, 4 * T, 4 * T, 4 * T * H, 12 * d):
+    for nbytes in (2 * T * d, 6 * T * d, 2 * T * d, 2 * T * d, 2 * T * ff, 4 * T, 4 * T, 4 * T * at.heads, 12 * d):
         offs.append(total)
         total += (nbytes + 255) & ~255
-    work = torch.empty(total, dtype=torch.uint8, device=dev)
-    y = torch.empty_like(x)
-    w0 = work.data_ptr()
-    g1, be1, g2, be2, bq, bk, bv, bo, b1, b2 = (t.data_ptr() for t in vecs)
-    rec = _BLOCK_PACK.pack(x.data_ptr(), y.data_ptr(), *(w0 + p for p in offs), *(w.data_ptr() for w in ws),
-                           g1, be1, g2, be2, bq, bk, bv, bo, b1, b2, B, S, d, ff, H, int(causal), int(not adjacent), K.OPS["add"], sms,
-                           nv.f32(n1.eps), nv.status_ptr(dev))
-    launches = C.c_int(0)
-    nv.check(nv.cuda().b200_block_fwd(rec, C.byref(launches), nv.stream_ptr()), "block_fwd")
-    nv.count_launch(launches.value)
-    return y
+    if work is None or work.numel() < total:
+        work = torch.empty(total, dtype=torch.uint8, device=x.device)
+    return _BlockCall(x, blk, causal, ws, vecs, work, offs)
+
+
+def block_calls(x, blocks):
+    """Calls for a stack of fused blocks that is applied several times in a forward pass, or None where any of them needs `transformer_block`."""
+    calls, work = [], None
+    for blk in blocks:
+        c = _block_call(x, blk, blk.causal, work)
+        if c is None:
+            return None
+        work = c.keep[2]
+        calls.append(c)
+    return calls
 
 
 def transformer_block(x, blk, causal):
-    """Run `blk` (a `models.looped_transformer.TransformerBlock`) through the fused function. Without gradients (and outside
-    torch.func transforms and forward-mode AD, whose tensors have no memory of their own, and tracing, which records a function
-    but not a kernel's writes) the forward is one native call."""
+    """Run `blk` (a `models.looped_transformer.TransformerBlock`) through the fused function. Without gradients (`plain_inference`) the
+    forward is one native call."""
     at = blk.attn
-    if (not torch.is_grad_enabled() and not nv.NVTX_ENABLED and torch._C._functorch.peek_interpreter_stack() is None
-            and torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None):
-        y = _block_forward(x, blk, causal)
-        if y is not None:
-            return y
+    if plain_inference():
+        call = _block_call(x, blk, causal)
+        if call is not None:
+            return call(x)
     return TransformerBlockFn.apply(
         x, blk.ln1.gamma, blk.ln1.beta, at.q_proj.weight, at.q_proj.bias, at.k_proj.weight, at.k_proj.bias,
         at.v_proj.weight, at.v_proj.bias, at.out_proj.weight, at.out_proj.bias, blk.ln2.gamma, blk.ln2.beta,
