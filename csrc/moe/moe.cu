@@ -242,6 +242,16 @@ __global__ void gather_sum_kernel(MoeRead tab, const int* __restrict__ dest, __n
   }
 }
 
+// Rows of an expert's buffer between its last token and the end of that token's 128-row tile: zeroed, because a contraction over the expert's
+// rows runs to the end of the tile. `fill` counts the slots claimed, also those past the capacity; `counts` (may be null) receives the rows in use.
+// One block per expert: at most 127 rows each, where clearing the whole buffer took 35 us (64 x 1024 x 1024).
+__global__ void moe_tail_kernel(const int* fill, int* counts, __nv_bfloat16* buf, int cap, int d) {
+  const int e = blockIdx.x, n = min(fill[e], cap), end = min((n + 127) / 128 * 128, cap);
+  if (counts && threadIdx.x == 0) counts[e] = n;
+  uint4* p = reinterpret_cast<uint4*>(buf + (long long)e * cap * d);
+  for (long long i = (long long)n * (d / 8) + threadIdx.x; i < (long long)end * (d / 8); i += blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Cross-rank barrier on the stream: everything this rank launched before it is complete and visible to the peers
 // once they leave it, and nothing launched after it starts before every rank has arrived. Replaces a host barrier
 // between the dispatch / expert-GEMM / combine phases, so an expert-parallel step can be captured into a CUDA graph.
@@ -326,6 +336,14 @@ int b200_moe_combine_bwd(void* const* ybuf, void* const* dybuf, int world, const
   MoeRead yt; MoeWrite dt;
   for (int r = 0; r < world; ++r) { yt.ybuf[r] = ybuf[r]; dt.dybuf[r] = dybuf[r]; }
   combine_bwd_kernel<<<warps_grid(tokens * k), 256, 0, st>>>(yt, dt, dest, w, (const __nv_bfloat16*)dout, dw, tokens, k, d, rows_per_rank);
+  return (int)cudaGetLastError();
+}
+
+// buf: [E, cap, d] bf16, d % 8 == 0
+int b200_moe_tail(const int* fill, int* counts, void* buf, int E, int cap, int d, cudaStream_t st) {
+  if (E <= 0 || cap <= 0) return 0;
+  if (d % 8) return -1;
+  moe_tail_kernel<<<(unsigned)E, 512, 0, st>>>(fill, counts, (__nv_bfloat16*)buf, cap, d);
   return (int)cudaGetLastError();
 }
 

@@ -38,6 +38,7 @@ nv.register_sigs({
     "b200_moe_combine_fwd": [C.POINTER(_P), C.c_int, _P, _P, _P, C.c_longlong, C.c_int, C.c_int, C.c_longlong, _P],
     "b200_moe_combine_bwd": [C.POINTER(_P), C.POINTER(_P), C.c_int, _P, _P, _P, _P, C.c_longlong, C.c_int, C.c_int, C.c_longlong, _P],
     "b200_moe_gather_sum": [C.POINTER(_P), C.c_int, _P, _P, C.c_longlong, C.c_int, C.c_int, C.c_longlong, _P],
+    "b200_moe_tail": [_P, _P, _P, C.c_int, C.c_int, C.c_int, _P],
     "b200_ep_barrier": [C.POINTER(_P), C.c_int, C.c_int, _P, C.c_longlong, _P, _P],
 })
 
@@ -235,6 +236,30 @@ def _fused_layer_forward(ep, xc, idx, w, W1, b1, W2, b2, act, cap, xbuf, xptrs, 
     return out, (dest, wc, xsave, h, pre, W1, b1, W2, b2, counts)
 
 
+def _owned(p) -> bool:
+    """Does the parameter carry a gradient in an optimizer's flat fp32 buffer, which kernels add into?"""
+    return getattr(p, "_fused_grad", False) and p.grad is not None and p.grad.dtype == torch.float32 and p.grad.is_contiguous()
+
+
+def _expert_wgrad(g, x, W, counts):
+    """dW[e] = g[e]^T x[e] over the rows in use; None where it went straight into the optimizer's buffer (an extra tensor of the weights' size
+    written, read and added took 125 us for 64 experts of 1024 x 512)."""
+    if _owned(W):
+        gemm(g, x, a_mn=True, b_mn=True, accumulate_into=W.grad, k_valid=counts)
+        return None
+    return gemm(g, x, a_mn=True, b_mn=True, out_dtype=torch.float32, k_valid=counts)
+
+
+def _expert_bgrad(g, b, counts):
+    if b is None:
+        return None
+    E, cap, n = g.shape
+    out = b.grad if _owned(b) else torch.zeros((E, n), dtype=torch.float32, device=g.device)
+    nv.check(nv.cuda().b200_colsum_batched(g.data_ptr(), out.data_ptr(), E, cap, n, n, cap * n, 1, nv.ptr(counts), nv.stream_ptr()), "colsum_batched")
+    nv.count_launch()
+    return None if out is b.grad else out
+
+
 class MoEExpertsFn(Function):
     """Routed experts: out[t] = sum_j w[t,j] * FFN_{idx[t,j]}(x[t]).  x [T, d] bf16 (CUDA).
 
@@ -259,8 +284,6 @@ class MoEExpertsFn(Function):
         rows = E_local * cap
         dev = x.device
         ep = ep or _LOCAL_EP
-        xbuf, xptrs = ep.buffer("x", rows * d, torch.bfloat16, dev)
-        fill, fptrs = ep.buffer("fill", max(E_local, 4), torch.int32, dev)
         ybuf, yptrs = ep.buffer("y", rows * d, torch.bfloat16, dev)
         dest = torch.empty((T, k), dtype=torch.int32, device=dev)
         lib = nv.cuda()
@@ -269,30 +292,49 @@ class MoEExpertsFn(Function):
         # faster: forward + backward of 8192 x 6 x 1024 1.79 against 1.90 ms, 16384 x 6 x 1024 2.75 against 3.03 ms, 16384 x 6 x 512
         # 1.58 against 1.72 ms; below that the single launch wins (4096 x 6 x 1024 1.48 against 1.55 ms).
         alone = world == 1 and T * k * d >= _ALONE_FROM
-        if ep.backend == "fused" and x.is_cuda and _FUSED_LAYER and d % 8 == 0 and not alone:
+        single = ep.backend == "fused" and x.is_cuda and _FUSED_LAYER and d % 8 == 0 and not alone
+        private = world == 1 and x.is_cuda and not single
+        if not private:
+            xbuf, xptrs = ep.buffer("x", rows * d, torch.bfloat16, dev)
+            fill, fptrs = ep.buffer("fill", max(E_local, 4), torch.int32, dev)
+        if single:
             out, saved = _fused_layer_forward(ep, xc, idx, w, W1, b1, W2, b2, act, cap, xbuf, xptrs, fill, fptrs, ybuf, yptrs, dest)
             ctx.save_for_backward(*saved)
             ctx.cfg = (act, cap, ep, T, d, k, E_local, hid)
             return out
-        nv.check(lib.b200_moe_dispatch(xc.data_ptr(), idx.data_ptr(), dest.data_ptr(), _ptr_array(xptrs), _ptr_array(fptrs), world,
-                                       T, k, d, E_local, cap, nv.stream_ptr()), "moe_dispatch")
-        ep.barrier(dev)                                           # all remote rows have landed
-        xb = xbuf.view(E_local, cap, d)
+        if private:
+            # nobody else writes here: the rows go straight into the tensor that the backward reads, and only the ends of the experts' last
+            # tiles are cleared (no clean shared buffer, no copy of it)
+            xsave = xb = torch.empty((E_local, cap, d), dtype=torch.bfloat16, device=dev)
+            claimed = torch.zeros(2 * E_local, dtype=torch.int32, device=dev)
+            counts = claimed[E_local:]
+            nv.check(lib.b200_moe_dispatch(xc.data_ptr(), idx.data_ptr(), dest.data_ptr(), _ptr_array([xsave.data_ptr()]), _ptr_array([claimed.data_ptr()]),
+                                           1, T, k, d, E_local, cap, nv.stream_ptr()), "moe_dispatch")
+            nv.check(lib.b200_moe_tail(claimed.data_ptr(), counts.data_ptr(), xsave.data_ptr(), E_local, cap, d, nv.stream_ptr()), "moe_tail")
+            nv.count_launch(2)
+        else:
+            nv.check(lib.b200_moe_dispatch(xc.data_ptr(), idx.data_ptr(), dest.data_ptr(), _ptr_array(xptrs), _ptr_array(fptrs), world,
+                                           T, k, d, E_local, cap, nv.stream_ptr()), "moe_dispatch")
+            nv.count_launch()
+            ep.barrier(dev)                                       # all remote rows have landed
+            xb = xbuf.view(E_local, cap, d)
+            counts = fill[:E_local].clamp(max=cap) if x.is_cuda else None
         W1l, W2l = F.lp(W1), F.lp(W2)
         # rows in use per local expert: the expert GEMMs skip the 128-row tiles past them (the capacity padding costs
         # nothing), and nothing downstream reads the rows they leave unwritten
-        counts = fill[:E_local].clamp(max=cap) if x.is_cuda else None
         h, pre = gemm(xb, W1l, bias=b1.detach() if b1 is not None else None, act=act, want_aux=True, m_valid=counts)   # [E, cap, hid]
-        y = gemm(h, W2l, bias=b2.detach() if b2 is not None else None, out=ybuf.view(E_local, cap, d), m_valid=counts)  # [E, cap, d], in the peers' reach
-        xsave = xb.clone()
+        gemm(h, W2l, bias=b2.detach() if b2 is not None else None, out=ybuf.view(E_local, cap, d), m_valid=counts)      # [E, cap, d], in the peers' reach
+        if not private:
+            xsave = xb.clone()
         ep.barrier(dev)                                           # every rank's expert outputs are in place
         out = torch.empty((T, d), dtype=torch.bfloat16, device=dev)
         wc = w.float().contiguous()
         nv.check(lib.b200_moe_combine_fwd(_ptr_array(yptrs), world, dest.data_ptr(), wc.data_ptr(), out.data_ptr(), T, k, d, rows,
                                           nv.stream_ptr()), "moe_combine_fwd")
-        nv.count_launch(2)
-        xbuf.zero_(); fill.zero_()
-        ep.barrier(dev)                                           # peers have read my outputs; everyone's input buffers are clear
+        nv.count_launch()
+        if not private:
+            xbuf.zero_(); fill.zero_()
+            ep.barrier(dev)                                       # peers have read my outputs; everyone's input buffers are clear
         ctx.save_for_backward(dest, wc, xsave, h, pre, W1, b1, W2, b2, counts if counts is not None else torch.empty(0))
         ctx.cfg = (act, cap, ep, T, d, k, E_local, hid)
         return out
@@ -316,24 +358,23 @@ class MoEExpertsFn(Function):
                                           dw.data_ptr(), T, k, d, rows, nv.stream_ptr()), "moe_combine_bwd")
         ep.barrier(dev)
         dy = dybuf.view(E_local, cap, d)
+        private = world == 1 and counts is not None
+        if private:                                               # as in the forward: only the ends of the last tiles are cleared
+            nv.check(lib.b200_moe_tail(counts.data_ptr(), 0, dybuf.data_ptr(), E_local, cap, d, nv.stream_ptr()), "moe_tail")
+            nv.count_launch()
         W1l, W2l = F.lp(W1), F.lp(W2)
         dh = gemm(dy, W2l, b_mn=True, aux_in=pre, dact=act, m_valid=counts)                   # [E, cap, hid]
-        dW2 = gemm(dy, h, a_mn=True, b_mn=True, out_dtype=torch.float32, k_valid=counts)       # [E, d, hid]
-        dW1 = gemm(dh, xb, a_mn=True, b_mn=True, out_dtype=torch.float32, k_valid=counts)      # [E, hid, d]
+        dW2 = _expert_wgrad(dy, h, W2, counts)                                                  # [E, d, hid]
+        dW1 = _expert_wgrad(dh, xb, W1, counts)                                                 # [E, hid, d]
         gemm(dh, W1l, b_mn=True, out=dxbuf.view(E_local, cap, d), m_valid=counts)               # [E, cap, d], pulled by the token owners
-        db1 = db2 = None
-        if b1 is not None:
-            db1 = torch.zeros((E_local, hid), dtype=torch.float32, device=dev)
-            nv.check(lib.b200_colsum_batched(dh.data_ptr(), db1.data_ptr(), E_local, cap, hid, hid, cap * hid, 1, nv.ptr(counts), nv.stream_ptr()), "colsum_batched")
-        if b2 is not None:
-            db2 = torch.zeros((E_local, d), dtype=torch.float32, device=dev)
-            nv.check(lib.b200_colsum_batched(dy.data_ptr(), db2.data_ptr(), E_local, cap, d, d, cap * d, 1, nv.ptr(counts), nv.stream_ptr()), "colsum_batched")
+        db1, db2 = _expert_bgrad(dh, b1, counts), _expert_bgrad(dy, b2, counts)
         # adjoint of dispatch: pull the token gradients back from the owning ranks
         ep.barrier(dev)
         dx = torch.empty((T, d), dtype=torch.bfloat16, device=dev)
         nv.check(lib.b200_moe_gather_sum(_ptr_array(dxptrs), world, dest.data_ptr(), dx.data_ptr(), T, k, d, rows, nv.stream_ptr()), "moe_gather_sum")
-        nv.count_launch(4)
-        dybuf.zero_()
+        nv.count_launch(2)
+        if not private:
+            dybuf.zero_()
         return dx, None, dw, dW1, db1, dW2, db2, None, None, None
 
 

@@ -165,3 +165,41 @@ def test_linear_attention_gpu(causal, kind):
     for name, a, b in (("dq", q, qr), ("dk", k, kr), ("dv", v, vr)):
         tol = 3e-2 if (name == "dq" and kind == "elu") else 1e-2
         assert rel_err(a.grad, b.grad) < tol, (name, rel_err(a.grad, b.grad))
+
+
+@pytest.mark.parametrize("T,E,k,cap", [(700, 8, 2, 256), (64, 16, 1, 128), (3, 4, 2, 128), (900, 4, 2, 130)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_expert_gradients_in_an_optimizers_buffer(monkeypatch, T, E, k, cap, fused):
+    """Weights whose gradients live in an optimizer's buffer: the products add into it (twice here); experts without tokens, with whole and broken tiles,
+    and past their capacity."""
+    monkeypatch.setattr(M, "_FUSED_LAYER", fused)
+    torch.manual_seed(T)
+    d, hid = 64, 128
+    x = (torch.randn(T, d, device="cuda") * 0.5).bfloat16().requires_grad_(True)
+    idx = torch.topk(torch.randn(T, E, device="cuda") + torch.linspace(0, 3, E, device="cuda"), k)[1].int().contiguous()
+    w = torch.rand(T, k, device="cuda")
+    g = torch.randn(T, d, device="cuda").bfloat16()
+    ws = [torch.nn.Parameter(torch.randn(*s, device="cuda") * 0.1) for s in ((E, hid, d), (E, hid), (E, d, hid), (E, d))]
+    M.MoEExpertsFn.apply(x, idx, w, *ws, "silu", cap, None).backward(g)
+    plain = [p.grad.clone() for p in ws]
+    for p in ws:
+        p._fused_grad, p.grad = True, torch.ones_like(p)
+    for _ in range(2):
+        M.MoEExpertsFn.apply(x, idx, w, *ws, "silu", cap, None).backward(g)
+    full = bool((torch.bincount(idx.flatten().long(), minlength=E) <= cap).all())
+    for p, one in zip(ws, plain):
+        if full:                                             # (which of an overfull expert's tokens are dropped depends on timing)
+            assert rel_err(p.grad, 1 + 2 * one) < 1e-3
+        assert torch.isfinite(p.grad).all()
+
+
+@pytest.mark.parametrize("rows,cols,ld", [(128, 8, 8), (300, 264, 264), (257, 40, 48), (64, 100, 100)])
+def test_batched_column_sums(rows, cols, ld):
+    from rust_neural_network_b200 import _native as nv
+    x = torch.randn(3, rows, ld, device="cuda").bfloat16()
+    valid = torch.tensor([0, 1, rows], dtype=torch.int32, device="cuda")
+    out = torch.ones(3, cols, device="cuda")
+    nv.check(nv.cuda().b200_colsum_batched(x.data_ptr(), out.data_ptr(), 3, rows, cols, ld, rows * ld, 1, valid.data_ptr(), nv.stream_ptr()), "colsum")
+    for b, n in enumerate([0, min(rows, 128), rows]):
+        want = 1 + x[b, :n, :cols].double().sum(0)
+        assert float((out[b].double() - want).abs().max()) < 1e-3
