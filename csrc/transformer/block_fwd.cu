@@ -2,10 +2,9 @@
 // projection, residual add + LayerNorm, GELU layer, second feed-forward layer with the residual. The launches are the ones
 // ops/transformer.py makes one by one when it has to keep tensors for a backward; a prompt of a few hundred tokens takes
 // 5 to 10 us on the GPU per launch, less than the 30 us that preparing a launch from Python took, so without gradients the
-// whole sequence is issued here from one record of pointers.
+// whole sequence is issued here from one record of pointers (each launcher goes through launch_pdl).
 #include <cmath>
 #include "../attention/flash_sm100.h"
-#include "../common/launch.cuh"
 #include "../gemm/gemm_sm100.h"
 
 extern "C" int b200_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd, long long rows, int d,
@@ -20,21 +19,13 @@ struct BlockArgs {
   // activations [T, d] and workspace, all bf16 and 16-byte aligned: h [T, d], qkv [T, 3d], o [T, d], y1 [T, d], a [T, ff]
   const void* x; void* y;
   void *h, *qkv, *o, *y1, *a;
-  float *mean, *rstd, *lse, *bqkv;               // fp32 [T], [T], [B, heads, S], [3d] (gathered from bq, bk, bv when bqkv_gather)
+  float *mean, *rstd, *lse;                      // fp32 [T], [T], [B, heads, S]
   const void *wqkv, *wo, *w1, *w2;               // bf16, K-major: [3d, d], [d, d], [ff, d], [d, ff]
-  const float *g1, *be1, *g2, *be2, *bq, *bk, *bv, *bo, *b1, *b2;
-  int B, S, d, ff, heads, causal, bqkv_gather, op_add, num_sms;
+  const float *g1, *be1, *g2, *be2, *bqkv, *bo, *b1, *b2;
+  int B, S, d, ff, heads, causal, op_add, num_sms;
   float eps;
   uint32_t* status;
 };
-
-// out[0 .. 3n) = a | b | c
-__global__ void gather3_kernel(const float* a, const float* b, const float* c, float* out, int n) {
-  pdl_trigger();
-  pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 3 * n) out[i] = __ldcg(i < n ? a + i : i < 2 * n ? b + (i - n) : c + (i - 2 * n));
-}
 
 static int block_gemm(const BlockArgs& b, const void* A, int M, int K, const void* W, int N, const float* bias, int act, const void* residual, void* C, cudaStream_t st) {
   GemmArgs g = {};
@@ -59,13 +50,7 @@ extern "C" int b200_block_fwd(const b200::BlockArgs* args, int* launches, cudaSt
   const int T = b.B * b.S, d = b.d, hd = d / b.heads;
   int n = 7;
   if (int rc = b200_layernorm_fwd(b.x, b.g1, b.be1, b.h, b.mean, b.rstd, T, d, b.eps, 1, st)) return rc;
-  const float* bqkv = b.bq;
-  if (b.bqkv_gather) {
-    const cudaError_t e = launch_pdl(gather3_kernel, dim3((3 * d + 255) / 256), dim3(256), 0, st, b.bq, b.bk, b.bv, b.bqkv, d);
-    if (e != cudaSuccess) return 400 + (int)e;
-    bqkv = b.bqkv; ++n;
-  }
-  if (int rc = block_gemm(b, b.h, T, d, b.wqkv, 3 * d, bqkv, ACT_NONE, nullptr, b.qkv, st)) return rc;
+  if (int rc = block_gemm(b, b.h, T, d, b.wqkv, 3 * d, b.bqkv, ACT_NONE, nullptr, b.qkv, st)) return rc;
   FlashArgs f = {};
   char* qkv = static_cast<char*>(b.qkv);
   AttnTensor* part[3] = {&f.q, &f.k, &f.v};

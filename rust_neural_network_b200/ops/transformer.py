@@ -171,7 +171,7 @@ class TransformerBlockFn(Function):
 
 
 nv.register_sigs({"b200_block_fwd": [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]})
-_BLOCK_PACK = struct.Struct("@25P9ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
+_BLOCK_PACK = struct.Struct("@22P8ifP")                       # `BlockArgs` of csrc/transformer/block_fwd.cu
 
 
 def _plain(*ts) -> bool:
@@ -195,8 +195,7 @@ class _BlockCall:
         w0 = work.data_ptr()
         self.keep = (ws, vecs, work)
         self.fields = (*(w0 + p for p in offs), *(w.data_ptr() for w in ws), *(t.data_ptr() for t in vecs), B, S, d, ws[2].shape[0], at.heads, int(causal),
-                       int(not _adjacent(at.q_proj.bias, at.k_proj.bias, at.v_proj.bias)), K.OPS["add"], _num_sms(x.device), nv.f32(blk.ln1.eps),
-                       nv.status_ptr(x.device))
+                       K.OPS["add"], _num_sms(x.device), nv.f32(blk.ln1.eps), nv.status_ptr(x.device))
 
     def __call__(self, x):
         x = x if x.is_contiguous() else x.contiguous()
@@ -224,10 +223,12 @@ def _block_call(x, blk, causal, work=None):
     ws = (wqkv[0] if _adjacent(*wqkv) else torch.cat(wqkv, 0), lp(o.weight), lp(f1.weight), lp(f2.weight))
     if any(w.data_ptr() % 16 or not w.is_contiguous() for w in ws):
         return None
+    bqkv = vecs[4] if _adjacent(*vecs[4:7]) else torch.cat([b.detach() for b in vecs[4:7]])
+    vecs = (*vecs[:4], bqkv, *vecs[7:])
     T = B * S
-    # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse, gathered bias (fp32)
+    # one workspace, carved at 256-byte boundaries: h, qkv, o, y1, a (bf16); mean, rstd, lse (fp32)
     offs, total = [], 0
-    for nbytes in (2 * T * d, 6 * T * d, 2 * T * d, 2 * T * d, 2 * T * ff, 4 * T, 4 * T, 4 * T * at.heads, 12 * d):
+    for nbytes in (2 * T * d, 6 * T * d, 2 * T * d, 2 * T * d, 2 * T * ff, 4 * T, 4 * T, 4 * T * at.heads):
         offs.append(total)
         total += (nbytes + 255) & ~255
     if work is None or work.numel() < total:
