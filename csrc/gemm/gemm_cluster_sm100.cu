@@ -244,13 +244,14 @@ static int launch_cluster(const GemmArgs& a, int ranks, cudaStream_t stream) {
 // CTAs per tile; 1: one CTA forms each sum. A cluster costs about 2 us (its CTAs start together, so the kernel's start hides less behind its
 // predecessor, and the partial tiles cross); a K block costs 0.2 us. Device time in a chain of launches, one CTA a tile (64-wide tiles, the
 // better of the two) against clusters of 8 / 4: 16 x 512 x 2048 10.0 / 7.7 us, 333 x 512 x 2048 10.6 / 8.4, with a residual 11.6 / 8.4,
-// 1024 x 512 x 2048 10.8 / 9.7 (4), 333 x 512 x 8192 29.9 / 10.9; 333 x 1024 x 1024 7.4 / 8.4 and 333 x 512 x 512 5.7 / 7.5: below 24
-// blocks the cluster loses. About 100 SMs are reached by clusters of 8 and 128 by clusters of 4 at once: more and a second wave
-// begins (32 tiles in clusters of 8: 24 us).
+// 333 x 512 x 8192 29.9 / 10.9; 333 x 1024 x 1024 7.4 / 8.4 and 333 x 512 x 512 5.7 / 7.5: below 24 blocks the cluster loses. About 100
+// SMs are reached by clusters of 8 at once: more and a second wave begins (32 tiles in clusters of 8: 24 us). Clusters of 4 win alone up to
+// 128 CTAs (1024 x 512 x 2048 10.8 / 9.7), but among a block's other launches, which they keep from starting early, 32 tiles lose: LM logits
+// of 512 tokens (16 tiles) 1330 -> 1163 us, of 1024 tokens (32 tiles) 1478 -> 1566.
 int gemm_cluster_ranks(const GemmArgs& a) {
   if (a.dtype != GEMM_BF16 || a.p.m_valid || a.p.k_valid || a.p.out_mode == OUT_I32 || a.K < 24 * 64) return 1;
   const long long tiles = (long long)((a.p.M + BM - 1) / BM) * ((a.p.N + CL_BN - 1) / CL_BN) * a.p.batch;
-  return tiles * 8 <= 96 ? 8 : tiles * 4 <= 128 ? 4 : 1;
+  return tiles * 8 <= 96 ? 8 : tiles * 4 <= 64 ? 4 : 1;
 }
 
 int gemm_cluster_launch(const GemmArgs& a, int ranks, cudaStream_t stream) {
