@@ -194,8 +194,7 @@ extern "C" int b200_gemm_init() {
   e |= gemm_set_attr<__nv_bfloat16, BN, true, false>(); e |= gemm_set_attr<__nv_bfloat16, BN, true, true>();
   B200_INIT_BN(64) B200_INIT_BN(128) B200_INIT_BN(256)
 #undef B200_INIT_BN
-  e |= gemm_set_attr<__nv_bfloat16, 64, false, false, true>() | gemm_set_attr<__nv_bfloat16, 128, false, false, true>() |
-       gemm_set_attr<__nv_bfloat16, 256, false, false, true>() | pair_set_attr<__nv_bfloat16, false, false, true>();
+  e |= gemm_set_attr<__nv_bfloat16, 64, false, false, true>() | gemm_set_attr<__nv_bfloat16, 256, false, false, true>() | pair_set_attr<__nv_bfloat16, false, false, true>();
   e |= pair_set_attr<__nv_bfloat16, false, false>(); e |= pair_set_attr<__nv_bfloat16, false, true>(); e |= pair_set_attr<__nv_bfloat16, true, false>(); e |= pair_set_attr<__nv_bfloat16, true, true>();
   e |= gemm_cluster_init() | gemm_kinds_init();
   return e;
@@ -206,12 +205,14 @@ extern "C" int b200_gemm_set_pair(int mode) { b200::g_pair_mode = mode < 0 ? 0 :
 
 extern "C" int b200_gemm_set_tma_store(int on) { b200::g_tma_store = on ? 1 : 0; return 0; }
 
-// Tiles of a bf16 product: bf16 results 64 columns while such tiles run at once, which shortens what a CTA loads and writes (device time, 64 / 128 wide:
-// 333 x 2048 x 512 5.9 / 6.6 us, 2048 x 512 x 512 (128 tiles) 5.9 / 6.6, x 2048 11.2 / 11.7; 1024 x 1536 x 512 (192 tiles) 8.1 / 6.8), 256
-// once such tiles fill the machine.
+// Tiles of a bf16 product: bf16 results of up to 512 rows 64 columns while such tiles run at once, which shortens what a CTA loads and writes
+// (device time, 64 / 128 wide: 333 x 2048 x 512 5.9 / 6.6 us, 512 x 512 x 512 5.6 / 6.4; 1024 x 1536 x 512 (192 tiles) 8.1 / 6.8), 256 once such
+// tiles fill the machine. Alone, 64 columns also win at 1024 x 512 (5.8 / 6.5 us), but a chain of products that alternates between kernels pays
+// about 3 us a change, and from 600 rows on a block's wider products are 128 wide: LM logits of 1024 tokens 1566 us mixed, 1480 all 128 wide;
+// up to 512 tokens all of them are narrow: 1305 -> 1169 us.
 static int bf16_tile(const b200::GemmArgs& a, int sms) {
   const long long m = (long long)((a.M + 127) / 128) * a.batch;
-  if (a.N <= 64 || (a.p.out_mode == b200::OUT_BF16 && m * ((a.N + 63) / 64) <= sms)) return 64;
+  if (a.N <= 64 || (a.p.out_mode == b200::OUT_BF16 && a.M <= 512 && m * ((a.N + 63) / 64) <= sms)) return 64;
   return a.N > 128 && m * ((a.N + 255) / 256) >= sms ? 256 : 128;
 }
 
